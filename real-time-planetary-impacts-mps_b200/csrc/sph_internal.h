@@ -59,7 +59,8 @@ struct Tree {
     float4 *locals = nullptr;       // [node_cap][kLocalQ]
     int32_t *lists[2] = {nullptr, nullptr}; // unchecked-node lists, [branch_cap][list_cap] each
     int32_t *meta = nullptr;        // device: [0] n_levels, [1] n_nodes, [2] tree_len
-    int2 *node_range = nullptr;     // [node_cap] by data pointer: (first, count) in the GPU tree's key order
+    int2 *node_range = nullptr;     // [node_cap] by data pointer, leaves of the GPU tree: (first, count) in key order
+    int32_t *parent = nullptr;      // [node_cap] by data pointer, GPU tree: the parent's tree offset, -1 at the root
     int64_t node_cap = 0;
     int64_t level_cap = 0;
     int64_t branch_cap = 0;         // list slots per level
@@ -74,16 +75,12 @@ struct Tree {
 // Scratch of the GPU tree builder (sph_tree.cu).
 struct TreeBuild {
     RadixSorter sorter;
-    int32_t *nstart = nullptr;  // [max_levels][level_cap]
-    int32_t *ncount = nullptr;  // [max_levels][level_cap]
-    int32_t *nparent = nullptr; // [max_levels][level_cap] parent index in previous level (or -1), octant in high bits
-    int64_t *scan = nullptr;    // [level_cap * 8 + 1] scan scratch
-    int64_t *scan_blocks = nullptr;
-    int32_t *per_particle = nullptr; // [3][n+1] ints at start, nodes at start, first level
-    int32_t *noffset = nullptr; // [max_levels][level_cap] tree offset of each node
-    int32_t *ndp = nullptr;     // [max_levels][level_cap] data pointer
+    uint8_t *levels = nullptr;  // [n] levels of the nodes that start at each particle (key order)
+    int32_t *ints = nullptr;    // [n] their ints
+    int32_t *at_int = nullptr, *at_node = nullptr;  // [n] first offset and data pointer of them
+    int64_t *totals = nullptr;  // block totals of the scans
+    uint32_t *ticket = nullptr; // blocks done (0 between builds)
     float *bbox = nullptr;      // device [6] lo.xyz, hi.xyz as ordered ints
-    int64_t scan_cap = 0;
     const uint32_t *order = nullptr;  // particle ids in the tree's key order (last GPU build)
     int32_t *walk_queues = nullptr;   // theta-form walk: node queues of the resident warps
     uint32_t *walk_counter = nullptr; // theta-form walk: group ticket
@@ -217,10 +214,6 @@ void sort_free(RadixSorter &s);
 int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t *health);
 sph_status launch_sort(sph_ctx *ctx, cudaStream_t st);
 void launch_init_cells(sph_ctx *ctx, cudaStream_t st);
-// 64-bit exclusive scan of `count` values (count read on the host side bound
-// `n_max`, actual count from *d_count when non-null) into out; *total at out[count].
-void scan_exclusive_i64(const int64_t *in, int64_t *out, int64_t *block_scratch, int n_max, const int32_t *d_count,
-                        cudaStream_t st);
 
 // sph_hydro.cu
 sph_status launch_density(sph_ctx *ctx, cudaStream_t st);

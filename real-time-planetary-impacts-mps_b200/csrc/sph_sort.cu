@@ -190,104 +190,7 @@ __global__ void k_init_cells(uint2 *cell_range, uint32_t count) {
         cell_range[i] = make_uint2(0xffffffffu, 0u);
 }
 
-// ---- 64-bit exclusive scan (reduce, scan of block sums, apply) -------------
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
-__device__ __forceinline__ int64_t block_excl_scan(int64_t v, int64_t *total) {
-    __shared__ int64_t warp_sums[kScanThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int64_t s = (lane < kScanThreads / 32) ? warp_sums[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int64_t y = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += y;
-        }
-        if (lane < kScanThreads / 32) warp_sums[lane] = s;
-    }
-    __syncthreads();
-    int64_t prefix = (warp > 0) ? warp_sums[warp - 1] : 0;
-    *total = warp_sums[kScanThreads / 32 - 1];
-    __syncthreads();
-    return prefix + x - v;
-}
-
-__global__ void k_scan_reduce(const int64_t *__restrict__ in, int64_t *__restrict__ blocks, int n_max,
-                              const int32_t *d_count) {
-    const int n = d_count ? min(*d_count, n_max) : n_max;
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-    int64_t s = 0;
-    for (int it = 0; it < kScanItems; ++it) {
-        int64_t i = base + (int64_t)it * kScanThreads + threadIdx.x;
-        if (i < n) s += in[i];
-    }
-    int64_t total;
-    block_excl_scan(s, &total);
-    if (threadIdx.x == 0) blocks[blockIdx.x] = total;
-}
-
-__global__ void k_scan_blocks(int64_t *blocks, int nb) {
-    // single block: exclusive scan of nb block sums in place, total at blocks[nb]
-    int64_t carry = 0;
-    for (int b0 = 0; b0 < nb; b0 += kScanThreads) {
-        int i = b0 + threadIdx.x;
-        int64_t v = (i < nb) ? blocks[i] : 0;
-        int64_t total;
-        int64_t e = block_excl_scan(v, &total);
-        if (i < nb) blocks[i] = carry + e;
-        carry += total;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) blocks[nb] = carry;
-}
-
-__global__ void k_scan_apply(const int64_t *__restrict__ in, int64_t *__restrict__ out,
-                             const int64_t *__restrict__ blocks, int n_max, const int32_t *d_count) {
-    const int n = d_count ? min(*d_count, n_max) : n_max;
-    const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-    int64_t loc[kScanItems];
-    int64_t s = 0;
-    for (int it = 0; it < kScanItems; ++it) {
-        int64_t i = base + it;
-        loc[it] = (i < n) ? in[i] : 0;
-        s += loc[it];
-    }
-    int64_t total;
-    int64_t e = block_excl_scan(s, &total) + blocks[blockIdx.x];
-    for (int it = 0; it < kScanItems; ++it) {
-        int64_t i = base + it;
-        if (i < n) out[i] = e;
-        e += loc[it];
-    }
-}
-
-__global__ void k_scan_total(const int64_t *__restrict__ in, int64_t *__restrict__ out, int n_max,
-                             const int32_t *d_count) {
-    const int n = d_count ? min(*d_count, n_max) : n_max;
-    out[n] = (n > 0) ? out[n - 1] + in[n - 1] : 0;
-}
-
 }  // namespace
-
-void scan_exclusive_i64(const int64_t *in, int64_t *out, int64_t *blocks, int n_max, const int32_t *d_count,
-                        cudaStream_t st) {
-    int nb = (n_max + kScanTile - 1) / kScanTile;
-    if (nb < 1) nb = 1;
-    k_scan_reduce<<<nb, kScanThreads, 0, st>>>(in, blocks, n_max, d_count);
-    k_scan_blocks<<<1, kScanThreads, 0, st>>>(blocks, nb);
-    k_scan_apply<<<nb, kScanThreads, 0, st>>>(in, out, blocks, n_max, d_count);
-    k_scan_total<<<1, 1, 0, st>>>(in, out, n_max, d_count);
-}
 
 sph_status sort_alloc(RadixSorter &s, int n) {
     s.n_cap = n;

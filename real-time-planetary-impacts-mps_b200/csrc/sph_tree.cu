@@ -16,20 +16,32 @@
 //     on it.  The split is geometric (cube midpoints) instead of the
 //     reference's per-subset mean.
 //
-// Build: bounding box -> keys (+ digit histograms) -> sort -> per level, each
-// branch finds its 8 octant ranges by binary search and a scan compacts the
-// children into the next level -> every node adds its size at its first
-// particle -> two scans give DFS offsets and data pointers -> nodes write
-// themselves and link into their parents.  Every launch size is a host-side
-// upper bound and the true counts stay on the device, so the whole build can
-// be captured in a CUDA graph.
+// Build: bounding box -> keys (+ digit histograms) -> sort -> three kernels.
+// The nodes follow from the sorted keys alone: with cl(a, b) the number of
+// leading triplets that two keys share, the run of particles of a node at
+// level l starts at i exactly when cl(i - 1, i) < l, it holds more than
+// leafcap particles exactly when cl(i, i + leafcap) >= l, and it is a node
+// exactly when its parent's run does.  So each particle knows, from a few
+// neighbouring keys, the levels first .. last at which nodes start at it (all
+// branches but the last), and an exclusive scan over the particles gives every
+// node's DFS offset, data pointer and place in its level's lists:
+//   k_tree_mark   levels and ints of each particle's nodes; block totals; the
+//                 last block to finish scans them
+//   k_tree_write  scans within the block, nodes, level lists, particle ids
+//   k_tree_link   the first node at each particle links itself into its
+//                 parent (the only node whose parent starts elsewhere)
+// With one set of launches per level (82 in all, most of them too small to
+// fill the device) the build was half of a gravity pass: tree, up and down
+// together, N = 1e6, leaf 32: 2.12 -> 1.62 ms; N = 1e5, leaf 4: 1.25 -> 0.86 ms.
+// Every launch size is a host-side upper bound and the true counts stay on
+// the device, so the whole build can be captured in a CUDA graph.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "sph_internal.h"
 
 namespace sph {
-
-void tree_bounds(int n, int leafcap, int depth, int64_t &nodes, int64_t &ints, int64_t &branches);
 
 namespace {
 
@@ -41,16 +53,26 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
+// Blocks of the passes that end in one set of global atomics per block.
+constexpr int kReduceThreads = 512;
+constexpr int kReduceBlocks = 296;
+int reduce_grid(int n) { return std::max(1, std::min(kReduceBlocks, (n + kReduceThreads - 1) / kReduceThreads)); }
+
 __global__ void k_bbox_init(uint32_t *bb) {
     if (threadIdx.x < 3) bb[threadIdx.x] = 0xffffffffu;
     else if (threadIdx.x < 6) bb[threadIdx.x] = 0u;
 }
 
-__global__ void k_bbox(const float4 *__restrict__ pos4, int n, uint32_t *bb) {
+// Few blocks (kReduceBlocks), each reduced to one value per bound before its
+// six atomics: with one set of atomics per warp of 2368 blocks the atomics
+// took the time (N = 1e6: 82 us).
+__global__ void __launch_bounds__(kReduceThreads) k_bbox(const float4 *__restrict__ pos4, int n, uint32_t *bb) {
+    __shared__ uint32_t s[6][kReduceThreads / 32];
     float lo[3] = {3.402823466e+38f, 3.402823466e+38f, 3.402823466e+38f};
     float hi[3] = {-3.402823466e+38f, -3.402823466e+38f, -3.402823466e+38f};
+#pragma unroll 4
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 p = pos4[i];
+        const float4 p = __ldg(pos4 + i);
         lo[0] = fminf(lo[0], p.x);
         lo[1] = fminf(lo[1], p.y);
         lo[2] = fminf(lo[2], p.z);
@@ -58,16 +80,23 @@ __global__ void k_bbox(const float4 *__restrict__ pos4, int n, uint32_t *bb) {
         hi[1] = fmaxf(hi[1], p.y);
         hi[2] = fmaxf(hi[2], p.z);
     }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        const uint32_t l = __reduce_min_sync(0xffffffffu, f2ord(lo[a]));
+        const uint32_t h = __reduce_max_sync(0xffffffffu, f2ord(hi[a]));
+        if (lane == 0) {
+            s[a][warp] = l;
+            s[3 + a][warp] = h;
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int a = 0; a < 3; ++a) {
-            atomicMin(bb + a, f2ord(lo[a]));
-            atomicMax(bb + 3 + a, f2ord(hi[a]));
+    __syncthreads();
+    if (warp < 6) {
+        const uint32_t v = s[warp][lane < kReduceThreads / 32 ? lane : 0];
+        const uint32_t r = warp < 3 ? __reduce_min_sync(0xffffffffu, v) : __reduce_max_sync(0xffffffffu, v);
+        if (lane == 0) {
+            if (warp < 3) atomicMin(bb + warp, r);
+            else atomicMax(bb + warp, r);
         }
     }
 }
@@ -104,221 +133,298 @@ __global__ void k_tree_keys(const float4 *__restrict__ pos4, int n, int depth, c
     }
 }
 
-struct LevelArgs {
-    int32_t *nstart, *ncount, *nparent, *nrank, *noffset;
-    int32_t *level_count;  // Tree::level_count
-    int32_t *scan_n;       // [16] 8 * level count
-    int64_t level_cap;
-    int64_t *cand;         // [8 * level_cap + 1]
-    int64_t *cand_scan;
-    int32_t *cstart;       // [8 * level_cap]
-    const uint32_t *keys;  // sorted tree keys
-    int depth, leafcap, n;
+// ---- nodes from the sorted keys ------------------------------------------------
+constexpr int kTreeThreads = 1024;  // particles per block of the three kernels
+// Scanned over the particles: nodes, ints, nodes per level (D + 1), branches
+// per level (D); D <= 10.
+constexpr int kTreeSeqs = 2 + 11 + 10;
+constexpr uint8_t kNoNodes = 0xff;
+
+struct TreeArgs {
+    const uint32_t *keys;   // sorted
+    const uint32_t *order;  // particle ids in key order
+    int n, depth, leafcap, blocks;
+    uint8_t *levels;        // [n] first | last << 4 level of the nodes starting at each particle, or kNoNodes
+    int32_t *ints;          // [n] ints of the nodes starting at each particle
+    int32_t *at_int, *at_node;  // [n] their first offset and data pointer
+    int64_t *totals;        // [kTreeSeqs][blocks] block totals, scanned in place by the last block
+    uint32_t *ticket;       // blocks of k_tree_mark that are done
+    int32_t *tree, *level_nodes, *level_count, *list_slot, *parent, *meta;
+    int2 *node_range;       // by data pointer, leaves: (first particle in key order, count)
+    int64_t level_cap, tree_cap, node_cap;
+    uint32_t *health;
 };
 
-__global__ void k_root(LevelArgs a) {
-    a.nstart[0] = 0;
-    a.ncount[0] = a.n;
-    a.nparent[0] = -1;
-    a.level_count[0] = 1;
-    for (int l = 1; l < 16; ++l) a.level_count[l] = 0;
+// Leading triplets shared by two keys of `depth` triplets.
+__device__ __forceinline__ int shared_levels(uint32_t a, uint32_t b, int depth) {
+    const uint32_t x = a ^ b;
+    return x ? depth - 1 - (31 - __clz(x)) / 3 : depth;
 }
 
-// first index in [lo, hi) whose octant digit (key >> shift & 7) is >= o
-__device__ __forceinline__ int digit_lower_bound(const uint32_t *keys, int lo, int hi, int shift, uint32_t o) {
+// First index in (i, hi] whose key leaves i's run at `level` (hi when none
+// does before it).
+__device__ __forceinline__ int run_end(const uint32_t *keys, uint32_t key, int i, int hi, int level, int depth) {
+    int lo = i + 1;
     while (lo < hi) {
-        int mid = lo + ((hi - lo) >> 1);
-        if (((keys[mid] >> shift) & 7u) < o)
-            lo = mid + 1;
-        else
-            hi = mid;
+        const int mid = lo + ((hi - lo) >> 1);
+        if (shared_levels(key, keys[mid], depth) >= level) lo = mid + 1;
+        else hi = mid;
     }
     return lo;
 }
 
-__global__ void k_children(LevelArgs a, int l) {
-    const int cnt = a.level_count[l];
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.scan_n[l] = 8 * cnt;
-    const int32_t *ns = a.nstart + (size_t)l * a.level_cap, *nc = a.ncount + (size_t)l * a.level_cap;
-    const int shift = 3 * (a.depth - l - 1);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-        const int s = ns[t], c = nc[t];
-        const bool branch = c > a.leafcap;
-        int b = s;
-        for (int o = 0; o < 8; ++o) {
-            int e = branch ? ((o == 7) ? s + c : digit_lower_bound(a.keys, b, s + c, shift, (uint32_t)o + 1u)) : b;
-            const int64_t nonempty = (e > b) ? 1 : 0;
-            const int64_t brf = (o == 0 && branch) ? 1 : 0;
-            a.cand[(size_t)t * 8 + o] = nonempty | (brf << 32);
-            a.cstart[(size_t)t * 8 + o] = b;
-            b = e;
+// First index of the run of i at `level`, not looked for before `lo`: steps
+// back that double, then a binary search, since most runs are short.
+__device__ __forceinline__ int run_start(const uint32_t *keys, uint32_t key, int i, int lo, int level, int depth) {
+    int in = i, out = lo - 1, step = 1;  // in: in the run; out: before it (or before lo)
+    while (in - step >= lo) {
+        if (shared_levels(key, keys[in - step], depth) < level) {
+            out = in - step;
+            break;
+        }
+        in -= step;
+        step += step;
+    }
+    while (in - out > 1) {
+        const int mid = out + ((in - out) >> 1);
+        if (shared_levels(key, keys[mid], depth) >= level) in = mid;
+        else out = mid;
+    }
+    return in;
+}
+
+__device__ __forceinline__ void unpack_levels(uint8_t v, int &first, int &last) {
+    first = v & 15;
+    last = v == kNoNodes ? -1 : v >> 4;  // none: an empty range
+}
+
+__global__ void __launch_bounds__(kTreeThreads) k_tree_mark(TreeArgs a) {
+    __shared__ int32_t s_tot[kTreeSeqs];
+    __shared__ bool s_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = blockIdx.x * kTreeThreads + tid;
+    const int D = a.depth, n = a.n;
+    if (tid < kTreeSeqs) s_tot[tid] = 0;
+    __syncthreads();
+    int first = 0, last = -1, ints = 0;
+    if (i < n) {
+        const uint32_t key = a.keys[i];
+        const int c = i ? shared_levels(a.keys[i - 1], key, D) : -1;
+        bool nodes = c < D;
+        if (nodes && c >= 0) {
+            // the run of level c that holds i - 1 and i is a branch: it has
+            // leafcap particles besides i within leafcap places of it
+            const bool right = i + a.leafcap - 1 < n && shared_levels(a.keys[i + a.leafcap - 1], key, D) >= c;
+            const bool left = i >= a.leafcap && shared_levels(a.keys[i - a.leafcap], key, D) >= c;
+            if (!right && !left) {
+                const int s = run_start(a.keys, key, i, max(i - a.leafcap, 0), c, D);
+                const int e = run_end(a.keys, key, i, min(i + a.leafcap, n), c, D);
+                nodes = e - s > a.leafcap;
+            }
+        }
+        if (nodes) {
+            const int far = i + a.leafcap;
+            const int q = far < n ? shared_levels(key, a.keys[far], D) : -1;
+            first = c + 1;
+            last = max(first, min(D, q + 1));
+            // the leaf's run ends within leafcap places unless it is cut off by the depth
+            const int e = q >= last ? run_end(a.keys, key, far, n, last, D)
+                                    : run_end(a.keys, key, i, min(far, n), last, D);
+            ints = 10 * (last - first) + 2 + (e - i);
+        }
+        a.levels[i] = nodes ? (uint8_t)(first | (last << 4)) : kNoNodes;
+        a.ints[i] = ints;
+    }
+    const int nodes = __reduce_add_sync(0xffffffffu, last - first + 1);
+    const int wints = __reduce_add_sync(0xffffffffu, ints);
+    if (lane == 0) {
+        atomicAdd(&s_tot[0], nodes);
+        atomicAdd(&s_tot[1], wints);
+    }
+    for (int l = 0; l <= D; ++l) {
+        const unsigned on = __ballot_sync(0xffffffffu, first <= l && l <= last);
+        const unsigned br = __ballot_sync(0xffffffffu, first <= l && l < last);
+        if (lane == 0 && on) {
+            atomicAdd(&s_tot[2 + l], __popc(on));
+            if (br) atomicAdd(&s_tot[3 + D + l], __popc(br));
         }
     }
-}
-
-__global__ void k_emit(LevelArgs a, int l) {
-    const int cnt = a.level_count[l];
-    const int64_t *sc = a.cand_scan;
-    const int32_t *nc = a.ncount + (size_t)l * a.level_cap;
-    int32_t *rank = a.nrank + (size_t)l * a.level_cap;
-    const size_t nb = (size_t)(l + 1) * a.level_cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-        const int64_t first = sc[(size_t)t * 8];
-        rank[t] = (nc[t] > a.leafcap) ? (int32_t)(first >> 32) : -1;
-        for (int o = 0; o < 8; ++o) {
-            const size_t q = (size_t)t * 8 + o;
-            const int64_t v = a.cand[q];
-            if ((v & 0xffffffffll) == 0) continue;
-            const int pos = (int)(sc[q] & 0xffffffffll);
-            const int s = a.cstart[q];
-            const int e = (o == 7) ? (a.cstart[(size_t)t * 8] + nc[t]) : a.cstart[q + 1];
-            a.nstart[nb + pos] = s;
-            a.ncount[nb + pos] = e - s;
-            a.nparent[nb + pos] = t | (o << 28);
+    __syncthreads();
+    const int seqs = 3 + 2 * D;
+    if (tid < seqs) a.totals[(size_t)tid * a.blocks + blockIdx.x] = s_tot[tid];
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    // the last block to get here: one warp scans each sequence of block totals
+    __threadfence();
+    if (tid == 0) *a.ticket = 0u;
+    if (warp < seqs) {
+        int64_t *t = a.totals + (size_t)warp * a.blocks;
+        int64_t carry = 0;
+        int64_t v = lane < a.blocks ? __ldcg(t + lane) : 0;
+        for (int b = lane; b - lane < a.blocks; b += 32) {
+            const int64_t next = b + 32 < a.blocks ? __ldcg(t + b + 32) : 0;
+            int64_t x = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (b < a.blocks) t[b] = carry + x - v;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+            v = next;
+        }
+        if (lane == 0) {
+            if (warp < 2) a.meta[1 + warp] = (int32_t)carry;
+            else if (warp < 3 + D) a.level_count[warp - 2] = (int32_t)carry;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.level_count[l + 1] = (int32_t)(sc[(size_t)cnt * 8] & 0xffffffffll);
+    if (tid < 16 && tid > D) a.level_count[tid] = 0;
 }
 
-// leaf-level nodes get rank -1 (no list)
-__global__ void k_rank_leaves(LevelArgs a, int l) {
-    const int cnt = a.level_count[l];
-    int32_t *rank = a.nrank + (size_t)l * a.level_cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) rank[t] = -1;
-}
-
-struct LayoutArgs {
-    const int32_t *nstart, *ncount, *nparent, *nrank;
-    int32_t *noffset;
-    const int32_t *level_count;
-    int64_t level_cap;
-    int64_t *ints_at, *nodes_at;  // per particle (n + 1)
-    int32_t *first_level;
-    const int64_t *ints_off, *dp_off;
-    int32_t *tree, *level_nodes, *list_slot;
-    int2 *node_range;  // by data pointer: (first particle in key order, count)
-    const uint32_t *order;
-    int depth, leafcap, n;
-    int64_t tree_cap, node_cap;
-    uint32_t *health;
-    int32_t *meta;
-};
-
-__global__ void k_layout_reset(LayoutArgs a) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= a.n; i += gridDim.x * blockDim.x) {
-        a.ints_at[i] = 0;
-        a.nodes_at[i] = 0;
-        a.first_level[i] = 0x7fffffff;
-    }
-}
-
-__device__ __forceinline__ bool is_branch(const LayoutArgs &a, int l, int count) {
-    return l < a.depth && count > a.leafcap;
-}
-
-__global__ void k_marks(LayoutArgs a, int l) {
-    const int cnt = a.level_count[l];
-    const int32_t *ns = a.nstart + (size_t)l * a.level_cap, *nc = a.ncount + (size_t)l * a.level_cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-        const int s = ns[t], c = nc[t];
-        const int size = is_branch(a, l, c) ? 10 : 2 + c;
-        atomicAdd((unsigned long long *)(a.ints_at + s), (unsigned long long)size);
-        atomicAdd((unsigned long long *)(a.nodes_at + s), 1ull);
-        atomicMin(a.first_level + s, l);
-    }
-}
-
-__global__ void k_write(LayoutArgs a, int l) {
-    const int cnt = a.level_count[l];
-    const size_t base = (size_t)l * a.level_cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-        const int s = a.nstart[base + t], c = a.ncount[base + t];
-        const int d = l - a.first_level[s];
-        const int64_t off = a.ints_off[s] + 10 * (int64_t)d;
-        const int64_t dp = a.dp_off[s] + d;
-        const bool br = is_branch(a, l, c);
-        if (off + (br ? 10 : 2 + c) > a.tree_cap || dp >= a.node_cap) {
-            raise_health(a.health, SPH_HEALTH_TREE_CAPACITY);
-            a.noffset[base + t] = 0;
-            continue;
+__global__ void __launch_bounds__(kTreeThreads) k_tree_write(TreeArgs a) {
+    __shared__ int32_t s_at[kTreeSeqs][32];  // first value of each warp
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i = blockIdx.x * kTreeThreads + tid;
+    const int D = a.depth, seqs = 3 + 2 * D;
+    const unsigned lt = (1u << lane) - 1u;
+    int first, last;
+    unpack_levels(i < a.n ? a.levels[i] : kNoNodes, first, last);
+    const bool has = last >= 0;
+    if (!has) first = 0;
+    const int nodes = has ? last - first + 1 : 0;
+    const int ints = has ? a.ints[i] : 0;
+    int xn = nodes, xi = ints;  // inclusive scans over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int yn = __shfl_up_sync(0xffffffffu, xn, o), yi = __shfl_up_sync(0xffffffffu, xi, o);
+        if (lane >= o) {
+            xn += yn;
+            xi += yi;
         }
-        a.noffset[base + t] = (int32_t)off;
-        a.level_nodes[base + t] = (int32_t)off;
+    }
+    if (lane == 31) {
+        s_at[0][warp] = xn;
+        s_at[1][warp] = xi;
+    }
+    for (int l = 0; l <= D; ++l) {
+        const unsigned on = __ballot_sync(0xffffffffu, first <= l && l <= last);
+        const unsigned br = __ballot_sync(0xffffffffu, first <= l && l < last);
+        if (lane == 0) {
+            s_at[2 + l][warp] = __popc(on);
+            if (l < D) s_at[3 + D + l][warp] = __popc(br);
+        }
+    }
+    __syncthreads();
+    if (warp < seqs) {
+        const int v = s_at[warp][lane];
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        s_at[warp][lane] = (int32_t)a.totals[(size_t)warp * a.blocks + blockIdx.x] + x - v;
+    }
+    __syncthreads();
+    const int dp0 = s_at[0][warp] + xn - nodes;
+    const int off0 = s_at[1][warp] + xi - ints;
+    const int64_t leaf_off = (int64_t)off0 + 10 * (last - first);
+    // a node whose record or data pointer lies past the storage is left out
+    // and flagged (k_tree_link leaves it out too)
+    const bool fits = has && (int64_t)off0 + ints <= a.tree_cap && (int64_t)dp0 + nodes <= a.node_cap;
+    if (has && !fits) raise_health(a.health, SPH_HEALTH_TREE_CAPACITY);
+    if (has) {
+        a.at_int[i] = off0;
+        a.at_node[i] = dp0;
+    }
+    const uint32_t key = has ? a.keys[i] : 0u;
+    for (int l = 0; l <= D; ++l) {
+        const bool on = first <= l && l <= last, br = first <= l && l < last;
+        const unsigned m_on = __ballot_sync(0xffffffffu, on), m_br = __ballot_sync(0xffffffffu, br);
+        if (!on || !fits) continue;
+        const int off = off0 + 10 * (l - first), dp = dp0 + (l - first);
+        a.level_nodes[(size_t)l * a.level_cap + s_at[2 + l][warp] + __popc(m_on & lt)] = off;
+        a.list_slot[dp] = br ? s_at[3 + D + l][warp] + __popc(m_br & lt) : -1;
+        if (l > first) a.parent[dp] = off - 10;
+        else if (l == 0) a.parent[dp] = -1;
         int32_t *T = a.tree + off;
-        T[0] = br ? 0 : c;
-        T[1] = (int32_t)dp;
+        T[1] = dp;
         if (br) {
-            for (int k = 0; k < 8; ++k) T[2 + k] = -1;
+            T[0] = 0;
+            // the child that starts at this particle is the next record
+            const int o = (int)((key >> (3 * (D - l - 1))) & 7u);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) T[2 + k] = k == o ? off + 10 : -1;
         } else {
-            for (int k = 0; k < c; ++k) T[2 + k] = (int32_t)a.order[s + k];
+            const int cnt = ints - 2 - 10 * (last - first);
+            T[0] = cnt;
+            a.node_range[dp] = make_int2(i, cnt);
         }
-        a.list_slot[dp] = br ? a.nrank[base + t] : -1;
-        a.node_range[dp] = make_int2(s, c);
     }
-    if (l == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
-        a.meta[1] = (int32_t)a.dp_off[a.n];
-        a.meta[2] = (int32_t)a.ints_off[a.n];
-    }
-}
-
-__global__ void k_link(LayoutArgs a, int l) {
-    // l >= 1: every node writes its offset into its parent's child slot
-    const int cnt = a.level_count[l];
-    const size_t base = (size_t)l * a.level_cap, pbase = (size_t)(l - 1) * a.level_cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-        const int pr = a.nparent[base + t];
-        const int pt = pr & 0x0fffffff, o = (pr >> 28) & 7;
-        const int32_t poff = a.noffset[pbase + pt];
-        a.tree[poff + 2 + o] = a.noffset[base + t];
+    // the leaves' particle ids, a warp per leaf
+    for (unsigned m = __ballot_sync(0xffffffffu, fits); m; m &= m - 1u) {
+        const int src = __ffs(m) - 1;
+        const int64_t off = __shfl_sync(0xffffffffu, leaf_off, src) + 2;
+        const int cnt = __shfl_sync(0xffffffffu, ints - 2 - 10 * (last - first), src);
+        const int p0 = i - lane + src;
+        for (int k = lane; k < cnt; k += 32) a.tree[off + k] = (int32_t)a.order[p0 + k];
     }
 }
 
-inline int grid_for(int64_t bound, int threads = 256) {
-    int64_t b = (bound + threads - 1) / threads;
-    if (b < 1) b = 1;
-    if (b > 148 * 16) b = 148 * 16;
-    return (int)b;
+__global__ void __launch_bounds__(256) k_tree_link(TreeArgs a) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < 1 || i >= a.n) return;
+    int first, last;
+    unpack_levels(a.levels[i], first, last);
+    if (last < 0 || first < 1) return;
+    const int off = a.at_int[i], dp = a.at_node[i];
+    if ((int64_t)off + a.ints[i] > a.tree_cap || (int64_t)dp + (last - first + 1) > a.node_cap) return;
+    const uint32_t key = a.keys[i];
+    const int level = first - 1;  // the parent's
+    const int s = run_start(a.keys, key, i, 0, level, a.depth);
+    int pf, pl;
+    unpack_levels(a.levels[s], pf, pl);
+    const int poff = a.at_int[s] + 10 * (level - pf);
+    a.tree[poff + 2 + (int)((key >> (3 * (a.depth - first))) & 7u)] = off;
+    a.parent[dp] = poff;
 }
 
 }  // namespace
 
 sph_status tree_alloc(sph_ctx *ctx) {
     TreeBuild &tb = ctx->tb;
-    if (tb.nstart) return SPH_OK;
+    if (tb.bbox) return SPH_OK;
     const int n = ctx->n;
-    const int D = ctx->params.max_tree_depth;
-    const int64_t cap = ctx->tree.level_cap;  // n
-    const int levels = D + 1;
     sph_status s = sort_alloc(tb.sorter, n);
     if (s != SPH_OK) return s;
+    const size_t blocks = (size_t)(n + kTreeThreads - 1) / kTreeThreads;
     cudaError_t e = cudaSuccess;
     auto chk = [&](cudaError_t r) {
         if (e == cudaSuccess) e = r;
     };
-    chk(cudaMalloc(&tb.nstart, sizeof(int32_t) * levels * cap));
-    chk(cudaMalloc(&tb.ncount, sizeof(int32_t) * levels * cap));
-    chk(cudaMalloc(&tb.nparent, sizeof(int32_t) * levels * cap));
-    chk(cudaMalloc(&tb.noffset, sizeof(int32_t) * levels * cap));
-    chk(cudaMalloc(&tb.ndp, sizeof(int32_t) * levels * cap));  // branch ranks per level
-    tb.scan_cap = 8 * cap + 1;
-    chk(cudaMalloc(&tb.scan, sizeof(int64_t) * 2 * tb.scan_cap));
-    chk(cudaMalloc(&tb.scan_blocks, sizeof(int64_t) * (tb.scan_cap / 2048 + 16)));
-    chk(cudaMalloc(&tb.per_particle, sizeof(int32_t) * 8 * (cap + 1)));  // cstart: 8 per node slot
-    chk(cudaMalloc(&tb.bbox, sizeof(uint32_t) * 8 + sizeof(int32_t) * 16));
+    chk(cudaMalloc(&tb.levels, sizeof(uint8_t) * (size_t)n));
+    chk(cudaMalloc(&tb.ints, sizeof(int32_t) * (size_t)n));
+    chk(cudaMalloc(&tb.at_int, sizeof(int32_t) * (size_t)n));
+    chk(cudaMalloc(&tb.at_node, sizeof(int32_t) * (size_t)n));
+    chk(cudaMalloc(&tb.totals, sizeof(int64_t) * kTreeSeqs * blocks));
+    chk(cudaMalloc(&tb.ticket, sizeof(uint32_t)));
+    if (e == cudaSuccess) chk(cudaMemset(tb.ticket, 0, sizeof(uint32_t)));
+    chk(cudaMalloc(&tb.bbox, sizeof(uint32_t) * 8));
     return cuda_status(e, "tree_alloc");
 }
 
 void tree_free(sph_ctx *ctx) {
     TreeBuild &tb = ctx->tb;
     sort_free(tb.sorter);
-    cudaFree(tb.nstart);
-    cudaFree(tb.ncount);
-    cudaFree(tb.nparent);
-    cudaFree(tb.noffset);
-    cudaFree(tb.ndp);
-    cudaFree(tb.scan);
-    cudaFree(tb.scan_blocks);
-    cudaFree(tb.per_particle);
+    cudaFree(tb.levels);
+    cudaFree(tb.ints);
+    cudaFree(tb.at_int);
+    cudaFree(tb.at_node);
+    cudaFree(tb.totals);
+    cudaFree(tb.ticket);
     cudaFree(tb.bbox);
     cudaFree(tb.walk_queues);
     cudaFree(tb.walk_counter);
@@ -332,94 +438,55 @@ sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st) {
     Tree &tr = ctx->tree;
     const int n = ctx->n;
     const int D = ctx->params.max_tree_depth;
-    const int leafcap = ctx->params.max_children_in_leaf;
-    const int64_t cap = tr.level_cap;
+    const int leafcap = std::min(ctx->params.max_children_in_leaf, n);  // more is the same
     const int bits = 3 * D;
     const int passes = (bits + 7) / 8;
     uint32_t *bb = (uint32_t *)tb.bbox;
-    int32_t *scan_n = (int32_t *)(bb + 8);
 
     k_bbox_init<<<1, 32, 0, st>>>(bb);
-    k_bbox<<<grid_for(n), 256, 0, st>>>(ctx->pos4, n, bb);
+    k_bbox<<<reduce_grid(n), kReduceThreads, 0, st>>>(ctx->pos4, n, bb);
     cudaMemsetAsync(tb.sorter.hist, 0, sizeof(uint32_t) * 256 * RadixSorter::kMaxPasses, st);
-    k_tree_keys<<<grid_for(n), 256, 0, st>>>(ctx->pos4, n, D, bb, tb.sorter.keys[0], tb.sorter.vals[0],
-                                              tb.sorter.hist, passes);
+    k_tree_keys<<<reduce_grid(n), kReduceThreads, 0, st>>>(ctx->pos4, n, D, bb, tb.sorter.keys[0], tb.sorter.vals[0],
+                                                           tb.sorter.hist, passes);
     const int fin = radix_sort_pairs(tb.sorter, n, bits, st, ctx->health);
-    const uint32_t *keys = tb.sorter.keys[fin];
-    const uint32_t *order = tb.sorter.vals[fin];
+    TreeArgs a;
+    a.keys = tb.sorter.keys[fin];
+    a.order = tb.sorter.vals[fin];
+    a.n = n;
+    a.depth = D;
+    a.leafcap = leafcap;
+    a.blocks = (n + kTreeThreads - 1) / kTreeThreads;
+    a.levels = tb.levels;
+    a.ints = tb.ints;
+    a.at_int = tb.at_int;
+    a.at_node = tb.at_node;
+    a.totals = tb.totals;
+    a.ticket = tb.ticket;
+    a.tree = tr.tree;
+    a.level_nodes = tr.level_nodes;
+    a.level_count = tr.level_count;
+    a.list_slot = tr.list_slot;
+    a.parent = tr.parent;
+    a.meta = tr.meta;
+    a.node_range = tr.node_range;
+    a.level_cap = tr.level_cap;
+    a.tree_cap = tr.tree_cap;
+    a.node_cap = tr.node_cap;
+    a.health = ctx->health;
+    tb.order = a.order;
+    k_tree_mark<<<a.blocks, kTreeThreads, 0, st>>>(a);
+    k_tree_write<<<a.blocks, kTreeThreads, 0, st>>>(a);
+    k_tree_link<<<(n + 255) / 256, 256, 0, st>>>(a);
 
-    LevelArgs la;
-    la.nstart = tb.nstart;
-    la.ncount = tb.ncount;
-    la.nparent = tb.nparent;
-    la.nrank = tb.ndp;
-    la.noffset = tb.noffset;
-    la.level_count = tr.level_count;
-    la.scan_n = scan_n;
-    la.level_cap = cap;
-    la.cand = tb.scan;
-    la.cand_scan = tb.scan + tb.scan_cap;
-    la.cstart = tb.per_particle;
-    la.keys = keys;
-    la.depth = D;
-    la.leafcap = leafcap;
-    la.n = n;
-    k_root<<<1, 1, 0, st>>>(la);
-    int64_t bound = 1;
-    for (int l = 0; l < D; ++l) {
-        k_children<<<grid_for(bound), 256, 0, st>>>(la, l);
-        scan_exclusive_i64(la.cand, la.cand_scan, tb.scan_blocks, (int)std::min<int64_t>(8 * bound, 8 * cap),
-                           scan_n + l, st);
-        k_emit<<<grid_for(bound), 256, 0, st>>>(la, l);
-        bound = std::min<int64_t>(bound * 8, cap);
-    }
-    k_rank_leaves<<<grid_for(bound), 256, 0, st>>>(la, D);
-
-    // DFS layout: per-particle size sums, then offsets
-    int64_t *ints_at = tb.scan, *nodes_at = tb.scan + (n + 1);
-    int64_t *ints_off = tb.scan + tb.scan_cap, *dp_off = tb.scan + tb.scan_cap + (n + 1);
-    int32_t *first_level = tb.per_particle;  // cstart no longer needed
-    LayoutArgs ya;
-    ya.nstart = tb.nstart;
-    ya.ncount = tb.ncount;
-    ya.nparent = tb.nparent;
-    ya.nrank = tb.ndp;
-    ya.noffset = tb.noffset;
-    ya.level_count = tr.level_count;
-    ya.level_cap = cap;
-    ya.ints_at = ints_at;
-    ya.nodes_at = nodes_at;
-    ya.first_level = first_level;
-    ya.ints_off = ints_off;
-    ya.dp_off = dp_off;
-    ya.tree = tr.tree;
-    ya.level_nodes = tr.level_nodes;
-    ya.list_slot = tr.list_slot;
-    ya.order = order;
-    ya.depth = D;
-    ya.leafcap = leafcap;
-    ya.n = n;
-    ya.tree_cap = tr.tree_cap;
-    ya.node_cap = tr.node_cap;
-    ya.health = ctx->health;
-    ya.meta = tr.meta;
-    ya.node_range = tr.node_range;
-    tb.order = order;
-    k_layout_reset<<<grid_for(n + 1), 256, 0, st>>>(ya);
-    int64_t lb[16];
-    bound = 1;
-    for (int l = 0; l <= D; ++l) {
-        lb[l] = bound;
-        k_marks<<<grid_for(bound), 256, 0, st>>>(ya, l);
-        bound = std::min<int64_t>(bound * 8, cap);
-    }
-    scan_exclusive_i64(ints_at, ints_off, tb.scan_blocks, n, nullptr, st);
-    scan_exclusive_i64(nodes_at, dp_off, tb.scan_blocks, n, nullptr, st);
-    for (int l = 0; l <= D; ++l) k_write<<<grid_for(lb[l]), 256, 0, st>>>(ya, l);
-    for (int l = 1; l <= D; ++l) k_link<<<grid_for(lb[l]), 256, 0, st>>>(ya, l);
-
+    // upper bounds of the level sizes: a level's nodes are children of the
+    // branches above it, each of which holds more than leafcap particles
     tr.n_levels_host = D + 1;
-    for (int l = 0; l < 16; ++l) tr.level_count_host[l] = (l <= D) ? (int)lb[l] : 0;
+    const int64_t branches = (int64_t)n / ((int64_t)leafcap + 1);
+    int64_t bound = 1;
+    for (int l = 0; l < 16; ++l) {
+        tr.level_count_host[l] = (l <= D) ? (int)bound : 0;
+        bound = std::max<int64_t>(1, std::min<int64_t>(n, 8 * std::min(bound, branches)));
+    }
     tr.valid = true;
     return cuda_status(cudaGetLastError(), "tree build");
 }

@@ -5,17 +5,18 @@
 //           M2L.metal:12-108, derivatives.metal:12-156, L2L.metal:12-104,
 //           L2P.metal:12-32, helpers.h:47-81 (leaf P2P)
 //
-// The tree is the reference's flattened int format.  Levels run in order
-// (deepest first up, root first down) as one launch each.  The up pass is one
-// thread per node.  The down pass gives each node a warp: the 32 lanes take
-// consecutive entries of the parent's unchecked list, evaluate the acceptance
-// test and the M2L kernels in parallel, and append rejected branch children
-// to the node's own list with a warp prefix sum, so the list keeps the
-// reference's order (entry-major, child-slot-minor) and the reference's
-// overflow rule (a child that finds the list full is force-accepted).  The
-// per-lane partial local expansions are summed across the warp at the end.
-// Leaves hand one particle to each lane for L2P plus the intra-leaf P2P sum,
-// which runs over the leaf's particles in the reference's order.
+// The tree is the reference's flattened int format.  The up pass is one thread
+// per node (sph_up.cuh: one launch for the GPU-built tree, one per level for a
+// host tree); the down pass runs level by level, one launch each, root first,
+// and gives each node a warp: the 32 lanes take consecutive entries of the
+// parent's unchecked list, evaluate the acceptance test and the M2L kernels in
+// parallel, and append rejected branch children to the node's own list with a
+// warp prefix sum, so the list keeps the reference's order (entry-major,
+// child-slot-minor) and the reference's overflow rule (a child that finds the
+// list full is force-accepted).  The per-lane partial local expansions are
+// summed across the warp at the end.  Leaves hand one particle to each lane
+// for L2P plus the intra-leaf P2P sum, which runs over the leaf's particles in
+// the reference's order.
 //
 // Lists are addressed by each branch's rank among the branches of its level
 // (the reference uses the node's index in its level list); only branches
@@ -23,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "sph_internal.h"
+#include "sph_up.cuh"
 
 namespace sph {
 
@@ -90,12 +92,15 @@ __device__ void p2m(const UpArgs &a, int tp, int dp) {
     bool act = false;
     float mxx = -3.402823466e+38f, mxy = mxx, mxz = mxx, mnx = 3.402823466e+38f, mny = mnx, mnz = mnx;
     const int gt = a.globals[0];
+    // (loads only, so that several particles' loads are in flight together)
+#pragma unroll 4
     for (int i = s; i < e; ++i) {
         const int p = T[i];
         const float4 q = a.pos4[p];
         // the reference's test as shipped is time <= next (every particle
         // active every step); the individual form uses README.md:62's
-        const bool ia = a.individual ? gt >= a.nat[p] : gt <= a.nat[p];
+        const int next = a.nat[p];
+        const bool ia = a.individual ? gt >= next : gt <= next;
         if (!act && ia) act = true;
         mxx = fmax_ref(mxx, q.x);
         mxy = fmax_ref(mxy, q.y);
@@ -107,13 +112,15 @@ __device__ void p2m(const UpArgs &a, int tp, int dp) {
         px += q.x * q.w;
         py += q.y * q.w;
         pz += q.z * q.w;
-        if (ia) mg = fmin_ref(mg, a.gnorm[p]);
+        const float g = a.gnorm[p];
+        if (ia) mg = fmin_ref(mg, g);
     }
     for (int i = s; i < e; ++i) a.active[T[i]] = act ? 1 : 0;
     px = px / m0;
     py = py / m0;
     pz = pz / m0;
     float ex[10] = {m0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
     for (int i = s; i < e; ++i) {
         const float4 q = a.pos4[T[i]];
         const float m = q.w;
@@ -143,22 +150,34 @@ __device__ void m2m(const UpArgs &a, int tp, int dp) {
     float mg = 3.402823466e+38f, px = 0.f, py = 0.f, pz = 0.f, mass = 0.f;
     bool act = false, all_leaves = true;
     float mxx = -3.402823466e+38f, mxy = mxx, mxz = mxx, mnx = 3.402823466e+38f, mny = mnx, mnz = mnx;
-    const int s = tp + 2, e = s + 8;
+    const int s = tp + 2;
     const int my_slot = a.list_slot[dp];
-    for (int i = s; i < e; ++i) {
-        const int c = T[i];
-        if (c == -1) continue;
-        const int cdp = T[c + 1];
-        a.parent_slot[cdp] = my_slot;
-        const float4 *cp = a.poles + (size_t)cdp * kPoleQ;
+    // the children's offsets, data pointers and records are loaded for all
+    // slots at once (an empty slot reads the node's own), so that a branch
+    // waits for memory three times and not once per child
+    int child[8], child_dp[8], child_n[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) child[k] = T[s + k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        child_dp[k] = child[k] != -1 ? T[child[k] + 1] : dp;
+        child_n[k] = child[k] != -1 ? T[child[k]] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (child[k] != -1) a.parent_slot[child_dp[k]] = my_slot;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float4 *cp = a.poles + (size_t)child_dp[k] * kPoleQ;
         const float4 c0 = cp[0], c1 = cp[1], c3 = cp[3], c4 = cp[4];
+        if (child[k] == -1) continue;
         mg = fmin_ref(c3.w, mg);
         mass += c1.x;
         px += c0.x * c1.x;
         py += c0.y * c1.x;
         pz += c0.z * c1.x;
         if (!act && c4.w != 0.f) act = true;
-        if (all_leaves && T[c] == 0) all_leaves = false;
+        if (child_n[k] == 0) all_leaves = false;
         mxx = fmax_ref(mxx, c4.x);
         mxy = fmax_ref(mxy, c4.y);
         mxz = fmax_ref(mxz, c4.z);
@@ -172,12 +191,12 @@ __device__ void m2m(const UpArgs &a, int tp, int dp) {
     py = py / mass;
     pz = pz / mass;
     float ex[10] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int i = s; i < e; ++i) {
-        const int c = T[i];
-        if (c == -1) continue;
-        const int cdp = T[c + 1];
-        float4 *cp = a.poles + (size_t)cdp * kPoleQ;
-        const float4 c0 = cp[0], c1 = cp[1], c2 = cp[2], c4 = cp[4], c5 = cp[5];
+    const bool sync = all_leaves && act;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float4 *cp = a.poles + (size_t)child_dp[k] * kPoleQ;
+        const float4 c0 = cp[0], c1 = cp[1], c2 = cp[2], c5 = cp[5];
+        if (child[k] == -1) continue;
         const float rx = px - c0.x, ry = py - c0.y, rz = pz - c0.z;
         const float cm = c1.x;
         ex[M] += cm;
@@ -191,10 +210,16 @@ __device__ void m2m(const UpArgs &a, int tp, int dp) {
         ex[YY] += c2.x + 0.5f * ry * ry * cm;
         ex[YZ] += c2.y + ry * rz * cm;
         ex[ZZ] += c2.z + 0.5f * rz * rz * c5.z;
-        if (all_leaves && act && c4.w == 0.f) {
+    }
+    if (sync) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int c = child[k];
+            if (c == -1) continue;
+            float4 *cp = a.poles + (size_t)child_dp[k] * kPoleQ;
+            if (cp[4].w != 0.f) continue;
             cp[4].w = 1.f;
-            const int cnp = T[c];
-            const int cs = c + 2, ce = s + cnp;
+            const int cs = c + 2, ce = s + child_n[k];
             for (int j = cs; j < ce; ++j) a.active[T[j]] = 1;
         }
     }
@@ -212,6 +237,10 @@ __global__ void k_up(UpArgs a, int level, int64_t level_cap) {
         else
             p2m(a, tp, dp);
     }
+}
+
+__global__ void __launch_bounds__(128) k_up_all(UpArgs a, UpNodes u) {
+    up_climb(u, [&](int tp, int dp) { p2m(a, tp, dp); }, [&](int tp, int dp) { m2m(a, tp, dp); });
 }
 
 // accept.metal:14-55.  A = (size, pos, minGrav) of the target; B = candidate.
@@ -579,11 +608,15 @@ sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st) {
     u.nat = ctx->nat;
     u.globals = ctx->globals;
     u.individual = ctx->form.timestep == SPH_TIMESTEP_INDIVIDUAL;
-    for (int l = L - 1; l >= 0; --l) {
-        int64_t bound = tr.level_count_host[l];
-        int blocks = (int)((bound + 127) / 128);
-        blocks = blocks < 1 ? 1 : (blocks > 148 * 32 ? 148 * 32 : blocks);
-        k_up<<<blocks, 128, 0, st>>>(u, l, tr.level_cap);
+    if (ctx->params.tree_source == SPH_TREE_GPU) {
+        k_up_all<<<up_blocks(tr, 128), 128, 0, st>>>(u, up_nodes(tr));
+    } else {
+        for (int l = L - 1; l >= 0; --l) {
+            int64_t bound = tr.level_count_host[l];
+            int blocks = (int)((bound + 127) / 128);
+            blocks = blocks < 1 ? 1 : (blocks > 148 * 32 ? 148 * 32 : blocks);
+            k_up<<<blocks, 128, 0, st>>>(u, l, tr.level_cap);
+        }
     }
     DownArgs d;
     d.T = tr.tree;

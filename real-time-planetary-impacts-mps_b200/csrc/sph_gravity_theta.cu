@@ -5,7 +5,7 @@
 // keeps integer-truncated softening coefficients (kernels.h:93,97).
 //
 // Tree: the GPU Morton octree (sph_tree.cu), whose leaves hold contiguous
-// runs of the particles in key order.  Up pass, one launch per level: per
+// runs of the particles in key order.  Up pass (sph_up.cuh, one launch): per
 // node the mass, centre of mass, the second moments Q_jk = sum m r_j r_k about
 // the centre of mass, and the radius of the smallest sphere about the centre
 // of mass that holds the node's box.
@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "sph_internal.h"
+#include "sph_up.cuh"
 
 namespace sph {
 
@@ -44,8 +45,6 @@ __device__ __forceinline__ float corner_radius(float cx, float cy, float cz, flo
 
 struct ThetaUpArgs {
     const int32_t *T;
-    const int32_t *level_nodes;
-    const int32_t *level_count;
     const int32_t *list_slot;
     int32_t *parent_slot;
     float4 *poles;
@@ -72,10 +71,11 @@ __device__ void p2m_theta(const ThetaUpArgs &a, int tp, int dp) {
         act = false;
         for (int i = 0; i < np && !act; ++i) act = gt >= a.nat[T[s + i]];
     }
+    for (int i = 0; i < np; ++i) a.active[T[s + i]] = act ? 1 : 0;
+    // (loads only, so that several particles' loads are in flight together)
+#pragma unroll 4
     for (int i = 0; i < np; ++i) {
-        const int p = T[s + i];
-        const float4 q = a.pos4[p];
-        a.active[p] = act ? 1 : 0;
+        const float4 q = a.pos4[T[s + i]];
         m += q.w;
         sx += q.w * (q.x - x0.x);
         sy += q.w * (q.y - x0.y);
@@ -89,6 +89,7 @@ __device__ void p2m_theta(const ThetaUpArgs &a, int tp, int dp) {
     }
     const float ox = sx / m, oy = sy / m, oz = sz / m;  // com - x0
     float qxx = 0.f, qxy = 0.f, qxz = 0.f, qyy = 0.f, qyz = 0.f, qzz = 0.f;
+#pragma unroll 4
     for (int i = 0; i < np; ++i) {
         const float4 q = a.pos4[T[s + i]];
         const float rx = (q.x - x0.x) - ox, ry = (q.y - x0.y) - oy, rz = (q.z - x0.z) - oz;
@@ -116,13 +117,21 @@ __device__ void m2m_theta(const ThetaUpArgs &a, int tp, int dp) {
     float4 c0f = make_float4(0.f, 0.f, 0.f, 0.f);
     float m = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
     float mnx = 3.402823466e+38f, mny = mnx, mnz = mnx, mxx = -mnx, mxy = -mnx, mxz = -mnx;
+    // all slots' loads at once (an empty slot reads the node's own record): a
+    // branch waits for memory three times and not once per child
+    int child[8], child_dp[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) child[k] = T[tp + 2 + k];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) child_dp[k] = child[k] != -1 ? T[child[k] + 1] : dp;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (child[k] != -1) a.parent_slot[child_dp[k]] = my_slot;
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int c = T[tp + 2 + k];
-        if (c == -1) continue;
-        const int cdp = T[c + 1];
-        a.parent_slot[cdp] = my_slot;
-        const float4 *cp = a.poles + (size_t)cdp * kPoleQ;
+        const float4 *cp = a.poles + (size_t)child_dp[k] * kPoleQ;
         const float4 q0 = cp[0], q1 = cp[1], q3 = cp[3], q4 = cp[4];
+        if (child[k] == -1) continue;
         if (first < 0) {
             first = k;
             c0f = q0;
@@ -140,11 +149,11 @@ __device__ void m2m_theta(const ThetaUpArgs &a, int tp, int dp) {
     }
     const float ox = sx / m, oy = sy / m, oz = sz / m;
     float qxx = 0.f, qxy = 0.f, qxz = 0.f, qyy = 0.f, qyz = 0.f, qzz = 0.f;
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int c = T[tp + 2 + k];
-        if (c == -1) continue;
-        const float4 *cp = a.poles + (size_t)T[c + 1] * kPoleQ;
+        const float4 *cp = a.poles + (size_t)child_dp[k] * kPoleQ;
         const float4 q0 = cp[0], q1 = cp[1], q2 = cp[2];
+        if (child[k] == -1) continue;
         const float rx = (q0.x - c0f.x) - ox, ry = (q0.y - c0f.y) - oy, rz = (q0.z - c0f.z) - oz;
         const float mc = q1.x;
         qxx += q1.y + mc * rx * rx;
@@ -161,17 +170,19 @@ __device__ void m2m_theta(const ThetaUpArgs &a, int tp, int dp) {
     if (a.individual) {
         act = false;
         bool all_leaves = true;
+#pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const int c = T[tp + 2 + k];
+            const int c = child[k];
             if (c == -1) continue;
-            if (a.poles[(size_t)T[c + 1] * kPoleQ + 4].w != 0.f) act = true;
+            if (a.poles[(size_t)child_dp[k] * kPoleQ + 4].w != 0.f) act = true;
             if (T[c] == 0) all_leaves = false;
         }
         if (act && all_leaves) {
+#pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const int c = T[tp + 2 + k];
+                const int c = child[k];
                 if (c == -1) continue;
-                a.poles[(size_t)T[c + 1] * kPoleQ + 4].w = 1.f;
+                a.poles[(size_t)child_dp[k] * kPoleQ + 4].w = 1.f;
                 for (int j = 0; j < T[c]; ++j) a.active[T[c + 2 + j]] = 1;
             }
         }
@@ -186,17 +197,9 @@ __device__ void m2m_theta(const ThetaUpArgs &a, int tp, int dp) {
     pr[5] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-__global__ void k_up_theta(ThetaUpArgs a, int level, int64_t level_cap) {
-    const int cnt = a.level_count[level];
-    const int32_t *nodes = a.level_nodes + (size_t)level * level_cap;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
-        const int tp = nodes[t];
-        const int dp = a.T[tp + 1];
-        if (a.T[tp] == 0)
-            m2m_theta(a, tp, dp);
-        else
-            p2m_theta(a, tp, dp);
-    }
+// (the walk needs the GPU-built tree, so the up pass is always the climb)
+__global__ void __launch_bounds__(128) k_up_theta(ThetaUpArgs a, UpNodes u) {
+    up_climb(u, [&](int tp, int dp) { p2m_theta(a, tp, dp); }, [&](int tp, int dp) { m2m_theta(a, tp, dp); });
 }
 
 // Cubic-spline softened pair kernel with its exact coefficients (the
@@ -603,11 +606,8 @@ static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t s
         return SPH_ERR_UNSUPPORTED;
     }
     const int n = ctx->n;
-    const int L = tr.n_levels_host;
     ThetaUpArgs u;
     u.T = tr.tree;
-    u.level_nodes = tr.level_nodes;
-    u.level_count = tr.level_count;
     u.list_slot = tr.list_slot;
     u.parent_slot = tr.parent_slot;
     u.poles = tr.poles;
@@ -618,12 +618,7 @@ static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t s
     // activity follows the next active times only when the accelerations are
     // computed (the potential for the diagnostics covers every particle)
     u.individual = acc && ctx->form.timestep == SPH_TIMESTEP_INDIVIDUAL;
-    for (int l = L - 1; l >= 0; --l) {
-        int64_t bound = tr.level_count_host[l];
-        int blocks = (int)((bound + 127) / 128);
-        blocks = blocks < 1 ? 1 : (blocks > 148 * 32 ? 148 * 32 : blocks);
-        k_up_theta<<<blocks, 128, 0, st>>>(u, l, tr.level_cap);
-    }
+    k_up_theta<<<up_blocks(tr, 128), 128, 0, st>>>(u, up_nodes(tr));
     // resident warps of the walk, each with its two node queues
     static int max_blocks_per_sm = 0;
     if (max_blocks_per_sm == 0) {

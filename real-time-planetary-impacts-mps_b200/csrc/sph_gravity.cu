@@ -23,6 +23,8 @@
 // write lists, so storage is bounded by the branch count.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "sph_internal.h"
 #include "sph_up.cuh"
 
@@ -353,13 +355,17 @@ struct DownArgs {
     uint32_t *health;
 };
 
-__device__ __forceinline__ void m2l_node(const DownArgs &a, int node, float lx, float ly, float lz, float *acc) {
-    const float4 *bp = a.poles + (size_t)a.T[node + 1] * kPoleQ;
-    m2l_add(lx, ly, lz, bp[0], bp[1], bp[2], acc);
-}
+constexpr int kDownThreads = 128;
 
-__global__ void __launch_bounds__(128) k_down(DownArgs a, int level, int64_t level_cap) {
+__global__ void __launch_bounds__(kDownThreads) k_down(DownArgs a, int level, int64_t level_cap) {
     const int lane = threadIdx.x & 31;
+#ifndef SPH_PARITY
+    __shared__ int32_t s_m2l[kDownThreads / 32][64];     // accepted nodes (data pointers)
+    __shared__ int32_t s_child[kDownThreads / 32][256];  // children of 32 rejected entries (tree offsets)
+    constexpr unsigned kFull = 0xffffffffu;
+    const int w = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+#endif
     const int warp0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int cnt = a.level_count[level];
@@ -452,9 +458,27 @@ __global__ void __launch_bounds__(128) k_down(DownArgs a, int level, int64_t lev
 #pragma unroll
         for (int j = 0; j < 10; ++j) le[j] = __shfl_sync(0xffffffffu, le[j], 0);
 #else
+        // Every lane works on every step: the entries' acceptance tests, the
+        // rejected entries' children and the accepted nodes' M2L each run 32 at
+        // a time.  Accepted nodes wait in s_m2l until 32 are there; the
+        // children of the rejected entries are numbered consecutively through
+        // s_child, which keeps the list's order (entry-major, slot-minor).
         float acc[10];
 #pragma unroll
         for (int j = 0; j < 10; ++j) acc[j] = 0.f;
+        int nm = 0;  // accepted nodes that wait
+        auto accepted = [&](bool yes, int node_dp) {
+            const unsigned m = __ballot_sync(kFull, yes);
+            if (yes) s_m2l[w][nm + __popc(m & lt)] = node_dp;
+            nm += __popc(m);
+            __syncwarp();
+            if (nm >= 32) {
+                nm -= 32;
+                const float4 *bp = a.poles + (size_t)s_m2l[w][nm + lane] * kPoleQ;
+                m2l_add(lx, ly, lz, bp[0], bp[1], bp[2], acc);
+                __syncwarp();
+            }
+        };
         for (int c0 = 0; c0 < cap; c0 += 32) {
             const int i = c0 + lane;
             int e = (i < cap) ? in[i] : -1;
@@ -462,58 +486,78 @@ __global__ void __launch_bounds__(128) k_down(DownArgs a, int level, int64_t lev
                 raise_health(a.health, SPH_HEALTH_LIST_CAPACITY);
                 e = -1;
             }
-            const uint32_t stop = __ballot_sync(0xffffffffu, e == -1);
+            const uint32_t stop = __ballot_sync(kFull, e == -1);
             const int nvalid = stop ? (__ffs(stop) - 1) : 32;
-            uint32_t cand = 0u;
-            if (lane < nvalid) {
-                const float4 *bp = a.poles + (size_t)T[e + 1] * kPoleQ;
+            const bool valid = lane < nvalid;
+            bool yes = false;
+            int edp = 0, kids = 0;
+            int child[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) child[k] = -1;
+            if (valid) {
+                edp = T[e + 1];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) child[k] = T[e + 2 + k];
+                const float4 *bp = a.poles + (size_t)edp * kPoleQ;
                 const float4 b0 = bp[0], b1 = bp[1], b2 = bp[2];
-                if (mac_accept(s0.w, s0.x, s0.y, s0.z, s_min_grav, b0, b1, b2)) {
-                    m2l_add(lx, ly, lz, b0, b1, b2, acc);
-                } else {
+                yes = mac_accept(s0.w, s0.x, s0.y, s0.z, s_min_grav, b0, b1, b2);
+                if (!yes) {
+#pragma unroll
                     for (int k = 0; k < 8; ++k) {
-                        const int c = T[e + 2 + k];
-                        if (c == tp || c == -1) continue;
-                        if (np != 0 || T[c] != 0) {
-                            // leaf target: every child forced (helpers.h:83-123, depth 1);
-                            // leaf child of a branch target: forced (helpers.h:141)
-                            m2l_node(a, c, lx, ly, lz, acc);
-                        } else {
-                            const float4 *cp = a.poles + (size_t)T[c + 1] * kPoleQ;
-                            const float4 c0v = cp[0], c1v = cp[1], c2v = cp[2];
-                            if (mac_accept(s0.w, s0.x, s0.y, s0.z, s_min_grav, c0v, c1v, c2v))
-                                m2l_add(lx, ly, lz, c0v, c1v, c2v, acc);
-                            else
-                                cand |= 1u << k;
-                        }
+                        if (child[k] == tp) child[k] = -1;
+                        kids += child[k] != -1;
                     }
                 }
             }
-            if (np == 0) {
-                // ordered append of the rejected branch children (entry-major)
-                const int mine = __popc(cand);
-                int incl = mine;
+            accepted(yes, edp);
+            int at = kids;  // inclusive, then exclusive scan
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                int pos = op + incl - mine;
-                while (cand) {
-                    const int k = __ffs(cand) - 1;
-                    cand &= cand - 1u;
-                    const int c = T[e + 2 + k];
-                    if (pos < cap)
-                        out[pos] = c;
-                    else
-                        m2l_node(a, c, lx, ly, lz, acc);  // list full: forced accept
-                    ++pos;
-                }
-                op = min(op + total, cap);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kFull, at, o);
+                if (lane >= o) at += y;
             }
+            const int total = __shfl_sync(kFull, at, 31);
+            at -= kids;
+            if (kids) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (child[k] != -1) s_child[w][at++] = child[k];
+            }
+            __syncwarp();
+            for (int j0 = 0; j0 < total; j0 += 32) {
+                const bool has = j0 + lane < total;
+                const int c = has ? s_child[w][j0 + lane] : 0;
+                const int cdp = has ? T[c + 1] : 0;
+                if (np != 0) {
+                    // leaf target: every child forced (helpers.h:83-123, depth 1)
+                    accepted(has, cdp);
+                    continue;
+                }
+                // leaf child of a branch target: forced (helpers.h:141)
+                bool take = has && T[c] != 0;
+                bool put = false;
+                if (has && !take) {
+                    const float4 *cp = a.poles + (size_t)cdp * kPoleQ;
+                    take = mac_accept(s0.w, s0.x, s0.y, s0.z, s_min_grav, cp[0], cp[1], cp[2]);
+                    put = !take;
+                }
+                const unsigned m = __ballot_sync(kFull, put);
+                const int pos = op + __popc(m & lt);
+                if (put) {
+                    if (pos < cap) out[pos] = c;
+                    else take = true;  // list full: forced accept
+                }
+                op = min(op + __popc(m), cap);
+                accepted(take, cdp);
+            }
+            __syncwarp();
             if (stop) break;
         }
+        if (lane < nm) {
+            const float4 *bp = a.poles + (size_t)s_m2l[w][lane] * kPoleQ;
+            m2l_add(lx, ly, lz, bp[0], bp[1], bp[2], acc);
+        }
+        __syncwarp();
         if (np == 0 && lane == 0 && op < cap) out[op] = -1;
         // sum the lanes' partial expansions
 #pragma unroll
@@ -560,27 +604,33 @@ __global__ void __launch_bounds__(128) k_down(DownArgs a, int level, int64_t lev
             const int s = tp + 2;
             for (int i0 = 0; i0 < np; i0 += 32) {
                 const int ii = i0 + lane;
-                if (ii >= np) continue;
-                const int p = T[s + ii];
-                if (!a.active[p]) continue;
-                const float4 xi = a.pos4[p];
+                const int p = ii < np ? T[s + ii] : -1;
+                const float4 xi = p >= 0 ? a.pos4[p] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const bool act = p >= 0 && a.active[p];
                 const float qx = xi.x - lx, qy = xi.y - ly, qz = xi.z - lz;
                 float ax = le[X], ay = le[Y], az = le[Z];
                 ax += qx * le[XX] + qy * le[XY] + qz * le[XZ];
                 ay += qx * le[XY] + qy * le[YY] + qz * le[YZ];
                 az += qx * le[XZ] + qy * le[YZ] + qz * le[ZZ];
-                for (int j = 0; j < np; ++j) {
-                    if (j == ii) continue;
-                    const float4 xj = a.pos4[T[s + j]];
-                    const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
-                    const float r = sqrtf(dx * dx + dy * dy + dz * dz);
-                    if (r == 0.f) continue;
-                    const float rhx = dx / r, rhy = dy / r, rhz = dz / r;
-                    const float fm = xj.w * grav_dphi_dr(r);
-                    ax -= fm * rhx;
-                    ay -= fm * rhy;
-                    az -= fm * rhz;
+                // the leaf's particles, 32 at a time from the lanes' registers
+                for (int j0 = 0; j0 < np; j0 += 32) {
+                    float4 xs = xi;
+                    if (j0 != i0) xs = j0 + lane < np ? a.pos4[T[s + j0 + lane]] : xi;
+                    const int cnt = min(32, np - j0);
+                    for (int j = 0; j < cnt; ++j) {
+                        const float xjx = __shfl_sync(0xffffffffu, xs.x, j), xjy = __shfl_sync(0xffffffffu, xs.y, j);
+                        const float xjz = __shfl_sync(0xffffffffu, xs.z, j), mj = __shfl_sync(0xffffffffu, xs.w, j);
+                        const float dx = xi.x - xjx, dy = xi.y - xjy, dz = xi.z - xjz;
+                        const float r = sqrtf(dx * dx + dy * dy + dz * dz);
+                        if (r == 0.f || j0 + j == ii) continue;
+                        const float rhx = dx / r, rhy = dy / r, rhz = dz / r;
+                        const float fm = mj * grav_dphi_dr(r);
+                        ax -= fm * rhx;
+                        ay -= fm * rhy;
+                        az -= fm * rhz;
+                    }
                 }
+                if (!act) continue;
                 const float4 old = a.acc4[p];
                 a.acc4[p] = make_float4(kG * ax, kG * ay, kG * az, old.w);
                 a.gnorm[p] = sqrtf(ax * ax + ay * ay + az * az);
@@ -638,9 +688,9 @@ sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st) {
         d.list_in = (l % 2 == 0) ? tr.lists[0] : tr.lists[1];
         d.list_out = (l % 2 == 0) ? tr.lists[1] : tr.lists[0];
         int64_t bound = tr.level_count_host[l];
-        int blocks = (int)((bound * 32 + 127) / 128);
-        blocks = blocks < 1 ? 1 : (blocks > 148 * 32 ? 148 * 32 : blocks);
-        k_down<<<blocks, 128, 0, st>>>(d, l, tr.level_cap);
+        int64_t want = (bound * 32 + kDownThreads - 1) / kDownThreads;
+        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(want, 148 * 32));
+        k_down<<<blocks, kDownThreads, 0, st>>>(d, l, tr.level_cap);
     }
     return cuda_status(cudaGetLastError(), "gravity");
 }

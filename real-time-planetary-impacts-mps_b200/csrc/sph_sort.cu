@@ -11,7 +11,7 @@
 //    histograms of all passes (the one-sweep "upsweep"); it also clears only
 //    the cell entries the previous sort filled, instead of all 2^24;
 //  * k_onesweep does one stable 8-bit pass per launch: warp-level ranking
-//    with match_any, a decoupled look-back across tiles for each digit (every
+//    with ballots, a decoupled look-back across tiles for each digit (every
 //    wait is bounded and raises a health bit instead of hanging), scatter;
 //    the top byte of the 24-bit keys is always zero, so three passes give the
 //    reference's four-pass order exactly;
@@ -19,6 +19,7 @@
 //    neighbouring keys, without atomics.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 
 #include "sph_internal.h"
@@ -38,22 +39,31 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// Blocks of the key kernels: each ends in one set of 768 global atomics, which
+// took the time with 2368 blocks (N = 1e6: 28 of the sort's 131 us).
+constexpr int kHashThreads = 512;
+constexpr int kHashBlocks = 296;
+int hash_grid(int n) { return std::max(1, std::min(kHashBlocks, (n + kHashThreads - 1) / kHashThreads)); }
+
 // Keys of the cell grid + all three digit histograms; clears the previous
-// sort's occupied cells first (they are read from the previous sorted keys,
-// which live in the buffer the first pass is about to overwrite).
-__global__ void k_hash_hist(const float4 *__restrict__ pos4, int n, uint32_t *__restrict__ keys,
-                            uint32_t *__restrict__ vals, uint32_t *__restrict__ hist,
-                            const uint32_t *__restrict__ prev_keys, uint2 *__restrict__ cell_range, int clear_prev) {
+// sort's occupied cells and units first (they are read from the previous
+// sorted keys, which live in the buffer the first pass is about to overwrite).
+__global__ void __launch_bounds__(kHashThreads)
+    k_hash_hist(const float4 *__restrict__ pos4, int n, uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
+                uint32_t *__restrict__ hist, const uint32_t *__restrict__ prev_keys, uint2 *__restrict__ cell_range,
+                uint2 *__restrict__ units, int clear_prev) {
     __shared__ uint32_t sh[3][256];
     for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x) (&sh[0][0])[i] = 0u;
     __syncthreads();
+#pragma unroll 2
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (clear_prev) {
-            uint32_t pk = prev_keys[i];
-            if (i == 0 || prev_keys[i - 1] != pk) cell_range[pk] = make_uint2(0xffffffffu, 0u);
+            const uint32_t pk = prev_keys[i], before = i ? prev_keys[i - 1] : ~pk;
+            if (before != pk) cell_range[pk] = make_uint2(0xffffffffu, 0u);
+            if ((before ^ pk) >> (3 * kUnitShift)) units[pk >> (3 * kUnitShift)] = make_uint2(0xffffffffu, 0xffffffffu);
         }
-        float4 p = pos4[i];
-        uint32_t k = cell_key(p.x, p.y, p.z);
+        const float4 p = __ldg(pos4 + i);
+        const uint32_t k = cell_key(p.x, p.y, p.z);
         keys[i] = k;
         vals[i] = (uint32_t)i;
         atomicAdd(&sh[0][k & 255u], 1u);
@@ -62,37 +72,56 @@ __global__ void k_hash_hist(const float4 *__restrict__ pos4, int n, uint32_t *__
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x) {
-        uint32_t v = (&sh[0][0])[i];
+        const uint32_t v = (&sh[0][0])[i];
         if (v) atomicAdd(hist + i, v);
     }
 }
 
-// One stable 8-bit LSD pass.
+// The valid lanes of the warp whose 8-bit digit equals this lane's, by a ballot
+// per bit: match_any takes a round per distinct digit.
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool ok) {
+    uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? m : ~m;
+    }
+    return peers;
+}
+
+// One stable 8-bit LSD pass over tiles of 256 x ITEMS keys.
+template <int ITEMS>
 __global__ void __launch_bounds__(RadixSorter::kThreads)
     k_onesweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int n, int shift,
                const uint32_t *__restrict__ hist, uint32_t *status, uint32_t *counter, uint32_t *health,
                int spin_limit) {
-    constexpr int T = RadixSorter::kThreads, I = RadixSorter::kItems, W = T / 32;
+    constexpr int T = RadixSorter::kThreads, I = ITEMS, W = T / 32;
+    constexpr int kWindow = 8;  // look-back words read at a time
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[W][256];
     __shared__ uint32_t s_base[256];
-    __shared__ uint32_t s_scan[256];
+    __shared__ uint32_t s_scan[W];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_tile = atomicAdd(counter, 1u);
     for (int i = tid; i < W * 256; i += T) (&s_warp[0][0])[i] = 0u;
-    // exclusive prefix of the global histogram over digits (Hillis-Steele in smem)
-    s_scan[tid] = hist[tid];
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {
-        uint32_t v = (tid >= off) ? s_scan[tid - off] : 0u;
-        __syncthreads();
-        s_scan[tid] += v;
-        __syncthreads();
+    // exclusive prefix of the global histogram over digits
+    const uint32_t count = hist[tid];
+    uint32_t incl = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
     }
-    const uint32_t global_excl = s_scan[tid] - hist[tid];
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    uint32_t global_excl = incl - count;
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+        if (w < warp) global_excl += s_scan[w];
     const uint32_t tile = s_tile;
-    const int64_t base = (int64_t)tile * RadixSorter::kTile + (int64_t)warp * (I * 32);
+    const int64_t base = (int64_t)tile * (T * I) + (int64_t)warp * (I * 32);
     const uint32_t lt = lanemask_lt();
 
     uint32_t k[I], v[I], rank[I];
@@ -105,11 +134,10 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
     }
 #pragma unroll
     for (int it = 0; it < I; ++it) {
-        int64_t idx = base + it * 32 + lane;
-        bool ok = idx < n;
-        uint32_t d = ok ? ((k[it] >> shift) & 255u) : 256u;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        uint32_t before = ok ? s_warp[warp][d] : 0u;
+        const bool ok = base + it * 32 + lane < n;
+        const uint32_t d = (k[it] >> shift) & 255u;
+        const uint32_t peers = digit_peers(d, ok);
+        const uint32_t before = s_warp[warp][d];
         rank[it] = before + __popc(peers & lt);
         __syncwarp();
         if (ok && (peers & lt) == 0u) s_warp[warp][d] = before + __popc(peers);
@@ -124,7 +152,8 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
         s_warp[w][tid] = tile_count;
         tile_count += c;
     }
-    // decoupled look-back for digit `tid`
+    // decoupled look-back for digit `tid`, kWindow predecessors per round trip
+    // (the words carry the counts themselves: nothing else has to be ordered)
     uint32_t excl = 0;
     volatile uint32_t *vs = status;
     if (tile == 0) {
@@ -133,22 +162,30 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
         vs[(size_t)tile * 256 + tid] = kFlagAgg | tile_count;
         int64_t j = (int64_t)tile - 1;
         int spins = 0;
-        while (j >= 0) {
-            uint32_t s = vs[(size_t)j * 256 + tid];
-            uint32_t flag = s & ~kValueMask;
-            if (flag == 0u) {
+        bool done = false;
+        while (!done) {
+            uint32_t s[kWindow];
+#pragma unroll
+            for (int q = 0; q < kWindow; ++q) s[q] = j - q >= 0 ? vs[(size_t)(j - q) * 256 + tid] : 2u << 30;
+            int got = 0;
+#pragma unroll
+            for (int q = 0; q < kWindow; ++q) {
+                const uint32_t flag = s[q] & ~kValueMask;
+                if (!done && got == q && flag != 0u) {
+                    excl += s[q] & kValueMask;
+                    ++got;
+                    done = flag == kFlagPrefix;
+                }
+            }
+            j -= got;
+            if (got == 0) {
                 if (++spins > spin_limit) {
                     raise_health(health, SPH_HEALTH_SORT_TIMEOUT);
                     break;
                 }
-                __nanosleep(64);
-                continue;
+                __nanosleep(32);
             }
-            excl += s & kValueMask;
-            if (flag == kFlagPrefix) break;
-            --j;
         }
-        __threadfence();
         vs[(size_t)tile * 256 + tid] = kFlagPrefix | ((excl + tile_count) & kValueMask);
     }
     s_base[tid] = global_excl + excl;
@@ -167,22 +204,27 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
     }
 }
 
-__global__ void k_cells(const uint32_t *__restrict__ keys, int n, uint2 *__restrict__ cell_range) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t k = keys[i];
-    if (i == 0 || keys[i - 1] != k) cell_range[k].x = (uint32_t)i;
-    if (i == n - 1 || keys[i + 1] != k) cell_range[k].y = (uint32_t)i;
+void launch_onesweep(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, int n,
+                     int shift, const uint32_t *hist, uint32_t *status, uint32_t *counter, uint32_t *health,
+                     int spin_limit, cudaStream_t st) {
+    const int tiles = RadixSorter::tiles(n), items = RadixSorter::items(n);
+    auto *kernel = items == 4 ? k_onesweep<4> : items == 8 ? k_onesweep<8> : k_onesweep<16>;
+    kernel<<<tiles, RadixSorter::kThreads, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n, shift, hist, status,
+                                                    counter, health, spin_limit);
 }
 
-// The unit table: (first, last) sorted index of every occupied 64-cell unit
-// (cell key >> 6); the table is cleared to 0xff bytes before.
-__global__ void k_units(const uint32_t *__restrict__ keys, int n, uint2 *__restrict__ units) {
+// Each occupied cell's (first, last) sorted index, and each occupied unit's
+// (cell key >> 6).
+__global__ void k_cells(const uint32_t *__restrict__ keys, int n, uint2 *__restrict__ cell_range,
+                        uint2 *__restrict__ units) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t u = keys[i] >> (3 * kUnitShift);
-    if (i == 0 || (keys[i - 1] >> (3 * kUnitShift)) != u) units[u].x = (uint32_t)i;
-    if (i == n - 1 || (keys[i + 1] >> (3 * kUnitShift)) != u) units[u].y = (uint32_t)i;
+    const uint32_t k = keys[i], u = k >> (3 * kUnitShift);
+    const uint32_t before = i ? keys[i - 1] : ~k, after = i < n - 1 ? keys[i + 1] : ~k;
+    if (before != k) cell_range[k].x = (uint32_t)i;
+    if (after != k) cell_range[k].y = (uint32_t)i;
+    if ((before >> (3 * kUnitShift)) != u) units[u].x = (uint32_t)i;
+    if ((after >> (3 * kUnitShift)) != u) units[u].y = (uint32_t)i;
 }
 
 __global__ void k_init_cells(uint2 *cell_range, uint32_t count) {
@@ -194,18 +236,18 @@ __global__ void k_init_cells(uint2 *cell_range, uint32_t count) {
 
 sph_status sort_alloc(RadixSorter &s, int n) {
     s.n_cap = n;
-    s.tiles_cap = (n + RadixSorter::kTile - 1) / RadixSorter::kTile;
-    if (s.tiles_cap < 1) s.tiles_cap = 1;
+    constexpr int kMinTile = RadixSorter::kThreads * RadixSorter::kMinItems;
+    const size_t tiles = (size_t)std::max(1, (n + kMinTile - 1) / kMinTile);
+    constexpr size_t kHead = 256 * RadixSorter::kMaxPasses + RadixSorter::kMaxPasses;
     size_t nb = sizeof(uint32_t) * (size_t)(n > 0 ? n : 1);
     cudaError_t e = cudaSuccess;
     for (int b = 0; b < 2; ++b) {
         if (e == cudaSuccess) e = cudaMalloc(&s.keys[b], nb);
         if (e == cudaSuccess) e = cudaMalloc(&s.vals[b], nb);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&s.hist, sizeof(uint32_t) * 256 * RadixSorter::kMaxPasses);
-    if (e == cudaSuccess)
-        e = cudaMalloc(&s.status, sizeof(uint32_t) * 256 * (size_t)s.tiles_cap * RadixSorter::kMaxPasses);
-    if (e == cudaSuccess) e = cudaMalloc(&s.counters, sizeof(uint32_t) * RadixSorter::kMaxPasses);
+    if (e == cudaSuccess) e = cudaMalloc(&s.hist, sizeof(uint32_t) * (kHead + 256 * tiles * RadixSorter::kMaxPasses));
+    s.counters = s.hist + 256 * RadixSorter::kMaxPasses;
+    s.status = s.hist + kHead;
     return cuda_status(e, "sort_alloc");
 }
 
@@ -216,23 +258,21 @@ void sort_free(RadixSorter &s) {
         s.keys[b] = s.vals[b] = nullptr;
     }
     cudaFree(s.hist);
-    cudaFree(s.status);
-    cudaFree(s.counters);
     s.hist = s.status = s.counters = nullptr;
+}
+
+void radix_clear(RadixSorter &s, int n, int bits, cudaStream_t st) {
+    const size_t words = (size_t)(s.status - s.hist) + 256 * (size_t)RadixSorter::tiles(n) * ((bits + 7) / 8);
+    cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * words, st);
 }
 
 int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t *health) {
     const int passes = (bits + 7) / 8;
-    const int tiles = (n + RadixSorter::kTile - 1) / RadixSorter::kTile;
     int cur = 0;
     if (n <= 0) return 0;
-    cudaMemsetAsync(s.status, 0, sizeof(uint32_t) * 256 * (size_t)tiles * passes, st);
-    cudaMemsetAsync(s.counters, 0, sizeof(uint32_t) * RadixSorter::kMaxPasses, st);
     for (int p = 0; p < passes; ++p) {
-        k_onesweep<<<tiles, RadixSorter::kThreads, 0, st>>>(s.keys[cur], s.vals[cur], s.keys[cur ^ 1],
-                                                             s.vals[cur ^ 1], n, 8 * p, s.hist + 256 * p,
-                                                             s.status + (size_t)256 * tiles * p, s.counters + p,
-                                                             health, s.spin_limit);
+        launch_onesweep(s.keys[cur], s.vals[cur], s.keys[cur ^ 1], s.vals[cur ^ 1], n, 8 * p, s.hist + 256 * p,
+                        s.status + (size_t)256 * RadixSorter::tiles(n) * p, s.counters + p, health, s.spin_limit, st);
         cur ^= 1;
     }
     return cur;
@@ -240,6 +280,7 @@ int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t 
 
 void launch_init_cells(sph_ctx *ctx, cudaStream_t st) {
     k_init_cells<<<148 * 8, 256, 0, st>>>(ctx->cell_range, kNumCells);
+    cudaMemsetAsync(ctx->units, 0xff, sizeof(uint2) * kNumUnits, st);
     ctx->cells_have_prev = false;
 }
 
@@ -247,10 +288,8 @@ sph_status launch_sort(sph_ctx *ctx, cudaStream_t st) {
     RadixSorter &s = ctx->cell_sort;
     const int n = ctx->n;
     if (n <= 0) return SPH_OK;
-    cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * 256 * RadixSorter::kMaxPasses, st);
+    radix_clear(s, n, 24, st);
     const int prev = ctx->cell_final;
-    int blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
     // the previous sorted keys live in keys[prev]; the hash writes keys[0] and
     // the first pass writes keys[1], so clearing must use keys[prev] before that
     uint32_t *clear_src = s.keys[prev];
@@ -258,16 +297,13 @@ sph_status launch_sort(sph_ctx *ctx, cudaStream_t st) {
         // never the case with 3 passes (result in buffer 1); kept for safety
         launch_init_cells(ctx, st);
     }
-    k_hash_hist<<<blocks, 256, 0, st>>>(ctx->pos4, n, s.keys[0], s.vals[0], s.hist, clear_src, ctx->cell_range,
-                                        (ctx->cells_have_prev && prev == 1) ? 1 : 0);
+    k_hash_hist<<<hash_grid(n), kHashThreads, 0, st>>>(ctx->pos4, n, s.keys[0], s.vals[0], s.hist, clear_src,
+                                                       ctx->cell_range, ctx->units,
+                                                       (ctx->cells_have_prev && prev == 1) ? 1 : 0);
     int fin = radix_sort_pairs(s, n, 24, st, ctx->health);
     ctx->cell_final = fin;
-    k_cells<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->cell_range);
+    k_cells<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->cell_range, ctx->units);
     ctx->cells_have_prev = true;
-    if (ctx->units) {
-        cudaMemsetAsync(ctx->units, 0xff, sizeof(uint2) * kNumUnits, st);
-        k_units<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->units);
-    }
     return cuda_status(cudaGetLastError(), "sort");
 }
 
@@ -286,7 +322,7 @@ sph_status launch_sort(sph_ctx *ctx, cudaStream_t st) {
 // outputs plus one fixed scratch array compiled into this library.
 //
 // The scratch is a file-scope __device__ array, so every GPU that loads the
-// library carries it (kNoAllocScratchBytes, about 2.2 MiB) until the process
+// library carries it (kNoAllocScratchBytes, about 2.8 MiB) until the process
 // exits.  On the host, the array's name is only a stand-in symbol, not a
 // device address; its device address is looked up with cudaGetSymbolAddress
 // on every call, for the device current at that call (the first lookup on a
@@ -303,7 +339,8 @@ namespace sph {
 namespace {
 
 constexpr int kNoAllocPasses = 3;  // 24-bit cell keys
-constexpr int kNoAllocTiles = (SPH_SORT_NOALLOC_MAX_N + RadixSorter::kTile - 1) / RadixSorter::kTile;
+constexpr int kNoAllocTiles = SPH_SORT_NOALLOC_MAX_N / (RadixSorter::kThreads * RadixSorter::kMinItems);
+static_assert(SPH_SORT_NOALLOC_MAX_N % (RadixSorter::kThreads * RadixSorter::kMinItems) == 0, "whole tiles");
 constexpr size_t kNoAllocKeysOff = 0;
 constexpr size_t kNoAllocValsOff = kNoAllocKeysOff + sizeof(uint32_t) * SPH_SORT_NOALLOC_MAX_N;
 // the words that must be zero when a call starts sit together from here on:
@@ -369,7 +406,7 @@ extern "C" sph_status sph_sort_cells_noalloc(const float *pos_xyz, int32_t n, ui
     sph_status st = noalloc_scratch(&s);
     if (st != SPH_OK) return st;
     cudaStream_t cs = (cudaStream_t)stream;
-    const int tiles = (n + RadixSorter::kTile - 1) / RadixSorter::kTile;
+    const int tiles = RadixSorter::tiles(n);
     uint32_t *tk = reinterpret_cast<uint32_t *>(s + kNoAllocKeysOff);
     uint32_t *tv = reinterpret_cast<uint32_t *>(s + kNoAllocValsOff);
     uint32_t *hist = reinterpret_cast<uint32_t *>(s + kNoAllocHistOff);
@@ -379,18 +416,15 @@ extern "C" sph_status sph_sort_cells_noalloc(const float *pos_xyz, int32_t n, ui
     const size_t zero_bytes = (kNoAllocStatusOff - kNoAllocHistOff) + sizeof(uint32_t) * 256 * (size_t)tiles * kNoAllocPasses;
     cudaError_t e = cudaMemsetAsync(s + kNoAllocHistOff, 0, zero_bytes, cs);
     if (e != cudaSuccess) return cuda_status(e, "sph_sort_cells_noalloc: clear scratch");
-    int blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    k_hash_hist_xyz<<<blocks, 256, 0, cs>>>(pos_xyz, n, tk, tv, hist);
+    k_hash_hist_xyz<<<hash_grid(n), kHashThreads, 0, cs>>>(pos_xyz, n, tk, tv, hist);
     // three stable 8-bit passes: scratch -> out -> scratch -> out
     uint32_t *kin[kNoAllocPasses] = {tk, cell_key, tk};
     uint32_t *vin[kNoAllocPasses] = {tv, cell_index, tv};
     uint32_t *kout[kNoAllocPasses] = {cell_key, tk, cell_key};
     uint32_t *vout[kNoAllocPasses] = {cell_index, tv, cell_index};
     for (int p = 0; p < kNoAllocPasses; ++p)
-        k_onesweep<<<tiles, RadixSorter::kThreads, 0, cs>>>(kin[p], vin[p], kout[p], vout[p], n, 8 * p, hist + 256 * p,
-                                                            status + (size_t)256 * tiles * p, counters + p, health,
-                                                            kSpinLimit);
+        launch_onesweep(kin[p], vin[p], kout[p], vout[p], n, 8 * p, hist + 256 * p,
+                        status + (size_t)256 * tiles * p, counters + p, health, kSpinLimit, cs);
     return cuda_status(cudaGetLastError(), "sph_sort_cells_noalloc");
 }
 
@@ -461,7 +495,7 @@ extern "C" sph_status sph_selftest_lookback_timeout(sph_ctx *ctx, int32_t spin_l
     }
     // the key/value buffers are valid device memory, though n = 0 touches none
     k_selftest_prepare<<<1, 256, 0, cs>>>(hist, status, counter);
-    k_onesweep<<<1, RadixSorter::kThreads, 0, cs>>>(kbuf, vbuf, kbuf, vbuf, 0, 0, hist, status, counter,
+    k_onesweep<RadixSorter::kMinItems><<<1, RadixSorter::kThreads, 0, cs>>>(kbuf, vbuf, kbuf, vbuf, 0, 0, hist, status, counter,
                                                     health, spin_limit);
     return cuda_status(cudaGetLastError(), "sph_selftest_lookback_timeout");
 }

@@ -445,7 +445,7 @@ sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st) {
 
     k_bbox_init<<<1, 32, 0, st>>>(bb);
     k_bbox<<<reduce_grid(n), kReduceThreads, 0, st>>>(ctx->pos4, n, bb);
-    cudaMemsetAsync(tb.sorter.hist, 0, sizeof(uint32_t) * 256 * RadixSorter::kMaxPasses, st);
+    radix_clear(tb.sorter, n, bits, st);
     k_tree_keys<<<reduce_grid(n), kReduceThreads, 0, st>>>(ctx->pos4, n, D, bb, tb.sorter.keys[0], tb.sorter.vals[0],
                                                            tb.sorter.hist, passes);
     const int fin = radix_sort_pairs(tb.sorter, n, bits, st, ctx->health);

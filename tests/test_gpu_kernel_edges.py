@@ -1,0 +1,86 @@
+"""The passes at the sizes and inputs where their kernels change what they do,
+against the parity build (the same sources without fused multiply-adds and with
+every sum in the reference's order), numpy, or the FP64 direct sum."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CELL = np.float32(0.18)
+
+
+def _keys(pos):
+    c = np.floor(pos.astype(np.float32) / CELL).astype(np.int64) % 256
+    key = np.zeros(len(pos), np.uint32)
+    for b in range(8):
+        for k in range(3):
+            key |= (((c[:, k] >> b) & 1) << (3 * b + k)).astype(np.uint32)
+    return key
+
+
+def _rel(a, b):
+    a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
+    floor = max(1e-3 * float(np.sqrt(np.mean(b * b))), 1e-30)
+    if a.ndim == 2:
+        return np.linalg.norm(a - b, axis=1) / np.maximum(np.linalg.norm(b, axis=1), floor)
+    return np.abs(a - b) / np.maximum(np.abs(b), floor)
+
+
+# keys per thread change at 2^18 and 2^21 particles; a tile is 256 threads' keys
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 262143, 262144, 262145, (1 << 21) + 1])
+def test_sort_at_its_tile_sizes(cuda, pkg, n):
+    import torch
+
+    ic = pkg.ic.make_cube(n, seed=n, side=20.0)
+    want = _keys(ic["pos"])
+    order = np.argsort(want, kind="stable")
+    with pkg.Compute(ic, max_children_in_leaf=32) as c:
+        for shift in (0.0, 0.5):  # the second sort clears the first one's cells
+            if shift:
+                c.upload("pos", ic["pos"] + np.float32(shift))
+                want = _keys(ic["pos"] + np.float32(shift))
+                order = np.argsort(want, kind="stable")
+            c.sort()
+            c.synchronize()
+            assert np.array_equal(c.download("cell_key"), want[order])
+            assert np.array_equal(c.download("cell_index"), order)
+        start, end = c.download("cell_start"), c.download("cell_end")
+        k, first = np.unique(want[order], return_index=True)
+        last = np.append(first[1:], n) - 1
+        assert np.array_equal(start[k], first) and np.array_equal(end[k], last)
+        assert int((start != 0xFFFFFFFF).sum()) == len(k)
+    if n <= 262144:
+        lib = pkg._lib.load()
+        pos = torch.from_numpy(ic["pos"] + np.float32(0.5)).cuda()
+        key = torch.zeros(n, dtype=torch.int32, device="cuda")
+        ind = torch.zeros(n, dtype=torch.int32, device="cuda")
+        vp = ctypes.c_void_p
+        assert lib.sph_sort_cells_noalloc(vp(pos.data_ptr()), n, vp(key.data_ptr()), vp(ind.data_ptr()), vp(0)) == 0
+        torch.cuda.synchronize()
+        assert np.array_equal(key.cpu().numpy().view(np.uint32), want[order])
+        assert np.array_equal(ind.cpu().numpy(), order)
+
+
+# down pass: lists that overflow at once (forced acceptance), leaves of more
+# than a warp's particles (cut off by the depth), single-particle leaves
+@pytest.mark.parametrize("n,leaf,depth,unchecked", [(3000, 4, 7, 1024), (3000, 4, 7, 16), (5000, 16, 3, 1024),
+                                                    (2000, 1, 7, 1024), (20000, 100, 7, 1024)])
+def test_reference_gravity_matches_the_parity_build(cuda, pkg, n, leaf, depth, unchecked):
+    ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=3)
+    got = []
+    for parity in (False, True):
+        with pkg.Compute(ic, max_children_in_leaf=leaf, max_tree_depth=depth, max_unchecked_pointers=unchecked,
+                         parity=parity) as c:
+            c.upload("grav_norm", np.full(n, 0.1, np.float32))
+            c.gravitationalPass()
+            c.synchronize()
+            got.append((c.download("acc"), c.download("active")))
+    e = _rel(got[0][0], got[1][0])
+    # fused multiply-adds move the reference's own gravity by up to 1.5e-3
+    # (tests/test_fp_sensitivity.py); its moments are taken 318 Mm from the origin
+    assert e.max() <= 1.2e-2 and np.median(e) <= 2e-4
+    assert np.array_equal(got[0][1], got[1][1])

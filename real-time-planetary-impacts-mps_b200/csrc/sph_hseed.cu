@@ -28,6 +28,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -68,6 +69,13 @@ constexpr uint32_t kD1 = 0, kD2 = 64, kD3 = 128, kD4 = 192, kD5 = 256;
 template <int MODE>
 __host__ __device__ constexpr uint32_t tmem_cols() { return MODE == 0 ? 128u : 512u; }
 
+// Eight consecutive K-columns of one row (16 bytes of a core matrix).
+__device__ __forceinline__ void st_bf16x8(unsigned char *base, uint32_t off, const float *v) {
+    __nv_bfloat162 p[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+    *reinterpret_cast<uint4 *>(base + off) = *reinterpret_cast<const uint4 *>(p);
+}
 __device__ __forceinline__ void st_bf16(unsigned char *base, uint32_t off, float v) {
     *reinterpret_cast<__nv_bfloat16 *>(base + off) = __float2bfloat16_rn(v);
 }
@@ -92,8 +100,10 @@ __global__ void k_hs_capture(HSeedArgs a) {
     if (i >= a.n) return;
     float f[kIn];
     raw_features(a, i, f);
+    static_assert(kIn % 4 == 0, "rows of whole float4");
 #pragma unroll
-    for (int k = 0; k < kIn; ++k) a.X[(size_t)i * kIn + k] = f[k];
+    for (int k = 0; k < kIn; k += 4)
+        *reinterpret_cast<float4 *>(a.X + (size_t)i * kIn + k) = make_float4(f[k], f[k + 1], f[k + 2], f[k + 3]);
     a.h0[i] = a.h[i];
 }
 
@@ -168,8 +178,10 @@ __device__ __forceinline__ int sample_row(uint32_t it, uint32_t row, int batch, 
     return (int)(((g * 0x9E3779B97F4A7C15ull) ^ salt) % (uint64_t)n);
 }
 
-// MODE 0: inference (features from the state, writes the seed); MODE 1:
-// gradients of the loss 1/2 mean (y - t)^2 over `batch` sampled rows.
+// MODE 0: inference (features from the state, writes the seed); each CTA keeps
+// the weights and takes tiles of 128 rows until none is left (one CTA per tile
+// spent most of its time on converting the weights: 144 us at N = 1e6).
+// MODE 1: gradients of the loss 1/2 mean (y - t)^2 over `batch` sampled rows.
 // MODE 1 samples its rows for iteration it + *it_base (it_base may be null).
 template <int MODE>
 __global__ void __launch_bounds__(kTile) k_mlp(HSeedArgs a, uint32_t it, int batch, const uint32_t *it_base) {
@@ -206,183 +218,191 @@ __global__ void __launch_bounds__(kTile) k_mlp(HSeedArgs a, uint32_t it, int bat
         for (int q = t; q < (kInPad - kIn) * kTile; q += kTile)
             st_bf16(sm + kSB5, tc::kmajor_off(kIn + q / kTile, q % kTile, kTile), 0.f);
     }
-    // --- this thread's row: features -> X ------------------------------------
-    int row = -1;
-    bool valid = false;
-    float x[kIn];
-    float target = 0.f;
-    if (MODE == 0) {
-        row = blockIdx.x * kTile + t;
-        valid = row < a.n;
-        if (valid) raw_features(a, row, x);
-    } else {
-        valid = (int)(blockIdx.x * kTile + t) < batch;
-        if (valid) {
-            row = sample_row(it + (it_base ? *it_base : 0u), blockIdx.x * kTile + t, batch, a.n, a.salt);
-#pragma unroll
-            for (int k = 0; k < kIn; ++k) x[k] = a.X[(size_t)row * kIn + k];
-            target = (a.y[row] - norm[2 * kIn]) / norm[2 * kIn + 1];
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < kIn; ++k) x[k] = valid ? (x[k] - norm[k]) * norm[kIn + k] : 0.f;
-#pragma unroll
-    for (int k = 0; k < kInPad; ++k) {
-        const float v = k < kIn ? x[k] : 0.f;
-        st_bf16(sm + kSA1, tc::kmajor_off(t, k, kInPad), v);
-        if (MODE == 1 && k < kIn) st_bf16(sm + kSB5, tc::kmajor_off(k, t, kTile), v);
-    }
-    tc::fence_async_smem();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tm = tmem_slot;
-    const uint32_t lane_base = tm + ((uint32_t)(warp * 32) << 16);
     const uint32_t sbase = tc::smem_u32(sm);
     uint32_t phase = 0;
     bool ok = true;
-    auto run = [&](auto &&issue) {
-        if (t == 0) {
-            issue();
-            tc::mma_commit(&bar);
-        }
-        if (!tc::mbar_wait(&bar, phase, kMbarLimit)) ok = false;
-        phase ^= 1u;
-        tc::fence_after_sync();
-    };
-    // --- layer 1 --------------------------------------------------------------
-    run([&] {
-        tc::mma_bf16(tm + kD1, tc::kmajor_desc(sbase + kSA1, kInPad), tc::kmajor_desc(sbase + kSW1, kInPad),
-                     tc::idesc_bf16_m128(kHid), false);
-    });
-    uint64_t mask1 = 0ull;
-    float v[16];
+    uint32_t tm = 0u;
+    const int tiles = MODE == 0 ? (a.n + kTile - 1) / kTile : 1;
+    for (int tile = MODE == 0 ? (int)blockIdx.x : 0; tile < tiles; tile += (int)gridDim.x) {
+        // --- this thread's row: features -> X ------------------------------------
+        int row = -1;
+        bool valid = false;
+        float x[kIn];
+        float target = 0.f;
+        if (MODE == 0) {
+            row = tile * kTile + t;
+            valid = row < a.n;
+            if (valid) raw_features(a, row, x);
+        } else {
+            valid = (int)(blockIdx.x * kTile + t) < batch;
+            if (valid) {
+                row = sample_row(it + (it_base ? *it_base : 0u), blockIdx.x * kTile + t, batch, a.n, a.salt);
 #pragma unroll
-    for (int c = 0; c < kHid; c += 16) {
-        tc::tmem_ld16(lane_base + kD1 + c, v);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int j = c + q;
-            const float z = v[q] + P[kOffB1 + j];
-            const float hval = z > 0.f ? z : 0.f;
-            if (z > 0.f) mask1 |= 1ull << j;
-            st_bf16(sm + kSA2, tc::kmajor_off(t, j, kHid), hval);
-            if (MODE == 1) st_bf16(sm + kSB4, tc::kmajor_off(j, t, kTile), hval);
-        }
-    }
-    tc::fence_before_sync();
-    tc::fence_async_smem();
-    __syncthreads();
-    tc::fence_after_sync();
-    // --- layer 2 --------------------------------------------------------------
-    run([&] {
-        for (int s = 0; s < kHid / 16; ++s)
-            tc::mma_bf16(tm + kD2, tc::kmajor_desc(sbase + kSA2 + s * 256, kHid),
-                         tc::kmajor_desc(sbase + kSW2 + s * 256, kHid), tc::idesc_bf16_m128(kHid), s > 0);
-    });
-    float yhat = P[kOffB3];
-    uint64_t mask2 = 0ull;
-    float h2[kHid];
-#pragma unroll
-    for (int c = 0; c < kHid; c += 16) {
-        tc::tmem_ld16(lane_base + kD2 + c, v);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            const int j = c + q;
-            const float z = v[q] + P[kOffB2 + j];
-            h2[j] = z > 0.f ? z : 0.f;
-            if (z > 0.f) mask2 |= 1ull << j;
-            yhat += h2[j] * P[kOffW3 + j];
-        }
-    }
-    if (MODE == 0) {
-        if (valid && ok) {
-            const float pred = norm[2 * kIn] + norm[2 * kIn + 1] * yhat;
-            a.seed[row] = a.h[row] * expf(pred);
-        }
-    } else {
-        // --- backward -----------------------------------------------------------
-        const float dy = valid ? (yhat - target) / (float)batch : 0.f;
-        if (valid) atomicAdd(a.loss, 0.5f * (yhat - target) * (yhat - target) / (float)batch);
-#pragma unroll
-        for (int j = 0; j < kHid; ++j) {
-            const float g = ((mask2 >> j) & 1ull) ? dy * P[kOffW3 + j] : 0.f;
-            st_bf16(sm + kSA3, tc::kmajor_off(t, j, kHid), g);
-            st_bf16(sm + kSA4, tc::kmajor_off(j, t, kTile), g);
-            // sums over the tile's rows: w3, b2
-            float s3 = dy * h2[j], s2 = g;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-                s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-            }
-            if (lane == 0) {
-                red_w3[warp][j] = s3;
-                red_b2[warp][j] = s2;
+                for (int k = 0; k < kIn; ++k) x[k] = a.X[(size_t)row * kIn + k];
+                target = (a.y[row] - norm[2 * kIn]) / norm[2 * kIn + 1];
             }
         }
-        float s = dy;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red_b3[warp] = s;
-        tc::fence_before_sync();
+        for (int k = 0; k < kIn; ++k) x[k] = valid ? (x[k] - norm[k]) * norm[kIn + k] : 0.f;
+        const float none[kIn] = {};
+        st_bf16x8(sm + kSA1, tc::kmajor_off(t, 0, kInPad), x);
+        st_bf16x8(sm + kSA1, tc::kmajor_off(t, kIn, kInPad), none);
+        if (MODE == 1)
+#pragma unroll
+            for (int k = 0; k < kIn; ++k) st_bf16(sm + kSB5, tc::kmajor_off(k, t, kTile), x[k]);
+        tc::fence_before_sync();  // the previous tile's TMEM reads
         tc::fence_async_smem();
-        __syncthreads();
+        // (a wait that gave up ends the CTA's work: the barrier's phase is unknown)
+        if (!__syncthreads_and(ok)) break;
         tc::fence_after_sync();
-        if (t < kHid) {
-            atomicAdd(a.grads + kOffW3 + t, red_w3[0][t] + red_w3[1][t] + red_w3[2][t] + red_w3[3][t]);
-            atomicAdd(a.grads + kOffB2 + t, red_b2[0][t] + red_b2[1][t] + red_b2[2][t] + red_b2[3][t]);
-        }
-        if (t == 0) atomicAdd(a.grads + kOffB3, red_b3[0] + red_b3[1] + red_b3[2] + red_b3[3]);
-        // dH1 = dH2 W2 and dW2 = dH2^T H1
+        tm = tmem_slot;
+        const uint32_t lane_base = tm + ((uint32_t)(warp * 32) << 16);
+        auto run = [&](auto &&issue) {
+            if (t == 0) {
+                issue();
+                tc::mma_commit(&bar);
+            }
+            if (!tc::mbar_wait(&bar, phase, kMbarLimit)) ok = false;
+            phase ^= 1u;
+            tc::fence_after_sync();
+        };
+        // --- layer 1 --------------------------------------------------------------
         run([&] {
-            for (int s2 = 0; s2 < kHid / 16; ++s2)
-                tc::mma_bf16(tm + kD3, tc::kmajor_desc(sbase + kSA3 + s2 * 256, kHid),
-                             tc::kmajor_desc(sbase + kSW2T + s2 * 256, kHid), tc::idesc_bf16_m128(kHid), s2 > 0);
-            for (int s2 = 0; s2 < kTile / 16; ++s2)
-                tc::mma_bf16(tm + kD4, tc::kmajor_desc(sbase + kSA4 + s2 * 256, kTile),
-                             tc::kmajor_desc(sbase + kSB4 + s2 * 256, kTile), tc::idesc_bf16_m128(kHid), s2 > 0);
+            tc::mma_bf16(tm + kD1, tc::kmajor_desc(sbase + kSA1, kInPad), tc::kmajor_desc(sbase + kSW1, kInPad),
+                         tc::idesc_bf16_m128(kHid), false);
         });
+        uint64_t mask1 = 0ull;
+        float v[16];
 #pragma unroll
         for (int c = 0; c < kHid; c += 16) {
-            tc::tmem_ld16(lane_base + kD3 + c, v);
+            tc::tmem_ld16(lane_base + kD1 + c, v);
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
                 const int j = c + q;
-                const float g = ((mask1 >> j) & 1ull) ? v[q] : 0.f;
-                st_bf16(sm + kSA5, tc::kmajor_off(j, t, kTile), g);
-                float s1 = g;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-                if (lane == 0) red_b1[warp][j] = s1;
+                const float z = v[q] + P[kOffB1 + j];
+                const float hval = z > 0.f ? z : 0.f;
+                if (MODE == 1 && z > 0.f) mask1 |= 1ull << j;
+                v[q] = hval;
+                if (MODE == 1) st_bf16(sm + kSB4, tc::kmajor_off(j, t, kTile), hval);
             }
-        }
-#pragma unroll
-        for (int c = 0; c < kHid; c += 16) {
-            tc::tmem_ld16(lane_base + kD4 + c, v);  // row t of dW2 (t < 64)
-            if (t < kHid && ok)
-#pragma unroll
-                for (int q = 0; q < 16; ++q) atomicAdd(a.grads + kOffW2 + t * kHid + c + q, v[q]);
+            st_bf16x8(sm + kSA2, tc::kmajor_off(t, c, kHid), v);
+            st_bf16x8(sm + kSA2, tc::kmajor_off(t, c + 8, kHid), v + 8);
         }
         tc::fence_before_sync();
         tc::fence_async_smem();
         __syncthreads();
         tc::fence_after_sync();
-        if (t < kHid) atomicAdd(a.grads + kOffB1 + t, red_b1[0][t] + red_b1[1][t] + red_b1[2][t] + red_b1[3][t]);
-        // dW1 = dH1^T X
+        // --- layer 2 --------------------------------------------------------------
         run([&] {
-            for (int s2 = 0; s2 < kTile / 16; ++s2)
-                tc::mma_bf16(tm + kD5, tc::kmajor_desc(sbase + kSA5 + s2 * 256, kTile),
-                             tc::kmajor_desc(sbase + kSB5 + s2 * 256, kTile), tc::idesc_bf16_m128(kInPad), s2 > 0);
+            for (int s = 0; s < kHid / 16; ++s)
+                tc::mma_bf16(tm + kD2, tc::kmajor_desc(sbase + kSA2 + s * 256, kHid),
+                             tc::kmajor_desc(sbase + kSW2 + s * 256, kHid), tc::idesc_bf16_m128(kHid), s > 0);
         });
-        tc::tmem_ld16(lane_base + kD5, v);
-        if (t < kHid && ok)
+        float yhat = P[kOffB3];
+        uint64_t mask2 = 0ull;
+        float h2[kHid];
 #pragma unroll
-            for (int q = 0; q < kIn; ++q) atomicAdd(a.grads + kOffW1 + t * kIn + q, v[q]);
+        for (int c = 0; c < kHid; c += 16) {
+            tc::tmem_ld16(lane_base + kD2 + c, v);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const int j = c + q;
+                const float z = v[q] + P[kOffB2 + j];
+                h2[j] = z > 0.f ? z : 0.f;
+                if (MODE == 1 && z > 0.f) mask2 |= 1ull << j;
+                yhat += h2[j] * P[kOffW3 + j];
+            }
+        }
+        if (MODE == 0) {
+            if (valid && ok) {
+                const float pred = norm[2 * kIn] + norm[2 * kIn + 1] * yhat;
+                a.seed[row] = a.h[row] * expf(pred);
+            }
+        } else {
+            // --- backward -----------------------------------------------------------
+            const float dy = valid ? (yhat - target) / (float)batch : 0.f;
+            if (valid) atomicAdd(a.loss, 0.5f * (yhat - target) * (yhat - target) / (float)batch);
+#pragma unroll
+            for (int j = 0; j < kHid; ++j) {
+                const float g = ((mask2 >> j) & 1ull) ? dy * P[kOffW3 + j] : 0.f;
+                st_bf16(sm + kSA3, tc::kmajor_off(t, j, kHid), g);
+                st_bf16(sm + kSA4, tc::kmajor_off(j, t, kTile), g);
+                // sums over the tile's rows: w3, b2
+                float s3 = dy * h2[j], s2 = g;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+                    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                }
+                if (lane == 0) {
+                    red_w3[warp][j] = s3;
+                    red_b2[warp][j] = s2;
+                }
+            }
+            float s = dy;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) red_b3[warp] = s;
+            tc::fence_before_sync();
+            tc::fence_async_smem();
+            __syncthreads();
+            tc::fence_after_sync();
+            if (t < kHid) {
+                atomicAdd(a.grads + kOffW3 + t, red_w3[0][t] + red_w3[1][t] + red_w3[2][t] + red_w3[3][t]);
+                atomicAdd(a.grads + kOffB2 + t, red_b2[0][t] + red_b2[1][t] + red_b2[2][t] + red_b2[3][t]);
+            }
+            if (t == 0) atomicAdd(a.grads + kOffB3, red_b3[0] + red_b3[1] + red_b3[2] + red_b3[3]);
+            // dH1 = dH2 W2 and dW2 = dH2^T H1
+            run([&] {
+                for (int s2 = 0; s2 < kHid / 16; ++s2)
+                    tc::mma_bf16(tm + kD3, tc::kmajor_desc(sbase + kSA3 + s2 * 256, kHid),
+                                 tc::kmajor_desc(sbase + kSW2T + s2 * 256, kHid), tc::idesc_bf16_m128(kHid), s2 > 0);
+                for (int s2 = 0; s2 < kTile / 16; ++s2)
+                    tc::mma_bf16(tm + kD4, tc::kmajor_desc(sbase + kSA4 + s2 * 256, kTile),
+                                 tc::kmajor_desc(sbase + kSB4 + s2 * 256, kTile), tc::idesc_bf16_m128(kHid), s2 > 0);
+            });
+#pragma unroll
+            for (int c = 0; c < kHid; c += 16) {
+                tc::tmem_ld16(lane_base + kD3 + c, v);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    const int j = c + q;
+                    const float g = ((mask1 >> j) & 1ull) ? v[q] : 0.f;
+                    st_bf16(sm + kSA5, tc::kmajor_off(j, t, kTile), g);
+                    float s1 = g;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+                    if (lane == 0) red_b1[warp][j] = s1;
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < kHid; c += 16) {
+                tc::tmem_ld16(lane_base + kD4 + c, v);  // row t of dW2 (t < 64)
+                if (t < kHid && ok)
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) atomicAdd(a.grads + kOffW2 + t * kHid + c + q, v[q]);
+            }
+            tc::fence_before_sync();
+            tc::fence_async_smem();
+            __syncthreads();
+            tc::fence_after_sync();
+            if (t < kHid) atomicAdd(a.grads + kOffB1 + t, red_b1[0][t] + red_b1[1][t] + red_b1[2][t] + red_b1[3][t]);
+            // dW1 = dH1^T X
+            run([&] {
+                for (int s2 = 0; s2 < kTile / 16; ++s2)
+                    tc::mma_bf16(tm + kD5, tc::kmajor_desc(sbase + kSA5 + s2 * 256, kTile),
+                                 tc::kmajor_desc(sbase + kSB5 + s2 * 256, kTile), tc::idesc_bf16_m128(kInPad), s2 > 0);
+            });
+            tc::tmem_ld16(lane_base + kD5, v);
+            if (t < kHid && ok)
+#pragma unroll
+                for (int q = 0; q < kIn; ++q) atomicAdd(a.grads + kOffW1 + t * kIn + q, v[q]);
+        }
     }
     if (!ok && t == 0) raise_health(a.health, SPH_HEALTH_MLP_TIMEOUT);
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tm, tmem_cols<MODE>());
+    if (warp == 0) tc::tmem_dealloc(tmem_slot, tmem_cols<MODE>());
 }
 
 // Adam on the FP32 master weights (one CTA); clears the gradient and counts
@@ -521,8 +541,11 @@ sph_status launch_hseed_targets(sph_ctx *ctx, cudaStream_t st) {
 sph_status launch_hseed_infer(sph_ctx *ctx, cudaStream_t st) {
     sph_status s = hseed_alloc(ctx);
     if (s != SPH_OK) return s;
-    const int tiles = (ctx->n + kTile - 1) / kTile;
-    k_mlp<0><<<tiles, kTile, kFwdBytes, st>>>(hseed_args(ctx), 0u, 0, nullptr);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    // as many CTAs as the SMs' 512 TMEM columns hold
+    const int blocks = std::min((ctx->n + kTile - 1) / kTile, sms * (int)(512u / tmem_cols<0>()));
+    k_mlp<0><<<blocks, kTile, kFwdBytes, st>>>(hseed_args(ctx), 0u, 0, nullptr);
     return cuda_status(cudaGetLastError(), "h seed inference");
 }
 

@@ -308,8 +308,9 @@ sph_status sph_destroy(sph_ctx *ctx) {
     drop_graphs(ctx);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
-    if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
-    if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+    if (ctx->gravity_stream) cudaStreamDestroy(ctx->gravity_stream);
+    for (cudaEvent_t e : {ctx->ev_fork, ctx->ev_join, ctx->ev_gfork, ctx->ev_up, ctx->ev_gjoin})
+        if (e) cudaEventDestroy(e);
     void *bufs[] = {ctx->pos4, ctx->vel4, ctx->acc4, ctx->rho, ctx->u, ctx->P, ctx->h, ctx->f, ctx->c,
                     ctx->du, ctx->B, ctx->dhdt, ctx->gnorm, ctx->phi, ctx->mat, ctx->nat, ctx->active, ctx->globals,
                     ctx->health, ctx->cell_range, ctx->sp4, ctx->sv4, ctx->sA, ctx->sB, ctx->sC,
@@ -882,8 +883,9 @@ sph_status sph_update_tree(sph_ctx *ctx, void *stream) {
 sph_status sph_sort(sph_ctx *ctx, void *stream) {
     return ctx ? launch_sort(ctx, (cudaStream_t)stream) : SPH_ERR_INVALID_ARG;
 }
-static sph_status gravity_pass(sph_ctx *ctx, cudaStream_t st) {
-    return ctx->form.gravity == SPH_GRAVITY_THETA ? launch_gravity_theta(ctx, st) : launch_gravity(ctx, st);
+static sph_status gravity_pass(sph_ctx *ctx, cudaStream_t st, cudaEvent_t up_done = nullptr) {
+    return ctx->form.gravity == SPH_GRAVITY_THETA ? launch_gravity_theta(ctx, st, up_done)
+                                                  : launch_gravity(ctx, st, up_done);
 }
 sph_status sph_gravity(sph_ctx *ctx, void *stream) {
     return ctx ? gravity_pass(ctx, (cudaStream_t)stream) : SPH_ERR_INVALID_ARG;
@@ -1072,46 +1074,77 @@ sph_status sph_step(sph_ctx *ctx, void *stream) {
 
 namespace sph {
 
-// One full step (Headless.cpp:43-51 without the snapshot) on `st`.
-// The side stream and the fork / join events of a step (created once).
-sph_status ensure_side(sph_ctx *ctx) {
+// The other streams and the events of a step (created once).
+sph_status ensure_streams(sph_ctx *ctx) {
     cudaError_t e = cudaSuccess;
-    if (!ctx->side_stream) e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess && !ctx->ev_fork) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess && !ctx->ev_join) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
-    return cuda_status(e, "side stream");
+    for (cudaStream_t *s : {&ctx->side_stream, &ctx->gravity_stream})
+        if (e == cudaSuccess && !*s) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+    for (cudaEvent_t *v : {&ctx->ev_fork, &ctx->ev_join, &ctx->ev_gfork, &ctx->ev_up, &ctx->ev_gjoin})
+        if (e == cudaSuccess && !*v) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+    return cuda_status(e, "step streams");
 }
 
-sph_status full_step(sph_ctx *ctx, cudaStream_t st) {
-    sph_status s = SPH_OK;
+// The passes of a step on st (Headless.cpp:43-51 without the snapshot), after
+// its inputs are there.  The tree and gravity passes run on a second stream
+// beside the sort and density passes: gravity reads the positions and writes
+// the acceleration, |a|, potential and active flags; density needs of these
+// only the flags (the up pass's), and the acceleration pass adds to gravity's
+// acceleration.  Small contexts are chains of launches that leave the device
+// mostly idle, and the two halves are about equally long (two steps at
+// N = 1.1e4: 1342 -> 1098 us, at 1e5: 3244 -> 3019 us).
+// `inputs` (may be null): joined before the density pass.  fork false: all on
+// st (an ensemble's instances already run beside one another).
+static sph_status step_passes(sph_ctx *ctx, cudaStream_t st, cudaEvent_t inputs, bool fork) {
+    cudaStream_t gs = fork ? ctx->gravity_stream : st;
+    cudaError_t e = cudaEventRecord(ctx->ev_gfork, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(gs, ctx->ev_gfork, 0);
+    sph_status s = cuda_status(e, "step fork");
+    // recorded here too: a gravity pass that does not get to its own record
+    // (no tree, an error) must not leave an older step's
+    cudaError_t eu = cudaEventRecord(ctx->ev_up, gs);
+    if (s == SPH_OK && ctx->params.tree_source == SPH_TREE_GPU) s = launch_tree_build(ctx, gs);
+    if (s == SPH_OK) s = gravity_pass(ctx, gs, ctx->ev_up);
+    cudaError_t ej = cudaEventRecord(ctx->ev_gjoin, gs);
+    if (s == SPH_OK) s = launch_sort(ctx, st);
+    if (eu == cudaSuccess) eu = cudaStreamWaitEvent(st, ctx->ev_up, 0);
+    // joined whatever happened, so that a capture ends well formed
+    if (inputs) {
+        const cudaError_t ei = cudaStreamWaitEvent(st, inputs, 0);
+        if (eu == cudaSuccess) eu = ei;
+    }
+    if (s == SPH_OK) s = cuda_status(eu, "step join");
+    if (s == SPH_OK) s = launch_density(ctx, st);
+    ctx->hs.trained_ahead = false;
+    if (ej == cudaSuccess) ej = cudaStreamWaitEvent(st, ctx->ev_gjoin, 0);
+    if (s == SPH_OK) s = cuda_status(ej, "step join");
+    if (s == SPH_OK) s = launch_acceleration(ctx, st);
+    if (s == SPH_OK) s = launch_step(ctx, st);
+    return s;
+}
+
+// One full step on `st`.
+sph_status full_step(sph_ctx *ctx, cudaStream_t st, bool fork) {
+    sph_status s = ensure_streams(ctx);
+    if (s != SPH_OK) return s;
     // the learned seed's online refresh runs beside the tree, sort and
     // gravity passes (it reads the previous density pass's pairs and writes
     // only the network) and is joined before the density pass
     const bool ahead = hseed_online_due(ctx);
     if (ahead) {
-        s = ensure_side(ctx);
-        cudaError_t e = cudaSuccess;
-        if (s == SPH_OK) e = cudaEventRecord(ctx->ev_fork, st);
-        if (s == SPH_OK && e == cudaSuccess) e = cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0);
-        if (s == SPH_OK && e != cudaSuccess) s = cuda_status(e, "full step fork");
+        cudaError_t e = cudaEventRecord(ctx->ev_fork, st);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0);
+        s = cuda_status(e, "full step fork");
         if (s == SPH_OK) s = launch_hseed_online(ctx, ctx->side_stream);
         // recorded whatever happened, so that a capture ends well formed
         cudaError_t ej = cudaEventRecord(ctx->ev_join, ctx->side_stream);
         if (s == SPH_OK && ej != cudaSuccess) s = cuda_status(ej, "full step join");
         ctx->hs.trained_ahead = s == SPH_OK;
+        if (s != SPH_OK) {
+            cudaStreamWaitEvent(st, ctx->ev_join, 0);
+            return s;
+        }
     }
-    if (s == SPH_OK && ctx->params.tree_source == SPH_TREE_GPU) s = launch_tree_build(ctx, st);
-    if (s == SPH_OK) s = launch_sort(ctx, st);
-    if (s == SPH_OK) s = gravity_pass(ctx, st);
-    if (ahead) {
-        cudaError_t ej = cudaStreamWaitEvent(st, ctx->ev_join, 0);
-        if (s == SPH_OK && ej != cudaSuccess) s = cuda_status(ej, "full step join");
-    }
-    if (s == SPH_OK) s = launch_density(ctx, st);
-    ctx->hs.trained_ahead = false;
-    if (s == SPH_OK) s = launch_acceleration(ctx, st);
-    if (s == SPH_OK) s = launch_step(ctx, st);
-    return s;
+    return step_passes(ctx, st, ahead ? ctx->ev_join : nullptr, fork);
 }
 
 void drop_graphs(sph_ctx *ctx) {
@@ -1184,16 +1217,11 @@ sph_status host_step(sph_ctx *ctx, const sph_host_state &in, const sph_host_stat
         ctx->hs.trained_ahead = s == SPH_OK;
     }
     ok(cudaEventRecord(ctx->ev_join, sd));
-    if (s == SPH_OK && ctx->params.tree_source == SPH_TREE_GPU) s = launch_tree_build(ctx, st);
-    if (s == SPH_OK) s = launch_sort(ctx, st);
-    if (s == SPH_OK) s = gravity_pass(ctx, st);
-    // joined whatever happened, so that a capture ends well formed
-    cudaError_t ej = cudaStreamWaitEvent(st, ctx->ev_join, 0);
-    if (s == SPH_OK && ej != cudaSuccess) s = cuda_status(ej, "sph_step_host join");
-    if (s == SPH_OK) s = launch_density(ctx, st);
-    ctx->hs.trained_ahead = false;
-    if (s == SPH_OK) s = launch_acceleration(ctx, st);
-    if (s == SPH_OK) s = launch_step(ctx, st);
+    if (s != SPH_OK) {
+        cudaStreamWaitEvent(st, ctx->ev_join, 0);  // so that a capture ends well formed
+        return s;
+    }
+    s = step_passes(ctx, st, ctx->ev_join, true);
     if (s != SPH_OK) return s;
     if (mixed && out.pos64) {
         k_unpack3d<<<blocks, 256, 0, st>>>(ctx->pos64, (double *)ctx->stage, n);
@@ -1280,7 +1308,7 @@ sph_status sph_step_host(sph_ctx *ctx, const sph_host_state *in, const sph_host_
     cudaError_t e = cudaSuccess;
     if (!ctx->own_stream) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_status(e, "sph_step_host stream");
-    sph_status s = ensure_side(ctx);
+    sph_status s = ensure_streams(ctx);
     if (s != SPH_OK) return s;
     const bool same = ctx->host_graph && std::memcmp(&ctx->host_in, in, sizeof(*in)) == 0 &&
                       std::memcmp(&ctx->host_out, out, sizeof(*out)) == 0;

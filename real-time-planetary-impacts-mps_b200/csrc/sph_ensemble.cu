@@ -77,7 +77,7 @@ sph_status gravity_median_error(sph_ctx *ctx, cudaStream_t st, float &err) {
     for (int i = 0; i < nt; ++i) tg[i] = (int32_t)(((int64_t)i * n) / nt);
     sph_status s = launch_tree_build(ctx, st);
     if (s == SPH_OK) s = launch_sort(ctx, st);
-    if (s == SPH_OK) s = launch_gravity_theta(ctx, st);
+    if (s == SPH_OK) s = launch_gravity_theta(ctx, st, nullptr);
     if (s != SPH_OK) return s;
     std::vector<float> acc(3 * (size_t)n);
     s = sph_download_async(ctx, SPH_FIELD_ACC, acc.data(), acc.size(), st);
@@ -171,7 +171,7 @@ sph_status build_graph(sph_ensemble *e) {
             s = cuda_status(err, "ensemble capture");
             break;
         }
-        s = full_step(c, e->capture);
+        s = full_step(c, e->capture, false);
         err = cudaStreamEndCapture(e->capture, &g);
         if (s == SPH_OK && err != cudaSuccess) s = cuda_status(err, "ensemble capture end");
         if (s == SPH_OK) {
@@ -278,7 +278,7 @@ sph_status sph_ensemble_step(sph_ensemble *e, void *stream, int32_t n_steps) {
         // the first step runs eagerly and puts every sort buffer in its steady
         // role (as sph_step_all does before capturing); then the graph is built
         for (sph_ctx *c : e->inst) {
-            sph_status s = full_step(c, st);
+            sph_status s = full_step(c, st, false);
             if (s != SPH_OK) return s;
         }
         cudaError_t err = cudaStreamSynchronize(st);

@@ -641,7 +641,7 @@ __global__ void __launch_bounds__(kDownThreads) k_down(DownArgs a, int level, in
 
 }  // namespace
 
-sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st) {
+sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st, cudaEvent_t up_done) {
     Tree &tr = ctx->tree;
     if (!tr.valid || ctx->n <= 0) return SPH_OK;
     const int L = tr.n_levels_host;
@@ -668,6 +668,7 @@ sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st) {
             k_up<<<blocks, 128, 0, st>>>(u, l, tr.level_cap);
         }
     }
+    if (up_done) cudaEventRecord(up_done, st);
     DownArgs d;
     d.T = tr.tree;
     d.level_nodes = tr.level_nodes;

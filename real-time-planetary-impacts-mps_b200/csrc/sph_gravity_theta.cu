@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(256) k_direct_f64(const float4 *__restrict__ p
 
 }  // namespace
 
-static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t st) {
+static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t st, cudaEvent_t up_done) {
     Tree &tr = ctx->tree;
     TreeBuild &tb = ctx->tb;
     if (!tr.valid || ctx->n <= 0) return SPH_OK;
@@ -619,6 +619,7 @@ static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t s
     // computed (the potential for the diagnostics covers every particle)
     u.individual = acc && ctx->form.timestep == SPH_TIMESTEP_INDIVIDUAL;
     k_up_theta<<<up_blocks(tr, 128), 128, 0, st>>>(u, up_nodes(tr));
+    if (up_done) cudaEventRecord(up_done, st);
     // resident warps of the walk, each with its two node queues
     static int max_blocks_per_sm = 0;
     if (max_blocks_per_sm == 0) {
@@ -646,7 +647,11 @@ static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t s
         cudaError_t e = cudaMalloc(&tb.walk_counter, sizeof(uint32_t));
         if (e != cudaSuccess) return cuda_status(e, "gravity (theta) walk counter");
     }
-    float4 *kp4 = ctx->sp4;  // free until the density pass gathers its own records
+    if (!tb.kp4) {
+        cudaError_t e = cudaMalloc(&tb.kp4, sizeof(float4) * (size_t)n);
+        if (e != cudaSuccess) return cuda_status(e, "gravity (theta) positions");
+    }
+    float4 *kp4 = tb.kp4;
     k_gather_key_order<<<(n + 255) / 256, 256, 0, st>>>(n, tb.order, ctx->pos4, kp4);
     cudaMemsetAsync(tb.walk_counter, 0, sizeof(uint32_t), st);
     WalkArgs w;
@@ -672,10 +677,12 @@ static sph_status theta_pass(sph_ctx *ctx, float theta, bool acc, cudaStream_t s
     return cuda_status(cudaGetLastError(), "gravity (theta)");
 }
 
-sph_status launch_gravity_theta(sph_ctx *ctx, cudaStream_t st) { return theta_pass(ctx, ctx->form.theta, true, st); }
+sph_status launch_gravity_theta(sph_ctx *ctx, cudaStream_t st, cudaEvent_t up_done) {
+    return theta_pass(ctx, ctx->form.theta, true, st, up_done);
+}
 
 sph_status launch_potential_theta(sph_ctx *ctx, float theta, cudaStream_t st) {
-    return theta_pass(ctx, theta, false, st);
+    return theta_pass(ctx, theta, false, st, nullptr);
 }
 
 sph_status launch_direct_f64(sph_ctx *ctx, const int32_t *d_targets, int nt, double *d_out, cudaStream_t st) {

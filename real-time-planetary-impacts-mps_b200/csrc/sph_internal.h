@@ -93,6 +93,7 @@ struct TreeBuild {
     int32_t *walk_queues = nullptr;   // theta-form walk: node queues of the resident warps
     uint32_t *walk_counter = nullptr; // theta-form walk: group ticket
     int64_t walk_queue_ints = 0;
+    float4 *kp4 = nullptr;            // theta-form walk: positions and masses in key order
 };
 
 // Learned smoothing-length seed (sph_hseed.cu): FP32 master weights and Adam
@@ -203,12 +204,13 @@ struct sph_ctx {
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
     cudaStream_t own_stream = nullptr;
-    // sph_step_host: its graph, the host buffers it was captured for, and the
-    // side stream and events of the overlapped input copies
+    // sph_step_host: its graph and the host buffers it was captured for
     cudaGraphExec_t host_graph = nullptr;
     sph_host_state host_in{}, host_out{};
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // a step's other streams and events: the seed's refresh and sph_step_host's
+    // input copies (side), the tree and gravity passes (gravity)
+    cudaStream_t side_stream = nullptr, gravity_stream = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_gfork = nullptr, ev_up = nullptr, ev_gjoin = nullptr;
 };
 
 namespace sph {
@@ -236,8 +238,9 @@ sph_status launch_pos_to64(sph_ctx *ctx, cudaStream_t st);
 // FP64 conservation sums into ctx->diag (see sph_diagnostics)
 sph_status launch_diag_sums(sph_ctx *ctx, cudaStream_t st);
 
-// sph_gravity.cu
-sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st);
+// sph_gravity.cu.  up_done (may be null) is recorded once the up pass, which
+// sets the particles' active flags, is enqueued.
+sph_status launch_gravity(sph_ctx *ctx, cudaStream_t st, cudaEvent_t up_done);
 
 // sph_hseed.cu
 sph_status hseed_alloc(sph_ctx *ctx);
@@ -252,7 +255,7 @@ sph_status launch_hseed_grad(sph_ctx *ctx, uint32_t it, bool counted, int batch,
 sph_status launch_hseed_adam(sph_ctx *ctx, float lr, cudaStream_t st);
 
 // sph_gravity_theta.cu
-sph_status launch_gravity_theta(sph_ctx *ctx, cudaStream_t st);
+sph_status launch_gravity_theta(sph_ctx *ctx, cudaStream_t st, cudaEvent_t up_done);
 // the potential alone (acceleration and |a| untouched), opening angle theta,
 // on the current GPU tree
 sph_status launch_potential_theta(sph_ctx *ctx, float theta, cudaStream_t st);
@@ -265,7 +268,8 @@ sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st);
 
 // sph_api.cu
 // One full step (tree, sort, gravity, density, acceleration, step) on st.
-sph_status full_step(sph_ctx *ctx, cudaStream_t st);
+// fork: the tree and gravity passes on a stream of their own.
+sph_status full_step(sph_ctx *ctx, cudaStream_t st, bool fork = true);
 // sph_hseed.cu: the online refresh of the learned seed (standardisation and
 // Adam steps on the last recorded pass) on st; whether one is due this step
 bool hseed_online_due(const sph_ctx *ctx);

@@ -427,6 +427,7 @@ void tree_free(sph_ctx *ctx) {
     cudaFree(tb.ticket);
     cudaFree(tb.bbox);
     cudaFree(tb.walk_queues);
+    cudaFree(tb.kp4);
     cudaFree(tb.walk_counter);
     tb = TreeBuild();
 }

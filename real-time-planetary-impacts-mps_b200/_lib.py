@@ -20,7 +20,7 @@ PARITY_LIB_PATH = os.path.join(HERE, "libsph_b200_parity.so")
 PARITY_FLAGS = ["-fmad=false", "-DSPH_PARITY"]
 SOURCES = ["sph_api.cu", "sph_sort.cu", "sph_hydro.cu", "sph_gravity.cu", "sph_gravity_theta.cu", "sph_tree.cu",
            "sph_hseed.cu", "sph_ensemble.cu"]
-HEADERS = ["sph_common.cuh", "sph_internal.h", "sph_tc.cuh", "sph_up.cuh"]
+HEADERS = ["sph_common.cuh", "sph_internal.h", "sph_tc.cuh", "sph_up.cuh", "sph_f32x2.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC,-ffp-contract=off", "-shared"]
 

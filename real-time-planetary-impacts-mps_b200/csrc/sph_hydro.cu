@@ -23,6 +23,7 @@
 
 #include <algorithm>
 
+#include "sph_f32x2.cuh"
 #include "sph_internal.h"
 
 namespace sph {
@@ -593,6 +594,12 @@ constexpr float kTileListReach = SPH_TILE_LIST_REACH;       // list radius / (2 
 // the staged box
 constexpr float kTileStageReach = SPH_TILE_STAGE_REACH;
 
+// Neighbours a particle's lanes keep in registers, as pairs per lane, through
+// the sweeps of its iteration; longer lists are read from shared memory in
+// every sweep.
+constexpr int kRegPairs = 7;
+constexpr int kRegList = 2 * kRegPairs * kTileLanes;        // 112 (a list holds ~75)
+
 struct TileShared {
     float4 pos[kTileStageMax];          // staged (x, y, z, m)
     uint32_t gidx[kTileStageMax];       // staged sorted index
@@ -760,6 +767,51 @@ __global__ void k_coarse_starts(int n, const uint32_t *__restrict__ skey, const 
     tiles[atomicAdd(ctr, 1u)] = make_uint2((uint32_t)k, l);
 }
 
+// 1 / (4 pi h^3), h1 = 1 / h: the norm of the cubic spline summed as
+// (2 - q)+^3 - 4 (1 - q)+^3.
+__device__ __forceinline__ float kernel_norm(float h1) { return 0.25f * kPi1 * h1 * h1 * h1; }
+
+// Where the spheres of a warp's four particles can reach, as one box of
+// centres and the largest radius (their z ranges row by row would be four
+// times the work for few slots less: the four are neighbours in cell order).
+struct Reach4 {
+    float x0, x1, y0, y1, z0, z1, r2;
+    // r2 < 0: a group that takes no part
+    __device__ __forceinline__ Reach4(float px, float py, float pz, float rr) {
+        constexpr unsigned kFull = 0xffffffffu;
+        constexpr int L = kTileLanes;
+        const float big = 3e38f;
+        const bool on = rr >= 0.f;
+        x0 = on ? px : big, y0 = on ? py : big, z0 = on ? pz : big;
+        x1 = on ? px : -big, y1 = on ? py : -big, z1 = on ? pz : -big;
+        r2 = rr;
+#pragma unroll
+        for (int o = L; o < 32; o <<= 1) {
+            x0 = fminf(x0, __shfl_xor_sync(kFull, x0, o));
+            y0 = fminf(y0, __shfl_xor_sync(kFull, y0, o));
+            z0 = fminf(z0, __shfl_xor_sync(kFull, z0, o));
+            x1 = fmaxf(x1, __shfl_xor_sync(kFull, x1, o));
+            y1 = fmaxf(y1, __shfl_xor_sync(kFull, y1, o));
+            z1 = fmaxf(z1, __shfl_xor_sync(kFull, z1, o));
+            r2 = fmaxf(r2, __shfl_xor_sync(kFull, r2, o));
+        }
+    }
+    // The z range, in U-units, of the row (x, y) of U-units that a sphere can
+    // reach; false when none does.
+    template <int U>
+    __device__ __forceinline__ bool row(int x, int y, int &zl, int &zh) const {
+        constexpr float w = kCellWidth * (1 << U), iw = 1.f / (kCellWidth * (1 << U));
+        const float gx = fmaxf(fmaxf((float)x * w - x1, x0 - (float)(x + 1) * w) - kCellMargin, 0.f);
+        const float gy = fmaxf(fmaxf((float)y * w - y1, y0 - (float)(y + 1) * w) - kCellMargin, 0.f);
+        const float left = r2 - (gx * gx + gy * gy);
+        if (left < 0.f) return false;
+        const float dz = left * rsqrtf(fmaxf(left, 1e-30f)) + kCellMargin;
+        zl = (int)floorf((z0 - dz) * iw - 1e-3f);
+        zh = (int)floorf((z1 + dz) * iw + 1e-3f);
+        return true;
+    }
+};
+
 // One warp: the density pass of sorted particles p0 .. p0 + 3 of the staged
 // tile (lane group g = lane / 8 takes p0 + g) whose pass is U (0 cell tiles,
 // kUnitShift coarse tiles; the staged box counts U-units), in lockstep so the warp never
@@ -846,20 +898,21 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
         const int v0 = __reduce_max_sync(kFull, b.hi0), v1 = __reduce_max_sync(kFull, b.hi1),
                   v2 = __reduce_max_sync(kFull, b.hi2);
         if (u0 > v0) return;  // no group builds
-        float qx[kTileGpw], qy[kTileGpw], qz[kTileGpw], qr[kTileGpw];
+        const Reach4 reach(px, py, pz, r2);
+        F2 nx[kTileGpw / 2], ny2[kTileGpw / 2], nz2[kTileGpw / 2];  // minus the positions, two particles each
+        float qr[kTileGpw];
 #pragma unroll
-        for (int k = 0; k < kTileGpw; ++k) {
-            qx[k] = __shfl_sync(kFull, px, k * L);
-            qy[k] = __shfl_sync(kFull, py, k * L);
-            qz[k] = __shfl_sync(kFull, pz, k * L);
-            qr[k] = __shfl_sync(kFull, r2, k * L);
+        for (int k = 0; k < kTileGpw; ++k) qr[k] = __shfl_sync(kFull, r2, k * L);
+#pragma unroll
+        for (int k = 0; k < kTileGpw / 2; ++k) {
+            nx[k] = f2(-__shfl_sync(kFull, px, 2 * k * L), -__shfl_sync(kFull, px, (2 * k + 1) * L));
+            ny2[k] = f2(-__shfl_sync(kFull, py, 2 * k * L), -__shfl_sync(kFull, py, (2 * k + 1) * L));
+            nz2[k] = f2(-__shfl_sync(kFull, pz, 2 * k * L), -__shfl_sync(kFull, pz, (2 * k + 1) * L));
         }
         int cnt[kTileGpw] = {};
         const unsigned below = (1u << lane) - 1u;
-        constexpr float w = kCellWidth;
-        constexpr float iw = 1.f / kCellWidth;
         // Rows (x, y) of the union box, 32 at a time, one per lane; each row is
-        // trimmed to the z cells that one of the four spheres reaches, and the
+        // trimmed to the z cells that the four spheres can reach, and the
         // trimmed rows are walked as one flat sequence of staged slots, 32
         // slots per step.
         const int nyu = v1 - u1 + 1;
@@ -869,27 +922,15 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
             uint32_t len = 0u, s0 = 0u;
             if (r < rows) {
                 const int x = u0 + r / nyu, y = u1 + r % nyu;
-                // the row's extent in x and y
-                const float x0 = (float)(x * (1 << U)) * w, x1 = (float)((x + 1) * (1 << U)) * w;
-                const float y0 = (float)(y * (1 << U)) * w, y1 = (float)((y + 1) * (1 << U)) * w;
-                int zl = 0x3fffffff, zh = -0x3fffffff;
-#pragma unroll
-                for (int k = 0; k < kTileGpw; ++k) {
-                    const float gx = fmaxf(fmaxf(x0 - qx[k], qx[k] - x1) - kCellMargin, 0.f);
-                    const float gy = fmaxf(fmaxf(y0 - qy[k], qy[k] - y1) - kCellMargin, 0.f);
-                    const float g2 = gx * gx + gy * gy;
-                    if (g2 <= qr[k]) {
-                        const float dz = sqrtf(qr[k] - g2);
-                        zl = min(zl, (int)floorf((qz[k] - dz) * iw - 1e-3f) >> U);
-                        zh = max(zh, (int)floorf((qz[k] + dz) * iw + 1e-3f) >> U);
+                int zl, zh;
+                if (reach.row<U>(x, y, zl, zh)) {
+                    zl = max(zl, u2);
+                    zh = min(zh, v2);
+                    if (zl <= zh) {
+                        const int c0 = ((x - lo0) * ny + (y - lo1)) * nz;
+                        s0 = S.off[c0 + (zl - lo2)];
+                        len = S.off[c0 + (zh - lo2) + 1] - s0;
                     }
-                }
-                zl = max(zl, u2);
-                zh = min(zh, v2);
-                if (zl <= zh) {
-                    const int c0 = ((x - lo0) * ny + (y - lo1)) * nz;
-                    s0 = S.off[c0 + (zl - lo2)];
-                    len = S.off[c0 + (zh - lo2) + 1] - s0;
                 }
             }
             uint32_t pre = len;  // inclusive scan of the row lengths
@@ -900,6 +941,7 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
             }
             const uint32_t excl = pre - len;
             const uint32_t total = __shfl_sync(kFull, pre, 31);
+            s0 -= excl;  // staged slot of flat index v in this row: s0 + v
             for (uint32_t vb = 0; vb < total; vb += 32u) {
                 const uint32_t v = vb + (uint32_t)lane;
                 int j = 0;  // the last row whose first flat index is <= v
@@ -908,20 +950,24 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
                     const uint32_t e = __shfl_sync(kFull, excl, j + step);
                     if (e <= v) j += step;
                 }
-                const uint32_t sj = __shfl_sync(kFull, s0, j), ej = __shfl_sync(kFull, excl, j);
+                const uint32_t s = __shfl_sync(kFull, s0, j) + v;
                 float4 q = make_float4(3e38f, 3e38f, 3e38f, 0.f);
-                const uint32_t s = sj + (v - ej);
                 if (v < total) q = S.pos[s];
+                const F2 qx = f2(q.x), qy = f2(q.y), qz = f2(q.z);
 #pragma unroll
-                for (int k = 0; k < kTileGpw; ++k) {
-                    const float dx = q.x - qx[k], dy = q.y - qy[k], dz = q.z - qz[k];
-                    const bool hit = dx * dx + dy * dy + dz * dz <= qr[k];
-                    const unsigned bal = __ballot_sync(kFull, hit);
-                    if (hit) {
-                        const int at = cnt[k] + __popc(bal & below);
-                        if (at < kTileList) lists[k][at] = (uint16_t)s;
+                for (int k = 0; k < kTileGpw / 2; ++k) {
+                    const F2 dx = qx + nx[k], dy = qy + ny2[k], dz = qz + nz2[k];
+                    float d[2];
+                    unpack(fma2(dz, dz, fma2(dy, dy, dx * dx)), d[0], d[1]);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int g2 = 2 * k + i;
+                        const bool hit = d[i] <= qr[g2];
+                        const unsigned bal = __ballot_sync(kFull, hit);
+                        const int at = cnt[g2] + __popc(bal & below);
+                        if (hit && at < kTileList) lists[g2][at] = (uint16_t)s;
+                        cnt[g2] += __popc(bal);
                     }
-                    cnt[k] += __popc(bal);
                 }
             }
         }
@@ -939,47 +985,66 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
             }
         }
     };
+    // Distance and mass of the pair of list entries (i, i + L); nothing (a
+    // massless neighbour far away) past the list's end.
+    auto entry_pair = [&](int i, F2 &r, F2 &m) {
+        float rr[2] = {1e30f, 1e30f}, mm[2] = {0.f, 0.f};
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (i + e * L < n_list) {
+                const float4 q = S.pos[list[i + e * L]];
+                const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
+                rr[e] = pair_sqrt(dx * dx + dy * dy + dz * dz);
+                mm[e] = q.w;
+            }
+        r = f2(rr[0], rr[1]);
+        m = f2(mm[0], mm[1]);
+    };
+    F2 rp[kRegPairs], mp[kRegPairs];
     bool iter = live;
     bool first = true, fell_back = false;
-    int sweeps = 0, count = 0, nn = 0;
+    int sweeps = 0, count = 0;
+    int maxn = 0;  // longest list of the warp
     float h2x4 = 4.f * hi * hi;
     float h1 = 1.f / hi;
-    float dens = 0.f, eps = 1.f;
-    float hs = hi, hs2x4 = h2x4;  // the h of the last full sweep
+    float w4 = 0.f, eps = 1.f;  // 4 pi h^3 x the density
     while (__any_sync(kFull, iter)) {
-        if (iter) {
-            hs = hi;
-            hs2x4 = h2x4;
-        }
-        const bool want = iter && (n_list < 0 || hs2x4 > list_r2);
+        const bool want = iter && (n_list < 0 || h2x4 > list_r2);
         if (__any_sync(kFull, want)) {
-            build(want, hs);
+            build(want, hi);
             iter = iter && live;
-        }
-        const int maxn = __reduce_max_sync(kFull, iter ? n_list : 0);
-        float part = 0.f;
-        int found = 0;
-#pragma unroll 4
-        for (int i = sub; i < maxn; i += L) {
-            if (iter && i < n_list) {
-                const float4 q = S.pos[list[i]];
-                const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 <= hs2x4) {
-                    const float r = pair_sqrt(r2);
-                    ++found;
-                    part += kernel_w(r, h1) * q.w;
-                }
+            maxn = __reduce_max_sync(kFull, live ? n_list : 0);
+            if (maxn <= kRegList) {
+#pragma unroll
+                for (int t = 0; t < kRegPairs; ++t)
+                    if (2 * t * L < maxn) entry_pair(sub + 2 * t * L, rp[t], mp[t]);
             }
         }
-        const float dsum = group_sum<L>(part, kFull);
-        const int fsum = group_sum_i<L>(found, kFull);
+        // the cubic spline as (2 - q)+^3 / 4 - (1 - q)+^3
+        const F2 nh = f2(-h1);
+        F2 acc = f2(0.f);
+        auto add = [&](F2 r, F2 m) {
+            const F2 t = clamp0(fma2(r, nh, f2(2.f))), u = clamp0(fma2(r, nh, f2(1.f)));
+            acc = fma2(m, fma2(f2(-4.f) * u, u * u, t * (t * t)), acc);
+        };
+        if (maxn <= kRegList) {
+#pragma unroll
+            for (int t = 0; t < kRegPairs; ++t)
+                if (2 * t * L < maxn) add(rp[t], mp[t]);
+        } else {
+            for (int i = sub; i < maxn; i += 2 * L) {
+                F2 r, m;
+                entry_pair(i, r, m);
+                add(r, m);
+            }
+        }
+        const float wsum = group_sum<L>(sum(acc), kFull);
         if (iter) {
-            dens = dsum;
-            nn = min(fsum, kNeighbourCache);
-            float nh = fmin_ref(kResolutionEta * powf(mi / dens, 1.f / 3), kMaxH);
-            nh = 0.5f * (hi + nh);
-            eps = fabsf(nh - hi) / hi;
+            w4 = wsum;
+            const float dens = kernel_norm(h1) * wsum;
+            float nh_ = fmin_ref(kResolutionEta * cbrtf(mi / dens), kMaxH);
+            nh_ = 0.5f * (hi + nh_);
+            eps = fabsf(nh_ - hi) * h1;
             ++sweeps;
             if (first && seeded && eps > kSeedFallback) {
                 // the seed disagrees with its own first sweep: start again from
@@ -989,68 +1054,92 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
                 hi = h_plain;
                 h1 = 1.f / hi;
                 h2x4 = 4.f * hi * hi;
-                nn = 0;
                 eps = 1.f;
             } else {
                 first = false;
                 if (eps > a.eta) {
-                    if (nh >= kMaxH) {
-                        defer();  // the reference's int max_h would leave 0 from here
+                    // at MAX_H the reference's int max_h would leave 0, and a
+                    // particle that does not converge ends on another h than
+                    // its last sweep's: the per-particle pass takes both
+                    if (nh_ >= kMaxH || ++count >= kMaxNR) {
+                        defer();
                     } else {
-                        hi = nh;
+                        hi = nh_;
                         h1 = 1.f / hi;
                         h2x4 = 4.f * hi * hi;
-                        count++;
                     }
                 }
             }
-            iter = live && eps > a.eta && count < kMaxNR;
+            iter = live && eps > a.eta;
         }
     }
-    // gradient sweep (density.metal:145-213), as in density_particle
-    const bool gcached = nn < kNeighbourCache;
-    const float g2 = gcached ? hs2x4 : h2x4;
+    // gradient sweep (density.metal:145-213) over the last sweep's neighbours,
+    // those within 2 h; with g' = 3 (1 - q)+^2 - 3 (2 - q)+^2 / 4 the spline's
+    // derivative, dW/dh = -(3 W + q g') / h (up to the norm), so of it only
+    // the sum of q g' is new
     const float h2 = hi + hi;
-    {
-        const bool want = live && g2 > list_r2;
-        if (__any_sync(kFull, want)) build(want, gcached ? hs : hi);
-    }
-    const int maxn = __reduce_max_sync(kFull, live ? n_list : 0);
     const float vix = mv.x, viy = mv.y, viz = mv.z;
-    float pdens = 0.f, dens_h = 0.f, vdiv = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-#pragma unroll 2
-    for (int i = sub; i < maxn; i += L) {
-        if (!(live && i < n_list)) continue;
-        const uint32_t s = list[i];
-        const float4 q = S.pos[s];
-        const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        if (r2 > g2) continue;
-        const float r = pair_sqrt(r2);
-        if (gcached && r > h2) continue;
-        const float mj = q.w;
-        if (!gcached) pdens += kernel_w(r, h1) * mj;
-        dens_h += mj * kernel_dwdh(r, h1);
-        if (r > 1e-12f) {
-            const float r1 = pair_rinv(r2, r);
-            const float4 vj = __ldg(a.sv4 + S.gidx[s]);
-            const float vx = vj.x - vix, vy = vj.y - viy, vz = vj.z - viz;
-            const float sc = kernel_gradw_scale(r, h1);
-            const float gx = sc * (dx * r1), gy = sc * (dy * r1), gz = sc * (dz * r1);
-            vdiv += mj * (vx * gx + vy * gy + vz * gz);
-            cx += mj * (vy * gz - vz * gy);
-            cy += mj * (vz * gx - vx * gz);
-            cz += mj * (vx * gy - vy * gx);
+    F2 qg = f2(0.f), vdiv2 = qg, cx2 = qg, cy2 = qg, cz2 = qg;
+    int nn = 0;
+    {
+        const F2 nh = f2(-h1);
+        const F2 npx = f2(-px), npy = f2(-py), npz = f2(-pz), nvx = f2(-vix), nvy = f2(-viy), nvz = f2(-viz);
+        auto add = [&](int i, F2 r, F2 m) {
+            const F2 t = clamp0(fma2(r, nh, f2(2.f))), u = clamp0(fma2(r, nh, f2(1.f)));
+            const F2 g = m * fma2(f2(3.f) * u, u, f2(-0.75f) * (t * t));
+            float re[2];
+            unpack(r, re[0], re[1]);
+            float4 q[2] = {me, me}, vj[2] = {mv, mv};
+            float rinv[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const bool in = re[e] <= h2 && live;
+                nn += in ? 1 : 0;
+                rinv[e] = in && re[e] > 1e-12f ? pdiv(1.f, re[e]) : 0.f;
+                if (in) {
+                    const uint32_t s = list[i + e * L];
+                    q[e] = S.pos[s];
+                    vj[e] = __ldg(a.sv4 + S.gidx[s]);
+                }
+            }
+            // (nh is -1/h: this adds minus the sum; far padding has g = 0)
+            qg = fma2(g * nh, f2(fminf(re[0], h2), fminf(re[1], h2)), qg);
+            const F2 gr = g * f2(rinv[0], rinv[1]);
+            const F2 gx = gr * (f2(q[0].x, q[1].x) + npx), gy = gr * (f2(q[0].y, q[1].y) + npy),
+                     gz = gr * (f2(q[0].z, q[1].z) + npz);
+            const F2 vx = f2(vj[0].x, vj[1].x) + nvx, vy = f2(vj[0].y, vj[1].y) + nvy,
+                     vz = f2(vj[0].z, vj[1].z) + nvz;
+            vdiv2 = fma2(vz, gz, fma2(vy, gy, fma2(vx, gx, vdiv2)));
+            cx2 = fma2(vy, gz, fma2(neg(vz), gy, cx2));
+            cy2 = fma2(vz, gx, fma2(neg(vx), gz, cy2));
+            cz2 = fma2(vx, gy, fma2(neg(vy), gx, cz2));
+        };
+        if (maxn <= kRegList) {
+#pragma unroll
+            for (int t = 0; t < kRegPairs; ++t)
+                if (2 * t * L < maxn) add(sub + 2 * t * L, rp[t], mp[t]);
+        } else {
+            for (int i = sub; i < maxn; i += 2 * L) {
+                F2 r, m;
+                entry_pair(i, r, m);
+                add(i, r, m);
+            }
         }
     }
-    pdens = group_sum<L>(pdens, kFull);
-    dens_h = group_sum<L>(dens_h, kFull);
-    vdiv = group_sum<L>(vdiv, kFull);
-    cx = group_sum<L>(cx, kFull);
-    cy = group_sum<L>(cy, kFull);
-    cz = group_sum<L>(cz, kFull);
+    nn = group_sum_i<L>(nn, kFull);
+    const float norm = kernel_norm(h1);  // 1 / (4 pi h^3)
+    const float nqg = group_sum<L>(sum(qg), kFull);
+    const float gnorm = 4.f * norm * h1;
+    float vdiv = gnorm * group_sum<L>(sum(vdiv2), kFull);
+    const float cx = gnorm * group_sum<L>(sum(cx2), kFull);
+    const float cy = gnorm * group_sum<L>(sum(cy2), kFull);
+    const float cz = gnorm * group_sum<L>(sum(cz2), kFull);
     if (!live || sub != 0) return;
-    if (!gcached) dens += pdens;
+    // 3 sum(W) + sum(q g') over sum(4 W): nqg is minus sum(q g')
+    const float dens_h = -gnorm * (0.75f * w4 - nqg);
+    float dens = norm * w4;
+    nn = min(nn, kNeighbourCache);
+    if (nn >= kNeighbourCache) dens += dens;  // the reference's full scan adds the density again
     if (a.stats) {
         atomicAdd(&stats[0], (uint32_t)sweeps);
         if (fell_back) atomicAdd(&stats[1], 1u);
@@ -1372,6 +1461,72 @@ __device__ __forceinline__ void accel_pair(const AccelI &I, AccelSum &S, const f
                      mj * (I.facti * (vx * gix + vy * giy + vz * giz) + 0.5f * nu * (vx * gx + vy * gy + vz * gz)));
     accel_add<KAHAN>(S.dh, S.kh, pdiv(mj, rhoj) * (vx * gix + vy * giy + vz * giz));
 }
+// The same for two neighbours per lane in packed arithmetic (product build's
+// tiles).  All of a pair's vector terms lie along the pair, so they are the
+// scalar factors below times (x_j - x_i) / r:
+//   si, sj       gradW(h_i), gradW(h_j) along the pair
+//   push         m_j (f_i si + f_j sj + nu (si + sj) / 2) / r
+//   w            (v_j - v_i) . (x_j - x_i) / r
+struct AccelSum2 {
+    F2 x = F2{0}, y = F2{0}, z = F2{0}, du = F2{0}, dh = F2{0};
+    F2 kx = F2{0}, ky = F2{0}, kz = F2{0}, ku = F2{0}, kh = F2{0};
+    float vsig = 1e-12f;
+};
+template <bool KAHAN>
+__device__ __forceinline__ void accel_add2(F2 &sum, F2 &comp, F2 v) {
+    if (KAHAN) {
+        const F2 minus = f2(-1.f);
+        const F2 y = fma2(comp, minus, v);
+        const F2 t = sum + y;
+        comp = fma2(y, minus, fma2(sum, minus, t));
+        sum = t;
+    } else {
+        sum = sum + v;
+    }
+}
+// pi h^4 times the spline's gradient along the pair at distance r: the
+// derivative of (2 - q)+^3 / 4 - (1 - q)+^3
+__device__ __forceinline__ F2 spline_slope(F2 r, F2 minus_h1) {
+    const F2 t = clamp0(fma2(r, minus_h1, f2(2.f))), u = clamp0(fma2(r, minus_h1, f2(1.f)));
+    return fma2(f2(3.f) * u, u, f2(-0.75f) * (t * t));
+}
+template <bool KAHAN>
+__device__ __forceinline__ void accel_pair2(const AccelI &I, float fac_i, AccelSum2 &S, const float4 (&A)[2],
+                                            const float4 (&B)[2], const float4 (&C)[2]) {
+    const F2 ex = f2(A[0].x, A[1].x) + f2(-I.xi), ey = f2(A[0].y, A[1].y) + f2(-I.yi),
+             ez = f2(A[0].z, A[1].z) + f2(-I.zi);
+    const F2 r2 = fma2(ez, ez, fma2(ey, ey, ex * ex));
+    const F2 r1 = rsqrt2(r2);
+    const F2 r = r2 * r1;
+    const F2 vx = f2(B[0].x, B[1].x) + f2(-I.vxi), vy = f2(B[0].y, B[1].y) + f2(-I.vyi),
+             vz = f2(B[0].z, B[1].z) + f2(-I.vzi);
+    const F2 w = fma2(vz, ez, fma2(vy, ey, vx * ex)) * r1;
+    float wa, wb;
+    unpack(w, wa, wb);
+    const F2 mu = f2(fminf(wa, 0.f), fminf(wb, 0.f));
+    const F2 vsig = fma2(f2(-3.f), mu, f2(B[0].w, B[1].w) + f2(I.ci));
+    float va, vb;
+    unpack(vsig, va, vb);
+    S.vsig = fmaxf(S.vsig, fmaxf(va, vb));
+    // -alpha B_ij mu vsig / (2 rho_ij), the halves of B_ij and rho_ij cancelled
+    const F2 bal = f2(C[0].w, C[1].w) + f2(I.Bi);
+    const F2 nu = f2(-0.5f * kViscosityAlpha) * bal * (mu * vsig) *
+                  f2(pdiv(1.f, I.rhoi + C[0].z), pdiv(1.f, I.rhoi + C[1].z));
+    const F2 nhj = f2(pdiv(-1.f, A[0].w), pdiv(-1.f, A[1].w));
+    const F2 hj2 = nhj * nhj;
+    const F2 si = f2(fac_i) * spline_slope(r, f2(-I.hi1));
+    const F2 sj = (f2(kPi1) * hj2) * hj2 * spline_slope(r, nhj);
+    const F2 mean = f2(0.5f) * (si + sj);
+    const F2 m = f2(C[0].x, C[1].x);
+    const F2 fsi = f2(I.facti) * si;
+    const F2 push = m * fma2(nu, mean, fma2(f2(C[0].y, C[1].y), sj, fsi)) * r1;
+    accel_add2<KAHAN>(S.x, S.kx, push * ex);
+    accel_add2<KAHAN>(S.y, S.ky, push * ey);
+    accel_add2<KAHAN>(S.z, S.kz, push * ez);
+    accel_add2<KAHAN>(S.du, S.ku, m * w * fma2(f2(0.5f) * nu, mean, fsi));
+    accel_add2<KAHAN>(S.dh, S.kh, m * w * si * f2(pdiv(1.f, C[0].z), pdiv(1.f, C[1].z)));
+}
+
 // The group's sums combined (every lane ends with the same bits).
 template <int L, bool KAHAN>
 __device__ __forceinline__ void accel_reduce(AccelSum &S, unsigned gm) {
@@ -1389,16 +1544,14 @@ __device__ __forceinline__ void accel_reduce(AccelSum &S, unsigned gm) {
     S.dh = group_sum<L>(S.dh, gm);
     S.vsig = group_max<L>(S.vsig, gm);
 }
-// accelerations.metal:129-140: the particle's timestep in ticks.
+// accelerations.metal:129-140: the particle's timestep in ticks, DT0 halved
+// until it is at most `goal` (kRMax times at most): the halvings are read off
+// the goal's exponent, 2^e <= goal < 2^(e + 1).
 __device__ __forceinline__ int accel_ticks(const AccelI &I, float vsig) {
     const float goal = 2.0f * kCFL * kGamma * I.hi / vsig;
-    int r = 0;
-    float cand = kDT0;
-    while (cand > goal && r < kRMax) {
-        cand *= 0.5f;
-        r++;
-    }
-    return (int)ceilf(1 / kDtMin1 * cand);
+    static_assert(kDT0 == 32.f, "5 below is log2 DT0");
+    const int e = (int)((__float_as_uint(goal) >> 23) & 255u) - 127;
+    return (1 << kRMax) >> min(max(5 - e, 0), kRMax);
 }
 __device__ __forceinline__ void accel_store(const AccelArgs &a, uint32_t ind, const AccelSum &S, int idt) {
     float4 acc = a.acc4[ind];
@@ -1521,11 +1674,10 @@ constexpr int kTileAccStage = 3072;  // staged particles per tile
 struct TileAccShared {
     float4 pos[kTileAccStage];          // staged sA (x, y, z, h)
     uint32_t gidx[kTileAccStage];       // staged sorted index
-    uint32_t scell[kTileAccStage];      // staged cell, box-relative: x | y << 10 | z << 20
+    uint32_t scell[kTileAccStage];      // staged cell, box-relative (pack_cell)
     uint32_t off[kTileCellsMax + 1];
     uint32_t first[kTileCellsMax];
     uint16_t list[kTileGroups][kTileList];
-    int gbox[kTileGroups][6];           // each group's box, box-relative lo xyz, hi xyz
     int box[6];
     uint32_t wsum[kTileThreads / 32];
     uint32_t start, end, tile, next;
@@ -1547,6 +1699,18 @@ __device__ __forceinline__ int accel_mode(float px, float py, float pz, float h,
     if (within_reach<0>(ox, oy, oz, b)) return 0;
     if (coarse && within_reach<kUnitShift>(ox, oy, oz, b)) return kUnitShift;
     return -1;
+}
+
+// Three cell coordinates below kBoxCellsMax in one word, each followed by a
+// guard bit: in_box subtracts all three at once, and a guard bit that a
+// subtraction borrows marks a coordinate past the bound.
+constexpr int kBoxCellsMax = 512;
+constexpr uint32_t kGuards = (1u << 9) | (1u << 19) | (1u << 29);
+__device__ __forceinline__ uint32_t pack_cell(int x, int y, int z) {
+    return (uint32_t)x | ((uint32_t)y << 10) | ((uint32_t)z << 20);
+}
+__device__ __forceinline__ bool in_box(uint32_t c, uint32_t lo, uint32_t hi) {
+    return (((c | kGuards) - lo) & ((hi | kGuards) - c) & kGuards) == kGuards;
 }
 
 // One warp: the acceleration pass of sorted particles p0 .. p0 + 3 of the
@@ -1598,14 +1762,10 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
         b.lo0 = b.lo1 = b.lo2 = kBig;
         b.hi0 = b.hi1 = b.hi2 = -kBig;
     }
-    if (want && sub == 0) {
-        int *gb = S.gbox[wslot * kTileGpw + g];
-        gb[0] = b.lo0 - lo0 * (1 << U);
-        gb[1] = b.lo1 - lo1 * (1 << U);
-        gb[2] = b.lo2 - lo2 * (1 << U);
-        gb[3] = b.hi0 - lo0 * (1 << U);
-        gb[4] = b.hi1 - lo1 * (1 << U);
-        gb[5] = b.hi2 - lo2 * (1 << U);
+    uint32_t blo = kGuards, bhi = 0u;  // the group's box, relative to the staged box
+    if (want) {
+        blo = pack_cell(b.lo0 - lo0 * (1 << U), b.lo1 - lo1 * (1 << U), b.lo2 - lo2 * (1 << U));
+        bhi = pack_cell(b.hi0 - lo0 * (1 << U), b.hi1 - lo1 * (1 << U), b.hi2 - lo2 * (1 << U));
     }
     const int u0 = __reduce_min_sync(kFull, b.lo0) >> U, u1 = __reduce_min_sync(kFull, b.lo1) >> U,
               u2 = __reduce_min_sync(kFull, b.lo2) >> U;
@@ -1615,16 +1775,23 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
     __syncwarp();
     // every accepted pair lies within 2 max(h_i, largest staged h) of the particle
     const float hm = fmaxf(I.hi, __int_as_float(S.hmax_bits));
-    float qx[kTileGpw], qy[kTileGpw], qz[kTileGpw], qr[kTileGpw], qR[kTileGpw];
+    const Reach4 reach(I.xi, I.yi, I.zi, want ? 4.f * hm * hm : -1.f);
+    F2 nx[kTileGpw / 2], ny2[kTileGpw / 2], nz2[kTileGpw / 2];  // minus the positions, two particles each
+    float qr[kTileGpw];
+    uint32_t klo[kTileGpw], khi[kTileGpw];
 #pragma unroll
     for (int k = 0; k < kTileGpw; ++k) {
-        qx[k] = __shfl_sync(kFull, I.xi, k * L);
-        qy[k] = __shfl_sync(kFull, I.yi, k * L);
-        qz[k] = __shfl_sync(kFull, I.zi, k * L);
         qr[k] = __shfl_sync(kFull, want ? I.hi2x4 : -1.f, k * L);
-        qR[k] = __shfl_sync(kFull, want ? 4.f * hm * hm : -1.f, k * L);
+        klo[k] = __shfl_sync(kFull, blo, k * L);
+        khi[k] = __shfl_sync(kFull, bhi, k * L);
     }
-    // box bounds of the four groups, for the row test (lane k * L holds group k's)
+#pragma unroll
+    for (int k = 0; k < kTileGpw / 2; ++k) {
+        nx[k] = f2(-__shfl_sync(kFull, I.xi, 2 * k * L), -__shfl_sync(kFull, I.xi, (2 * k + 1) * L));
+        ny2[k] = f2(-__shfl_sync(kFull, I.yi, 2 * k * L), -__shfl_sync(kFull, I.yi, (2 * k + 1) * L));
+        nz2[k] = f2(-__shfl_sync(kFull, I.zi, 2 * k * L), -__shfl_sync(kFull, I.zi, (2 * k + 1) * L));
+    }
+    uint16_t (*const lists)[kTileList] = &S.list[wslot * kTileGpw];
     int cnt[kTileGpw] = {};
     const unsigned below = (1u << lane) - 1u;
     const int nyu = v1 - u1 + 1;
@@ -1632,39 +1799,19 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
     for (int rb = 0; rb < rows; rb += 32) {
         const int r = rb + lane;
         uint32_t len = 0u, s0 = 0u;
-        int zl = kBig, zh = -kBig;
-        int x = 0, y = 0;
         if (r < rows) {
-            x = u0 + r / nyu;
-            y = u1 + r % nyu;
-        }
-        // the z range of the boxes that contain row (x, y), trimmed to the
-        // sphere that holds every accepted pair
-        constexpr float w = kCellWidth;
-        constexpr float iw = 1.f / kCellWidth;
-        const float x0 = (float)(x * (1 << U)) * w, x1 = (float)((x + 1) * (1 << U)) * w;
-        const float y0 = (float)(y * (1 << U)) * w, y1 = (float)((y + 1) * (1 << U)) * w;
-#pragma unroll
-        for (int k = 0; k < kTileGpw; ++k) {
-            // group k's box in U-units (empty boxes stay empty: kBig >> U > -kBig >> U)
-            const int bl0 = __shfl_sync(kFull, b.lo0, k * L) >> U, bh0 = __shfl_sync(kFull, b.hi0, k * L) >> U;
-            const int bl1 = __shfl_sync(kFull, b.lo1, k * L) >> U, bh1 = __shfl_sync(kFull, b.hi1, k * L) >> U;
-            const int bl2 = __shfl_sync(kFull, b.lo2, k * L) >> U, bh2 = __shfl_sync(kFull, b.hi2, k * L) >> U;
-            if (r < rows && x >= bl0 && x <= bh0 && y >= bl1 && y <= bh1) {
-                const float gx = fmaxf(fmaxf(x0 - qx[k], qx[k] - x1) - kCellMargin, 0.f);
-                const float gy = fmaxf(fmaxf(y0 - qy[k], qy[k] - y1) - kCellMargin, 0.f);
-                const float g2 = gx * gx + gy * gy;
-                if (g2 <= qR[k]) {
-                    const float dz = sqrtf(qR[k] - g2);
-                    zl = min(zl, max(bl2, (int)floorf((qz[k] - dz) * iw - 1e-3f) >> U));
-                    zh = max(zh, min(bh2, (int)floorf((qz[k] + dz) * iw + 1e-3f) >> U));
+            // the row's z range that an accepted pair of the four can have
+            const int x = u0 + r / nyu, y = u1 + r % nyu;
+            int zl, zh;
+            if (reach.row<U>(x, y, zl, zh)) {
+                zl = max(zl, u2);
+                zh = min(zh, v2);
+                if (zl <= zh) {
+                    const int c0 = ((x - lo0) * ny + (y - lo1)) * nz;
+                    s0 = S.off[c0 + (zl - lo2)];
+                    len = S.off[c0 + (zh - lo2) + 1] - s0;
                 }
             }
-        }
-        if (zl <= zh) {
-            const int c0 = ((x - lo0) * ny + (y - lo1)) * nz;
-            s0 = S.off[c0 + (zl - lo2)];
-            len = S.off[c0 + (zh - lo2) + 1] - s0;
         }
         uint32_t pre = len;
 #pragma unroll
@@ -1674,6 +1821,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
         }
         const uint32_t excl = pre - len;
         const uint32_t total = __shfl_sync(kFull, pre, 31);
+        s0 -= excl;  // staged slot of flat index v in this row: s0 + v
         for (uint32_t vb = 0; vb < total; vb += 32u) {
             const uint32_t v = vb + (uint32_t)lane;
             int j = 0;
@@ -1682,8 +1830,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
                 const uint32_t e = __shfl_sync(kFull, excl, j + step);
                 if (e <= v) j += step;
             }
-            const uint32_t sj = __shfl_sync(kFull, s0, j), ej = __shfl_sync(kFull, excl, j);
-            const uint32_t s = sj + (v - ej);
+            const uint32_t s = __shfl_sync(kFull, s0, j) + v;
             float4 q = make_float4(3e38f, 3e38f, 3e38f, 0.f);
             uint32_t sc = 0u;
             if (v < total) {
@@ -1691,26 +1838,21 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
                 sc = S.scell[s];
             }
             const float hj2x4 = q.w * q.w * 4.f;
+            const F2 qx = f2(q.x), qy = f2(q.y), qz = f2(q.z);
+            float d[kTileGpw];
+#pragma unroll
+            for (int k = 0; k < kTileGpw / 2; ++k) {
+                const F2 dx = qx + nx[k], dy = qy + ny2[k], dz = qz + nz2[k];
+                unpack(fma2(dz, dz, fma2(dy, dy, dx * dx)), d[2 * k], d[2 * k + 1]);
+            }
 #pragma unroll
             for (int k = 0; k < kTileGpw; ++k) {
-                const float dx = qx[k] - q.x, dy = qy[k] - q.y, dz = qz[k] - q.z;
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                const bool near = r2 >= 1e-12f;
-                bool hit = near && r2 <= qr[k];
-                // r > 2 h_i but r <= 2 h_j: only when the neighbour's cell is in the box
-                const bool maybe = near && !hit && qr[k] >= 0.f && r2 <= hj2x4;
-                if (__any_sync(kFull, maybe)) {
-                    const int *gb = S.gbox[wslot * kTileGpw + k];
-                    const int cx = (int)(sc & 1023u), cy = (int)((sc >> 10) & 1023u), cz = (int)(sc >> 20);
-                    if (maybe && cx >= gb[0] && cx <= gb[3] && cy >= gb[1] && cy <= gb[4] && cz >= gb[2] &&
-                        cz <= gb[5])
-                        hit = true;
-                }
+                // r <= 2 h_i, or r <= 2 h_j with the neighbour's cell in the
+                // particle's box (empty for a group that takes no part)
+                const bool hit = d[k] >= 1e-12f && (d[k] <= qr[k] || (d[k] <= hj2x4 && in_box(sc, klo[k], khi[k])));
                 const unsigned bal = __ballot_sync(kFull, hit);
-                if (hit) {
-                    const int at = cnt[k] + __popc(bal & below);
-                    if (at < kTileList) S.list[wslot * kTileGpw + k][at] = (uint16_t)s;
-                }
+                const int at = cnt[k] + __popc(bal & below);
+                if (hit && at < kTileList) lists[k][at] = (uint16_t)s;
                 cnt[k] += __popc(bal);
             }
         }
@@ -1725,16 +1867,33 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
         live = false;
     }
     const int maxn = __reduce_max_sync(kFull, live ? n_list : 0);
-    AccelSum Sm;
-#pragma unroll 2
-    for (int i = sub; i < maxn; i += L) {
-        if (live && i < n_list) {
-            const uint32_t s = list[i];
-            const uint32_t gj = S.gidx[s];
-            accel_pair<KAHAN>(I, Sm, S.pos[s], __ldg(a.sB + gj), __ldg(a.sC + gj));
-        }
+    AccelSum2 S2;
+    const float hi2 = I.hi1 * I.hi1, fac_i = kPi1 * hi2 * hi2;
+    for (int i = sub; i < maxn; i += 2 * L) {
+        // (past the list's end: no mass, no relative motion, far away)
+        const float4 none = make_float4(I.xi + 1e15f, I.yi, I.zi, 1.f);
+        float4 Aj[2] = {none, none}, Bj[2], Cj[2];
+        Bj[0] = Bj[1] = make_float4(I.vxi, I.vyi, I.vzi, -1e30f);
+        Cj[0] = Cj[1] = make_float4(0.f, 0.f, 1.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            if (live && i + e * L < n_list) {
+                const uint32_t s = list[i + e * L];
+                const uint32_t gj = S.gidx[s];
+                Aj[e] = S.pos[s];
+                Bj[e] = __ldg(a.sB + gj);
+                Cj[e] = __ldg(a.sC + gj);
+            }
+        accel_pair2<KAHAN>(I, fac_i, S2, Aj, Bj, Cj);
     }
-    accel_reduce<L, KAHAN>(Sm, kFull);
+    AccelSum Sm;
+    Sm.dvx = KAHAN ? sum(fma2(S2.kx, f2(-1.f), S2.x)) : sum(S2.x);
+    Sm.dvy = KAHAN ? sum(fma2(S2.ky, f2(-1.f), S2.y)) : sum(S2.y);
+    Sm.dvz = KAHAN ? sum(fma2(S2.kz, f2(-1.f), S2.z)) : sum(S2.z);
+    Sm.du = KAHAN ? sum(fma2(S2.ku, f2(-1.f), S2.du)) : sum(S2.du);
+    Sm.dh = KAHAN ? sum(fma2(S2.kh, f2(-1.f), S2.dh)) : sum(S2.dh);
+    Sm.vsig = S2.vsig;
+    accel_reduce<L, false>(Sm, kFull);
     int idt = idt_inactive;
     if (live) {
         idt = accel_ticks(I, Sm.vsig);
@@ -1846,7 +2005,9 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                       nz = any ? S.box[5] - lo2 + 1 : 0;
             int ncell = 0;
             if (any) {
-                if (nx * ny * nz > kTileCellsMax) {
+                // (pack_cell's range: such a box holds particles of cells that
+                // are only alike modulo the grid)
+                if (nx * ny * nz > kTileCellsMax || max(nx, max(ny, nz)) > (kBoxCellsMax >> U)) {
                     if (tid == 0) S.defer_all = 1;
                 } else {
                     ncell = nx * ny * nz;
@@ -1923,7 +2084,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                         iy = (iy << U) | dy;
                         iz = (iz << U) | dz;
                     }
-                    S.scell[s] = (uint32_t)ix | ((uint32_t)iy << 10) | ((uint32_t)iz << 20);
+                    S.scell[s] = pack_cell(ix, iy, iz);
                     hmax = fmaxf(hmax, q.w);
                 }
             }

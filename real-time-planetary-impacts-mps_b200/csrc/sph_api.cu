@@ -315,7 +315,8 @@ sph_status sph_destroy(sph_ctx *ctx) {
                     ctx->du, ctx->B, ctx->dhdt, ctx->gnorm, ctx->phi, ctx->mat, ctx->nat, ctx->active, ctx->globals,
                     ctx->health, ctx->cell_range, ctx->sp4, ctx->sv4, ctx->sA, ctx->sB, ctx->sC,
                     ctx->eos_forsterite, ctx->eos_fe, ctx->stage, ctx->snapshot, ctx->pos64, ctx->dglob,
-                    ctx->diag, ctx->tiles, ctx->tile_ctr, ctx->deferred, ctx->units, ctx->coarse_flags};
+                    ctx->diag, ctx->tiles, ctx->tile_ctr, ctx->deferred, ctx->units, ctx->coarse_flags,
+                    ctx->tile_mode, ctx->tile_h, ctx->octets};
     for (void *b : bufs) cudaFree(b);
     sort_free(ctx->cell_sort);
     hseed_free(ctx);
@@ -394,7 +395,10 @@ sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out)
     chk(dmalloc(&ctx->tiles, (size_t)n));
     chk(dmalloc(&ctx->tile_ctr, 16));
     chk(dmalloc(&ctx->deferred, (size_t)n));
+    chk(dmalloc(&ctx->tile_mode, (size_t)n));
+    chk(dmalloc(&ctx->tile_h, (size_t)n));
     chk(dmalloc(&ctx->units, (size_t)kNumUnits));
+    chk(dmalloc(&ctx->octets, (size_t)kNumOctets));
     chk(dmalloc(&ctx->coarse_flags, (size_t)kNumCoarseBlocks));
     if (e == cudaSuccess) e = cudaMemset(ctx->coarse_flags, 0, kNumCoarseBlocks);
     if (e != cudaSuccess) {

@@ -88,10 +88,8 @@ __device__ __forceinline__ uint32_t cell_index_of(int x, int y, int z) {
 constexpr int kUnitShift = 2;  // cells per unit edge = 1 << kUnitShift
 constexpr uint32_t kNumUnits = kNumCells >> (3 * kUnitShift);
 constexpr uint32_t kNumCoarseBlocks = kNumUnits >> 3;
-__device__ __forceinline__ uint32_t unit_index_of(int x, int y, int z) {
-    const int mask = (kCellsPerDim >> kUnitShift) - 1;
-    return morton3((uint32_t)(x & mask), (uint32_t)(y & mask), (uint32_t)(z & mask));
-}
+// Octets: 2 x 2 x 2 cells, the cells whose keys agree above the low three bits.
+constexpr uint32_t kNumOctets = kNumCells >> 3;
 struct CellBox {
     int lo0, lo1, lo2, hi0, hi1, hi2;
 };

@@ -264,9 +264,12 @@ struct DensityArgs {
     const uint32_t *cidx;
     const uint32_t *skey;  // sorted cell keys (tile passes)
     const uint2 *cells;
+    const uint2 *octets;   // 8-cell octet ranges and
     const uint2 *units;    // 64-cell unit ranges (coarse tiles)
     uint8_t *cflags;       // per 512-cell block: holds a coarse-tile particle
     int coarse;            // coarse tiles on
+    uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_tile_plan
+    float *start_h;        // [n] the h its staged box is built for, written by k_tile_plan
     const float4 *sp4, *sv4;
     float *h, *rho, *f, *P, *c, *B;
     const float *u;
@@ -604,7 +607,6 @@ struct TileShared {
     float4 pos[kTileStageMax];          // staged (x, y, z, m)
     uint32_t gidx[kTileStageMax];       // staged sorted index
     uint32_t off[kTileCellsMax + 1];    // first staged slot of each box cell; off[cells] = staged count
-    uint32_t first[kTileCellsMax];      // first sorted index of each box cell
     uint16_t list[kTileGroups][kTileList];
     int box[6];                         // staged box: lo x y z, hi x y z (unwrapped cell coordinates)
     uint32_t wsum[kTileThreads / 32];
@@ -631,12 +633,33 @@ __device__ __forceinline__ void tile_box(float px, float py, float pz, float hb,
     b.hi2 = (int)floorf((pz + rl) * iw + widen);
 }
 
-// The (first, last) sorted range of tiling unit (x, y, z): a cell (U = 0) or a
-// 64-cell unit (U = kUnitShift); first is 0xffffffff when it is empty.
+// Units of a box, or some number past any limit (particles of one cell that
+// are only alike modulo the grid can span thousands of cells).
+__device__ __forceinline__ int64_t box_units(int nx, int ny, int nz) {
+    return (int64_t)min(nx, 1 << 20) * min(ny, 1 << 20) * min(nz, 1 << 20);
+}
+
+// Tiling units of the staged box: cells (shift 0, the cell tiles), 2 x 2 x 2
+// octets (shift 1) or 4 x 4 x 4-cell units (shift 2) for the coarse tiles,
+// which take the octets whenever their box has few enough of them: finer
+// units stage fewer particles and trim the lists' rows closer (h of 2 cells,
+// reach 5: half the staged particles), while at a reach of 7 cells and more
+// their 200 rows cost more than they trim.
 template <int U>
-__device__ __forceinline__ uint2 unit_range(const uint2 *cells, const uint2 *units, int x, int y, int z) {
-    if (U == 0) return __ldg(cells + cell_index_of(x, y, z));
-    return __ldg(units + unit_index_of(x, y, z));
+__device__ __forceinline__ int unit_shift(const int (&box)[6]) {
+    if (U == 0) return 0;
+    return box_units((box[3] >> 1) - (box[0] >> 1) + 1, (box[4] >> 1) - (box[1] >> 1) + 1,
+                     (box[5] >> 1) - (box[2] >> 1) + 1) <= kTileCellsMax
+               ? 1
+               : kUnitShift;
+}
+// The (first, last) sorted range of unit (x, y, z); first is 0xffffffff when
+// it is empty.
+__device__ __forceinline__ uint2 unit_range(const uint2 *cells, const uint2 *octets, const uint2 *units, int shift,
+                                            int x, int y, int z) {
+    const int mask = (kCellsPerDim >> shift) - 1;
+    const uint2 *t = shift == 0 ? cells : shift == 1 ? octets : units;
+    return __ldg(t + morton3((uint32_t)(x & mask), (uint32_t)(y & mask), (uint32_t)(z & mask)));
 }
 
 // Whether a cell box reaches at most kTileReach tiling units (cells for U = 0,
@@ -652,8 +675,7 @@ __device__ __forceinline__ bool within_reach(int ox, int oy, int oz, const CellB
 // radius 2 hb kTileListReach: 0 the cell tiles, kUnitShift the coarse tiles
 // (a box past kTileReach cells, within kTileReach units), -1 the per-particle
 // pass (h at MAX_H, where the reference's neighbour cache comes into play, or
-// coarse tiles off).  Every pass evaluates it from the same inputs, so each
-// particle is taken by exactly one.
+// coarse tiles off).
 __device__ __forceinline__ int density_mode(float px, float py, float pz, float hb, int coarse) {
     if (!(hb < kMaxH)) return -1;
     constexpr float iw = 1.f / kCellWidth;
@@ -663,6 +685,48 @@ __device__ __forceinline__ int density_mode(float px, float py, float pz, float 
     if (within_reach<0>(ox, oy, oz, b)) return 0;
     if (coarse && within_reach<kUnitShift>(ox, oy, oz, b)) return kUnitShift;
     return -1;
+}
+
+// Staging: a warp copies the particles of its lanes' units (cnt and first of
+// kTileCellsPerThread consecutive units per lane), which are consecutive
+// staged slots from the warp's first: 32 slots at a time, each lane finding the
+// lane and unit its slot belongs to, so that a unit with many particles is
+// shared out.  excl, incl: the lane's slots within the warp.  copy(slot
+// within the warp's, sorted index, unit counted from the warp's first).
+template <class Copy>
+__device__ __forceinline__ void stage_units(const uint32_t (&cnt)[kTileCellsPerThread],
+                                            const uint32_t (&first)[kTileCellsPerThread], uint32_t excl,
+                                            uint32_t incl, int lane, Copy &&copy) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+#pragma unroll 2
+    for (uint32_t vb = 0; vb < total; vb += 32u) {
+        const uint32_t v = vb + (uint32_t)lane;
+        int j = 0;  // the last lane whose first slot is <= v
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+            const uint32_t e = __shfl_sync(kFull, excl, j + step);
+            if (e <= v) j += step;
+        }
+        uint32_t at = v - __shfl_sync(kFull, excl, j);
+        uint32_t g = 0u;
+        int unit = 0;
+        bool found = false;
+#pragma unroll
+        for (int k = 0; k < kTileCellsPerThread; ++k) {
+            const uint32_t c = __shfl_sync(kFull, cnt[k], j), f = __shfl_sync(kFull, first[k], j);
+            if (!found) {
+                if (at < c) {
+                    g = f + at;
+                    unit = kTileCellsPerThread * j + k;
+                    found = true;
+                } else {
+                    at -= c;
+                }
+            }
+        }
+        if (v < total) copy(v, g, unit);
+    }
 }
 
 // The starting h of an active particle's iteration (the learned seed when it
@@ -679,72 +743,102 @@ __device__ __forceinline__ float tile_start_h(const DensityArgs &a, uint32_t ind
     return h_plain;
 }
 
-// Tiles: at the first sorted particle of every occupied 128-cell block (the
-// cells whose keys differ in the low seven bits, 4 x 4 x 8), the block's
-// octet ranges (from its 128 cell ranges); the block is one tile when it
-// holds at most big_max particles, else each 64-cell half is one when it
-// holds at most block_max, else each 16-cell quarter when it holds at most
+// The pass that takes a sorted particle, decided once per pass by k_tile_plan
+// from the particle's starting h: the density pass changes h as it goes, so a
+// second look could give a particle to two passes (10 % of them on a 2e5
+// impact) or to none.
+constexpr uint8_t kModeWalk = 0xfe;      // the per-particle pass
+constexpr uint8_t kModeInactive = 0xff;  // no neighbours needed (cell-tile pass)
+static_assert(kUnitShift < kModeWalk, "0 and kUnitShift: the tile passes");
+
+// A warp: the tiles of the 128-cell block `blk` (the cells whose keys differ
+// in the low seven bits, 4 x 4 x 8), four cells per lane, so an octet is two
+// lanes, a 16-cell quarter of a half four, a 64-cell half sixteen: the block
+// is one tile when it holds at most big_max particles, else each half is one
+// when it holds at most block_max, else each quarter when it holds at most
 // half_max, else each octet.  (first, one past last) per tile, in ticket
-// order.  ctr[0] counts tiles; ctr[1] is the CTAs' tile ticket, ctr[2] the
-// deferred count.
-__global__ void k_tile_starts(int n, const uint32_t *__restrict__ skey, const uint2 *__restrict__ cells,
-                              uint2 *__restrict__ tiles, uint32_t *ctr, int32_t *globals, uint32_t block_max,
-                              uint32_t half_max, uint32_t big_max) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0 && globals) globals[1] = (int32_t)(kDT0 * 1 / kDtMin1);  // density.metal:34-36
-    if (k >= n) return;
-    const uint32_t blk = skey[k] >> 7;
-    if (k > 0 && (skey[k - 1] >> 7) == blk) return;
-    uint32_t ofirst[16], oend[16];  // octet ranges; oend == 0 when empty
+// order; ctr[0] counts tiles.
+__device__ __forceinline__ void plan_block(uint32_t blk, const uint2 *cells, uint2 *tiles, uint32_t *ctr,
+                                           uint32_t block_max, uint32_t half_max, uint32_t big_max, int lane) {
+    constexpr unsigned kFull = 0xffffffffu;
+    uint32_t f = 0xffffffffu, l = 0u;
+    const uint4 *c4 = reinterpret_cast<const uint4 *>(cells + (size_t)blk * 128u + 4u * (uint32_t)lane);
 #pragma unroll
-    for (int o = 0; o < 16; ++o) {
-        uint32_t f = 0xffffffffu, l = 0u;
-        for (int j = 0; j < 8; ++j) {
-            const uint2 r = cells[blk * 128u + (uint32_t)(o * 8 + j)];
-            if (r.x != 0xffffffffu) {
-                f = min(f, r.x);
-                l = max(l, r.y + 1u);
-            }
-        }
-        ofirst[o] = f;
-        oend[o] = l;
+    for (int j = 0; j < 2; ++j) {
+        const uint4 r = __ldg(c4 + j);
+        if (r.x != 0xffffffffu) f = min(f, r.x), l = max(l, r.y + 1u);
+        if (r.z != 0xffffffffu) f = min(f, r.z), l = max(l, r.w + 1u);
     }
-    auto emit = [&](uint32_t f, uint32_t l) {
-        if (l > f) tiles[atomicAdd(ctr, 1u)] = make_uint2(f, l);
+    uint32_t first = 0u, end = 0u;  // the tile this lane leads
+    bool fits = false;              // a larger block already holds the lane's cells
+    uint32_t lf[5], ll[5];          // ranges of 2, 4, 8, 16 and 32 lanes
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        f = min(f, __shfl_xor_sync(kFull, f, 1 << k));
+        l = max(l, __shfl_xor_sync(kFull, l, 1 << k));
+        lf[k] = f;
+        ll[k] = l;
+    }
+    auto take = [&](int k, uint32_t most) {
+        if (fits || ll[k] <= lf[k] || ll[k] - lf[k] > most) return;
+        fits = true;
+        if ((lane & ((2 << k) - 1)) == 0) {
+            first = lf[k];
+            end = ll[k];
+        }
     };
-    auto span = [&](int o0, int o1, uint32_t &f, uint32_t &l) {  // octets o0 .. o1 - 1
-        f = 0xffffffffu;
-        l = 0u;
-        for (int o = o0; o < o1; ++o)
-            if (oend[o]) {
-                f = min(f, ofirst[o]);
-                l = max(l, oend[o]);
-            }
-    };
-    uint32_t f, l;
-    span(0, 16, f, l);
-    if (l - f <= big_max) {
-        emit(f, l);
-        return;
+    take(4, big_max);
+    take(3, block_max);
+    take(1, half_max);
+    take(0, 0xffffffffu);
+    const unsigned m = __ballot_sync(kFull, end > first);
+    uint32_t at = 0u;
+    if (lane == 0) at = atomicAdd(ctr, (uint32_t)__popc(m));
+    at = __shfl_sync(kFull, at, 0);
+    if (end > first) tiles[at + (uint32_t)__popc(m & ((1u << lane) - 1u))] = make_uint2(first, end);
+}
+
+// One thread per sorted particle: its pass (Mode(p), which also flags the
+// 512-cell blocks that hold a coarse-tile particle), and, a warp per occupied
+// 128-cell block that starts among its particles, the tiles.  (With one thread
+// per block, whose 128 cell reads ran one after another, the tiles alone took
+// 20 us at N = 1e6.)
+template <class Mode>
+__device__ __forceinline__ void tile_plan(int n, const uint32_t *skey, const uint2 *cells, uint8_t *cflags,
+                                          uint8_t *mode, uint2 *tiles, uint32_t *ctr, uint32_t block_max,
+                                          uint32_t half_max, uint32_t big_max, Mode &&of) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    uint32_t key = 0u;
+    bool start = false;
+    if (k < n) {
+        key = skey[k];
+        start = k == 0 || ((skey[k - 1] ^ key) >> 7) != 0u;
+        const uint8_t m = of(k);
+        mode[k] = m;
+        if (m == kUnitShift) cflags[key >> (3 * kUnitShift + 3)] = 1;
     }
-    for (int hh = 0; hh < 2; ++hh) {
-        span(8 * hh, 8 * hh + 8, f, l);
-        if (l <= f) continue;
-        if (l - f <= block_max) {
-            emit(f, l);
-            continue;
-        }
-        for (int q = 4 * hh; q < 4 * hh + 4; ++q) {
-            span(2 * q, 2 * q + 2, f, l);
-            if (l <= f) continue;
-            if (l - f <= half_max) {
-                emit(f, l);
-            } else {
-                emit(ofirst[2 * q], oend[2 * q]);
-                emit(ofirst[2 * q + 1], oend[2 * q + 1]);
-            }
-        }
-    }
+    for (unsigned s = __ballot_sync(0xffffffffu, start); s; s &= s - 1u)
+        plan_block(__shfl_sync(0xffffffffu, key, __ffs(s) - 1) >> 7, cells, tiles, ctr, block_max, half_max, big_max,
+                   lane);
+}
+
+__global__ void __launch_bounds__(256) k_density_plan(DensityArgs a, uint2 *tiles, uint32_t *ctr, uint32_t block_max,
+                                                      uint32_t half_max, uint32_t big_max) {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        a.globals[1] = (int32_t)(kDT0 * 1 / kDtMin1);  // density.metal:34-36
+    tile_plan(a.n, a.skey, a.cells, a.cflags, a.mode, tiles, ctr, block_max, half_max, big_max, [&](int p) -> uint8_t {
+        const uint32_t ind = a.cidx[p];
+        const float4 me = a.sp4[p];
+        const float h_plain = a.h[ind];
+        const bool on = a.active[ind];
+        bool seeded;
+        const float hb = fmaxf(tile_start_h(a, ind, h_plain, seeded), h_plain);
+        a.start_h[p] = hb;
+        if (!on) return kModeInactive;
+        const int m = density_mode(me.x, me.y, me.z, hb, a.coarse);
+        return m < 0 ? kModeWalk : (uint8_t)m;
+    });
 }
 
 // Coarse tiles: at the first sorted particle of every 512-cell block (2 x 2 x
@@ -796,11 +890,9 @@ struct Reach4 {
             r2 = fmaxf(r2, __shfl_xor_sync(kFull, r2, o));
         }
     }
-    // The z range, in U-units, of the row (x, y) of U-units that a sphere can
-    // reach; false when none does.
-    template <int U>
-    __device__ __forceinline__ bool row(int x, int y, int &zl, int &zh) const {
-        constexpr float w = kCellWidth * (1 << U), iw = 1.f / (kCellWidth * (1 << U));
+    // The z range of the row (x, y) of units (w wide, iw = 1 / w) that a sphere
+    // can reach; false when none does.
+    __device__ __forceinline__ bool row(int x, int y, float w, float iw, int &zl, int &zh) const {
         const float gx = fmaxf(fmaxf((float)x * w - x1, x0 - (float)(x + 1) * w) - kCellMargin, 0.f);
         const float gy = fmaxf(fmaxf((float)y * w - y1, y0 - (float)(y + 1) * w) - kCellMargin, 0.f);
         const float left = r2 - (gx * gx + gy * gy);
@@ -814,7 +906,7 @@ struct Reach4 {
 
 // One warp: the density pass of sorted particles p0 .. p0 + 3 of the staged
 // tile (lane group g = lane / 8 takes p0 + g) whose pass is U (0 cell tiles,
-// kUnitShift coarse tiles; the staged box counts U-units), in lockstep so the warp never
+// kUnitShift coarse tiles; the staged box is counted in units), in lockstep so the warp never
 // runs its groups one after another: the list build is transposed (each lane
 // takes one staged slot of a row and tests it against all four particles), and
 // the sweeps run over the longest of the four lists with the others predicated
@@ -835,13 +927,15 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
     bool live = p < end;  // the group iterates its particle (uniform within the group)
     uint32_t ind = 0u;
     float4 me = make_float4(0.f, 0.f, 0.f, 0.f), mv = me;
+    const uint8_t mode = live ? a.mode[p] : kModeInactive;
+    if (live && mode != U && (U != 0 || mode == kUnitShift)) live = false;  // another pass takes it
     if (live) {
         ind = a.cidx[p];
         me = a.sp4[p];
         mv = a.sv4[p];
-        if (!a.active[ind]) {
+        if (mode == kModeInactive) {
             // density.metal:40-55: EOS only (in the cell-tile pass)
-            if (U == 0 && sub == 0) {
+            if (sub == 0) {
                 float2 pc = eos_lookup(a.eos, a.mat[ind], a.rho[ind], a.u[ind]);
                 a.P[ind] = pc.x;
                 a.c[ind] = pc.y;
@@ -863,16 +957,14 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
     if (live) {
         h_plain = a.h[ind];
         hi = tile_start_h(a, ind, h_plain, seeded);
-        const int m = density_mode(px, py, pz, fmaxf(hi, h_plain), a.coarse);
-        if (m != U) {
-            if (U == 0 && m < 0) defer();
-            else live = false;  // another tile pass takes it
-        } else if (S.defer_all) {
-            defer();
-        }
+        if (mode != U || S.defer_all) defer();
     }
-    const int lo0 = S.box[0], lo1 = S.box[1], lo2 = S.box[2];
-    const int ny = S.box[4] - lo1 + 1, nz = S.box[5] - lo2 + 1;
+    // the staged box in its units
+    const int us = unit_shift<U>(S.box);
+    const float uw = kCellWidth * (float)(1 << us), uiw = (1.f / kCellWidth) / (float)(1 << us);
+    const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
+    const int hi0 = S.box[3] >> us, hi1 = S.box[4] >> us, hi2 = S.box[5] >> us;
+    const int ny = hi1 - lo1 + 1, nz = hi2 - lo2 + 1;
     // the group's list: staged slots within 2 hb kTileListReach
     int n_list = -1;
     float list_r2 = 0.f;
@@ -880,9 +972,9 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
         CellBox b;
         if (want) {
             tile_box(px, py, pz, hb, b);
-            b.lo0 >>= U, b.lo1 >>= U, b.lo2 >>= U, b.hi0 >>= U, b.hi1 >>= U, b.hi2 >>= U;  // U-units
-            if (!(hb < kMaxH) || b.lo0 < lo0 || b.lo1 < lo1 || b.lo2 < lo2 || b.hi0 > S.box[3] || b.hi1 > S.box[4] ||
-                b.hi2 > S.box[5]) {
+            b.lo0 >>= us, b.lo1 >>= us, b.lo2 >>= us, b.hi0 >>= us, b.hi1 >>= us, b.hi2 >>= us;
+            if (!(hb < kMaxH) || b.lo0 < lo0 || b.lo1 < lo1 || b.lo2 < lo2 || b.hi0 > hi0 || b.hi1 > hi1 ||
+                b.hi2 > hi2) {
                 defer();
                 want = false;
             }
@@ -923,7 +1015,7 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
             if (r < rows) {
                 const int x = u0 + r / nyu, y = u1 + r % nyu;
                 int zl, zh;
-                if (reach.row<U>(x, y, zl, zh)) {
+                if (reach.row(x, y, uw, uiw, zl, zh)) {
                     zl = max(zl, u2);
                     zh = min(zh, v2);
                     if (zl <= zh) {
@@ -1231,28 +1323,19 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                 // cell-tile pass, for the inactive (EOS only) and deferred ones
                 bool need = false;
                 for (uint32_t p = start + tid; p < end; p += kTileThreads) {
-                    const uint32_t ind = a.cidx[p];
-                    if (!a.active[ind]) {
-                        need |= U == 0;
-                        continue;
-                    }
-                    const float4 me = a.sp4[p];
-                    const float h_plain = a.h[ind];
-                    bool seeded;
-                    const float h0 = tile_start_h(a, ind, h_plain, seeded);
-                    const float hb = fmaxf(h0, h_plain);
-                    const int m = density_mode(me.x, me.y, me.z, hb, a.coarse);
-                    if (U == 0 && m == kUnitShift) a.cflags[a.skey[p] >> (3 * kUnitShift + 3)] = 1;
-                    need |= m == U || (U == 0 && m < 0);
+                    const uint8_t m = a.mode[p];
+                    need |= m == U || (U == 0 && m != kUnitShift);
                     if (m != U) continue;
+                    const float4 me = a.sp4[p];
+                    const float hb = a.start_h[p];
                     CellBox cb;
                     tile_box(me.x, me.y, me.z, hb, cb, fmaxf(kTileStageReach, kTileListReach));
-                    b[0] = min(b[0], cb.lo0 >> U);
-                    b[1] = min(b[1], cb.lo1 >> U);
-                    b[2] = min(b[2], cb.lo2 >> U);
-                    b[3] = max(b[3], cb.hi0 >> U);
-                    b[4] = max(b[4], cb.hi1 >> U);
-                    b[5] = max(b[5], cb.hi2 >> U);
+                    b[0] = min(b[0], cb.lo0);
+                    b[1] = min(b[1], cb.lo1);
+                    b[2] = min(b[2], cb.lo2);
+                    b[3] = max(b[3], cb.hi0);
+                    b[4] = max(b[4], cb.hi1);
+                    b[5] = max(b[5], cb.hi2);
                 }
     #pragma unroll
                 for (int k = 0; k < 3; ++k) {
@@ -1269,13 +1352,18 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                 }
             }
             __syncthreads();
-            const int lo0 = S.box[0], lo1 = S.box[1], lo2 = S.box[2];
-            const bool any = lo0 <= S.box[3];  // some particle of the tile takes the tile path
-            const int nx = any ? S.box[3] - lo0 + 1 : 0, ny = any ? S.box[4] - lo1 + 1 : 0,
-                      nz = any ? S.box[5] - lo2 + 1 : 0;
+            if (!S.need) {  // nothing in the range for this pass
+                r0 = end;
+                continue;
+            }
+            const bool any = S.box[0] <= S.box[3];  // some particle of the tile takes the tile path
+            const int us = unit_shift<U>(S.box);
+            const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
+            const int nx = any ? (S.box[3] >> us) - lo0 + 1 : 0, ny = any ? (S.box[4] >> us) - lo1 + 1 : 0,
+                      nz = any ? (S.box[5] >> us) - lo2 + 1 : 0;
             int ncell = 0;
             if (any) {
-                if (nx * ny * nz > kTileCellsMax) {
+                if (box_units(nx, ny, nz) > kTileCellsMax) {
                     if (tid == 0) S.defer_all = 1;
                 } else {
                     ncell = nx * ny * nz;
@@ -1283,18 +1371,18 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             }
             // cell counts (kTileCellsPerThread consecutive cells per thread) and
             // their exclusive scan
-            uint32_t c_cnt[kTileCellsPerThread];
+            uint32_t c_cnt[kTileCellsPerThread], c_first[kTileCellsPerThread];
             uint32_t tsum = 0u;
     #pragma unroll
             for (int k = 0; k < kTileCellsPerThread; ++k) {
                 const int c = kTileCellsPerThread * tid + k;
-                c_cnt[k] = 0u;
+                c_cnt[k] = c_first[k] = 0u;
                 if (c < ncell) {
                     const int ix = c / (ny * nz), rem = c - ix * ny * nz, iy = rem / nz, iz = rem - iy * nz;
-                    const uint2 r = unit_range<U>(a.cells, a.units, lo0 + ix, lo1 + iy, lo2 + iz);
+                    const uint2 r = unit_range(a.cells, a.octets, a.units, us, lo0 + ix, lo1 + iy, lo2 + iz);
                     if (r.x != 0xffffffffu) {
                         c_cnt[k] = r.y - r.x + 1u;
-                        S.first[c] = r.x;
+                        c_first[k] = r.x;
                     }
                 }
                 tsum += c_cnt[k];
@@ -1326,23 +1414,14 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                 continue;
             }
             if (!S.defer_all) {
-                const uint32_t total = S.off[ncell];
-                for (uint32_t s = tid; s < total; s += kTileThreads) {
-                    int lo = 0, hi = ncell - 1;  // the last cell whose first slot is <= s
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (S.off[mid] <= s) lo = mid;
-                        else hi = mid - 1;
-                    }
-                    const uint32_t g = S.first[lo] + (s - S.off[lo]);
-                    S.pos[s] = __ldg(a.sp4 + g);
-                    S.gidx[s] = g;
-                }
+                stage_units(c_cnt, c_first, inc - tsum, inc, lane, [&](uint32_t v, uint32_t g, int) {
+                    S.pos[wbase + v] = __ldg(a.sp4 + g);
+                    S.gidx[wbase + v] = g;
+                });
             }
             __syncthreads();
-            // warps take the tile's particles four at a time (none when no
-            // particle of the range needs this pass)
-            for (bool more = S.need != 0; more;) {
+            // warps take the tile's particles four at a time
+            for (bool more = true; more;) {
                 uint32_t j = 0u;
                 if (lane == 0) j = atomicAdd(&S.next, (uint32_t)kTileGpw);
                 j = __shfl_sync(0xffffffffu, j, 0);
@@ -1369,9 +1448,11 @@ struct AccelArgs {
     const uint32_t *cidx;
     const uint32_t *skey;  // sorted cell keys (tile passes)
     const uint2 *cells;
+    const uint2 *octets;   // 8-cell octet ranges and
     const uint2 *units;    // 64-cell unit ranges (coarse tiles)
     uint8_t *cflags;       // per 512-cell block: holds a coarse-tile particle
     int coarse;            // coarse tiles on
+    uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_tile_plan
     const float4 *sA, *sB, *sC;
     float4 *acc4;
     float *du, *dhdt;
@@ -1657,7 +1738,7 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L)
 
 // ---- acceleration over cell tiles (product build) ---------------------------
 //
-// The tiles of the density pass (k_tile_starts), staged the same way with the
+// The tiles of the density pass (k_density_plan), staged the same way with the
 // sA records (x, y, z, h) of the union of the tile particles' boxes of radius
 // 2 min(h, MAX_H) -- the reference's box, exact (cell_box) -- plus each staged
 // particle's cell within the staged box.  Warps take four particles at a time:
@@ -1676,7 +1757,6 @@ struct TileAccShared {
     uint32_t gidx[kTileAccStage];       // staged sorted index
     uint32_t scell[kTileAccStage];      // staged cell, box-relative (pack_cell)
     uint32_t off[kTileCellsMax + 1];
-    uint32_t first[kTileCellsMax];
     uint16_t list[kTileGroups][kTileList];
     int box[6];
     uint32_t wsum[kTileThreads / 32];
@@ -1730,10 +1810,14 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
     bool live = p < end;
     uint32_t ind = 0u;
     int idt_inactive = 0x7fffffff;
+    const uint8_t mode = live ? a.mode[p] : kModeInactive;
+    if (live && mode != U && (U != 0 || mode == kUnitShift)) live = false;  // another pass takes it
     if (live) {
         ind = a.cidx[p];
-        live = a.active[ind] != 0;
-        if (!live && U == 0) idt_inactive = inactive_ticks(a, ind);
+        if (mode == kModeInactive) {
+            idt_inactive = inactive_ticks(a, ind);
+            live = false;
+        }
     }
     float4 A = make_float4(0.f, 0.f, 0.f, 1.f), Bv = A, Cv = A;
     if (live) {
@@ -1742,19 +1826,19 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
         Cv = a.sC[p];
     }
     const AccelI I = accel_i(A, Bv, Cv);
-    const int lo0 = S.box[0], lo1 = S.box[1], lo2 = S.box[2];
-    const int ny = S.box[4] - lo1 + 1, nz = S.box[5] - lo2 + 1;
+    // the staged box in its units
+    const int us = unit_shift<U>(S.box);
+    const float uw = kCellWidth * (float)(1 << us), uiw = (1.f / kCellWidth) / (float)(1 << us);
+    const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
+    const int ny = (S.box[4] >> us) - lo1 + 1, nz = (S.box[5] >> us) - lo2 + 1;
     CellBox b;
     bool want = false;
     if (live) {
-        const int m = accel_mode(I.xi, I.yi, I.zi, I.hi, b, a.coarse);
-        if (m != U) {
-            if (U == 0 && m < 0 && sub == 0) deferred[atomicAdd(dctr, 1u)] = p;
-            live = false;  // deferred, or another tile pass takes it
-        } else if (S.defer_all) {
+        if (mode != U || S.defer_all) {
             if (sub == 0) deferred[atomicAdd(dctr, 1u)] = p;
             live = false;
         } else {
+            b = cell_box(I.xi, I.yi, I.zi, fmin_ref(I.hi, kMaxH));
             want = true;
         }
     }
@@ -1764,13 +1848,13 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
     }
     uint32_t blo = kGuards, bhi = 0u;  // the group's box, relative to the staged box
     if (want) {
-        blo = pack_cell(b.lo0 - lo0 * (1 << U), b.lo1 - lo1 * (1 << U), b.lo2 - lo2 * (1 << U));
-        bhi = pack_cell(b.hi0 - lo0 * (1 << U), b.hi1 - lo1 * (1 << U), b.hi2 - lo2 * (1 << U));
+        blo = pack_cell(b.lo0 - (lo0 << us), b.lo1 - (lo1 << us), b.lo2 - (lo2 << us));
+        bhi = pack_cell(b.hi0 - (lo0 << us), b.hi1 - (lo1 << us), b.hi2 - (lo2 << us));
     }
-    const int u0 = __reduce_min_sync(kFull, b.lo0) >> U, u1 = __reduce_min_sync(kFull, b.lo1) >> U,
-              u2 = __reduce_min_sync(kFull, b.lo2) >> U;
-    const int v0 = __reduce_max_sync(kFull, b.hi0) >> U, v1 = __reduce_max_sync(kFull, b.hi1) >> U,
-              v2 = __reduce_max_sync(kFull, b.hi2) >> U;
+    const int u0 = __reduce_min_sync(kFull, b.lo0) >> us, u1 = __reduce_min_sync(kFull, b.lo1) >> us,
+              u2 = __reduce_min_sync(kFull, b.lo2) >> us;
+    const int v0 = __reduce_max_sync(kFull, b.hi0) >> us, v1 = __reduce_max_sync(kFull, b.hi1) >> us,
+              v2 = __reduce_max_sync(kFull, b.hi2) >> us;
     if (u0 > v0) return __reduce_min_sync(kFull, idt_inactive);  // no active particle takes the tile path
     __syncwarp();
     // every accepted pair lies within 2 max(h_i, largest staged h) of the particle
@@ -1803,7 +1887,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
             // the row's z range that an accepted pair of the four can have
             const int x = u0 + r / nyu, y = u1 + r % nyu;
             int zl, zh;
-            if (reach.row<U>(x, y, zl, zh)) {
+            if (reach.row(x, y, uw, uiw, zl, zh)) {
                 zl = max(zl, u2);
                 zh = min(zh, v2);
                 if (zl <= zh) {
@@ -1902,6 +1986,17 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
     return __reduce_min_sync(kFull, idt);
 }
 
+__global__ void __launch_bounds__(256) k_acceleration_plan(AccelArgs a, uint2 *tiles, uint32_t *ctr,
+                                                           uint32_t block_max, uint32_t half_max, uint32_t big_max) {
+    tile_plan(a.n, a.skey, a.cells, a.cflags, a.mode, tiles, ctr, block_max, half_max, big_max, [&](int p) -> uint8_t {
+        const float4 A = a.sA[p];
+        if (!a.active[a.cidx[p]]) return kModeInactive;
+        CellBox b;
+        const int m = accel_mode(A.x, A.y, A.z, A.w, b, a.coarse);
+        return m < 0 ? kModeWalk : (uint8_t)m;
+    });
+}
+
 // The acceleration tile pass U over `tiles` (ctr[0] of them, ctr[1] the
 // ticket), as k_density_tile; deferred particles are counted in *dctr.
 template <bool KAHAN, int U>
@@ -1967,22 +2062,17 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                 // the step) and deferred ones
                 bool need = false;
                 for (uint32_t p = start + tid; p < end; p += kTileThreads) {
-                    if (!a.active[a.cidx[p]]) {
-                        need |= U == 0;
-                        continue;
-                    }
-                    const float4 A = a.sA[p];
-                    CellBox cb;
-                    const int m = accel_mode(A.x, A.y, A.z, A.w, cb, a.coarse);
-                    if (U == 0 && m == kUnitShift) a.cflags[a.skey[p] >> (3 * kUnitShift + 3)] = 1;
-                    need |= m == U || (U == 0 && m < 0);
+                    const uint8_t m = a.mode[p];
+                    need |= m == U || (U == 0 && m != kUnitShift);
                     if (m != U) continue;
-                    b[0] = min(b[0], cb.lo0 >> U);
-                    b[1] = min(b[1], cb.lo1 >> U);
-                    b[2] = min(b[2], cb.lo2 >> U);
-                    b[3] = max(b[3], cb.hi0 >> U);
-                    b[4] = max(b[4], cb.hi1 >> U);
-                    b[5] = max(b[5], cb.hi2 >> U);
+                    const float4 A = a.sA[p];
+                    const CellBox cb = cell_box(A.x, A.y, A.z, fmin_ref(A.w, kMaxH));
+                    b[0] = min(b[0], cb.lo0);
+                    b[1] = min(b[1], cb.lo1);
+                    b[2] = min(b[2], cb.lo2);
+                    b[3] = max(b[3], cb.hi0);
+                    b[4] = max(b[4], cb.hi1);
+                    b[5] = max(b[5], cb.hi2);
                 }
     #pragma unroll
                 for (int k = 0; k < 3; ++k) {
@@ -1999,32 +2089,37 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                 }
             }
             __syncthreads();
-            const int lo0 = S.box[0], lo1 = S.box[1], lo2 = S.box[2];
-            const bool any = lo0 <= S.box[3];
-            const int nx = any ? S.box[3] - lo0 + 1 : 0, ny = any ? S.box[4] - lo1 + 1 : 0,
-                      nz = any ? S.box[5] - lo2 + 1 : 0;
+            if (!S.need) {  // nothing in the range for this pass
+                r0 = end;
+                continue;
+            }
+            const bool any = S.box[0] <= S.box[3];
+            const int us = unit_shift<U>(S.box);
+            const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
+            const int nx = any ? (S.box[3] >> us) - lo0 + 1 : 0, ny = any ? (S.box[4] >> us) - lo1 + 1 : 0,
+                      nz = any ? (S.box[5] >> us) - lo2 + 1 : 0;
             int ncell = 0;
             if (any) {
                 // (pack_cell's range: such a box holds particles of cells that
                 // are only alike modulo the grid)
-                if (nx * ny * nz > kTileCellsMax || max(nx, max(ny, nz)) > (kBoxCellsMax >> U)) {
+                if (box_units(nx, ny, nz) > kTileCellsMax || max(nx, max(ny, nz)) > (kBoxCellsMax >> us)) {
                     if (tid == 0) S.defer_all = 1;
                 } else {
                     ncell = nx * ny * nz;
                 }
             }
-            uint32_t c_cnt[kTileCellsPerThread];
+            uint32_t c_cnt[kTileCellsPerThread], c_first[kTileCellsPerThread];
             uint32_t tsum = 0u;
     #pragma unroll
             for (int k = 0; k < kTileCellsPerThread; ++k) {
                 const int c = kTileCellsPerThread * tid + k;
-                c_cnt[k] = 0u;
+                c_cnt[k] = c_first[k] = 0u;
                 if (c < ncell) {
                     const int ix = c / (ny * nz), rem = c - ix * ny * nz, iy = rem / nz, iz = rem - iy * nz;
-                    const uint2 r = unit_range<U>(a.cells, a.units, lo0 + ix, lo1 + iy, lo2 + iz);
+                    const uint2 r = unit_range(a.cells, a.octets, a.units, us, lo0 + ix, lo1 + iy, lo2 + iz);
                     if (r.x != 0xffffffffu) {
                         c_cnt[k] = r.y - r.x + 1u;
-                        S.first[c] = r.x;
+                        c_first[k] = r.x;
                     }
                 }
                 tsum += c_cnt[k];
@@ -2057,36 +2152,30 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             }
             float hmax = 0.f;
             if (!S.defer_all) {
-                const uint32_t total = S.off[ncell];
-                for (uint32_t s = tid; s < total; s += kTileThreads) {
-                    int lo = 0, hi = ncell - 1;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) >> 1;
-                        if (S.off[mid] <= s) lo = mid;
-                        else hi = mid - 1;
-                    }
-                    const uint32_t gi = S.first[lo] + (s - S.off[lo]);
-                    const float4 q = __ldg(a.sA + gi);
-                    S.pos[s] = q;
-                    S.gidx[s] = gi;
-                    int ix = lo / (ny * nz), rem = lo - ix * ny * nz, iy = rem / nz, iz = rem - iy * nz;
+                stage_units(c_cnt, c_first, inc - tsum, inc, lane, [&](uint32_t v, uint32_t g, int c) {
+                    const float4 q = __ldg(a.sA + g);
+                    c += kTileCellsPerThread * (tid - lane);
+                    int ix = c / (ny * nz), rem = c - ix * ny * nz, iy = rem / nz, iz = rem - iy * nz;
                     if (U > 0) {
-                        // the particle's cell within its unit: the low 3U bits of its key
-                        const uint32_t key = a.skey[gi];
+                        // the particle's cell within its unit: the low bits of its key
+                        const uint32_t key = a.skey[g];
                         int dx = 0, dy = 0, dz = 0;
 #pragma unroll
-                        for (int bit = 0; bit < U; ++bit) {
+                        for (int bit = 0; bit < kUnitShift; ++bit) {
                             dx |= (int)((key >> (3 * bit)) & 1u) << bit;
                             dy |= (int)((key >> (3 * bit + 1)) & 1u) << bit;
                             dz |= (int)((key >> (3 * bit + 2)) & 1u) << bit;
                         }
-                        ix = (ix << U) | dx;
-                        iy = (iy << U) | dy;
-                        iz = (iz << U) | dz;
+                        const int low = (1 << us) - 1;
+                        ix = (ix << us) | (dx & low);
+                        iy = (iy << us) | (dy & low);
+                        iz = (iz << us) | (dz & low);
                     }
-                    S.scell[s] = pack_cell(ix, iy, iz);
+                    S.pos[wbase + v] = q;
+                    S.gidx[wbase + v] = g;
+                    S.scell[wbase + v] = pack_cell(ix, iy, iz);
                     hmax = fmaxf(hmax, q.w);
-                }
+                });
             }
             {
                 float v = hmax;
@@ -2096,7 +2185,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             }
             __syncthreads();
             int wmin = 0x7fffffff;
-            for (bool more = S.need != 0; more;) {  // none when no particle of the range needs this pass
+            for (bool more = true; more;) {
                 uint32_t j = 0u;
                 if (lane == 0) j = atomicAdd(&S.next, (uint32_t)kTileGpw);
                 j = __shfl_sync(0xffffffffu, j, 0);
@@ -2317,9 +2406,12 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     a.cidx = cidx;
     a.skey = ctx->cell_sort.keys[ctx->cell_final];
     a.cells = ctx->cell_range;
+    a.octets = ctx->octets;
     a.units = ctx->units;
     a.cflags = ctx->coarse_flags;
     a.coarse = ctx->tile_coarse;
+    a.mode = ctx->tile_mode;
+    a.start_h = ctx->tile_h;
     a.sp4 = ctx->sp4;
     a.sv4 = ctx->sv4;
     a.h = ctx->h;
@@ -2365,8 +2457,8 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     const int sms = tile_smem_opt_in();
     uint32_t *ctr = ctx->tile_ctr;
     cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * 8, st);
-    k_tile_starts<<<(n + 255) / 256, 256, 0, st>>>(n, a.skey, ctx->cell_range, ctx->tiles, ctr, ctx->globals,
-                                                   ctx->tile_block_max, ctx->tile_half_max, ctx->tile_big_max);
+    k_density_plan<<<(n + 255) / 256, 256, 0, st>>>(a, ctx->tiles, ctr, ctx->tile_block_max, ctx->tile_half_max,
+                                                    ctx->tile_big_max);
     const unsigned tgrid = tile_grid(n, sms);
     k_density_tile<0><<<tgrid, kTileThreads, sizeof(TileShared), st>>>(a, ctx->tiles, ctr, ctx->deferred, ctr + 2);
     if (a.coarse) {
@@ -2391,9 +2483,11 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     a.cidx = ctx->cell_sort.vals[ctx->cell_final];
     a.skey = ctx->cell_sort.keys[ctx->cell_final];
     a.cells = ctx->cell_range;
+    a.octets = ctx->octets;
     a.units = ctx->units;
     a.cflags = ctx->coarse_flags;
     a.coarse = ctx->tile_coarse;
+    a.mode = ctx->tile_mode;
     a.sA = ctx->sA;
     a.sB = ctx->sB;
     a.sC = ctx->sC;
@@ -2420,8 +2514,8 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     const int sms = tile_smem_opt_in();
     uint32_t *ctr = ctx->tile_ctr + 8;
     cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * 8, st);
-    k_tile_starts<<<(n + 255) / 256, 256, 0, st>>>(n, a.skey, ctx->cell_range, ctx->tiles, ctr, nullptr,
-                                                   ctx->tile_block_max, ctx->tile_half_max, ctx->tile_big_max);
+    k_acceleration_plan<<<(n + 255) / 256, 256, 0, st>>>(a, ctx->tiles, ctr, ctx->tile_block_max,
+                                                         ctx->tile_half_max, ctx->tile_big_max);
     const unsigned tgrid = tile_grid(n, sms);
     const size_t tsm = sizeof(TileAccShared);
     if (kahan)

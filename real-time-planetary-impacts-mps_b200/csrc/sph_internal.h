@@ -173,6 +173,8 @@ struct sph_ctx {
     uint2 *tiles = nullptr;
     uint32_t *tile_ctr = nullptr;
     uint32_t *deferred = nullptr;
+    uint8_t *tile_mode = nullptr;  // [n] the pass that takes each sorted particle
+    float *tile_h = nullptr;       // [n] density: the h its staged box is built for
     // tile sizes: a 128-cell block is one tile up to tile_big_max particles
     // (0: never; measured slower at N = 1e6: such tiles overflow shared memory
     // and fall back to octets), else its 64-cell halves up to tile_block_max,
@@ -187,6 +189,7 @@ struct sph_ctx {
     // and cleared when the coarse tiles are listed.  tile_coarse 0 hands
     // those particles to the per-particle pass instead.
     uint2 *units = nullptr;
+    uint2 *octets = nullptr;  // the same per 8-cell octet (cell key >> 3)
     uint8_t *coarse_flags = nullptr;
     int tile_coarse = 1;
     float2 *eos_forsterite = nullptr, *eos_fe = nullptr;

@@ -46,12 +46,12 @@ constexpr int kHashBlocks = 296;
 int hash_grid(int n) { return std::max(1, std::min(kHashBlocks, (n + kHashThreads - 1) / kHashThreads)); }
 
 // Keys of the cell grid + all three digit histograms; clears the previous
-// sort's occupied cells and units first (they are read from the previous
+// sort's occupied cells, octets and units first (they are read from the previous
 // sorted keys, which live in the buffer the first pass is about to overwrite).
 __global__ void __launch_bounds__(kHashThreads)
     k_hash_hist(const float4 *__restrict__ pos4, int n, uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
                 uint32_t *__restrict__ hist, const uint32_t *__restrict__ prev_keys, uint2 *__restrict__ cell_range,
-                uint2 *__restrict__ units, int clear_prev) {
+                uint2 *__restrict__ octets, uint2 *__restrict__ units, int clear_prev) {
     __shared__ uint32_t sh[3][256];
     for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x) (&sh[0][0])[i] = 0u;
     __syncthreads();
@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(kHashThreads)
         if (clear_prev) {
             const uint32_t pk = prev_keys[i], before = i ? prev_keys[i - 1] : ~pk;
             if (before != pk) cell_range[pk] = make_uint2(0xffffffffu, 0u);
+            if ((before ^ pk) >> 3) octets[pk >> 3] = make_uint2(0xffffffffu, 0xffffffffu);
             if ((before ^ pk) >> (3 * kUnitShift)) units[pk >> (3 * kUnitShift)] = make_uint2(0xffffffffu, 0xffffffffu);
         }
         const float4 p = __ldg(pos4 + i);
@@ -213,16 +214,18 @@ void launch_onesweep(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t 
                                                     counter, health, spin_limit);
 }
 
-// Each occupied cell's (first, last) sorted index, and each occupied unit's
-// (cell key >> 6).
+// Each occupied cell's (first, last) sorted index, and each occupied octet's
+// (cell key >> 3) and unit's (cell key >> 6).
 __global__ void k_cells(const uint32_t *__restrict__ keys, int n, uint2 *__restrict__ cell_range,
-                        uint2 *__restrict__ units) {
+                        uint2 *__restrict__ octets, uint2 *__restrict__ units) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t k = keys[i], u = k >> (3 * kUnitShift);
     const uint32_t before = i ? keys[i - 1] : ~k, after = i < n - 1 ? keys[i + 1] : ~k;
     if (before != k) cell_range[k].x = (uint32_t)i;
     if (after != k) cell_range[k].y = (uint32_t)i;
+    if ((before ^ k) >> 3) octets[k >> 3].x = (uint32_t)i;
+    if ((after ^ k) >> 3) octets[k >> 3].y = (uint32_t)i;
     if ((before >> (3 * kUnitShift)) != u) units[u].x = (uint32_t)i;
     if ((after >> (3 * kUnitShift)) != u) units[u].y = (uint32_t)i;
 }
@@ -280,6 +283,7 @@ int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t 
 
 void launch_init_cells(sph_ctx *ctx, cudaStream_t st) {
     k_init_cells<<<148 * 8, 256, 0, st>>>(ctx->cell_range, kNumCells);
+    cudaMemsetAsync(ctx->octets, 0xff, sizeof(uint2) * kNumOctets, st);
     cudaMemsetAsync(ctx->units, 0xff, sizeof(uint2) * kNumUnits, st);
     ctx->cells_have_prev = false;
 }
@@ -298,11 +302,11 @@ sph_status launch_sort(sph_ctx *ctx, cudaStream_t st) {
         launch_init_cells(ctx, st);
     }
     k_hash_hist<<<hash_grid(n), kHashThreads, 0, st>>>(ctx->pos4, n, s.keys[0], s.vals[0], s.hist, clear_src,
-                                                       ctx->cell_range, ctx->units,
+                                                       ctx->cell_range, ctx->octets, ctx->units,
                                                        (ctx->cells_have_prev && prev == 1) ? 1 : 0);
     int fin = radix_sort_pairs(s, n, 24, st, ctx->health);
     ctx->cell_final = fin;
-    k_cells<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->cell_range, ctx->units);
+    k_cells<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->cell_range, ctx->octets, ctx->units);
     ctx->cells_have_prev = true;
     return cuda_status(cudaGetLastError(), "sort");
 }

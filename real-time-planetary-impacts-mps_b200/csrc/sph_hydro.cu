@@ -77,6 +77,12 @@ constexpr int kLanesPerParticle = 1;
 #endif
 constexpr int kLanesPerParticle = SPH_HYDRO_LANES;
 #endif
+// Lanes per particle of the deferred particles' walk, a whole warp: its cost
+// is the walk over the thousands of cells of a box that no tile can hold, one
+// look-up per lane at a time, and a few particles at the end of a pass are
+// nothing but latency (N = 2e4, 3 particles: the density pass 434 us
+// with 8 lanes a particle, 278 with 32).
+constexpr int kWalkLanes = 32;
 
 // Squared distance from (px, py, pz) to the box of cell (x, y, z), each axis
 // gap shortened by the margin.
@@ -2446,9 +2452,10 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     if (s != SPH_OK) return s;
     a.nn_out = ctx->hs.nn;
     a.stats = ctx->hs.stats;
-    constexpr int parts = parts_per_block<kLanesPerParticle>();
     const size_t smem = list_smem_opt_in();
+    static_assert(parts_per_block<kWalkLanes>() <= parts_per_block<kLanesPerParticle>(), "the lists' shared memory");
 #ifdef SPH_PARITY
+    constexpr int parts = parts_per_block<kLanesPerParticle>();
     // one lane per particle, in the reference's order
     k_density<kLanesPerParticle><<<(unsigned)((n + parts - 1) / parts), parts * kLanesPerParticle, smem, st>>>(a);
 #else
@@ -2467,8 +2474,8 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
         k_density_tile<kUnitShift>
             <<<tgrid, kTileThreads, sizeof(TileShared), st>>>(a, ctx->tiles, ctr + 4, ctx->deferred, ctr + 2);
     }
-    k_density_deferred<kLanesPerParticle><<<tgrid * 4, parts * kLanesPerParticle, smem, st>>>(a, ctx->deferred,
-                                                                                           ctr + 2);
+    k_density_deferred<kWalkLanes><<<tgrid * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(
+        a, ctx->deferred, ctr + 2);
 #endif
     if (ctx->hs.capture) s = launch_hseed_targets(ctx, st);
     if (s != SPH_OK) return s;
@@ -2498,10 +2505,10 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     a.active = ctx->active;
     a.globals = ctx->globals;
     a.individual = ctx->form.timestep == SPH_TIMESTEP_INDIVIDUAL;
-    constexpr int parts = parts_per_block<kLanesPerParticle>();
     const size_t smem = list_smem_opt_in();
     const bool kahan = ctx->form.precision == SPH_PRECISION_MIXED;
 #ifdef SPH_PARITY
+    constexpr int parts = parts_per_block<kLanesPerParticle>();
     // one lane per particle, in the reference's order
     const unsigned blocks = (unsigned)((n + parts - 1) / parts);
     if (kahan)
@@ -2533,11 +2540,11 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
                 <<<tgrid, kTileThreads, tsm, st>>>(a, ctx->tiles, ctr + 4, ctx->deferred, ctr + 2);
     }
     if (kahan)
-        k_acceleration_deferred<kLanesPerParticle, true>
-            <<<tgrid * 4, parts * kLanesPerParticle, smem, st>>>(a, ctx->deferred, ctr + 2);
+        k_acceleration_deferred<kWalkLanes, true>
+            <<<tgrid * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(a, ctx->deferred, ctr + 2);
     else
-        k_acceleration_deferred<kLanesPerParticle, false>
-            <<<tgrid * 4, parts * kLanesPerParticle, smem, st>>>(a, ctx->deferred, ctr + 2);
+        k_acceleration_deferred<kWalkLanes, false>
+            <<<tgrid * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(a, ctx->deferred, ctr + 2);
 #endif
     return cuda_status(cudaGetLastError(), "acceleration");
 }

@@ -84,3 +84,24 @@ def test_reference_gravity_matches_the_parity_build(cuda, pkg, n, leaf, depth, u
     # (tests/test_fp_sensitivity.py); its moments are taken 318 Mm from the origin
     assert e.max() <= 1.2e-2 and np.median(e) <= 2e-4
     assert np.array_equal(got[0][1], got[1][1])
+
+
+# odd counts of staged nodes and particles, groups that are not full, and pairs
+# inside the softening
+@pytest.mark.parametrize("n,leaf,side", [(1, 4, 10.0), (2, 1, 0.05), (31, 4, 10.0), (33, 32, 0.3), (65, 1, 10.0),
+                                         (1001, 16, 1.0), (5003, 7, 10.0)])
+def test_opening_angle_gravity_matches_the_direct_sum(cuda, pkg, n, leaf, side):
+    ic = pkg.ic.make_cube(n, seed=n, side=side)
+    with pkg.Compute(ic, max_children_in_leaf=leaf, max_tree_depth=10) as c:
+        c.set_form(gravity="theta", theta=0.2)
+        c.gravitationalPass()
+        c.synchronize()
+        acc, phi, gn = c.download("acc").astype(np.float64), c.download("potential"), c.download("grav_norm")
+        ref = c.gravity_direct_f64(np.arange(n))
+        assert c.health() == 0
+    scale = np.sqrt(np.mean(ref[:, :3] ** 2)) + 1e-30
+    # theta = 0.2: the octupole left out is below theta^3 / 8 = 1e-3 of a node's
+    # force, and nodes' errors do not add up
+    assert np.max(np.linalg.norm(acc - ref[:, :3], axis=1)) <= 1e-3 * scale * np.sqrt(3.0)
+    assert np.max(np.abs(phi - ref[:, 3])) <= 1e-4 * np.max(np.abs(ref[:, 3]))
+    assert np.allclose(gn * 6.67e-5, np.linalg.norm(acc, axis=1), rtol=1e-5)

@@ -316,7 +316,8 @@ sph_status sph_destroy(sph_ctx *ctx) {
                     ctx->health, ctx->cell_range, ctx->sp4, ctx->sv4, ctx->sA, ctx->sB, ctx->sC,
                     ctx->eos_forsterite, ctx->eos_fe, ctx->stage, ctx->snapshot, ctx->pos64, ctx->dglob,
                     ctx->diag, ctx->tiles, ctx->tile_ctr, ctx->deferred, ctx->units, ctx->coarse_flags,
-                    ctx->tile_mode, ctx->tile_h, ctx->octets};
+                    ctx->tile_mode, ctx->tile_h, ctx->octets,
+                    ctx->nlist, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     for (void *b : bufs) cudaFree(b);
     sort_free(ctx->cell_sort);
     hseed_free(ctx);
@@ -397,6 +398,9 @@ sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out)
     chk(dmalloc(&ctx->deferred, (size_t)n));
     chk(dmalloc(&ctx->tile_mode, (size_t)n));
     chk(dmalloc(&ctx->tile_h, (size_t)n));
+    chk(dmalloc(&ctx->nlist_count, (size_t)n));
+    chk(dmalloc(&ctx->nlist_reach2, (size_t)n));
+    chk(dmalloc(&ctx->grown, (size_t)kNumUnits));
     chk(dmalloc(&ctx->units, (size_t)kNumUnits));
     chk(dmalloc(&ctx->octets, (size_t)kNumOctets));
     chk(dmalloc(&ctx->coarse_flags, (size_t)kNumCoarseBlocks));
@@ -420,6 +424,14 @@ sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out)
         sph_destroy(ctx);
         return s;
     }
+    // the neighbour lists (640 B a particle) are worth their storage but not
+    // needed: without it the acceleration pass looks for the neighbours again
+    if (dmalloc(&ctx->nlist, neighbour_list_entries(n)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->nlist = nullptr;
+    }
+    if (e == cudaSuccess) e = cudaMemset(ctx->nlist_count, 0xff, (size_t)n);
+    if (e == cudaSuccess) e = cudaMemset(ctx->grown, 0, sizeof(int) * kNumUnits);
     // EOS tables and the derived lookup constants (density.metal:45-46)
     chk(cudaMemcpy(ctx->eos_forsterite, tf.data(), sizeof(float) * tf.size(), cudaMemcpyHostToDevice));
     chk(cudaMemcpy(ctx->eos_fe, te.data(), sizeof(float) * te.size(), cudaMemcpyHostToDevice));

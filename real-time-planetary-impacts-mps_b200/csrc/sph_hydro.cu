@@ -42,7 +42,7 @@ __device__ __forceinline__ float pair_sqrt(float r2) {
 #ifdef SPH_PARITY
     return sqrtf(r2);
 #else
-    return r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
+    return r2 > 1e-30f ? r2 * rsqrt_hw(r2) : 0.f;
 #endif
 }
 
@@ -53,7 +53,7 @@ __device__ __forceinline__ float pair_rinv(float r2, float r) {
     return 1.f / r;
 #else
     (void)r;
-    return rsqrtf(r2);
+    return rsqrt_hw(r2);
 #endif
 }
 
@@ -63,7 +63,7 @@ __device__ __forceinline__ float pdiv(float a, float b) {
 #ifdef SPH_PARITY
     return a / b;
 #else
-    return __fdividef(a, b);
+    return a * rcp_hw(b);
 #endif
 }
 
@@ -265,6 +265,22 @@ __device__ __forceinline__ int group_collect(float px, float py, float pz, float
     return cnt;
 }
 
+// Neighbour lists that the density tiles leave for the acceleration pass, so
+// that it need not look for the same neighbours again.  A particle's list
+// holds every particle within 2 kTileListReach x max(its h, the other's h),
+// the h at the start of the density pass (the last h a list was built for, its
+// own), as far as its box of cells reaches: all pairs the acceleration pass can
+// accept, unless a neighbour's h has outgrown its start by more than
+// kTileListReach: the largest such h is kept per 64-cell unit in `grown`, and a
+// particle's list is complete as long as that h reaches no further than it.
+struct NeighbourLists {
+    uint32_t *entries;  // [n][kTileList] sorted indices
+    uint8_t *count;     // [n], kNoList: none
+    float *reach2;      // [n] everything within this squared distance is listed
+    int *grown;         // [units] float bits, 0: none
+};
+constexpr uint8_t kNoList = 0xff;
+
 struct DensityArgs {
     int n;
     const uint32_t *cidx;
@@ -274,8 +290,9 @@ struct DensityArgs {
     const uint2 *units;    // 64-cell unit ranges (coarse tiles)
     uint8_t *cflags;       // per 512-cell block: holds a coarse-tile particle
     int coarse;            // coarse tiles on
-    uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_tile_plan
-    float *start_h;        // [n] the h its staged box is built for, written by k_tile_plan
+    uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_density_plan
+    float *start_h;        // [n] the h its staged box is built for, written by k_density_plan
+    NeighbourLists lists;  // out, for the acceleration pass
     const float4 *sp4, *sv4;
     float *h, *rho, *f, *P, *c, *B;
     const float *u;
@@ -307,6 +324,8 @@ constexpr int kListMax = 192;       // list entries per particle
 template <int L>
 __host__ __device__ constexpr int parts_per_block() { return 16 * L >= 32 ? 16 : 32 / L; }
 constexpr float kListReach = 1.15f; // list radius / (2 h)
+
+__device__ __forceinline__ void mark_grown(const DensityArgs &a, uint32_t p, float h);
 
 // density.metal:12-239 for one sorted particle per lane group.  The group
 // keeps the reference's per-particle iteration state (h, the int max_h, the
@@ -515,6 +534,9 @@ __device__ __forceinline__ void density_particle(const DensityArgs &a, int index
     float fi = 1.f / (1.f + (hi / (3.f * dens)) * dens_h);
     float2 pc = eos_lookup(a.eos, a.mat[ind], dens, a.u[ind]);
     float bal = vdiv / (vdiv + acurl + 1e-4f * (pc.y / hi));
+#ifndef SPH_PARITY
+    mark_grown(a, (uint32_t)index, hi);
+#endif
     a.h[ind] = hi;
     a.rho[ind] = dens;
     a.f[ind] = fi;
@@ -559,67 +581,85 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L)
     }
 }
 
-// ---- density over cell tiles (product build) --------------------------------
+// ---- density over neighbour lists (product build) ---------------------------
 //
-// A tile is an aligned Morton block of cells -- 64 cells (4 x 4 x 4), or, where
-// such a block holds many particles, its 16-cell halves of halves or its
-// octets -- so its particles are one contiguous run of the sorted order.  A CTA
-// takes tiles from a ticket counter; per tile it stages, once, every particle
-// of the box of cells that the tile's neighbour lists can reach (float4
-// position + mass and the sorted index) into shared memory, in cell order
-// x-major, then y, z innermost, so a row of cells along z is one contiguous
-// run of staged slots.  Warps then take the tile's particles four at a time
-// (density_tile_warp): the list build reads the particles' rows of the staged
-// box, every h-iteration sweep reads the list, and no sweep touches the cell
-// table or global positions again.  A particle whose list box reaches more
-// than kTileReach cells beyond its own cell, whose h is at least
-// MAX_SMOOTHING_LENGTH (where the reference's neighbour cache comes into play),
-// whose list overflows or whose growing h leaves the staged box is handed to
-// k_density_deferred, which runs the per-particle walk above; so is every
-// particle of a tile whose box exceeds the shared-memory budget.
-constexpr int kTileThreads = 384;
+// k_lists finds every particle's neighbours over tiles: a tile is an aligned
+// Morton block of cells -- 64 cells (4 x 4 x 4), or, where such a block holds
+// many particles, its 16-cell quarters or its octets -- so its particles are
+// one contiguous run of the sorted order.  A CTA takes tiles from a ticket
+// counter; per tile it stages, once, every particle of the box of cells that
+// the tile's lists can reach (position, sorted index, starting h) into shared
+// memory, in cell order x-major, then y, z innermost, so a row of cells along z
+// is one contiguous run of staged slots.  Warps then take the tile's particles
+// four at a time (lists_tile_warp) and write their lists.
+//
+// k_density_list iterates h from the lists alone, eight lanes a particle: the
+// distances and masses stay in registers through the sweeps, and no sweep
+// touches memory.  The acceleration pass reads the same lists.  (Search and
+// iteration were one kernel, whose registers and shared memory left room for
+// 24 warps per SM and whose 77 KB of code did not fit the instruction caches:
+// N = 1e6, 3.05 ms the pass; the two kernels 2.02.)
+//
+// A particle whose list box reaches more than kTileReach units beyond its own,
+// whose h is at least MAX_SMOOTHING_LENGTH (where the reference's neighbour
+// cache comes into play), whose list overflows or whose growing h leaves its
+// list is handed to k_density_deferred, which runs the per-particle walk above;
+// so is every particle of a tile whose box exceeds the shared-memory budget.
 #ifndef SPH_TILE_LANES
 #define SPH_TILE_LANES 8
 #endif
 constexpr int kTileLanes = SPH_TILE_LANES;                  // lanes per particle
 constexpr int kTileGpw = 32 / kTileLanes;                   // particles per warp
-constexpr int kTileGroups = kTileThreads / kTileLanes;      // particles in flight per CTA
-constexpr int kTileStageMax = 3840;                         // staged particles per tile
-constexpr int kTileCellsMax = 1024;                         // cells of a tile's staged box
-constexpr int kTileCellsPerThread = (kTileCellsMax + kTileThreads - 1) / kTileThreads;
+constexpr int kTileCellsMax = 1024;                         // units of a tile's staged box
 #ifndef SPH_TILE_REACH_CELLS
 #define SPH_TILE_REACH_CELLS 3
 #endif
-constexpr int kTileReach = SPH_TILE_REACH_CELLS;            // cells a list box may extend past its own cell
-constexpr int kTileList = 256;                              // list entries per particle (staged slots)
+constexpr int kTileReach = SPH_TILE_REACH_CELLS;            // units a list box may extend past its own
+constexpr int kTileList = 160;                              // list entries per particle
 #ifndef SPH_TILE_LIST_REACH
-#define SPH_TILE_LIST_REACH 1.05f
+#define SPH_TILE_LIST_REACH 1.08f
 #endif
-constexpr float kTileListReach = SPH_TILE_LIST_REACH;       // list radius / (2 h)
-#ifndef SPH_TILE_STAGE_REACH
-#define SPH_TILE_STAGE_REACH 1.15f
-#endif
-// staged box radius / (2 h): room for h to grow before a list rebuild leaves
-// the staged box
-constexpr float kTileStageReach = SPH_TILE_STAGE_REACH;
-
+// list radius / (2 h), for the h that k_density_plan expects: a list costs as
+// much as several sweeps, and a particle whose h outgrows it is walked for on
+// its own
+constexpr float kTileListReach = SPH_TILE_LIST_REACH;
+// staged box radius / (2 h): room for the second, wider search of a particle
+// that finds too few neighbours
+constexpr float kTileStageReach = 1.25f;
+// neighbours within 2 kTileListReach h of a particle at its fixed point,
+// 4/3 pi (2 RESOLUTION_ETA kTileListReach)^3
+constexpr float kListFull = 4.18879f * 8.f * kResolutionEta * kResolutionEta * kResolutionEta * kTileListReach *
+                            kTileListReach * kTileListReach;
 // Neighbours a particle's lanes keep in registers, as pairs per lane, through
-// the sweeps of its iteration; longer lists are read from shared memory in
-// every sweep.
-constexpr int kRegPairs = 7;
-constexpr int kRegList = 2 * kRegPairs * kTileLanes;        // 112 (a list holds ~75)
+// the sweeps of its iteration; longer lists are read again in every sweep.
+constexpr int kRegPairs = 6;
+constexpr int kRegList = 2 * kRegPairs * kTileLanes;        // 96 (a list holds ~85)
 
-struct TileShared {
-    float4 pos[kTileStageMax];          // staged (x, y, z, m)
-    uint32_t gidx[kTileStageMax];       // staged sorted index
-    uint32_t off[kTileCellsMax + 1];    // first staged slot of each box cell; off[cells] = staged count
-    uint16_t list[kTileGroups][kTileList];
-    int box[6];                         // staged box: lo x y z, hi x y z (unwrapped cell coordinates)
-    uint32_t wsum[kTileThreads / 32];
+// CTAs of the tile passes.  Cell tiles: three of 320 threads fill an SM's
+// registers (64 each) and shared memory.  Coarse tiles stage more per particle,
+// and one that overflows is taken again unit by unit, a few particles at a
+// time: two larger CTAs (N = 1e5, whose boxes are mostly coarse, two steps: 2032
+// us with the cell tiles' shape, 1791 with this; the cell tiles with this shape
+// 2.18 ms at N = 1e6 instead of 2.02).
+template <int U>
+struct ListTile {
+    static constexpr int kThreads = U == 0 ? 320 : 512;
+    static constexpr int kCtas = U == 0 ? 3 : 2;      // per SM
+    static constexpr int kStage = U == 0 ? 2944 : 4096;  // staged particles
+};
+template <int U>
+struct ListShared {
+    float4 pos[ListTile<U>::kStage];       // staged (x, y, z, m)
+    uint32_t gidx[ListTile<U>::kStage];    // staged sorted index
+    float hs[ListTile<U>::kStage];         // staged starting h
+    uint32_t off[kTileCellsMax + 1];       // first staged slot of each box unit; off[units] = staged count
+    int box[6];                            // staged box: lo x y z, hi x y z (unwrapped cell coordinates)
+    int hmax_bits;                         // largest staged starting h (float bits; h > 0)
+    uint32_t wsum[ListTile<U>::kThreads / 32];
+    uint32_t rows[ListTile<U>::kThreads / 32][32];  // each warp's rows: staged slot minus flat index
     uint32_t start, end, tile, next;
-    uint32_t stats[4];
     int defer_all;
-    int need;                           // some particle of the range needs the warp pass
+    int need;                              // some particle of the range needs the warp pass
 };
 
 // The list box of a tile particle at smoothing length hb: the cells within
@@ -643,6 +683,14 @@ __device__ __forceinline__ void tile_box(float px, float py, float pz, float hb,
 // are only alike modulo the grid can span thousands of cells).
 __device__ __forceinline__ int64_t box_units(int nx, int ny, int nz) {
     return (int64_t)min(nx, 1 << 20) * min(ny, 1 << 20) * min(nz, 1 << 20);
+}
+
+// The particle's h is final: note it when the lists of its neighbours may lack
+// it (a little early, for the rounding of the lists' squared reach; NaN counts
+// as grown).
+__device__ __forceinline__ void mark_grown(const DensityArgs &a, uint32_t p, float h) {
+    if (!(h <= (kTileListReach - 1e-4f) * a.start_h[p]))
+        atomicMax(a.lists.grown + (a.skey[p] >> (3 * kUnitShift)), __float_as_int(h));
 }
 
 // Tiling units of the staged box: cells (shift 0, the cell tiles), 2 x 2 x 2
@@ -694,14 +742,13 @@ __device__ __forceinline__ int density_mode(float px, float py, float pz, float 
 }
 
 // Staging: a warp copies the particles of its lanes' units (cnt and first of
-// kTileCellsPerThread consecutive units per lane), which are consecutive
+// PER consecutive units per lane), which are consecutive
 // staged slots from the warp's first: 32 slots at a time, each lane finding the
 // lane and unit its slot belongs to, so that a unit with many particles is
 // shared out.  excl, incl: the lane's slots within the warp.  copy(slot
 // within the warp's, sorted index, unit counted from the warp's first).
-template <class Copy>
-__device__ __forceinline__ void stage_units(const uint32_t (&cnt)[kTileCellsPerThread],
-                                            const uint32_t (&first)[kTileCellsPerThread], uint32_t excl,
+template <int PER, class Copy>
+__device__ __forceinline__ void stage_units(const uint32_t (&cnt)[PER], const uint32_t (&first)[PER], uint32_t excl,
                                             uint32_t incl, int lane, Copy &&copy) {
     constexpr unsigned kFull = 0xffffffffu;
     const uint32_t total = __shfl_sync(kFull, incl, 31);
@@ -719,12 +766,12 @@ __device__ __forceinline__ void stage_units(const uint32_t (&cnt)[kTileCellsPerT
         int unit = 0;
         bool found = false;
 #pragma unroll
-        for (int k = 0; k < kTileCellsPerThread; ++k) {
+        for (int k = 0; k < PER; ++k) {
             const uint32_t c = __shfl_sync(kFull, cnt[k], j), f = __shfl_sync(kFull, first[k], j);
             if (!found) {
                 if (at < c) {
                     g = f + at;
-                    unit = kTileCellsPerThread * j + k;
+                    unit = PER * j + k;
                     found = true;
                 } else {
                     at -= c;
@@ -755,6 +802,7 @@ __device__ __forceinline__ float tile_start_h(const DensityArgs &a, uint32_t ind
 // impact) or to none.
 constexpr uint8_t kModeWalk = 0xfe;      // the per-particle pass
 constexpr uint8_t kModeInactive = 0xff;  // no neighbours needed (cell-tile pass)
+constexpr uint8_t kModeList = 0xfd;      // acceleration: the density pass's list
 static_assert(kUnitShift < kModeWalk, "0 and kUnitShift: the tile passes");
 
 // A warp: the tiles of the 128-cell block `blk` (the cells whose keys differ
@@ -839,8 +887,15 @@ __global__ void __launch_bounds__(256) k_density_plan(DensityArgs a, uint2 *tile
         const float h_plain = a.h[ind];
         const bool on = a.active[ind];
         bool seeded;
-        const float hb = fmaxf(tile_start_h(a, ind, h_plain, seeded), h_plain);
+        float hb = fmaxf(tile_start_h(a, ind, h_plain, seeded), h_plain);
+        // the list is built for the h the iteration is on its way to, as the
+        // last pass's density (moved on by the step) has it
+        if (on && hb < kMaxH) {
+            const float to = kResolutionEta * cbrtf(me.w / a.rho[ind]);
+            hb = fmaxf(hb, fminf(fminf(to, 1.2f * hb), 0.999f * kMaxH));
+        }
         a.start_h[p] = hb;
+        a.lists.count[p] = kNoList;
         if (!on) return kModeInactive;
         const int m = density_mode(me.x, me.y, me.z, hb, a.coarse);
         return m < 0 ? kModeWalk : (uint8_t)m;
@@ -903,116 +958,84 @@ struct Reach4 {
         const float gy = fmaxf(fmaxf((float)y * w - y1, y0 - (float)(y + 1) * w) - kCellMargin, 0.f);
         const float left = r2 - (gx * gx + gy * gy);
         if (left < 0.f) return false;
-        const float dz = left * rsqrtf(fmaxf(left, 1e-30f)) + kCellMargin;
+        const float dz = left * rsqrt_hw(fmaxf(left, 1e-30f)) + kCellMargin;
         zl = (int)floorf((z0 - dz) * iw - 1e-3f);
         zh = (int)floorf((z1 + dz) * iw + 1e-3f);
         return true;
     }
 };
 
-// One warp: the density pass of sorted particles p0 .. p0 + 3 of the staged
+// One warp: the neighbour lists of sorted particles p0 .. p0 + 3 of the staged
 // tile (lane group g = lane / 8 takes p0 + g) whose pass is U (0 cell tiles,
-// kUnitShift coarse tiles; the staged box is counted in units), in lockstep so the warp never
-// runs its groups one after another: the list build is transposed (each lane
-// takes one staged slot of a row and tests it against all four particles), and
-// the sweeps run over the longest of the four lists with the others predicated
-// off.  A particle that the tile path cannot finish is appended to `deferred`
-// (sorted index) with nothing written; k_density_deferred takes it from the
-// start.  The iteration is density_particle's with the neighbour cache never
-// in use (h < MAX_H throughout, so the reference's int max_h stays 0).
-template <int U, class Stage>
-__device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S, uint32_t *stats, uint32_t p0,
-                                                  uint32_t end, int lane, uint16_t (*lists)[kTileList],
-                                                  uint32_t *deferred, uint32_t *dctr) {
+// kUnitShift coarse tiles; the staged box is counted in units).  The search is
+// transposed: each lane takes one staged slot of a row and tests it against all
+// four particles.  A list holds the staged particles within 2 kTileListReach x
+// the particle's starting h or x their own (see NeighbourLists).
+template <int U>
+__device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared<U> &S, uint32_t p0, uint32_t end,
+                                                int lane) {
     constexpr int L = kTileLanes;
     constexpr unsigned kFull = 0xffffffffu;
     constexpr int kBig = 0x3fffffff;
+    constexpr float kFar2 = 4.f * kTileListReach * kTileListReach;
     const int g = lane / L, sub = lane & (L - 1);
-    uint16_t *list = lists[g];
     const uint32_t p = p0 + (uint32_t)g;
-    bool live = p < end;  // the group iterates its particle (uniform within the group)
-    uint32_t ind = 0u;
-    float4 me = make_float4(0.f, 0.f, 0.f, 0.f), mv = me;
-    const uint8_t mode = live ? a.mode[p] : kModeInactive;
-    if (live && mode != U && (U != 0 || mode == kUnitShift)) live = false;  // another pass takes it
-    if (live) {
-        ind = a.cidx[p];
-        me = a.sp4[p];
-        mv = a.sv4[p];
-        if (mode == kModeInactive) {
-            // density.metal:40-55: EOS only (in the cell-tile pass)
-            if (sub == 0) {
-                float2 pc = eos_lookup(a.eos, a.mat[ind], a.rho[ind], a.u[ind]);
-                a.P[ind] = pc.x;
-                a.c[ind] = pc.y;
-                float hh = a.h[ind], rho = a.rho[ind], fi = a.f[ind];
-                a.sA[p] = make_float4(me.x, me.y, me.z, hh);
-                a.sB[p] = make_float4(mv.x, mv.y, mv.z, pc.y);
-                a.sC[p] = make_float4(me.w, (fi * pc.x / (rho * rho)), rho, a.B[ind]);
-            }
-            live = false;
-        }
-    }
-    auto defer = [&]() {
-        if (sub == 0) deferred[atomicAdd(dctr, 1u)] = p;
-        live = false;
-    };
-    const float px = me.x, py = me.y, pz = me.z, mi = me.w;
-    float h_plain = 0.5f, hi = 0.5f;
-    bool seeded = false;
-    if (live) {
-        h_plain = a.h[ind];
-        hi = tile_start_h(a, ind, h_plain, seeded);
-        if (mode != U || S.defer_all) defer();
-    }
+    bool want = p < end && a.mode[p] == U;
+    float4 me = make_float4(3e38f, 3e38f, 3e38f, 0.f);  // (a group without a particle is nowhere near)
+    float hb = 0.f;
     // the staged box in its units
     const int us = unit_shift<U>(S.box);
     const float uw = kCellWidth * (float)(1 << us), uiw = (1.f / kCellWidth) / (float)(1 << us);
     const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
     const int hi0 = S.box[3] >> us, hi1 = S.box[4] >> us, hi2 = S.box[5] >> us;
     const int ny = hi1 - lo1 + 1, nz = hi2 - lo2 + 1;
-    // the group's list: staged slots within 2 hb kTileListReach
-    int n_list = -1;
-    float list_r2 = 0.f;
-    auto build = [&](bool want, float hb) {
+    if (want) {
+        me = a.sp4[p];
+        hb = a.start_h[p];
+    }
+    // a second search, wider, for the particles that found too few neighbours
+    // for their h to stay within the first one's reach (a body's surface at its
+    // first step)
+    for (int round = 0; round < 2; ++round) {
         CellBox b;
+        b.lo0 = b.lo1 = b.lo2 = kBig;
+        b.hi0 = b.hi1 = b.hi2 = -kBig;
         if (want) {
-            tile_box(px, py, pz, hb, b);
-            b.lo0 >>= us, b.lo1 >>= us, b.lo2 >>= us, b.hi0 >>= us, b.hi1 >>= us, b.hi2 >>= us;
-            if (!(hb < kMaxH) || b.lo0 < lo0 || b.lo1 < lo1 || b.lo2 < lo2 || b.hi0 > hi0 || b.hi1 > hi1 ||
-                b.hi2 > hi2) {
-                defer();
-                want = false;
+            tile_box(me.x, me.y, me.z, hb, b);
+            if (round == 1 && ((b.lo0 >> us) < lo0 || (b.lo1 >> us) < lo1 || (b.lo2 >> us) < lo2 ||
+                               (b.hi0 >> us) > hi0 || (b.hi1 >> us) > hi1 || (b.hi2 >> us) > hi2)) {
+                hb = a.start_h[p] * (kTileStageReach / kTileListReach);  // what is staged for it
+                tile_box(me.x, me.y, me.z, hb, b);
             }
+            b.lo0 = max(b.lo0 >> us, lo0), b.lo1 = max(b.lo1 >> us, lo1), b.lo2 = max(b.lo2 >> us, lo2);
+            b.hi0 = min(b.hi0 >> us, hi0), b.hi1 = min(b.hi1 >> us, hi1), b.hi2 = min(b.hi2 >> us, hi2);
         }
-        if (!want) {
-            b.lo0 = b.lo1 = b.lo2 = kBig;
-            b.hi0 = b.hi1 = b.hi2 = -kBig;
-        }
-        const float rl = 2.f * hb * kTileListReach;
-        const float r2 = want ? rl * rl : -1.f;
+        const float r2 = kFar2 * hb * hb;
         const int u0 = __reduce_min_sync(kFull, b.lo0), u1 = __reduce_min_sync(kFull, b.lo1),
                   u2 = __reduce_min_sync(kFull, b.lo2);
         const int v0 = __reduce_max_sync(kFull, b.hi0), v1 = __reduce_max_sync(kFull, b.hi1),
                   v2 = __reduce_max_sync(kFull, b.hi2);
-        if (u0 > v0) return;  // no group builds
-        const Reach4 reach(px, py, pz, r2);
+        if (u0 > v0) return;  // nothing (more) to search for
+        const float hm = fmaxf(hb, __int_as_float(S.hmax_bits));
+        const Reach4 reach(me.x, me.y, me.z, want ? kFar2 * hm * hm : -1.f);
         F2 nx[kTileGpw / 2], ny2[kTileGpw / 2], nz2[kTileGpw / 2];  // minus the positions, two particles each
         float qr[kTileGpw];
+        const float qpx = want ? me.x : 3e38f;
 #pragma unroll
         for (int k = 0; k < kTileGpw; ++k) qr[k] = __shfl_sync(kFull, r2, k * L);
 #pragma unroll
         for (int k = 0; k < kTileGpw / 2; ++k) {
-            nx[k] = f2(-__shfl_sync(kFull, px, 2 * k * L), -__shfl_sync(kFull, px, (2 * k + 1) * L));
-            ny2[k] = f2(-__shfl_sync(kFull, py, 2 * k * L), -__shfl_sync(kFull, py, (2 * k + 1) * L));
-            nz2[k] = f2(-__shfl_sync(kFull, pz, 2 * k * L), -__shfl_sync(kFull, pz, (2 * k + 1) * L));
+            nx[k] = f2(-__shfl_sync(kFull, qpx, 2 * k * L), -__shfl_sync(kFull, qpx, (2 * k + 1) * L));
+            ny2[k] = f2(-__shfl_sync(kFull, me.y, 2 * k * L), -__shfl_sync(kFull, me.y, (2 * k + 1) * L));
+            nz2[k] = f2(-__shfl_sync(kFull, me.z, 2 * k * L), -__shfl_sync(kFull, me.z, (2 * k + 1) * L));
         }
+        uint32_t *const out = a.lists.entries + (size_t)p0 * kTileList;  // of particle k: + k kTileList
         int cnt[kTileGpw] = {};
         const unsigned below = (1u << lane) - 1u;
+        uint32_t *const rows_of = S.rows[threadIdx.x >> 5];
         // Rows (x, y) of the union box, 32 at a time, one per lane; each row is
-        // trimmed to the z cells that the four spheres can reach, and the
-        // trimmed rows are walked as one flat sequence of staged slots, 32
-        // slots per step.
+        // trimmed to the z cells that the four spheres can reach, and the trimmed
+        // rows are walked as one flat sequence of staged slots, 32 slots per step.
         const int nyu = v1 - u1 + 1;
         const int rows = (v0 - u0 + 1) * nyu;
         for (int rb = 0; rb < rows; rb += 32) {
@@ -1039,18 +1062,29 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
             }
             const uint32_t excl = pre - len;
             const uint32_t total = __shfl_sync(kFull, pre, 31);
-            s0 -= excl;  // staged slot of flat index v in this row: s0 + v
+            // rows that have slots, in order: the staged slot of flat index v
+            // in row j is rows[j] + v
+            const unsigned some = __ballot_sync(kFull, len > 0u);
+            __syncwarp();
+            if (len) rows_of[__popc(some & below)] = s0 - excl;
+            __syncwarp();
+            int row0 = -1;  // the last row that starts before the step's slots
             for (uint32_t vb = 0; vb < total; vb += 32u) {
                 const uint32_t v = vb + (uint32_t)lane;
-                int j = 0;  // the last row whose first flat index is <= v
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const uint32_t e = __shfl_sync(kFull, excl, j + step);
-                    if (e <= v) j += step;
+                const uint32_t at0 = excl - vb;
+                const unsigned starts = __reduce_or_sync(kFull, len && at0 < 32u ? 1u << at0 : 0u);
+                const int j = row0 + __popc(starts & ((below << 1) | 1u));
+                row0 += __popc(starts);
+                const uint32_t s = rows_of[j] + v;
+                float4 q = make_float4(-3e38f, -3e38f, -3e38f, 0.f);
+                float hr = 0.f;
+                uint32_t gi = 0u;
+                if (v < total) {
+                    q = S.pos[s];
+                    const float h = S.hs[s];
+                    hr = kFar2 * h * h;
+                    gi = S.gidx[s];
                 }
-                const uint32_t s = __shfl_sync(kFull, s0, j) + v;
-                float4 q = make_float4(3e38f, 3e38f, 3e38f, 0.f);
-                if (v < total) q = S.pos[s];
                 const F2 qx = f2(q.x), qy = f2(q.y), qz = f2(q.z);
 #pragma unroll
                 for (int k = 0; k < kTileGpw / 2; ++k) {
@@ -1060,64 +1094,284 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const int g2 = 2 * k + i;
-                        const bool hit = d[i] <= qr[g2];
+                        const bool hit = d[i] <= fmaxf(qr[g2], hr);
                         const unsigned bal = __ballot_sync(kFull, hit);
                         const int at = cnt[g2] + __popc(bal & below);
-                        if (hit && at < kTileList) lists[g2][at] = (uint16_t)s;
+                        if (hit && at < kTileList) out[g2 * kTileList + at] = gi;
                         cnt[g2] += __popc(bal);
                     }
                 }
             }
         }
-        __syncwarp();
         if (want) {
             int c = 0;
 #pragma unroll
             for (int k = 0; k < kTileGpw; ++k)
                 if (g == k) c = cnt[k];
-            if (c > kTileList) {
-                defer();
-            } else {
-                n_list = c;
-                list_r2 = r2;
+            if (sub == 0) {
+                a.lists.count[p] = c <= kTileList ? (uint8_t)c : kNoList;
+                a.lists.reach2[p] = r2;
+            }
+            const float to = hb * cbrtf(kListFull / (float)max(c, 1));
+            want = round == 0 && to > kTileListReach * hb && to < kMaxH;
+            if (want) hb = fminf(1.02f * to, 0.999f * kMaxH);
+        }
+    }
+}
+
+// The tile pass U over the tiles of `tiles` (ctr[0] of them, ctr[1] the tile
+// ticket): U = 0 the cell tiles, U = kUnitShift the coarse tiles (512-cell
+// blocks).
+template <int U>
+__global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
+    k_lists(DensityArgs a, const uint2 *__restrict__ tiles, uint32_t *ctr) {
+    constexpr int T = ListTile<U>::kThreads;
+    constexpr int kPer = (kTileCellsMax + T - 1) / T;  // units per thread
+    extern __shared__ float4 s_tile_raw[];
+    ListShared<U> &S = *reinterpret_cast<ListShared<U> *>(s_tile_raw);
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t ntiles = ctr[0];
+    for (;;) {
+        __syncthreads();  // the previous tile is done with the staged data
+        if (tid == 0) {
+            const uint32_t t = atomicAdd(ctr + 1, 1u);
+            S.tile = t;
+            if (t < ntiles) {
+                const uint2 r = tiles[t];
+                S.start = r.x;
+                S.end = r.y;
             }
         }
+        __syncthreads();
+        if (S.tile >= ntiles) break;
+        const uint32_t tstart = S.start, tend = S.end;
+        // a tile whose staged box overflows shared memory is taken again as
+        // its octets (coarse tiles: its units), one at a time; one that still
+        // overflows is left to the per-particle pass
+        constexpr int kSplit = U == 0 ? 3 : 3 * U;
+        const bool splittable = (a.skey[tstart] >> kSplit) != (a.skey[tend - 1] >> kSplit);
+        bool whole = true;
+        uint32_t r0 = tstart;
+        while (r0 < tend) {
+            __syncthreads();
+            if (tid == 0) {
+                uint32_t r1 = tend;
+                if (!whole) {  // the rest of r0's octet / unit
+                    const uint32_t o = a.skey[r0] >> kSplit;
+                    r1 = max(r0 + 1u, (U == 0 ? a.octets : a.units)[o].y + 1u);
+                }
+                S.end = r1;
+                S.next = 0u;
+                S.box[0] = S.box[1] = S.box[2] = 0x7fffffff;
+                S.box[3] = S.box[4] = S.box[5] = -0x7fffffff;
+                S.defer_all = 0;
+                S.need = 0;
+                S.hmax_bits = 0;
+            }
+            __syncthreads();
+            const uint32_t start = r0, end = S.end;
+            // the staged box: union of the list boxes of the pass's particles
+            {
+                int b[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, -0x7fffffff, -0x7fffffff, -0x7fffffff};
+                bool need = false;
+                for (uint32_t p = start + tid; p < end; p += T) {
+                    if (a.mode[p] != U) continue;
+                    need = true;
+                    const float4 me = a.sp4[p];
+                    CellBox cb;
+                    tile_box(me.x, me.y, me.z, a.start_h[p], cb, kTileStageReach);
+                    b[0] = min(b[0], cb.lo0);
+                    b[1] = min(b[1], cb.lo1);
+                    b[2] = min(b[2], cb.lo2);
+                    b[3] = max(b[3], cb.hi0);
+                    b[4] = max(b[4], cb.hi1);
+                    b[5] = max(b[5], cb.hi2);
+                }
+                if (__any_sync(0xffffffffu, need)) {
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        b[k] = __reduce_min_sync(0xffffffffu, b[k]);
+                        b[k + 3] = __reduce_max_sync(0xffffffffu, b[k + 3]);
+                    }
+                    if (lane == 0) {
+                        S.need = 1;
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            atomicMin(&S.box[k], b[k]);
+                            atomicMax(&S.box[k + 3], b[k + 3]);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            if (!S.need) {  // nothing in the range for this pass
+                r0 = end;
+                continue;
+            }
+            const int us = unit_shift<U>(S.box);
+            const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
+            const int nx = (S.box[3] >> us) - lo0 + 1, ny = (S.box[4] >> us) - lo1 + 1, nz = (S.box[5] >> us) - lo2 + 1;
+            const bool too_many = box_units(nx, ny, nz) > kTileCellsMax;
+            const int ncell = too_many ? 0 : nx * ny * nz;
+            // unit counts (kPer consecutive units per thread) and their
+            // exclusive scan
+            uint32_t c_cnt[kPer], c_first[kPer];
+            uint32_t tsum = 0u;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                const int c = kPer * tid + k;
+                c_cnt[k] = c_first[k] = 0u;
+                if (c < ncell) {
+                    const int ix = c / (ny * nz), rem = c - ix * ny * nz, iy = rem / nz, iz = rem - iy * nz;
+                    const uint2 r = unit_range(a.cells, a.octets, a.units, us, lo0 + ix, lo1 + iy, lo2 + iz);
+                    if (r.x != 0xffffffffu) {
+                        c_cnt[k] = r.y - r.x + 1u;
+                        c_first[k] = r.x;
+                    }
+                }
+                tsum += c_cnt[k];
+            }
+            uint32_t inc = tsum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane == 31) S.wsum[tid >> 5] = inc;
+            __syncthreads();
+            uint32_t wbase = 0u;
+            for (int w = 0; w < (tid >> 5); ++w) wbase += S.wsum[w];
+            uint32_t run = wbase + inc - tsum;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                const int c = kPer * tid + k;
+                if (c < ncell) S.off[c] = run;
+                run += c_cnt[k];
+            }
+            if (tid == T - 1) {
+                S.off[ncell] = run;
+                if (too_many || run > (uint32_t)ListTile<U>::kStage) S.defer_all = 1;
+            }
+            __syncthreads();
+            if (S.defer_all) {
+                if (whole && splittable) whole = false;
+                else r0 = end;  // its particles are left without a list
+                continue;
+            }
+            float hmax = 0.f;
+            stage_units(c_cnt, c_first, inc - tsum, inc, lane, [&](uint32_t v, uint32_t g, int) {
+                const float h = __ldg(a.start_h + g);
+                S.pos[wbase + v] = __ldg(a.sp4 + g);
+                S.gidx[wbase + v] = g;
+                S.hs[wbase + v] = h;
+                hmax = fmaxf(hmax, h);
+            });
+            const int hbits = __reduce_max_sync(0xffffffffu, __float_as_int(hmax));
+            if (lane == 0 && hbits > 0) atomicMax(&S.hmax_bits, hbits);
+            __syncthreads();
+            // warps take the tile's particles four at a time
+            for (;;) {
+                uint32_t j = 0u;
+                if (lane == 0) j = atomicAdd(&S.next, (uint32_t)kTileGpw);
+                j = __shfl_sync(0xffffffffu, j, 0);
+                if (start + j >= end) break;
+                lists_tile_warp<U>(a, S, start + j, end, lane);
+            }
+            r0 = end;
+        }
+    }
+}
+
+// The density pass over the lists: a warp takes four consecutive sorted
+// particles, eight lanes each, in lockstep so it never runs its groups one after
+// another.  Particles without a list, and those whose h outgrows theirs, are
+// appended to `deferred` (sorted index) with nothing written;
+// k_density_deferred takes them from the start.  The iteration is
+// density_particle's with the neighbour cache never in use (h < MAX_H
+// throughout, so the reference's int max_h stays 0).
+constexpr int kListThreads = 256;
+__global__ void __launch_bounds__(kListThreads, 4)
+    k_density_list(DensityArgs a, uint32_t *__restrict__ deferred, uint32_t *dctr) {
+    constexpr int L = kTileLanes;
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & (L - 1);
+    const int p = (int)((blockIdx.x * (unsigned)kListThreads + threadIdx.x) / L);
+    const uint8_t mode = p < a.n ? a.mode[p] : kModeInactive;
+    bool live = p < a.n;  // the group iterates its particle (uniform within the group)
+    uint32_t ind = 0u;
+    float4 me = make_float4(0.f, 0.f, 0.f, 0.f), mv = me;
+    float h_plain = 0.5f;
+    int n_list = -1;
+    if (live) {
+        ind = a.cidx[p];
+        me = a.sp4[p];
+        mv = a.sv4[p];
+        h_plain = a.h[ind];
+        if (mode == kModeInactive) {
+            // density.metal:40-55: EOS only
+            if (sub == 0) {
+                float2 pc = eos_lookup(a.eos, a.mat[ind], a.rho[ind], a.u[ind]);
+                a.P[ind] = pc.x;
+                a.c[ind] = pc.y;
+                float rho = a.rho[ind], fi = a.f[ind];
+                a.sA[p] = make_float4(me.x, me.y, me.z, h_plain);
+                a.sB[p] = make_float4(mv.x, mv.y, mv.z, pc.y);
+                a.sC[p] = make_float4(me.w, (fi * pc.x / (rho * rho)), rho, a.B[ind]);
+            }
+            live = false;
+        }
+    }
+    auto defer = [&]() {
+        if (sub == 0) {
+            deferred[atomicAdd(dctr, 1u)] = (uint32_t)p;
+            a.lists.count[p] = kNoList;  // (too short for the acceleration pass too)
+        }
+        live = false;
     };
+    const uint32_t *list = a.lists.entries + (size_t)(p < a.n ? p : 0) * kTileList;
+    float hi = 0.5f, list_r2 = 0.f;
+    bool seeded = false;
+    if (live) {
+        const uint8_t c = a.lists.count[p];
+        if (c == kNoList) {
+            defer();
+        } else {
+            n_list = c;
+            list_r2 = a.lists.reach2[p];
+            hi = tile_start_h(a, ind, h_plain, seeded);
+        }
+    }
+    const float px = me.x, py = me.y, pz = me.z, mi = me.w;
+    const int maxn = __reduce_max_sync(kFull, n_list);
+    // The sorted index behind list entry i, this particle's own past the list's
+    // end: loads without branches, so that many are in flight together.
+    const int self = min(p, a.n - 1);
+    auto entry = [&](int i) { return i < n_list ? (int)__ldg(list + i) : self; };
     // Distance and mass of the pair of list entries (i, i + L); nothing (a
     // massless neighbour far away) past the list's end.
     auto entry_pair = [&](int i, F2 &r, F2 &m) {
-        float rr[2] = {1e30f, 1e30f}, mm[2] = {0.f, 0.f};
+        float rr[2], mm[2];
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-            if (i + e * L < n_list) {
-                const float4 q = S.pos[list[i + e * L]];
-                const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
-                rr[e] = pair_sqrt(dx * dx + dy * dy + dz * dz);
-                mm[e] = q.w;
-            }
+        for (int e = 0; e < 2; ++e) {
+            const float4 q = __ldg(a.sp4 + entry(i + e * L));
+            const float dx = q.x - px, dy = q.y - py, dz = q.z - pz;
+            const bool in = i + e * L < n_list;
+            rr[e] = in ? pair_sqrt(dx * dx + dy * dy + dz * dz) : 1e30f;
+            mm[e] = in ? q.w : 0.f;
+        }
         r = f2(rr[0], rr[1]);
         m = f2(mm[0], mm[1]);
     };
     F2 rp[kRegPairs], mp[kRegPairs];
+#pragma unroll
+    for (int t = 0; t < kRegPairs; ++t) entry_pair(sub + 2 * t * L, rp[t], mp[t]);
     bool iter = live;
     bool first = true, fell_back = false;
     int sweeps = 0, count = 0;
-    int maxn = 0;  // longest list of the warp
     float h2x4 = 4.f * hi * hi;
     float h1 = 1.f / hi;
     float w4 = 0.f, eps = 1.f;  // 4 pi h^3 x the density
     while (__any_sync(kFull, iter)) {
-        const bool want = iter && (n_list < 0 || h2x4 > list_r2);
-        if (__any_sync(kFull, want)) {
-            build(want, hi);
-            iter = iter && live;
-            maxn = __reduce_max_sync(kFull, live ? n_list : 0);
-            if (maxn <= kRegList) {
-#pragma unroll
-                for (int t = 0; t < kRegPairs; ++t)
-                    if (2 * t * L < maxn) entry_pair(sub + 2 * t * L, rp[t], mp[t]);
-            }
-        }
         // the cubic spline as (2 - q)+^3 / 4 - (1 - q)+^3
         const F2 nh = f2(-h1);
         F2 acc = f2(0.f);
@@ -1125,49 +1379,40 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
             const F2 t = clamp0(fma2(r, nh, f2(2.f))), u = clamp0(fma2(r, nh, f2(1.f)));
             acc = fma2(m, fma2(f2(-4.f) * u, u * u, t * (t * t)), acc);
         };
-        if (maxn <= kRegList) {
 #pragma unroll
-            for (int t = 0; t < kRegPairs; ++t)
-                if (2 * t * L < maxn) add(rp[t], mp[t]);
-        } else {
-            for (int i = sub; i < maxn; i += 2 * L) {
-                F2 r, m;
-                entry_pair(i, r, m);
-                add(r, m);
-            }
+        for (int t = 0; t < kRegPairs; ++t) add(rp[t], mp[t]);
+        for (int i = kRegList + sub; i < maxn; i += 2 * L) {
+            F2 r, m;
+            entry_pair(i, r, m);
+            add(r, m);
         }
         const float wsum = group_sum<L>(sum(acc), kFull);
         if (iter) {
             w4 = wsum;
             const float dens = kernel_norm(h1) * wsum;
-            float nh_ = fmin_ref(kResolutionEta * cbrtf(mi / dens), kMaxH);
+            float nh_ = fmin_ref(kResolutionEta * cbrtf(pdiv(mi, dens)), kMaxH);
             nh_ = 0.5f * (hi + nh_);
             eps = fabsf(nh_ - hi) * h1;
             ++sweeps;
             if (first && seeded && eps > kSeedFallback) {
                 // the seed disagrees with its own first sweep: start again from
                 // the plain guess
-                first = false;
                 fell_back = true;
                 hi = h_plain;
                 h1 = 1.f / hi;
                 h2x4 = 4.f * hi * hi;
                 eps = 1.f;
-            } else {
-                first = false;
-                if (eps > a.eta) {
-                    // at MAX_H the reference's int max_h would leave 0, and a
-                    // particle that does not converge ends on another h than
-                    // its last sweep's: the per-particle pass takes both
-                    if (nh_ >= kMaxH || ++count >= kMaxNR) {
-                        defer();
-                    } else {
-                        hi = nh_;
-                        h1 = 1.f / hi;
-                        h2x4 = 4.f * hi * hi;
-                    }
-                }
+            } else if (eps > a.eta) {
+                // at MAX_H the reference's int max_h would leave 0, and a
+                // particle that does not converge ends on another h than its
+                // last sweep's: the per-particle pass takes both, and those
+                // whose list is too short for the new h
+                hi = nh_;
+                h1 = 1.f / hi;
+                h2x4 = 4.f * hi * hi;
+                if (nh_ >= kMaxH || ++count >= kMaxNR || !(h2x4 <= list_r2)) defer();
             }
+            first = false;
             iter = live && eps > a.eta;
         }
     }
@@ -1175,54 +1420,48 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
     // those within 2 h; with g' = 3 (1 - q)+^2 - 3 (2 - q)+^2 / 4 the spline's
     // derivative, dW/dh = -(3 W + q g') / h (up to the norm), so of it only
     // the sum of q g' is new
-    const float h2 = hi + hi;
     const float vix = mv.x, viy = mv.y, viz = mv.z;
     F2 qg = f2(0.f), vdiv2 = qg, cx2 = qg, cy2 = qg, cz2 = qg;
     int nn = 0;
-    {
-        const F2 nh = f2(-h1);
-        const F2 npx = f2(-px), npy = f2(-py), npz = f2(-pz), nvx = f2(-vix), nvy = f2(-viy), nvz = f2(-viz);
-        auto add = [&](int i, F2 r, F2 m) {
-            const F2 t = clamp0(fma2(r, nh, f2(2.f))), u = clamp0(fma2(r, nh, f2(1.f)));
-            const F2 g = m * fma2(f2(3.f) * u, u, f2(-0.75f) * (t * t));
-            float re[2];
-            unpack(r, re[0], re[1]);
-            float4 q[2] = {me, me}, vj[2] = {mv, mv};
-            float rinv[2];
+    const F2 nh = f2(-h1);
+#pragma unroll 2
+    for (int i = sub; i < maxn; i += 2 * L) {
+        // (a neighbour past 2 h, or the list's end: this particle itself)
+        float4 q[2], vj[2];
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const bool in = re[e] <= h2 && live;
-                nn += in ? 1 : 0;
-                rinv[e] = in && re[e] > 1e-12f ? pdiv(1.f, re[e]) : 0.f;
-                if (in) {
-                    const uint32_t s = list[i + e * L];
-                    q[e] = S.pos[s];
-                    vj[e] = __ldg(a.sv4 + S.gidx[s]);
-                }
-            }
-            // (nh is -1/h: this adds minus the sum; far padding has g = 0)
-            qg = fma2(g * nh, f2(fminf(re[0], h2), fminf(re[1], h2)), qg);
-            const F2 gr = g * f2(rinv[0], rinv[1]);
-            const F2 gx = gr * (f2(q[0].x, q[1].x) + npx), gy = gr * (f2(q[0].y, q[1].y) + npy),
-                     gz = gr * (f2(q[0].z, q[1].z) + npz);
-            const F2 vx = f2(vj[0].x, vj[1].x) + nvx, vy = f2(vj[0].y, vj[1].y) + nvy,
-                     vz = f2(vj[0].z, vj[1].z) + nvz;
-            vdiv2 = fma2(vz, gz, fma2(vy, gy, fma2(vx, gx, vdiv2)));
-            cx2 = fma2(vy, gz, fma2(neg(vz), gy, cx2));
-            cy2 = fma2(vz, gx, fma2(neg(vx), gz, cy2));
-            cz2 = fma2(vx, gy, fma2(neg(vy), gx, cz2));
-        };
-        if (maxn <= kRegList) {
-#pragma unroll
-            for (int t = 0; t < kRegPairs; ++t)
-                if (2 * t * L < maxn) add(sub + 2 * t * L, rp[t], mp[t]);
-        } else {
-            for (int i = sub; i < maxn; i += 2 * L) {
-                F2 r, m;
-                entry_pair(i, r, m);
-                add(i, r, m);
-            }
+        for (int e = 0; e < 2; ++e) {
+            const int gi = entry(i + e * L);
+            q[e] = __ldg(a.sp4 + gi);
+            vj[e] = __ldg(a.sv4 + gi);
         }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const float dx = q[e].x - px, dy = q[e].y - py, dz = q[e].z - pz;
+            const bool in = dx * dx + dy * dy + dz * dz <= h2x4 && i + e * L < n_list;
+            if (!in) {
+                q[e] = me;
+                vj[e] = mv;
+            }
+            nn += in ? 1 : 0;
+        }
+        const F2 dx = f2(q[0].x, q[1].x) + f2(-px), dy = f2(q[0].y, q[1].y) + f2(-py),
+                 dz = f2(q[0].z, q[1].z) + f2(-pz);
+        const F2 r2 = fma2(dz, dz, fma2(dy, dy, dx * dx));
+        float ra, rb;
+        unpack(r2, ra, rb);
+        const F2 rinv = f2(ra > 1e-24f ? rsqrt_hw(ra) : 0.f, rb > 1e-24f ? rsqrt_hw(rb) : 0.f);
+        const F2 r = r2 * rinv;
+        const F2 t = clamp0(fma2(r, nh, f2(2.f))), u = clamp0(fma2(r, nh, f2(1.f)));
+        const F2 g = f2(q[0].w, q[1].w) * fma2(f2(3.f) * u, u, f2(-0.75f) * (t * t));
+        qg = fma2(g, r * nh, qg);  // (nh is -1/h: minus the sum)
+        const F2 gr = g * rinv;
+        const F2 gx = gr * dx, gy = gr * dy, gz = gr * dz;
+        const F2 vx = f2(vj[0].x, vj[1].x) + f2(-vix), vy = f2(vj[0].y, vj[1].y) + f2(-viy),
+                 vz = f2(vj[0].z, vj[1].z) + f2(-viz);
+        vdiv2 = fma2(vz, gz, fma2(vy, gy, fma2(vx, gx, vdiv2)));
+        cx2 = fma2(vy, gz, fma2(neg(vz), gy, cx2));
+        cy2 = fma2(vz, gx, fma2(neg(vx), gz, cy2));
+        cz2 = fma2(vx, gy, fma2(neg(vy), gx, cz2));
     }
     nn = group_sum_i<L>(nn, kFull);
     const float norm = kernel_norm(h1);  // 1 / (4 pi h^3)
@@ -1232,18 +1471,36 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
     const float cx = gnorm * group_sum<L>(sum(cx2), kFull);
     const float cy = gnorm * group_sum<L>(sum(cy2), kFull);
     const float cz = gnorm * group_sum<L>(sum(cz2), kFull);
+    if (a.stats) {
+        const uint32_t mine = live && sub == 0 ? 1u : 0u;
+        const uint32_t sw = __reduce_add_sync(kFull, mine * (uint32_t)sweeps);
+        const uint32_t fb = __reduce_add_sync(kFull, mine * (fell_back ? 1u : 0u));
+        const uint32_t mx = __reduce_max_sync(kFull, mine * (uint32_t)sweeps);
+        const uint32_t np = __reduce_add_sync(kFull, mine);
+        __shared__ uint32_t s_stats[4];
+        if (threadIdx.x < 4) s_stats[threadIdx.x] = 0u;
+        __syncthreads();
+        if (lane == 0) {
+            atomicAdd(&s_stats[0], sw);
+            atomicAdd(&s_stats[1], fb);
+            atomicMax(&s_stats[2], mx);
+            atomicAdd(&s_stats[3], np);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && s_stats[3]) {
+            atomicAdd(a.stats + 0, s_stats[0]);
+            if (s_stats[1]) atomicAdd(a.stats + 1, s_stats[1]);
+            atomicMax(a.stats + 2, s_stats[2]);
+            atomicAdd(a.stats + 3, s_stats[3]);
+        }
+    }
     if (!live || sub != 0) return;
     // 3 sum(W) + sum(q g') over sum(4 W): nqg is minus sum(q g')
     const float dens_h = -gnorm * (0.75f * w4 - nqg);
     float dens = norm * w4;
     nn = min(nn, kNeighbourCache);
     if (nn >= kNeighbourCache) dens += dens;  // the reference's full scan adds the density again
-    if (a.stats) {
-        atomicAdd(&stats[0], (uint32_t)sweeps);
-        if (fell_back) atomicAdd(&stats[1], 1u);
-        atomicMax(&stats[2], (uint32_t)sweeps);
-        atomicAdd(&stats[3], 1u);
-    }
+    mark_grown(a, (uint32_t)p, hi);
     if (a.nn_out) a.nn_out[ind] = (float)nn;
     vdiv = fabsf(vdiv) / dens;
     float acurl = sqrtf(cx * cx + cy * cy + cz * cz) / dens;
@@ -1262,193 +1519,6 @@ __device__ __forceinline__ void density_tile_warp(const DensityArgs &a, Stage &S
     a.sC[p] = make_float4(mi, (fi * pc.x / (dens * dens)), dens, bal);
 }
 
-// The density tile pass U over the tiles of `tiles` (ctr[0] of them, ctr[1]
-// the tile ticket): U = 0 the cell tiles, whose staged box counts cells;
-// U = kUnitShift the coarse tiles (512-cell blocks), whose staged box counts
-// 64-cell units.  Deferred particles are appended to `deferred`, counted in
-// *dctr.
-template <int U>
-__global__ void __launch_bounds__(kTileThreads, 2)
-    k_density_tile(DensityArgs a, const uint2 *__restrict__ tiles, uint32_t *ctr, uint32_t *__restrict__ deferred,
-                   uint32_t *dctr) {
-    extern __shared__ float4 s_tile_raw[];
-    TileShared &S = *reinterpret_cast<TileShared *>(s_tile_raw);
-    const int tid = threadIdx.x, lane = tid & 31;
-    if (tid < 4) S.stats[tid] = 0u;
-    const uint32_t ntiles = ctr[0];
-    for (;;) {
-        __syncthreads();  // the previous tile is done with the staged data
-        if (tid == 0) {
-            const uint32_t t = atomicAdd(ctr + 1, 1u);
-            S.tile = t;
-            if (t < ntiles) {
-                const uint2 r = tiles[t];
-                S.start = r.x;
-                S.end = r.y;
-            }
-        }
-        __syncthreads();
-        if (S.tile >= ntiles) break;
-        const uint32_t tstart = S.start, tend = S.end;
-        // a tile whose staged box overflows shared memory is taken again as
-        // its octets (coarse tiles: its units), one at a time; one that still
-        // overflows is handed to the per-particle pass
-        constexpr int kSplit = U == 0 ? 3 : 3 * U;
-        const bool splittable = (a.skey[tstart] >> kSplit) != (a.skey[tend - 1] >> kSplit);
-        bool whole = true;
-        uint32_t r0 = tstart;
-        while (r0 < tend) {
-            __syncthreads();
-            if (tid == 0) {
-                uint32_t r1 = tend;
-                if (!whole) {  // the rest of r0's octet / unit
-                    const uint32_t o = a.skey[r0] >> kSplit;
-                    r1 = r0 + 1u;
-                    if (U == 0) {
-                        for (int j = 0; j < 8; ++j) {
-                            const uint2 r = a.cells[o * 8u + (uint32_t)j];
-                            if (r.x != 0xffffffffu) r1 = max(r1, r.y + 1u);
-                        }
-                    } else {
-                        r1 = max(r1, a.units[o].y + 1u);
-                    }
-                }
-                S.end = r1;
-                S.next = 0u;
-                S.box[0] = S.box[1] = S.box[2] = 0x7fffffff;
-                S.box[3] = S.box[4] = S.box[5] = -0x7fffffff;
-                S.defer_all = 0;
-                S.need = 0;
-            }
-            __syncthreads();
-            const uint32_t start = r0, end = S.end;
-            // the staged box: union of the list boxes of the tile's active particles
-            {
-                int b[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, -0x7fffffff, -0x7fffffff, -0x7fffffff};
-                // the warp pass is needed for this pass's particles and, in the
-                // cell-tile pass, for the inactive (EOS only) and deferred ones
-                bool need = false;
-                for (uint32_t p = start + tid; p < end; p += kTileThreads) {
-                    const uint8_t m = a.mode[p];
-                    need |= m == U || (U == 0 && m != kUnitShift);
-                    if (m != U) continue;
-                    const float4 me = a.sp4[p];
-                    const float hb = a.start_h[p];
-                    CellBox cb;
-                    tile_box(me.x, me.y, me.z, hb, cb, fmaxf(kTileStageReach, kTileListReach));
-                    b[0] = min(b[0], cb.lo0);
-                    b[1] = min(b[1], cb.lo1);
-                    b[2] = min(b[2], cb.lo2);
-                    b[3] = max(b[3], cb.hi0);
-                    b[4] = max(b[4], cb.hi1);
-                    b[5] = max(b[5], cb.hi2);
-                }
-    #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    b[k] = __reduce_min_sync(0xffffffffu, b[k]);
-                    b[k + 3] = __reduce_max_sync(0xffffffffu, b[k + 3]);
-                }
-                if (__any_sync(0xffffffffu, need) && lane == 0) S.need = 1;
-                if (lane == 0) {
-    #pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        atomicMin(&S.box[k], b[k]);
-                        atomicMax(&S.box[k + 3], b[k + 3]);
-                    }
-                }
-            }
-            __syncthreads();
-            if (!S.need) {  // nothing in the range for this pass
-                r0 = end;
-                continue;
-            }
-            const bool any = S.box[0] <= S.box[3];  // some particle of the tile takes the tile path
-            const int us = unit_shift<U>(S.box);
-            const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
-            const int nx = any ? (S.box[3] >> us) - lo0 + 1 : 0, ny = any ? (S.box[4] >> us) - lo1 + 1 : 0,
-                      nz = any ? (S.box[5] >> us) - lo2 + 1 : 0;
-            int ncell = 0;
-            if (any) {
-                if (box_units(nx, ny, nz) > kTileCellsMax) {
-                    if (tid == 0) S.defer_all = 1;
-                } else {
-                    ncell = nx * ny * nz;
-                }
-            }
-            // cell counts (kTileCellsPerThread consecutive cells per thread) and
-            // their exclusive scan
-            uint32_t c_cnt[kTileCellsPerThread], c_first[kTileCellsPerThread];
-            uint32_t tsum = 0u;
-    #pragma unroll
-            for (int k = 0; k < kTileCellsPerThread; ++k) {
-                const int c = kTileCellsPerThread * tid + k;
-                c_cnt[k] = c_first[k] = 0u;
-                if (c < ncell) {
-                    const int ix = c / (ny * nz), rem = c - ix * ny * nz, iy = rem / nz, iz = rem - iy * nz;
-                    const uint2 r = unit_range(a.cells, a.octets, a.units, us, lo0 + ix, lo1 + iy, lo2 + iz);
-                    if (r.x != 0xffffffffu) {
-                        c_cnt[k] = r.y - r.x + 1u;
-                        c_first[k] = r.x;
-                    }
-                }
-                tsum += c_cnt[k];
-            }
-            uint32_t inc = tsum;
-    #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            if (lane == 31) S.wsum[tid >> 5] = inc;
-            __syncthreads();
-            uint32_t wbase = 0u;
-            for (int w = 0; w < (tid >> 5); ++w) wbase += S.wsum[w];
-            uint32_t run = wbase + inc - tsum;
-    #pragma unroll
-            for (int k = 0; k < kTileCellsPerThread; ++k) {
-                const int c = kTileCellsPerThread * tid + k;
-                if (c < ncell) S.off[c] = run;
-                run += c_cnt[k];
-            }
-            if (tid == kTileThreads - 1) {
-                S.off[ncell] = run;
-                if (run > (uint32_t)kTileStageMax) S.defer_all = 1;
-            }
-            __syncthreads();
-            if (S.defer_all && whole && splittable) {
-                whole = false;
-                continue;
-            }
-            if (!S.defer_all) {
-                stage_units(c_cnt, c_first, inc - tsum, inc, lane, [&](uint32_t v, uint32_t g, int) {
-                    S.pos[wbase + v] = __ldg(a.sp4 + g);
-                    S.gidx[wbase + v] = g;
-                });
-            }
-            __syncthreads();
-            // warps take the tile's particles four at a time
-            for (bool more = true; more;) {
-                uint32_t j = 0u;
-                if (lane == 0) j = atomicAdd(&S.next, (uint32_t)kTileGpw);
-                j = __shfl_sync(0xffffffffu, j, 0);
-                more = start + j < end;
-                if (!more) break;
-                density_tile_warp<U>(a, S, S.stats, start + j, end, lane, &S.list[(tid >> 5) * kTileGpw], deferred,
-                                     dctr);
-            }
-            r0 = end;
-        }
-    }
-    if (a.stats && tid == 0) {
-        if (S.stats[3]) {
-            atomicAdd(a.stats + 0, S.stats[0]);
-            if (S.stats[1]) atomicAdd(a.stats + 1, S.stats[1]);
-            atomicMax(a.stats + 2, S.stats[2]);
-            atomicAdd(a.stats + 3, S.stats[3]);
-        }
-    }
-}
-
 struct AccelArgs {
     int n;
     const uint32_t *cidx;
@@ -1458,7 +1528,8 @@ struct AccelArgs {
     const uint2 *units;    // 64-cell unit ranges (coarse tiles)
     uint8_t *cflags;       // per 512-cell block: holds a coarse-tile particle
     int coarse;            // coarse tiles on
-    uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_tile_plan
+    uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_acceleration_plan
+    NeighbourLists lists;  // the density pass's
     const float4 *sA, *sB, *sC;
     float4 *acc4;
     float *du, *dhdt;
@@ -1614,6 +1685,20 @@ __device__ __forceinline__ void accel_pair2(const AccelI &I, float fac_i, AccelS
     accel_add2<KAHAN>(S.dh, S.kh, m * w * si * f2(pdiv(1.f, C[0].z), pdiv(1.f, C[1].z)));
 }
 
+// A lane's two halves (with their compensations) as one.
+template <bool KAHAN>
+__device__ __forceinline__ AccelSum accel_close(const AccelSum2 &S) {
+    const F2 minus = f2(-1.f);
+    AccelSum r;
+    r.dvx = sum(KAHAN ? fma2(S.kx, minus, S.x) : S.x);
+    r.dvy = sum(KAHAN ? fma2(S.ky, minus, S.y) : S.y);
+    r.dvz = sum(KAHAN ? fma2(S.kz, minus, S.z) : S.z);
+    r.du = sum(KAHAN ? fma2(S.ku, minus, S.du) : S.du);
+    r.dh = sum(KAHAN ? fma2(S.kh, minus, S.dh) : S.dh);
+    r.vsig = S.vsig;
+    return r;
+}
+
 // The group's sums combined (every lane ends with the same bits).
 template <int L, bool KAHAN>
 __device__ __forceinline__ void accel_reduce(AccelSum &S, unsigned gm) {
@@ -1693,7 +1778,8 @@ __device__ __forceinline__ int accel_particle(const AccelArgs &a, int index, int
     return idt;
 }
 
-// Block-wide minimum of the timesteps, then one atomic per block.
+// Block-wide minimum of the timesteps, then one atomic per block that lowers
+// the global one.
 __device__ __forceinline__ void block_min_dt(int idt, int32_t *dt) {
     __shared__ int wmin[32];
     const int lane = threadIdx.x & 31;
@@ -1703,7 +1789,7 @@ __device__ __forceinline__ void block_min_dt(int idt, int32_t *dt) {
     if (threadIdx.x < 32) {
         int v = (threadIdx.x < ((blockDim.x + 31) >> 5)) ? wmin[threadIdx.x] : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (threadIdx.x == 0 && v != 0x7fffffff) atomicMin(dt, v);
+        if (threadIdx.x == 0 && v < *(volatile int32_t *)dt) atomicMin(dt, v);
     }
 }
 
@@ -1756,7 +1842,10 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L)
 // Particles whose box reaches more than kTileReach cells past their own cell,
 // whose list overflows, and every particle of a tile whose staged box exceeds
 // the budget go to k_acceleration_deferred.
-constexpr int kTileAccStage = 3072;  // staged particles per tile
+constexpr int kTileThreads = 384;
+constexpr int kTileGroups = kTileThreads / kTileLanes;  // particles in flight per CTA
+constexpr int kTileAccStage = 3072;                     // staged particles per tile
+constexpr int kTileCellsPerThread = (kTileCellsMax + kTileThreads - 1) / kTileThreads;
 
 struct TileAccShared {
     float4 pos[kTileAccStage];          // staged sA (x, y, z, h)
@@ -1817,7 +1906,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
     uint32_t ind = 0u;
     int idt_inactive = 0x7fffffff;
     const uint8_t mode = live ? a.mode[p] : kModeInactive;
-    if (live && mode != U && (U != 0 || mode == kUnitShift)) live = false;  // another pass takes it
+    if (live && mode != U && (U != 0 || mode < kModeWalk)) live = false;  // another pass takes it
     if (live) {
         ind = a.cidx[p];
         if (mode == kModeInactive) {
@@ -1976,13 +2065,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
             }
         accel_pair2<KAHAN>(I, fac_i, S2, Aj, Bj, Cj);
     }
-    AccelSum Sm;
-    Sm.dvx = KAHAN ? sum(fma2(S2.kx, f2(-1.f), S2.x)) : sum(S2.x);
-    Sm.dvy = KAHAN ? sum(fma2(S2.ky, f2(-1.f), S2.y)) : sum(S2.y);
-    Sm.dvz = KAHAN ? sum(fma2(S2.kz, f2(-1.f), S2.z)) : sum(S2.z);
-    Sm.du = KAHAN ? sum(fma2(S2.ku, f2(-1.f), S2.du)) : sum(S2.du);
-    Sm.dh = KAHAN ? sum(fma2(S2.kh, f2(-1.f), S2.dh)) : sum(S2.dh);
-    Sm.vsig = S2.vsig;
+    AccelSum Sm = accel_close<KAHAN>(S2);
     accel_reduce<L, false>(Sm, kFull);
     int idt = idt_inactive;
     if (live) {
@@ -1999,7 +2082,22 @@ __global__ void __launch_bounds__(256) k_acceleration_plan(AccelArgs a, uint2 *t
         if (!a.active[a.cidx[p]]) return kModeInactive;
         CellBox b;
         const int m = accel_mode(A.x, A.y, A.z, A.w, b, a.coarse);
-        return m < 0 ? kModeWalk : (uint8_t)m;
+        if (m < 0) return kModeWalk;
+        // the list is complete when no neighbour the box can hold has outgrown it
+        // (a NaN h counts as larger than any)
+        if (a.lists.entries && a.lists.count[p] != kNoList) {
+            int grown = 0;
+            for (int x = b.lo0 >> kUnitShift; x <= b.hi0 >> kUnitShift; ++x)
+                for (int y = b.lo1 >> kUnitShift; y <= b.hi1 >> kUnitShift; ++y)
+                    for (int z = b.lo2 >> kUnitShift; z <= b.hi2 >> kUnitShift; ++z) {
+                        const int mask = (kCellsPerDim >> kUnitShift) - 1;
+                        grown = max(grown, __ldg(a.lists.grown + morton3((uint32_t)(x & mask), (uint32_t)(y & mask),
+                                                                         (uint32_t)(z & mask))));
+                    }
+            const float hg = __int_as_float(grown);
+            if (4.f * hg * hg <= 0.9999f * a.lists.reach2[p]) return kModeList;
+        }
+        return (uint8_t)m;
     });
 }
 
@@ -2069,7 +2167,7 @@ __global__ void __launch_bounds__(kTileThreads, 2)
                 bool need = false;
                 for (uint32_t p = start + tid; p < end; p += kTileThreads) {
                     const uint8_t m = a.mode[p];
-                    need |= m == U || (U == 0 && m != kUnitShift);
+                    need |= m == U || (U == 0 && m >= kModeWalk);
                     if (m != U) continue;
                     const float4 A = a.sA[p];
                     const CellBox cb = cell_box(A.x, A.y, A.z, fmin_ref(A.w, kMaxH));
@@ -2204,6 +2302,91 @@ __global__ void __launch_bounds__(kTileThreads, 2)
         }
     }
     if (tid == 0 && S.dtmin != 0x7fffffff) atomicMin(a.globals + 1, S.dtmin);
+}
+
+// The particles whose list the density pass left (kModeList): eight lanes
+// each, two neighbours per lane and step, all neighbour records read by sorted
+// index (they are neighbours in that order too, so most come from L1).  Same
+// pairs and arithmetic as the tiles; what is saved is the search, which was
+// 70 % of a tile's time.  Measured, acceleration pass at N = 1e6: 1.61 -> 0.86 ms
+// (24 warps per SM; with 32 and spilled sums 0.93).
+template <bool KAHAN>
+__global__ void __launch_bounds__(kListThreads, 3) k_acceleration_list(AccelArgs a) {
+    constexpr int L = kTileLanes;
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & (L - 1);
+    const int p = (int)((blockIdx.x * (unsigned)kListThreads + threadIdx.x) / L);
+    const bool live = p < a.n && a.mode[p] == kModeList;
+    int idt = 0x7fffffff;
+    if (__any_sync(kFull, live)) {
+        float4 A = make_float4(0.f, 0.f, 0.f, 1.f), Bv = A, Cv = A;
+        int n_list = 0;
+        if (live) {
+            A = a.sA[p];
+            Bv = a.sB[p];
+            Cv = a.sC[p];
+            n_list = a.lists.count[p];
+        }
+        const AccelI I = accel_i(A, Bv, Cv);
+        CellBox box = cell_box(I.xi, I.yi, I.zi, fmin_ref(I.hi, kMaxH));
+        const uint32_t *list = a.lists.entries + (size_t)(live ? p : 0) * kTileList;
+        const float hi2 = I.hi1 * I.hi1, fac_i = kPi1 * hi2 * hi2;
+        const int maxn = __reduce_max_sync(kFull, n_list);
+        AccelSum2 S2;
+        // the sorted index behind list entry i, this particle's own past the end
+        const int self = min(p, a.n - 1);
+        auto entry = [&](int i) { return i < n_list ? (int)__ldg(list + i) : self; };
+        int g[2] = {entry(sub), entry(sub + L)};
+        float4 Aj[2] = {__ldg(a.sA + g[0]), __ldg(a.sA + g[1])};
+#pragma unroll 1
+        for (int i = sub; i < maxn; i += 2 * L) {
+            // the next step's neighbours are on their way while this one's count
+            const int gn[2] = {entry(i + 2 * L), entry(i + 3 * L)};
+            float4 Bj[2], Cj[2], An[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                Bj[e] = __ldg(a.sB + g[e]);
+                Cj[e] = __ldg(a.sC + g[e]);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) An[e] = __ldg(a.sA + gn[e]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float dx = Aj[e].x - I.xi, dy = Aj[e].y - I.yi, dz = Aj[e].z - I.zi;
+                const float d = dx * dx + dy * dy + dz * dz;
+                bool hit = d >= 1e-12f && d <= I.hi2x4;
+                if (!hit && d >= 1e-12f && d <= Aj[e].w * Aj[e].w * 4.f) {
+                    // seen only through the neighbour's h: only when its
+                    // cell lies in the particle's box
+                    const int cx = (int)floorf(__fdiv_rn(Aj[e].x, kCellWidth)),
+                              cy = (int)floorf(__fdiv_rn(Aj[e].y, kCellWidth)),
+                              cz = (int)floorf(__fdiv_rn(Aj[e].z, kCellWidth));
+                    hit = cx >= box.lo0 && cx <= box.hi0 && cy >= box.lo1 && cy <= box.hi1 && cz >= box.lo2 &&
+                          cz <= box.hi2;
+                }
+                if (!hit || i + e * L >= n_list) {
+                    // no pair: no mass, no relative motion, far away
+                    Aj[e] = make_float4(I.xi + 1e15f, I.yi, I.zi, 1.f);
+                    Bj[e] = make_float4(I.vxi, I.vyi, I.vzi, -1e30f);
+                    Cj[e] = make_float4(0.f, 0.f, 1.f, 0.f);
+                }
+            }
+            accel_pair2<KAHAN>(I, fac_i, S2, Aj, Bj, Cj);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                g[e] = gn[e];
+                Aj[e] = An[e];
+            }
+        }
+        AccelSum Sm = accel_close<KAHAN>(S2);
+        accel_reduce<L, false>(Sm, kFull);
+        if (live) {
+            idt = accel_ticks(I, Sm.vsig);
+            if (sub == 0) accel_store(a, a.cidx[p], Sm, idt);
+        }
+    }
+    idt = __reduce_min_sync(kFull, idt);
+    if (lane == 0 && idt < *(volatile int32_t *)(a.globals + 1)) atomicMin(a.globals + 1, idt);
 }
 
 struct StepArgs {
@@ -2374,9 +2557,9 @@ int tile_smem_opt_in() {
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!sms[dev]) {
-        cudaFuncSetAttribute(k_density_tile<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TileShared));
-        cudaFuncSetAttribute(k_density_tile<kUnitShift>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(TileShared));
+        cudaFuncSetAttribute(k_lists<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ListShared<0>));
+        cudaFuncSetAttribute(k_lists<kUnitShift>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(ListShared<kUnitShift>));
         cudaFuncSetAttribute(k_acceleration_tile<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(TileAccShared));
         cudaFuncSetAttribute(k_acceleration_tile<true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2392,15 +2575,17 @@ int tile_smem_opt_in() {
     return sms[dev];
 }
 
-// Persistent CTAs of the tile passes: two per SM, but no more than one per
-// ~48 particles (a tile holds ~100-300), so a small context -- an ensemble
-// instance -- leaves the rest of the device to the others.
-unsigned tile_grid(int n, int sms) {
+// Persistent CTAs of the tile passes: as many as are resident, but no more
+// than one per ~48 particles (a tile holds ~100-300), so a small context -- an
+// ensemble instance -- leaves the rest of the device to the others.
+unsigned tile_grid(int n, int resident) {
     const int want = (n + 47) / 48;
-    return (unsigned)std::max(1, std::min(sms * 2, want));
+    return (unsigned)std::max(1, std::min(resident, want));
 }
 
 }  // namespace
+
+size_t neighbour_list_entries(int n) { return (size_t)n * kTileList; }
 
 sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     const int n = ctx->n;
@@ -2418,6 +2603,7 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     a.coarse = ctx->tile_coarse;
     a.mode = ctx->tile_mode;
     a.start_h = ctx->tile_h;
+    a.lists = NeighbourLists{ctx->nlist, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     a.sp4 = ctx->sp4;
     a.sv4 = ctx->sv4;
     a.h = ctx->h;
@@ -2459,22 +2645,29 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     // one lane per particle, in the reference's order
     k_density<kLanesPerParticle><<<(unsigned)((n + parts - 1) / parts), parts * kLanesPerParticle, smem, st>>>(a);
 #else
-    // cell tiles, then the coarse tiles of the blocks they flagged (the tile
-    // list is reused), then the per-particle pass over what both deferred
+    // the lists over cell tiles, then over the coarse tiles of the flagged
+    // blocks (the tile list is reused); the iteration; the per-particle pass
+    // over what it deferred
     const int sms = tile_smem_opt_in();
     uint32_t *ctr = ctx->tile_ctr;
     cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * 8, st);
+    cudaMemsetAsync(ctx->grown, 0, sizeof(int) * kNumUnits, st);
     k_density_plan<<<(n + 255) / 256, 256, 0, st>>>(a, ctx->tiles, ctr, ctx->tile_block_max, ctx->tile_half_max,
                                                     ctx->tile_big_max);
-    const unsigned tgrid = tile_grid(n, sms);
-    k_density_tile<0><<<tgrid, kTileThreads, sizeof(TileShared), st>>>(a, ctx->tiles, ctr, ctx->deferred, ctr + 2);
-    if (a.coarse) {
+    // (without the lists' storage every particle is left to the walk)
+    if (ctx->nlist)
+        k_lists<0><<<tile_grid(n, sms * ListTile<0>::kCtas), ListTile<0>::kThreads, sizeof(ListShared<0>), st>>>(
+            a, ctx->tiles, ctr);
+    if (ctx->nlist && a.coarse) {
+        constexpr int U = kUnitShift;
         k_coarse_starts<<<(n + 255) / 256, 256, 0, st>>>(n, a.skey, ctx->units, ctx->coarse_flags, ctx->tiles,
                                                          ctr + 4);
-        k_density_tile<kUnitShift>
-            <<<tgrid, kTileThreads, sizeof(TileShared), st>>>(a, ctx->tiles, ctr + 4, ctx->deferred, ctr + 2);
+        k_lists<U><<<tile_grid(n, sms * ListTile<U>::kCtas), ListTile<U>::kThreads, sizeof(ListShared<U>), st>>>(
+            a, ctx->tiles, ctr + 4);
     }
-    k_density_deferred<kWalkLanes><<<tgrid * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(
+    const unsigned lgrid = (unsigned)(((int64_t)n * kTileLanes + kListThreads - 1) / kListThreads);
+    k_density_list<<<lgrid, kListThreads, 0, st>>>(a, ctx->deferred, ctr + 2);
+    k_density_deferred<kWalkLanes><<<tile_grid(n, sms * 2) * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(
         a, ctx->deferred, ctr + 2);
 #endif
     if (ctx->hs.capture) s = launch_hseed_targets(ctx, st);
@@ -2495,6 +2688,7 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     a.cflags = ctx->coarse_flags;
     a.coarse = ctx->tile_coarse;
     a.mode = ctx->tile_mode;
+    a.lists = NeighbourLists{ctx->nlist, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     a.sA = ctx->sA;
     a.sB = ctx->sB;
     a.sC = ctx->sC;
@@ -2523,8 +2717,13 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     cudaMemsetAsync(ctr, 0, sizeof(uint32_t) * 8, st);
     k_acceleration_plan<<<(n + 255) / 256, 256, 0, st>>>(a, ctx->tiles, ctr, ctx->tile_block_max,
                                                          ctx->tile_half_max, ctx->tile_big_max);
-    const unsigned tgrid = tile_grid(n, sms);
+    const unsigned tgrid = tile_grid(n, sms * 2);
     const size_t tsm = sizeof(TileAccShared);
+    if (ctx->nlist) {
+        const unsigned lgrid = (unsigned)(((int64_t)n * kTileLanes + kListThreads - 1) / kListThreads);
+        if (kahan) k_acceleration_list<true><<<lgrid, kListThreads, 0, st>>>(a);
+        else k_acceleration_list<false><<<lgrid, kListThreads, 0, st>>>(a);
+    }
     if (kahan)
         k_acceleration_tile<true, 0><<<tgrid, kTileThreads, tsm, st>>>(a, ctx->tiles, ctr, ctx->deferred, ctr + 2);
     else

@@ -175,6 +175,12 @@ struct sph_ctx {
     uint32_t *deferred = nullptr;
     uint8_t *tile_mode = nullptr;  // [n] the pass that takes each sorted particle
     float *tile_h = nullptr;       // [n] density: the h its staged box is built for
+    // neighbour lists of the density tiles, read by the acceleration pass
+    // (none when their storage could not be had: the tiles look again)
+    uint32_t *nlist = nullptr;
+    uint8_t *nlist_count = nullptr;
+    float *nlist_reach2 = nullptr;
+    int *grown = nullptr;          // per 64-cell unit
     // tile sizes: a 128-cell block is one tile up to tile_big_max particles
     // (0: never; measured slower at N = 1e6: such tiles overflow shared memory
     // and fall back to octets), else its 64-cell halves up to tile_block_max,
@@ -232,6 +238,7 @@ sph_status launch_sort(sph_ctx *ctx, cudaStream_t st);
 void launch_init_cells(sph_ctx *ctx, cudaStream_t st);
 
 // sph_hydro.cu
+size_t neighbour_list_entries(int n);
 sph_status launch_density(sph_ctx *ctx, cudaStream_t st);
 sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st);
 sph_status launch_step(sph_ctx *ctx, cudaStream_t st);

@@ -276,7 +276,8 @@ __device__ __forceinline__ int group_collect(float px, float py, float pz, float
 struct NeighbourLists {
     uint32_t *entries;  // [n][kTileList] sorted indices
     uint8_t *count;     // [n], kNoList: none
-    float *reach2;      // [n] everything within this squared distance is listed
+    float *reach2;      // [n] everything within this squared distance is listed;
+                        // negative: nothing else is (no use to the acceleration pass)
     int *grown;         // [units] float bits, 0: none
 };
 constexpr uint8_t kNoList = 0xff;
@@ -615,7 +616,7 @@ constexpr int kTileCellsMax = 1024;                         // units of a tile's
 #define SPH_TILE_REACH_CELLS 3
 #endif
 constexpr int kTileReach = SPH_TILE_REACH_CELLS;            // units a list box may extend past its own
-constexpr int kTileList = 160;                              // list entries per particle
+constexpr int kTileList = 192;                              // list entries per particle
 #ifndef SPH_TILE_LIST_REACH
 #define SPH_TILE_LIST_REACH 1.08f
 #endif
@@ -660,6 +661,7 @@ struct ListShared {
     uint32_t start, end, tile, next;
     int defer_all;
     int need;                              // some particle of the range needs the warp pass
+    float reach;                           // staged box radius / (2 h)
 };
 
 // The list box of a tile particle at smoothing length hb: the cells within
@@ -993,18 +995,21 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
         me = a.sp4[p];
         hb = a.start_h[p];
     }
-    // a second search, wider, for the particles that found too few neighbours
+    // a second search: wider, for the particles that found too few neighbours
     // for their h to stay within the first one's reach (a body's surface at its
-    // first step)
+    // first step), or just as far as the iteration's first sweep needs, for
+    // those that found more than a list holds (a body that contracts)
+    float hscale = kFar2;  // 0: the neighbours' own reach does not count
+    bool narrow = false;
     for (int round = 0; round < 2; ++round) {
         CellBox b;
         b.lo0 = b.lo1 = b.lo2 = kBig;
         b.hi0 = b.hi1 = b.hi2 = -kBig;
         if (want) {
             tile_box(me.x, me.y, me.z, hb, b);
-            if (round == 1 && ((b.lo0 >> us) < lo0 || (b.lo1 >> us) < lo1 || (b.lo2 >> us) < lo2 ||
+            if (round == 1 && !narrow && ((b.lo0 >> us) < lo0 || (b.lo1 >> us) < lo1 || (b.lo2 >> us) < lo2 ||
                                (b.hi0 >> us) > hi0 || (b.hi1 >> us) > hi1 || (b.hi2 >> us) > hi2)) {
-                hb = a.start_h[p] * (kTileStageReach / kTileListReach);  // what is staged for it
+                hb = a.start_h[p] * (S.reach / kTileListReach);  // what is staged for it
                 tile_box(me.x, me.y, me.z, hb, b);
             }
             b.lo0 = max(b.lo0 >> us, lo0), b.lo1 = max(b.lo1 >> us, lo1), b.lo2 = max(b.lo2 >> us, lo2);
@@ -1082,7 +1087,7 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
                 if (v < total) {
                     q = S.pos[s];
                     const float h = S.hs[s];
-                    hr = kFar2 * h * h;
+                    hr = hscale * h * h;
                     gi = S.gidx[s];
                 }
                 const F2 qx = f2(q.x), qy = f2(q.y), qz = f2(q.z);
@@ -1110,12 +1115,23 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
                 if (g == k) c = cnt[k];
             if (sub == 0) {
                 a.lists.count[p] = c <= kTileList ? (uint8_t)c : kNoList;
-                a.lists.reach2[p] = r2;
+                a.lists.reach2[p] = hscale > 0.f ? r2 : -r2;
             }
             const float to = hb * cbrtf(kListFull / (float)max(c, 1));
-            want = round == 0 && to > kTileListReach * hb && to < kMaxH;
-            if (want) hb = fminf(1.02f * to, 0.999f * kMaxH);
+            narrow = c > kTileList;
+            want = round == 0 && (narrow || (to > kTileListReach * hb && to < kMaxH && S.reach > kTileListReach));
+            if (want && narrow) {
+                const uint32_t ind = a.cidx[p];
+                const float h_plain = a.h[ind];
+                bool seeded;
+                hb = fmaxf(tile_start_h(a, ind, h_plain, seeded), h_plain) * (1.00001f / kTileListReach);
+            } else if (want) {
+                hb = fminf(1.02f * to, 0.999f * kMaxH);
+            }
         }
+        // (a warp's second searches are alike: rare, and the test of a slot
+        // stays the same for all)
+        if (__any_sync(kFull, want && narrow)) hscale = 0.f;
     }
 }
 
@@ -1146,20 +1162,25 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
         if (S.tile >= ntiles) break;
         const uint32_t tstart = S.start, tend = S.end;
         // a tile whose staged box overflows shared memory is taken again as
-        // its octets (coarse tiles: its units), one at a time; one that still
-        // overflows is left to the per-particle pass
-        constexpr int kSplit = U == 0 ? 3 : 3 * U;
+        // its octets (coarse tiles: its units), one at a time, an octet that
+        // still does as its cells (a unit: its octets) and without the margin
+        // for wider searches (a body under compression); what overflows even
+        // so is left to the per-particle pass
+        constexpr int kSplit = U == 0 ? 3 : 3 * U, kSplit2 = kSplit - 3;
         const bool splittable = (a.skey[tstart] >> kSplit) != (a.skey[tend - 1] >> kSplit);
-        bool whole = true;
+        int level = 0;  // 0 the tile, 1 its octets, 2 their cells
         uint32_t r0 = tstart;
         while (r0 < tend) {
             __syncthreads();
             if (tid == 0) {
                 uint32_t r1 = tend;
-                if (!whole) {  // the rest of r0's octet / unit
-                    const uint32_t o = a.skey[r0] >> kSplit;
-                    r1 = max(r0 + 1u, (U == 0 ? a.octets : a.units)[o].y + 1u);
+                if (level == 1) {  // the rest of r0's octet / unit
+                    r1 = (U == 0 ? a.octets : a.units)[a.skey[r0] >> kSplit].y + 1u;
+                } else if (level == 2) {
+                    r1 = (U == 0 ? a.cells : a.octets)[a.skey[r0] >> kSplit2].y + 1u;
                 }
+                r1 = min(max(r0 + 1u, r1), tend);
+                S.reach = level < 2 ? kTileStageReach : kTileListReach;
                 S.end = r1;
                 S.next = 0u;
                 S.box[0] = S.box[1] = S.box[2] = 0x7fffffff;
@@ -1179,7 +1200,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
                     need = true;
                     const float4 me = a.sp4[p];
                     CellBox cb;
-                    tile_box(me.x, me.y, me.z, a.start_h[p], cb, kTileStageReach);
+                    tile_box(me.x, me.y, me.z, a.start_h[p], cb, S.reach);
                     b[0] = min(b[0], cb.lo0);
                     b[1] = min(b[1], cb.lo1);
                     b[2] = min(b[2], cb.lo2);
@@ -1254,7 +1275,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
             }
             __syncthreads();
             if (S.defer_all) {
-                if (whole && splittable) whole = false;
+                if (level < 2) level = level == 0 && splittable ? 1 : 2;
                 else r0 = end;  // its particles are left without a list
                 continue;
             }
@@ -1278,6 +1299,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
                 lists_tile_warp<U>(a, S, start + j, end, lane);
             }
             r0 = end;
+            if (level == 2 && r0 < tend && ((a.skey[r0] ^ a.skey[r0 - 1u]) >> kSplit) != 0u) level = 1;
         }
     }
 }
@@ -1337,7 +1359,7 @@ __global__ void __launch_bounds__(kListThreads, 4)
             defer();
         } else {
             n_list = c;
-            list_r2 = a.lists.reach2[p];
+            list_r2 = fabsf(a.lists.reach2[p]);
             hi = tile_start_h(a, ind, h_plain, seeded);
         }
     }
@@ -1844,6 +1866,7 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L)
 // the budget go to k_acceleration_deferred.
 constexpr int kTileThreads = 384;
 constexpr int kTileGroups = kTileThreads / kTileLanes;  // particles in flight per CTA
+constexpr int kTileAccList = 256;                       // list entries per particle
 constexpr int kTileAccStage = 3072;                     // staged particles per tile
 constexpr int kTileCellsPerThread = (kTileCellsMax + kTileThreads - 1) / kTileThreads;
 
@@ -1852,7 +1875,7 @@ struct TileAccShared {
     uint32_t gidx[kTileAccStage];       // staged sorted index
     uint32_t scell[kTileAccStage];      // staged cell, box-relative (pack_cell)
     uint32_t off[kTileCellsMax + 1];
-    uint16_t list[kTileGroups][kTileList];
+    uint16_t list[kTileGroups][kTileAccList];
     int box[6];
     uint32_t wsum[kTileThreads / 32];
     uint32_t start, end, tile, next;
@@ -1970,7 +1993,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
         ny2[k] = f2(-__shfl_sync(kFull, I.yi, 2 * k * L), -__shfl_sync(kFull, I.yi, (2 * k + 1) * L));
         nz2[k] = f2(-__shfl_sync(kFull, I.zi, 2 * k * L), -__shfl_sync(kFull, I.zi, (2 * k + 1) * L));
     }
-    uint16_t (*const lists)[kTileList] = &S.list[wslot * kTileGpw];
+    uint16_t (*const lists)[kTileAccList] = &S.list[wslot * kTileGpw];
     int cnt[kTileGpw] = {};
     const unsigned below = (1u << lane) - 1u;
     const int nyu = v1 - u1 + 1;
@@ -2031,7 +2054,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
                 const bool hit = d[k] >= 1e-12f && (d[k] <= qr[k] || (d[k] <= hj2x4 && in_box(sc, klo[k], khi[k])));
                 const unsigned bal = __ballot_sync(kFull, hit);
                 const int at = cnt[k] + __popc(bal & below);
-                if (hit && at < kTileList) lists[k][at] = (uint16_t)s;
+                if (hit && at < kTileAccList) lists[k][at] = (uint16_t)s;
                 cnt[k] += __popc(bal);
             }
         }
@@ -2041,7 +2064,7 @@ __device__ __forceinline__ int accel_tile_warp(const AccelArgs &a, TileAccShared
 #pragma unroll
     for (int k = 0; k < kTileGpw; ++k)
         if (g == k) n_list = cnt[k];
-    if (live && n_list > kTileList) {
+    if (live && n_list > kTileAccList) {
         if (sub == 0) deferred[atomicAdd(dctr, 1u)] = p;
         live = false;
     }
@@ -2084,7 +2107,8 @@ __global__ void __launch_bounds__(256) k_acceleration_plan(AccelArgs a, uint2 *t
         const int m = accel_mode(A.x, A.y, A.z, A.w, b, a.coarse);
         if (m < 0) return kModeWalk;
         // the list is complete when no neighbour the box can hold has outgrown it
-        // (a NaN h counts as larger than any)
+        // (a NaN h counts as larger than any; a list without the neighbours' own
+        // reach has a negative one)
         if (a.lists.entries && a.lists.count[p] != kNoList) {
             int grown = 0;
             for (int x = b.lo0 >> kUnitShift; x <= b.hi0 >> kUnitShift; ++x)

@@ -115,17 +115,21 @@ def test_opening_angle_gravity_matches_the_direct_sum(cuda, pkg, n, leaf, side):
     assert np.allclose(gn * 6.67e-5, np.linalg.norm(acc, axis=1), rtol=1e-5)
 
 
-# lists that fit the lanes' registers, that do not (h too large), and that fit
-# no list; unequal masses; cell tiles (n = 4e5, small h), octets, units
-@pytest.mark.parametrize("n,scale,masses", [(4000, 1.0, False), (20480, 1.0, True), (20480, 1.2, False),
-                                            (20480, 1.5, True), (60000, 1.0, True), (60000, 0.7, False),
-                                            (100000, 1.25, False), (400000, 1.0, False), (400000, 1.3, True)])
+# lists that fit the lanes' registers, that do not (h too large), that hold only
+# the first sweep's neighbours, and that fit no list; unequal masses; cell tiles
+# (n = 4e5, small h), octets, units; bodies so dense that a tile's box does not
+# fit the staging and is split (squeeze)
+@pytest.mark.parametrize("n,scale,masses,squeeze", [
+    (4000, 1.0, False, 1.0), (20480, 1.0, True, 1.0), (20480, 1.2, False, 1.0), (20480, 1.5, True, 1.0),
+    (60000, 1.0, True, 1.0), (60000, 0.7, False, 1.0), (60000, 1.35, False, 1.0), (100000, 1.25, False, 1.0),
+    (100000, 0.8, True, 0.7), (400000, 1.0, False, 1.0), (400000, 1.3, True, 1.0), (400000, 0.9, False, 0.8)])
 @pytest.mark.parametrize("precision", ["reference", "mixed"])
-def test_hydro_matches_the_parity_build(cuda, pkg, n, scale, masses, precision):
+def test_hydro_matches_the_parity_build(cuda, pkg, n, scale, masses, squeeze, precision):
     if precision == "mixed" and n > 100000:
         pytest.skip("the plain sums cover the large sizes")
     rng = np.random.default_rng(n)
     ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=5)
+    ic["pos"] = (ic["pos"] * np.float32(squeeze)).astype(np.float32)
     ic["h"] = np.minimum(ic["h"] * np.float32(scale) * rng.uniform(0.95, 1.05, n), 0.99).astype(np.float32)
     ic["vel"] = (ic["vel"] + rng.normal(size=(n, 3)) * 1e-3).astype(np.float32)
     if masses:

@@ -37,20 +37,23 @@ struct RadixSorter {
     // one allocation, cleared by radix_clear before a sort:
     uint32_t *hist = nullptr;     // [kMaxPasses][256] digit counts, filled by the key producer
     uint32_t *counters = nullptr; // [kMaxPasses] tile tickets
-    uint32_t *status = nullptr;   // [passes][tiles][256] look-back words
+    uint32_t *status = nullptr;   // [passes][tiles + groups of tiles][256] look-back words
     int n_cap = 0;
     int spin_limit = 1 << 22;     // polls before a look-back wait gives up
     static constexpr int kThreads = 256;
     static constexpr int kMaxPasses = 4;
     // Keys per thread, so that small sorts still spread over the device's SMs
-    // (a tile is one block) and large ones do not pay the per-tile work, 256
-    // digits' look-back, more often than needed (whole
-    // sort, N = 2e4: 46 us with 16 keys a thread, 27 with 4)
-    static constexpr int kMinItems = 4;
+    // (a tile is one block) and large ones have few tiles: 256 digits' look-back
+    // per tile, and waiting tiles' polls hold up the words they wait for.
+    // Whole sort in us, N = 1e5, 3e5, 5e5, 1e6: 4 keys 38, 47, 77, 286; 8 keys
+    // 42, 43, 54, 93; 16 keys 49, 53, 55, 76.
+    static constexpr int kMinItems = 4, kMaxItems = 16;
+    static constexpr int kGroup = 16;  // tiles per look-back group
     static int items(int n) {
-        return n <= (1 << 18) ? 4 : n <= (1 << 21) ? 8 : 16;
+        return n <= (1 << 18) ? 4 : n <= (1 << 19) ? 8 : 16;
     }
     static int tiles(int n) { return (n + kThreads * items(n) - 1) / (kThreads * items(n)); }
+    static constexpr size_t rows(int tiles) { return (size_t)tiles + (tiles + kGroup - 1) / kGroup; }
 };
 
 // Device-resident octree in the reference's flattened format plus the node

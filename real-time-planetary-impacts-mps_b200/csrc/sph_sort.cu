@@ -31,6 +31,9 @@ namespace {
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kValueMask = (1u << 30) - 1u;
+constexpr uint32_t kArrived = 1u << 27;  // group words: tiles added, above the sum of their counts
+static_assert(RadixSorter::kGroup * RadixSorter::kThreads * RadixSorter::kMaxItems < kArrived &&
+                  RadixSorter::kGroup < 32, "group words");
 constexpr int kSpinLimit = 1 << 22;
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
@@ -96,10 +99,13 @@ template <int ITEMS>
 __global__ void __launch_bounds__(RadixSorter::kThreads)
     k_onesweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int n, int shift,
-               const uint32_t *__restrict__ hist, uint32_t *status, uint32_t *counter, uint32_t *health,
+               const uint32_t *__restrict__ hist, uint32_t *status, int tiles, uint32_t *counter, uint32_t *health,
                int spin_limit) {
-    constexpr int T = RadixSorter::kThreads, I = ITEMS, W = T / 32;
-    constexpr int kWindow = 8;  // look-back words read at a time
+    constexpr int T = RadixSorter::kThreads, I = ITEMS, W = T / 32, G = RadixSorter::kGroup;
+    // tiles, groups read at a time (the polls of all waiting tiles meet in a few
+    // lines of L2: with twice as many, N = 1e6 in tiles of 2048 keys takes 171
+    // instead of 93 us)
+    constexpr int kWindow = 4, kGroupWindow = 4;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[W][256];
     __shared__ uint32_t s_base[256];
@@ -153,42 +159,68 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
         s_warp[w][tid] = tile_count;
         tile_count += c;
     }
-    // decoupled look-back for digit `tid`, kWindow predecessors per round trip
-    // (the words carry the counts themselves: nothing else has to be ordered)
+    // Decoupled look-back for digit `tid` (the words carry the counts
+    // themselves: nothing else has to be ordered).  All tiles of a sort of 1e6
+    // keys run at once, so that most words hold only their own tile's count and
+    // a walk over single tiles reads all before it.  So a tile also adds its
+    // count to its group's word, and the walk goes by tiles to the group's start
+    // and then by groups, whichever of a group's sum and its last tile's prefix
+    // is there.
     uint32_t excl = 0;
     volatile uint32_t *vs = status;
-    if (tile == 0) {
-        vs[tid] = kFlagPrefix | tile_count;
-    } else {
-        vs[(size_t)tile * 256 + tid] = kFlagAgg | tile_count;
-        int64_t j = (int64_t)tile - 1;
-        int spins = 0;
-        bool done = false;
-        while (!done) {
-            uint32_t s[kWindow];
+    uint32_t *const groups = status + (size_t)tiles * 256;
+    volatile uint32_t *vg = groups;
+    const int64_t group = tile / G, first = group * G;
+    vs[(size_t)tile * 256 + tid] = (tile == 0 ? kFlagPrefix : kFlagAgg) | tile_count;
+    if (tiles > G) atomicAdd(groups + group * 256 + tid, kArrived | tile_count);
+    int spins = 0;
+    bool done = tile == 0;
+    auto wait = [&]() {  // false: given up
+        if (++spins > spin_limit) {
+            raise_health(health, SPH_HEALTH_SORT_TIMEOUT);
+            return false;
+        }
+        __nanosleep(32);
+        return true;
+    };
+    for (int64_t j = (int64_t)tile - 1; !done && j >= first;) {
+        uint32_t s[kWindow];
 #pragma unroll
-            for (int q = 0; q < kWindow; ++q) s[q] = j - q >= 0 ? vs[(size_t)(j - q) * 256 + tid] : 2u << 30;
-            int got = 0;
+        for (int q = 0; q < kWindow; ++q) s[q] = j - q >= first ? vs[(size_t)(j - q) * 256 + tid] : 0u;
+        int got = 0;
 #pragma unroll
-            for (int q = 0; q < kWindow; ++q) {
-                const uint32_t flag = s[q] & ~kValueMask;
-                if (!done && got == q && flag != 0u) {
-                    excl += s[q] & kValueMask;
-                    ++got;
-                    done = flag == kFlagPrefix;
-                }
-            }
-            j -= got;
-            if (got == 0) {
-                if (++spins > spin_limit) {
-                    raise_health(health, SPH_HEALTH_SORT_TIMEOUT);
-                    break;
-                }
-                __nanosleep(32);
+        for (int q = 0; q < kWindow; ++q) {
+            const uint32_t flag = s[q] & ~kValueMask;
+            if (!done && got == q && flag != 0u) {
+                excl += s[q] & kValueMask;
+                ++got;
+                done = flag == kFlagPrefix;
             }
         }
-        vs[(size_t)tile * 256 + tid] = kFlagPrefix | ((excl + tile_count) & kValueMask);
+        j -= got;
+        if (got == 0 && !wait()) done = true;
     }
+    for (int64_t j = group - 1; !done && j >= 0;) {
+        uint32_t s[kGroupWindow], e[kGroupWindow];
+#pragma unroll
+        for (int q = 0; q < kGroupWindow; ++q) {
+            s[q] = j - q >= 0 ? vg[(size_t)(j - q) * 256 + tid] : 0u;
+            e[q] = j - q >= 0 ? vs[(size_t)((j - q) * G + G - 1) * 256 + tid] : 0u;
+        }
+        int got = 0;
+#pragma unroll
+        for (int q = 0; q < kGroupWindow; ++q) {
+            const bool prefix = (e[q] & ~kValueMask) == kFlagPrefix;
+            if (!done && got == q && (prefix || s[q] / kArrived == G)) {
+                excl += prefix ? e[q] & kValueMask : s[q] % kArrived;
+                ++got;
+                done = prefix;
+            }
+        }
+        j -= got;
+        if (got == 0 && !wait()) done = true;
+    }
+    if (tile != 0) vs[(size_t)tile * 256 + tid] = kFlagPrefix | ((excl + tile_count) & kValueMask);
     s_base[tid] = global_excl + excl;
     __syncthreads();
 #pragma unroll
@@ -211,7 +243,7 @@ void launch_onesweep(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t 
     const int tiles = RadixSorter::tiles(n), items = RadixSorter::items(n);
     auto *kernel = items == 4 ? k_onesweep<4> : items == 8 ? k_onesweep<8> : k_onesweep<16>;
     kernel<<<tiles, RadixSorter::kThreads, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n, shift, hist, status,
-                                                    counter, health, spin_limit);
+                                                    tiles, counter, health, spin_limit);
 }
 
 // Each occupied cell's (first, last) sorted index, and each occupied octet's
@@ -240,7 +272,7 @@ __global__ void k_init_cells(uint2 *cell_range, uint32_t count) {
 sph_status sort_alloc(RadixSorter &s, int n) {
     s.n_cap = n;
     constexpr int kMinTile = RadixSorter::kThreads * RadixSorter::kMinItems;
-    const size_t tiles = (size_t)std::max(1, (n + kMinTile - 1) / kMinTile);
+    const size_t rows = RadixSorter::rows(std::max(1, (n + kMinTile - 1) / kMinTile));
     constexpr size_t kHead = 256 * RadixSorter::kMaxPasses + RadixSorter::kMaxPasses;
     size_t nb = sizeof(uint32_t) * (size_t)(n > 0 ? n : 1);
     cudaError_t e = cudaSuccess;
@@ -248,7 +280,7 @@ sph_status sort_alloc(RadixSorter &s, int n) {
         if (e == cudaSuccess) e = cudaMalloc(&s.keys[b], nb);
         if (e == cudaSuccess) e = cudaMalloc(&s.vals[b], nb);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&s.hist, sizeof(uint32_t) * (kHead + 256 * tiles * RadixSorter::kMaxPasses));
+    if (e == cudaSuccess) e = cudaMalloc(&s.hist, sizeof(uint32_t) * (kHead + 256 * rows * RadixSorter::kMaxPasses));
     s.counters = s.hist + 256 * RadixSorter::kMaxPasses;
     s.status = s.hist + kHead;
     return cuda_status(e, "sort_alloc");
@@ -265,7 +297,7 @@ void sort_free(RadixSorter &s) {
 }
 
 void radix_clear(RadixSorter &s, int n, int bits, cudaStream_t st) {
-    const size_t words = (size_t)(s.status - s.hist) + 256 * (size_t)RadixSorter::tiles(n) * ((bits + 7) / 8);
+    const size_t words = (size_t)(s.status - s.hist) + 256 * RadixSorter::rows(RadixSorter::tiles(n)) * ((bits + 7) / 8);
     cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * words, st);
 }
 
@@ -275,7 +307,7 @@ int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t 
     if (n <= 0) return 0;
     for (int p = 0; p < passes; ++p) {
         launch_onesweep(s.keys[cur], s.vals[cur], s.keys[cur ^ 1], s.vals[cur ^ 1], n, 8 * p, s.hist + 256 * p,
-                        s.status + (size_t)256 * RadixSorter::tiles(n) * p, s.counters + p, health, s.spin_limit, st);
+                        s.status + 256 * RadixSorter::rows(RadixSorter::tiles(n)) * p, s.counters + p, health, s.spin_limit, st);
         cur ^= 1;
     }
     return cur;
@@ -349,12 +381,12 @@ constexpr size_t kNoAllocKeysOff = 0;
 constexpr size_t kNoAllocValsOff = kNoAllocKeysOff + sizeof(uint32_t) * SPH_SORT_NOALLOC_MAX_N;
 // the words that must be zero when a call starts sit together from here on:
 // histograms, tile tickets, the health word, then the look-back words of the
-// three passes, each pass using 256 x (tiles of this call) words
+// three passes, each pass using 256 x (rows of this call) words
 constexpr size_t kNoAllocHistOff = kNoAllocValsOff + sizeof(uint32_t) * SPH_SORT_NOALLOC_MAX_N;
 constexpr size_t kNoAllocCountOff = kNoAllocHistOff + sizeof(uint32_t) * 256 * kNoAllocPasses;
 constexpr size_t kNoAllocHealthOff = kNoAllocCountOff + sizeof(uint32_t) * kNoAllocPasses;
 constexpr size_t kNoAllocStatusOff = kNoAllocHealthOff + sizeof(uint32_t);
-constexpr size_t kNoAllocScratchBytes = kNoAllocStatusOff + sizeof(uint32_t) * 256 * kNoAllocTiles * kNoAllocPasses;
+constexpr size_t kNoAllocScratchBytes = kNoAllocStatusOff + sizeof(uint32_t) * 256 * RadixSorter::rows(kNoAllocTiles) * kNoAllocPasses;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -410,14 +442,14 @@ extern "C" sph_status sph_sort_cells_noalloc(const float *pos_xyz, int32_t n, ui
     sph_status st = noalloc_scratch(&s);
     if (st != SPH_OK) return st;
     cudaStream_t cs = (cudaStream_t)stream;
-    const int tiles = RadixSorter::tiles(n);
+    const size_t rows = RadixSorter::rows(RadixSorter::tiles(n));
     uint32_t *tk = reinterpret_cast<uint32_t *>(s + kNoAllocKeysOff);
     uint32_t *tv = reinterpret_cast<uint32_t *>(s + kNoAllocValsOff);
     uint32_t *hist = reinterpret_cast<uint32_t *>(s + kNoAllocHistOff);
     uint32_t *counters = reinterpret_cast<uint32_t *>(s + kNoAllocCountOff);
     uint32_t *health = reinterpret_cast<uint32_t *>(s + kNoAllocHealthOff);
     uint32_t *status = reinterpret_cast<uint32_t *>(s + kNoAllocStatusOff);
-    const size_t zero_bytes = (kNoAllocStatusOff - kNoAllocHistOff) + sizeof(uint32_t) * 256 * (size_t)tiles * kNoAllocPasses;
+    const size_t zero_bytes = (kNoAllocStatusOff - kNoAllocHistOff) + sizeof(uint32_t) * 256 * rows * kNoAllocPasses;
     cudaError_t e = cudaMemsetAsync(s + kNoAllocHistOff, 0, zero_bytes, cs);
     if (e != cudaSuccess) return cuda_status(e, "sph_sort_cells_noalloc: clear scratch");
     k_hash_hist_xyz<<<hash_grid(n), kHashThreads, 0, cs>>>(pos_xyz, n, tk, tv, hist);
@@ -428,7 +460,7 @@ extern "C" sph_status sph_sort_cells_noalloc(const float *pos_xyz, int32_t n, ui
     uint32_t *vout[kNoAllocPasses] = {cell_index, tv, cell_index};
     for (int p = 0; p < kNoAllocPasses; ++p)
         launch_onesweep(kin[p], vin[p], kout[p], vout[p], n, 8 * p, hist + 256 * p,
-                        status + (size_t)256 * tiles * p, counters + p, health, kSpinLimit, cs);
+                        status + 256 * rows * p, counters + p, health, kSpinLimit, cs);
     return cuda_status(cudaGetLastError(), "sph_sort_cells_noalloc");
 }
 
@@ -464,6 +496,7 @@ __global__ void k_selftest_prepare(uint32_t *hist, uint32_t *status, uint32_t *c
     hist[t] = 0u;
     status[t] = 0u;
     status[256 + t] = 0u;
+    status[512 + t] = 0u;  // the group's word
     if (t == 0) *counter = 1u;
 }
 }  // namespace
@@ -499,7 +532,7 @@ extern "C" sph_status sph_selftest_lookback_timeout(sph_ctx *ctx, int32_t spin_l
     }
     // the key/value buffers are valid device memory, though n = 0 touches none
     k_selftest_prepare<<<1, 256, 0, cs>>>(hist, status, counter);
-    k_onesweep<RadixSorter::kMinItems><<<1, RadixSorter::kThreads, 0, cs>>>(kbuf, vbuf, kbuf, vbuf, 0, 0, hist, status, counter,
-                                                    health, spin_limit);
+    k_onesweep<RadixSorter::kMinItems><<<1, RadixSorter::kThreads, 0, cs>>>(kbuf, vbuf, kbuf, vbuf, 0, 0, hist, status, 2,
+                                                                            counter, health, spin_limit);
     return cuda_status(cudaGetLastError(), "sph_selftest_lookback_timeout");
 }

@@ -38,8 +38,10 @@ def _rel(a, b):
     return np.abs(a - b) / np.maximum(np.abs(b), floor)
 
 
-# keys per thread change at 2^18 and 2^21 particles; a tile is 256 threads' keys
-@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 262143, 262144, 262145, (1 << 21) + 1])
+# keys per thread change at 2^18 and 2^19 particles; a tile is 256 threads' keys,
+# a look-back group 16 tiles
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 16384, 16385, 262143, 262144, 262145, 524288, 524289,
+                               (1 << 21) + 1])
 def test_sort_at_its_tile_sizes(cuda, pkg, n):
     import torch
 

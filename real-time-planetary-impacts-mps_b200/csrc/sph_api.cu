@@ -424,9 +424,16 @@ sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out)
         sph_destroy(ctx);
         return s;
     }
-    // the neighbour lists (640 B a particle) are worth their storage but not
-    // needed: without it the acceleration pass looks for the neighbours again
-    if (dmalloc(&ctx->nlist, neighbour_list_entries(n)) != cudaSuccess) {
+    // The neighbour lists (768 B a particle) are worth their storage but not
+    // needed: without it density walks the cells particle by particle and the
+    // acceleration tiles search for themselves.  Taken only when 256 B a
+    // particle stay free for what is allocated later (FP64 positions, the
+    // learned seed's records, a larger tree).
+    size_t free_bytes = 0, total_bytes = 0;
+    const size_t entries = neighbour_list_entries(n);
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess ||
+        free_bytes / 256 < entries * sizeof(uint32_t) / 256 + (size_t)n ||
+        dmalloc(&ctx->nlist, entries) != cudaSuccess) {
         cudaGetLastError();
         ctx->nlist = nullptr;
     }

@@ -2126,7 +2126,8 @@ __global__ void __launch_bounds__(256) k_acceleration_plan(AccelArgs a, uint2 *t
 }
 
 // The acceleration tile pass U over `tiles` (ctr[0] of them, ctr[1] the
-// ticket), as k_density_tile; deferred particles are counted in *dctr.
+// ticket), staged and taken as in k_lists; deferred particles are counted in
+// *dctr.
 template <bool KAHAN, int U>
 __global__ void __launch_bounds__(kTileThreads, 2)
     k_acceleration_tile(AccelArgs a, const uint2 *__restrict__ tiles, uint32_t *ctr, uint32_t *__restrict__ deferred,

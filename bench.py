@@ -57,30 +57,29 @@ PASSES = ("tree", "sort", "gravity", "density", "acceleration", "step")
 # compulsory HBM bytes per particle per pass (each array touched once)
 ALGO_BYTES = {"tree": 76, "sort": 92, "gravity": 44, "density": 65, "acceleration": 88, "step": 92}
 PASS_KERNELS = {
-    "tree": "k_bbox, k_tree_keys, k_onesweep x3, k_children/k_emit/scan x7, k_marks, k_write, k_link",
+    "tree": "k_bbox, k_tree_keys, k_onesweep x3, k_mark, k_write, k_link",
     "sort": "k_hash_hist, k_onesweep x3, k_cells",
-    "gravity": "plain: k_up x8, k_down x8; chosen: k_up_theta x8, k_gather_key_order, k_walk",
-    "density": "k_gather, [k_mlp (learned seed)], k_tile_starts, k_density_tile, k_density_deferred",
-    "acceleration": "k_tile_starts, k_acceleration_tile, k_acceleration_deferred",
+    "gravity": "plain: k_up_all, k_down x8; chosen: k_up_theta, k_gather_key_order, k_walk",
+    "density": "k_gather, [k_mlp (learned seed)], k_density_plan, k_lists, k_density_list, k_density_deferred",
+    "acceleration": "k_acceleration_plan, k_acceleration_list, k_acceleration_tile, k_acceleration_deferred",
     "step": "k_step",
 }
 
 
 def launches_per_step(depth: int, chosen: bool, online_iters: int = 0, seed: bool | None = None) -> int:
     """Kernels of one step (memsets excluded), counted from the pass structure
-    (matches the ncu launch list: 116 plain, 131 chosen with 8 online Adam
+    (matches the ncu launch list: 37 plain, 52 chosen with 8 online Adam
     steps, at depth 7)."""
-    scan = 4  # reduce, blocks, apply, total
-    tree = 3 + 3 + 1 + depth * (1 + scan + 1) + 1 + 1 + (depth + 1) + 2 * scan + (depth + 1) + depth
-    sort = 1 + 3 + 1 + 1                 # hash, 3 passes, cells, units
-    gravity = (depth + 1) + 2 if chosen else 2 * (depth + 1)
-    # gather, tile starts, tile pass, coarse starts, coarse tile pass, deferred pass
-    density = 6
+    tree = 3 + 3 + 3                     # box (2), keys, 3 sort passes, marks, write, link
+    sort = 1 + 3 + 1                     # hash, 3 passes, cells
+    gravity = 3 if chosen else 1 + (depth + 1)
+    # gather, plan, lists, coarse starts, coarse lists, iteration, deferred pass
+    density = 7
     if chosen if seed is None else seed:
         density += 3                     # seed inference, pair capture, targets
         if online_iters > 0:
             density += 2 + 2 * online_iters  # standardisation, gradient + Adam per step
-    acceleration = 5                     # tile starts, tile pass, coarse starts, coarse pass, deferred pass
+    acceleration = 6                     # plan, list pass, tile pass, coarse starts, coarse pass, deferred pass
     return tree + sort + gravity + density + acceleration + 1
 
 

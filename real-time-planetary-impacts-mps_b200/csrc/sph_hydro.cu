@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L)
 // touches memory.  The acceleration pass reads the same lists.  (Search and
 // iteration were one kernel, whose registers and shared memory left room for
 // 24 warps per SM and whose 77 KB of code did not fit the instruction caches:
-// N = 1e6, 3.05 ms the pass; the two kernels 2.02.)
+// N = 1e6, 3.05 ms the pass; the two kernels 2.06.)
 //
 // A particle whose list box reaches more than kTileReach units beyond its own,
 // whose h is at least MAX_SMOOTHING_LENGTH (where the reference's neighbour

@@ -21,6 +21,11 @@ pytestmark = pytest.mark.gpu
 CELL = np.float32(0.18)
 
 
+@pytest.fixture(scope="module", autouse=True)
+def _parity_library(cuda, pkg):
+    pkg.build(parity=True)
+
+
 def _keys(pos):
     c = np.floor(pos.astype(np.float32) / CELL).astype(np.int64) % 256
     key = np.zeros(len(pos), np.uint32)

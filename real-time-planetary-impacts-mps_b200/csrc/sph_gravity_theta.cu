@@ -368,7 +368,9 @@ __device__ __forceinline__ void eval_parts(const PartPair *part, int np, float4 
         const F2 r2 = fma2(rz, rz, fma2(ry, ry, rx * rx));
         float r2a, r2b;
         unpack(r2, r2a, r2b);
-        if (fminf(r2a, r2b) >= soft2x4) {
+        // (both compared, so that a NaN position takes the other branch, where
+        // its pair is left out)
+        if (r2a >= soft2x4 && r2b >= soft2x4) {
             const F2 rinv = f2(rsqrt_hw(r2a), rsqrt_hw(r2b));
             const F2 mr = at2(q.c[3]) * rinv;
             const F2 s = mr * rinv * rinv;
@@ -381,6 +383,8 @@ __device__ __forceinline__ void eval_parts(const PartPair *part, int np, float4 
             unpack(rx, xa, xb);
             unpack(ry, ya, yb);
             unpack(rz, za, zb);
+            if (!(r2a > 0.f)) xa = ya = za = 0.f;
+            if (!(r2b > 0.f)) xb = yb = zb = 0.f;
             const float2 a = near_pair(r2a, q.c[3][0]), b = near_pair(r2b, q.c[3][1]);
             sx += a.x * xa + b.x * xb;
             sy += a.x * ya + b.x * yb;

@@ -122,6 +122,33 @@ def test_opening_angle_gravity_matches_the_direct_sum(cuda, pkg, n, leaf, side):
     assert np.allclose(gn * 6.67e-5, np.linalg.norm(acc, axis=1), rtol=1e-5)
 
 
+# A position that is no number (a run that blew up; sph_create refuses it, an
+# upload does not) leaves the pairs of its particle out and no others: the rest
+# feel the same as without its mass.  It stands last or in the middle of a
+# staged batch, alone in its leaf or among others.
+@pytest.mark.parametrize("n,leaf,which", [(2001, 16, (0,)), (2001, 1, (1000,)), (3000, 7, (5, 6, 2999))])
+def test_opening_angle_gravity_leaves_out_a_nan_position(cuda, pkg, n, leaf, which):
+    ic = pkg.ic.make_cube(n, seed=n, side=10.0)
+    bad = list(which)
+    rest = np.setdiff1d(np.arange(n), bad)
+    with pkg.Compute({**ic, "mass": np.where(np.isin(np.arange(n), bad), np.float32(1e-30), ic["mass"])},
+                     max_children_in_leaf=leaf, max_tree_depth=10) as c:
+        ref = c.gravity_direct_f64(rest.astype(np.int32))
+    with pkg.Compute(ic, max_children_in_leaf=leaf, max_tree_depth=10) as c:
+        c.set_form(gravity="theta", theta=0.2)
+        pos = ic["pos"].copy()
+        pos[bad] = np.float32("nan")
+        c.upload("pos", pos)
+        c.updateOctreeBuffer()
+        c.gravitationalPass()
+        c.synchronize()
+        acc, phi = c.download("acc").astype(np.float64)[rest], c.download("potential")[rest]
+    # the bounds of test_opening_angle_gravity_matches_the_direct_sum
+    scale = np.sqrt(np.mean(ref[:, :3] ** 2))
+    assert np.max(np.linalg.norm(acc - ref[:, :3], axis=1)) <= 1e-3 * scale * np.sqrt(3.0)
+    assert np.max(np.abs(phi - ref[:, 3])) <= 1e-4 * np.max(np.abs(ref[:, 3]))
+
+
 # lists that fit the lanes' registers, that do not (h too large), that hold only
 # the first sweep's neighbours, and that fit no list; unequal masses; cell tiles
 # (n = 4e5, small h), octets, units; bodies so dense that a tile's box does not

@@ -328,6 +328,14 @@ sph_status sph_sort_cells_noalloc_health(void *stream, uint32_t *word);
  * returns SPH_ERR_TIMEOUT).  The GPU stays usable; clear the word afterwards
  * (sph_clear_health, or the next sph_sort_cells_noalloc call). */
 sph_status sph_selftest_lookback_timeout(sph_ctx *ctx, int32_t spin_limit, void *stream);
+/* Self-test of what follows such a time-out (no counterpart in the reference):
+ * one tree build and one cell sort run with the first tile of every sort pass
+ * withheld and the waits limited to spin_limit polls (1..2^22), so that both
+ * sorts give up and raise SPH_HEALTH_SORT_TIMEOUT.  The passes may then run on
+ * their results (a tree of no meaning and a cell grid without particles) and
+ * stay within their buffers; the next build and sort are whole.  SPH_TREE_GPU
+ * contexts of more than 1024 particles only. */
+sph_status sph_selftest_sort_timeout(sph_ctx *ctx, int32_t spin_limit, void *stream);
 /* Self-test of the GPU tree build's capacity check (no counterpart in the
  * reference): one tree build runs with its storage bound lowered to 16 ints,
  * so the layout kernels find the tree too large, skip the writes that would

@@ -37,6 +37,7 @@ struct RadixSorter {
     // one allocation, cleared by radix_clear before a sort:
     uint32_t *hist = nullptr;     // [kMaxPasses][256] digit counts, filled by the key producer
     uint32_t *counters = nullptr; // [kMaxPasses] tile tickets
+    uint32_t *failed = nullptr;   // set by a look-back wait that gave up: the result is not sorted
     uint32_t *status = nullptr;   // [passes][tiles + groups of tiles][256] look-back words
     int n_cap = 0;
     int spin_limit = 1 << 22;     // polls before a look-back wait gives up
@@ -235,9 +236,13 @@ void sort_free(RadixSorter &s);
 void radix_clear(RadixSorter &s, int n, int bits, cudaStream_t st);
 // Sort keys[0]/vals[0] (n pairs, `bits` significant key bits) whose digit
 // histograms the producer already accumulated into s.hist.  Returns the buffer
-// index (0/1) that holds the result.
-int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t *health);
-sph_status launch_sort(sph_ctx *ctx, cudaStream_t st);
+// index (0/1) that holds the result.  After a look-back wait that gave up
+// (*s.failed) the result holds keys and values of this or earlier sorts, in
+// range but neither sorted nor a permutation; what is built on it has to look.
+// withhold: the first tile of every pass is left out, so that the others' waits
+// give up (self-test; n of more than one tile).
+int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t *health, bool withhold = false);
+sph_status launch_sort(sph_ctx *ctx, cudaStream_t st, bool withhold = false);
 void launch_init_cells(sph_ctx *ctx, cudaStream_t st);
 
 // sph_hydro.cu
@@ -277,7 +282,7 @@ sph_status launch_direct_f64(sph_ctx *ctx, const int32_t *d_targets, int nt, dou
 // sph_tree.cu
 sph_status tree_alloc(sph_ctx *ctx);
 void tree_free(sph_ctx *ctx);
-sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st);
+sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st, bool withhold = false);
 
 // sph_api.cu
 // One full step (tree, sort, gravity, density, acceleration, step) on st.

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
     k_onesweep(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, int n, int shift,
                const uint32_t *__restrict__ hist, uint32_t *status, int tiles, uint32_t *counter, uint32_t *health,
-               int spin_limit) {
+               uint32_t *failed, int spin_limit) {
     constexpr int T = RadixSorter::kThreads, I = ITEMS, W = T / 32, G = RadixSorter::kGroup;
     // tiles, groups read at a time (the polls of all waiting tiles meet in a few
     // lines of L2: with twice as many, N = 1e6 in tiles of 2048 keys takes 171
@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
     auto wait = [&]() {  // false: given up
         if (++spins > spin_limit) {
             raise_health(health, SPH_HEALTH_SORT_TIMEOUT);
+            if (failed) *failed = 1u;
             return false;
         }
         __nanosleep(32);
@@ -239,19 +240,24 @@ __global__ void __launch_bounds__(RadixSorter::kThreads)
 
 void launch_onesweep(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, int n,
                      int shift, const uint32_t *hist, uint32_t *status, uint32_t *counter, uint32_t *health,
-                     int spin_limit, cudaStream_t st) {
+                     uint32_t *failed, int spin_limit, cudaStream_t st, bool withhold = false) {
     const int tiles = RadixSorter::tiles(n), items = RadixSorter::items(n);
     auto *kernel = items == 4 ? k_onesweep<4> : items == 8 ? k_onesweep<8> : k_onesweep<16>;
-    kernel<<<tiles, RadixSorter::kThreads, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n, shift, hist, status,
-                                                    tiles, counter, health, spin_limit);
+    kernel<<<withhold ? tiles - 1 : tiles, RadixSorter::kThreads, 0, st>>>(
+        keys_in, vals_in, keys_out, vals_out, n, shift, hist, status, tiles, counter, health, failed, spin_limit);
 }
 
+// Self-test: the tickets of all passes start behind the first tile.
+__global__ void k_withhold(uint32_t *counters) { counters[threadIdx.x] = 1u; }
+
 // Each occupied cell's (first, last) sorted index, and each occupied octet's
-// (cell key >> 3) and unit's (cell key >> 6).
+// (cell key >> 3) and unit's (cell key >> 6).  Of keys that are not sorted there
+// are no ranges: all cells stay empty (a first index behind the last would be a
+// run over most of memory).
 __global__ void k_cells(const uint32_t *__restrict__ keys, int n, uint2 *__restrict__ cell_range,
-                        uint2 *__restrict__ octets, uint2 *__restrict__ units) {
+                        uint2 *__restrict__ octets, uint2 *__restrict__ units, const uint32_t *__restrict__ failed) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || *failed) return;
     const uint32_t k = keys[i], u = k >> (3 * kUnitShift);
     const uint32_t before = i ? keys[i - 1] : ~k, after = i < n - 1 ? keys[i + 1] : ~k;
     if (before != k) cell_range[k].x = (uint32_t)i;
@@ -273,15 +279,19 @@ sph_status sort_alloc(RadixSorter &s, int n) {
     s.n_cap = n;
     constexpr int kMinTile = RadixSorter::kThreads * RadixSorter::kMinItems;
     const size_t rows = RadixSorter::rows(std::max(1, (n + kMinTile - 1) / kMinTile));
-    constexpr size_t kHead = 256 * RadixSorter::kMaxPasses + RadixSorter::kMaxPasses;
+    constexpr size_t kHead = 256 * RadixSorter::kMaxPasses + RadixSorter::kMaxPasses + 1;
     size_t nb = sizeof(uint32_t) * (size_t)(n > 0 ? n : 1);
     cudaError_t e = cudaSuccess;
     for (int b = 0; b < 2; ++b) {
         if (e == cudaSuccess) e = cudaMalloc(&s.keys[b], nb);
         if (e == cudaSuccess) e = cudaMalloc(&s.vals[b], nb);
+        // (in range from the start: a sort that fails leaves entries unwritten)
+        if (e == cudaSuccess) e = cudaMemset(s.keys[b], 0, nb);
+        if (e == cudaSuccess) e = cudaMemset(s.vals[b], 0, nb);
     }
     if (e == cudaSuccess) e = cudaMalloc(&s.hist, sizeof(uint32_t) * (kHead + 256 * rows * RadixSorter::kMaxPasses));
     s.counters = s.hist + 256 * RadixSorter::kMaxPasses;
+    s.failed = s.counters + RadixSorter::kMaxPasses;
     s.status = s.hist + kHead;
     return cuda_status(e, "sort_alloc");
 }
@@ -293,7 +303,7 @@ void sort_free(RadixSorter &s) {
         s.keys[b] = s.vals[b] = nullptr;
     }
     cudaFree(s.hist);
-    s.hist = s.status = s.counters = nullptr;
+    s.hist = s.status = s.counters = s.failed = nullptr;
 }
 
 void radix_clear(RadixSorter &s, int n, int bits, cudaStream_t st) {
@@ -301,13 +311,15 @@ void radix_clear(RadixSorter &s, int n, int bits, cudaStream_t st) {
     cudaMemsetAsync(s.hist, 0, sizeof(uint32_t) * words, st);
 }
 
-int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t *health) {
+int radix_sort_pairs(RadixSorter &s, int n, int bits, cudaStream_t st, uint32_t *health, bool withhold) {
     const int passes = (bits + 7) / 8;
     int cur = 0;
     if (n <= 0) return 0;
+    if (withhold) k_withhold<<<1, RadixSorter::kMaxPasses, 0, st>>>(s.counters);
     for (int p = 0; p < passes; ++p) {
         launch_onesweep(s.keys[cur], s.vals[cur], s.keys[cur ^ 1], s.vals[cur ^ 1], n, 8 * p, s.hist + 256 * p,
-                        s.status + 256 * RadixSorter::rows(RadixSorter::tiles(n)) * p, s.counters + p, health, s.spin_limit, st);
+                        s.status + 256 * RadixSorter::rows(RadixSorter::tiles(n)) * p, s.counters + p, health, s.failed,
+                        s.spin_limit, st, withhold);
         cur ^= 1;
     }
     return cur;
@@ -320,7 +332,7 @@ void launch_init_cells(sph_ctx *ctx, cudaStream_t st) {
     ctx->cells_have_prev = false;
 }
 
-sph_status launch_sort(sph_ctx *ctx, cudaStream_t st) {
+sph_status launch_sort(sph_ctx *ctx, cudaStream_t st, bool withhold) {
     RadixSorter &s = ctx->cell_sort;
     const int n = ctx->n;
     if (n <= 0) return SPH_OK;
@@ -336,9 +348,10 @@ sph_status launch_sort(sph_ctx *ctx, cudaStream_t st) {
     k_hash_hist<<<hash_grid(n), kHashThreads, 0, st>>>(ctx->pos4, n, s.keys[0], s.vals[0], s.hist, clear_src,
                                                        ctx->cell_range, ctx->octets, ctx->units,
                                                        (ctx->cells_have_prev && prev == 1) ? 1 : 0);
-    int fin = radix_sort_pairs(s, n, 24, st, ctx->health);
+    int fin = radix_sort_pairs(s, n, 24, st, ctx->health, withhold);
     ctx->cell_final = fin;
-    k_cells<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->cell_range, ctx->octets, ctx->units);
+    k_cells<<<(n + 255) / 256, 256, 0, st>>>(s.keys[fin], n, ctx->cell_range, ctx->octets, ctx->units,
+                                              s.failed);
     ctx->cells_have_prev = true;
     return cuda_status(cudaGetLastError(), "sort");
 }
@@ -460,7 +473,7 @@ extern "C" sph_status sph_sort_cells_noalloc(const float *pos_xyz, int32_t n, ui
     uint32_t *vout[kNoAllocPasses] = {cell_index, tv, cell_index};
     for (int p = 0; p < kNoAllocPasses; ++p)
         launch_onesweep(kin[p], vin[p], kout[p], vout[p], n, 8 * p, hist + 256 * p,
-                        status + 256 * rows * p, counters + p, health, kSpinLimit, cs);
+                        status + 256 * rows * p, counters + p, health, nullptr, kSpinLimit, cs);
     return cuda_status(cudaGetLastError(), "sph_sort_cells_noalloc");
 }
 
@@ -533,6 +546,25 @@ extern "C" sph_status sph_selftest_lookback_timeout(sph_ctx *ctx, int32_t spin_l
     // the key/value buffers are valid device memory, though n = 0 touches none
     k_selftest_prepare<<<1, 256, 0, cs>>>(hist, status, counter);
     k_onesweep<RadixSorter::kMinItems><<<1, RadixSorter::kThreads, 0, cs>>>(kbuf, vbuf, kbuf, vbuf, 0, 0, hist, status, 2,
-                                                                            counter, health, spin_limit);
+                                                                            counter, health, nullptr, spin_limit);
     return cuda_status(cudaGetLastError(), "sph_selftest_lookback_timeout");
+}
+
+// The same for what follows a sort whose waits gave up: a tree build and a cell
+// sort whose first tiles are withheld.
+extern "C" sph_status sph_selftest_sort_timeout(sph_ctx *ctx, int32_t spin_limit, void *stream) {
+    using namespace sph;
+    if (!ctx || ctx->params.tree_source != SPH_TREE_GPU || RadixSorter::tiles(ctx->n) < 2 || spin_limit < 1 ||
+        spin_limit > (1 << 22)) {
+        set_error("sph_selftest_sort_timeout: needs a context with the GPU tree and more than one sort tile, and a "
+                  "spin limit in 1..%d", 1 << 22);
+        return SPH_ERR_INVALID_ARG;
+    }
+    cudaSetDevice(ctx->device);
+    RadixSorter *const sorters[] = {&ctx->tb.sorter, &ctx->cell_sort};
+    for (RadixSorter *r : sorters) r->spin_limit = spin_limit;
+    sph_status s = launch_tree_build(ctx, (cudaStream_t)stream, true);
+    if (s == SPH_OK) s = launch_sort(ctx, (cudaStream_t)stream, true);
+    for (RadixSorter *r : sorters) r->spin_limit = kSpinLimit;
+    return s;
 }

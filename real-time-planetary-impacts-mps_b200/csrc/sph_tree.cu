@@ -140,8 +140,24 @@ constexpr int kTreeThreads = 1024;  // particles per block of the three kernels
 constexpr int kTreeSeqs = 2 + 11 + 10;
 constexpr uint8_t kNoNodes = 0xff;
 
+// The sorted keys.  After a sort whose look-back gave up they are in no order,
+// and the rules below would make a tree without bounds on its nodes: then the
+// particles' places stand for their keys, spread evenly over the key range, so
+// that the tree is a whole one (of no meaning; the health word says so).
+__device__ __noinline__ uint32_t place_key(int i, int n, int bits) {
+    return (uint32_t)(((uint64_t)(uint32_t)i << bits) / (uint32_t)n);
+}
+struct TreeKeys {
+    const uint32_t *k;
+    const uint32_t *failed;
+    int n, bits;
+    bool bad;  // read once per kernel (load)
+    __device__ __forceinline__ void load() { bad = *failed != 0u; }
+    __device__ __forceinline__ uint32_t operator[](int i) const { return bad ? place_key(i, n, bits) : k[i]; }
+};
+
 struct TreeArgs {
-    const uint32_t *keys;   // sorted
+    TreeKeys keys;
     const uint32_t *order;  // particle ids in key order
     int n, depth, leafcap, blocks;
     uint8_t *levels;        // [n] first | last << 4 level of the nodes starting at each particle, or kNoNodes
@@ -163,7 +179,7 @@ __device__ __forceinline__ int shared_levels(uint32_t a, uint32_t b, int depth) 
 
 // First index in (i, hi] whose key leaves i's run at `level` (hi when none
 // does before it).
-__device__ __forceinline__ int run_end(const uint32_t *keys, uint32_t key, int i, int hi, int level, int depth) {
+__device__ __forceinline__ int run_end(const TreeKeys &keys, uint32_t key, int i, int hi, int level, int depth) {
     int lo = i + 1;
     while (lo < hi) {
         const int mid = lo + ((hi - lo) >> 1);
@@ -175,7 +191,7 @@ __device__ __forceinline__ int run_end(const uint32_t *keys, uint32_t key, int i
 
 // First index of the run of i at `level`, not looked for before `lo`: steps
 // back that double, then a binary search, since most runs are short.
-__device__ __forceinline__ int run_start(const uint32_t *keys, uint32_t key, int i, int lo, int level, int depth) {
+__device__ __forceinline__ int run_start(const TreeKeys &keys, uint32_t key, int i, int lo, int level, int depth) {
     int in = i, out = lo - 1, step = 1;  // in: in the run; out: before it (or before lo)
     while (in - step >= lo) {
         if (shared_levels(key, keys[in - step], depth) < level) {
@@ -204,6 +220,7 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_mark(TreeArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i = blockIdx.x * kTreeThreads + tid;
     const int D = a.depth, n = a.n;
+    a.keys.load();
     if (tid < kTreeSeqs) s_tot[tid] = 0;
     __syncthreads();
     int first = 0, last = -1, ints = 0;
@@ -289,6 +306,7 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_write(TreeArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int i = blockIdx.x * kTreeThreads + tid;
     const int D = a.depth, seqs = 3 + 2 * D;
+    a.keys.load();
     const unsigned lt = (1u << lane) - 1u;
     int first, last;
     unpack_levels(i < a.n ? a.levels[i] : kNoNodes, first, last);
@@ -381,6 +399,7 @@ __global__ void __launch_bounds__(256) k_tree_link(TreeArgs a) {
     unpack_levels(a.levels[i], first, last);
     if (last < 0 || first < 1) return;
     const int off = a.at_int[i], dp = a.at_node[i];
+    a.keys.load();
     if ((int64_t)off + a.ints[i] > a.tree_cap || (int64_t)dp + (last - first + 1) > a.node_cap) return;
     const uint32_t key = a.keys[i];
     const int level = first - 1;  // the parent's
@@ -432,7 +451,7 @@ void tree_free(sph_ctx *ctx) {
     tb = TreeBuild();
 }
 
-sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st) {
+sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st, bool withhold) {
     sph_status s = tree_alloc(ctx);
     if (s != SPH_OK) return s;
     TreeBuild &tb = ctx->tb;
@@ -449,9 +468,9 @@ sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st) {
     radix_clear(tb.sorter, n, bits, st);
     k_tree_keys<<<reduce_grid(n), kReduceThreads, 0, st>>>(ctx->pos4, n, D, bb, tb.sorter.keys[0], tb.sorter.vals[0],
                                                            tb.sorter.hist, passes);
-    const int fin = radix_sort_pairs(tb.sorter, n, bits, st, ctx->health);
+    const int fin = radix_sort_pairs(tb.sorter, n, bits, st, ctx->health, withhold);
     TreeArgs a;
-    a.keys = tb.sorter.keys[fin];
+    a.keys = TreeKeys{tb.sorter.keys[fin], tb.sorter.failed, n, bits, false};
     a.order = tb.sorter.vals[fin];
     a.n = n;
     a.depth = D;

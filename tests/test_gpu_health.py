@@ -35,6 +35,46 @@ def test_lookback_timeout_is_reported_and_context_recovers(cuda, pkg):
         assert np.all(np.isfinite(c.download("pos")))
 
 
+# what is built on a sort whose waits gave up -- the tree, and the cell ranges
+# with all that walks them -- stays within its buffers, in both gravity forms
+@pytest.mark.parametrize("n,leaf,depth,theta", [(2560, 16, 7, None), (20481, 1, 7, None), (20481, 4, 10, 0.6),
+                                                (300000, 32, 7, 0.6)])
+def test_passes_after_a_sort_timeout_and_recovery(cuda, pkg, n, leaf, depth, theta):
+    lib = pkg._lib.load()
+    ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=4)
+    gn = np.full(n, 0.1, np.float32)
+    got = []
+    for disturbed in (True, False):
+        with pkg.Compute(ic, max_children_in_leaf=leaf, max_tree_depth=depth) as c:
+            if theta:
+                c.set_form(gravity="theta", theta=theta)
+            for _ in range(2 if disturbed else 0):
+                assert lib.sph_selftest_sort_timeout(c._h, 200, None) == 0
+                tree = c.get_tree()
+                # a whole tree: every particle place in one leaf, every node reached once
+                assert tree["n_nodes"] == sum(np.diff(tree["level_offsets"]))
+                start = c.download("cell_start")
+                assert np.all(start == 0xFFFFFFFF)
+                c.gravitationalPass()
+                c.densityPass()
+                c.accelerationPass()
+                assert lib.sph_synchronize(c._h, None) == SPH_ERR_TIMEOUT
+                assert c.health() & pkg._lib.HEALTH["sort_timeout"]
+                c.clear_health()
+            for f in ("h", "rho"):
+                c.upload(f, ic[f])
+            c.upload("grav_norm", gn)
+            c.updateOctreeBuffer()
+            c.sort()
+            c.gravitationalPass()
+            c.densityPass()
+            c.accelerationPass()
+            c.synchronize()
+            got.append([c.get_tree()["tree"]] + [c.download(f) for f in ("cell_start", "cell_end", "h", "rho", "acc")])
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
 def test_non_finite_density_is_reported(cuda, pkg):
     lib = pkg._lib.load()
     ic = pkg.ic.make_impact(2048, 512, seed=4)

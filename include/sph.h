@@ -331,7 +331,8 @@ sph_status sph_selftest_lookback_timeout(sph_ctx *ctx, int32_t spin_limit, void 
 /* Self-test of what follows such a time-out (no counterpart in the reference):
  * one tree build and one cell sort run with the first tile of every sort pass
  * withheld and the waits limited to spin_limit polls (1..2^22), so that both
- * sorts give up and raise SPH_HEALTH_SORT_TIMEOUT.  The passes may then run on
+ * sorts give up and raise SPH_HEALTH_SORT_TIMEOUT; the up pass's counters of
+ * finished children are set to nonsense before it.  The passes may then run on
  * their results (a tree of no meaning and a cell grid without particles) and
  * stay within their buffers; the next build and sort are whole.  SPH_TREE_GPU
  * contexts of more than 1024 particles only. */

@@ -72,7 +72,7 @@ struct Tree {
     int32_t *meta = nullptr;        // device: [0] n_levels, [1] n_nodes, [2] tree_len
     int2 *node_range = nullptr;     // [node_cap] by data pointer, leaves of the GPU tree: (first, count) in key order
     int32_t *parent = nullptr;      // [node_cap] by data pointer, GPU tree: the parent's tree offset, -1 at the root
-    int32_t *arrived = nullptr;     // [node_cap] up pass: children done (0 between passes)
+    int32_t *arrived = nullptr;     // [node_cap] up pass: children done (0 from the tree build on, between passes)
     int64_t node_cap = 0;
     int64_t level_cap = 0;
     int64_t branch_cap = 0;         // list slots per level

@@ -562,6 +562,8 @@ extern "C" sph_status sph_selftest_sort_timeout(sph_ctx *ctx, int32_t spin_limit
     }
     cudaSetDevice(ctx->device);
     RadixSorter *const sorters[] = {&ctx->tb.sorter, &ctx->cell_sort};
+    // (what an up pass over a tree that is none leaves behind)
+    cudaMemsetAsync(ctx->tree.arrived, 1, sizeof(int32_t) * ctx->tree.node_cap, (cudaStream_t)stream);
     for (RadixSorter *r : sorters) r->spin_limit = spin_limit;
     sph_status s = launch_tree_build(ctx, (cudaStream_t)stream, true);
     if (s == SPH_OK) s = launch_sort(ctx, (cudaStream_t)stream, true);

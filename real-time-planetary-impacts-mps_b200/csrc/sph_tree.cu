@@ -165,7 +165,7 @@ struct TreeArgs {
     int32_t *at_int, *at_node;  // [n] their first offset and data pointer
     int64_t *totals;        // [kTreeSeqs][blocks] block totals, scanned in place by the last block
     uint32_t *ticket;       // blocks of k_tree_mark that are done
-    int32_t *tree, *level_nodes, *level_count, *list_slot, *parent, *meta;
+    int32_t *tree, *level_nodes, *level_count, *list_slot, *parent, *arrived, *meta;
     int2 *node_range;       // by data pointer, leaves: (first particle in key order, count)
     int64_t level_cap, tree_cap, node_cap;
     uint32_t *health;
@@ -366,6 +366,7 @@ __global__ void __launch_bounds__(kTreeThreads) k_tree_write(TreeArgs a) {
         const int off = off0 + 10 * (l - first), dp = dp0 + (l - first);
         a.level_nodes[(size_t)l * a.level_cap + s_at[2 + l][warp] + __popc(m_on & lt)] = off;
         a.list_slot[dp] = br ? s_at[3 + D + l][warp] + __popc(m_br & lt) : -1;
+        a.arrived[dp] = 0;
         if (l > first) a.parent[dp] = off - 10;
         else if (l == 0) a.parent[dp] = -1;
         int32_t *T = a.tree + off;
@@ -487,6 +488,7 @@ sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st, bool withhold) {
     a.level_count = tr.level_count;
     a.list_slot = tr.list_slot;
     a.parent = tr.parent;
+    a.arrived = tr.arrived;
     a.meta = tr.meta;
     a.node_range = tr.node_range;
     a.level_cap = tr.level_cap;

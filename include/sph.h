@@ -337,6 +337,11 @@ sph_status sph_selftest_lookback_timeout(sph_ctx *ctx, int32_t spin_limit, void 
  * stay within their buffers; the next build and sort are whole.  SPH_TREE_GPU
  * contexts of more than 1024 particles only. */
 sph_status sph_selftest_sort_timeout(sph_ctx *ctx, int32_t spin_limit, void *stream);
+/* Self-test of the learned seed's bounded tensor-core waits (no counterpart in
+ * the reference): one CTA's thread `thread` (0..127) waits for a barrier at which
+ * nothing arrives, at most `limit` polls (1..1024), and the CTA reports it as the
+ * seed's kernels do: SPH_HEALTH_MLP_TIMEOUT, whichever thread it was. */
+sph_status sph_selftest_mlp_timeout(sph_ctx *ctx, int32_t thread, int32_t limit, void *stream);
 /* Self-test of the GPU tree build's capacity check (no counterpart in the
  * reference): one tree build runs with its storage bound lowered to 16 ints,
  * so the layout kernels find the tree too large, skip the writes that would

@@ -178,6 +178,19 @@ __device__ __forceinline__ int sample_row(uint32_t it, uint32_t row, int batch, 
     return (int)(((g * 0x9E3779B97F4A7C15ull) ^ salt) % (uint64_t)n);
 }
 
+// The CTA's bounded waits are over: reported when any thread's gave up.
+__device__ __forceinline__ void report_waits(bool ok, uint32_t *health) {
+    if (__syncthreads_or(!ok) && threadIdx.x == 0) raise_health(health, SPH_HEALTH_MLP_TIMEOUT);
+}
+
+// Self-test: one thread waits for a barrier at which nothing arrives.
+__global__ void __launch_bounds__(kTile) k_selftest_wait(int thread, int limit, uint32_t *health) {
+    __shared__ uint64_t bar;
+    if (threadIdx.x == 0) tc::mbar_init(&bar, 1);
+    __syncthreads();
+    report_waits((int)threadIdx.x != thread || tc::mbar_wait(&bar, 0u, limit), health);
+}
+
 // MODE 0: inference (features from the state, writes the seed); each CTA keeps
 // the weights and takes tiles of 128 rows until none is left (one CTA per tile
 // spent most of its time on converting the weights: 144 us at N = 1e6, now 88).
@@ -262,7 +275,10 @@ __global__ void __launch_bounds__(kTile) k_mlp(HSeedArgs a, uint32_t it, int bat
                 issue();
                 tc::mma_commit(&bar);
             }
-            if (!tc::mbar_wait(&bar, phase, kMbarLimit)) ok = false;
+            if (!tc::mbar_wait(&bar, phase, kMbarLimit)) {
+                ok = false;
+                tc::mbar_wait(&bar, phase, kMbarLimit);  // the MMAs in flight, before their TMEM is freed
+            }
             phase ^= 1u;
             tc::fence_after_sync();
         };
@@ -399,9 +415,8 @@ __global__ void __launch_bounds__(kTile) k_mlp(HSeedArgs a, uint32_t it, int bat
                 for (int q = 0; q < kIn; ++q) atomicAdd(a.grads + kOffW1 + t * kIn + q, v[q]);
         }
     }
-    if (!ok && t == 0) raise_health(a.health, SPH_HEALTH_MLP_TIMEOUT);
     tc::fence_before_sync();
-    __syncthreads();
+    report_waits(ok, a.health);
     if (warp == 0) tc::tmem_dealloc(tmem_slot, tmem_cols<MODE>());
 }
 
@@ -758,6 +773,16 @@ sph_status sph_hseed_get_stats(sph_ctx *ctx, sph_hseed_stats *out) {
     out->max_sweeps = v[2];
     out->particles = v[3];
     return SPH_OK;
+}
+
+sph_status sph_selftest_mlp_timeout(sph_ctx *ctx, int32_t thread, int32_t limit, void *stream) {
+    if (!ctx || thread < 0 || thread >= kTile || limit < 1 || limit > 1024) {
+        set_error("sph_selftest_mlp_timeout: thread must be in 0..%d and limit in 1..1024", kTile - 1);
+        return SPH_ERR_INVALID_ARG;
+    }
+    cudaSetDevice(ctx->device);
+    k_selftest_wait<<<1, kTile, 0, (cudaStream_t)stream>>>(thread, limit, ctx->health);
+    return cuda_status(cudaGetLastError(), "sph_selftest_mlp_timeout");
 }
 
 }  // extern "C"

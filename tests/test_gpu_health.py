@@ -75,6 +75,20 @@ def test_passes_after_a_sort_timeout_and_recovery(cuda, pkg, n, leaf, depth, the
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("thread", [0, 1, 77, 127])
+def test_a_tensor_core_wait_that_gives_up_is_reported_by_any_thread(cuda, pkg, thread):
+    lib = pkg._lib.load()
+    ic = pkg.ic.make_impact(2048, 512, seed=4)
+    with pkg.Compute(ic, max_children_in_leaf=16) as c:
+        assert lib.sph_selftest_mlp_timeout(c._h, 128, 16, None) == 1  # no such thread
+        assert lib.sph_selftest_mlp_timeout(c._h, thread, 16, None) == 0
+        assert lib.sph_synchronize(c._h, None) == SPH_ERR_TIMEOUT
+        assert c.health() == pkg._lib.HEALTH["mlp_timeout"]
+        c.clear_health()
+        c.step()
+        c.synchronize()
+
+
 def test_non_finite_density_is_reported(cuda, pkg):
     lib = pkg._lib.load()
     ic = pkg.ic.make_impact(2048, 512, seed=4)

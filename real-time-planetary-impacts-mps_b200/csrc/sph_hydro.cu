@@ -681,11 +681,15 @@ __device__ __forceinline__ void tile_box(float px, float py, float pz, float hb,
     b.hi2 = (int)floorf((pz + rl) * iw + widen);
 }
 
-// Units of a box, or some number past any limit (particles of one cell that
-// are only alike modulo the grid can span thousands of cells).
-__device__ __forceinline__ int64_t box_units(int nx, int ny, int nz) {
-    return (int64_t)min(nx, 1 << 20) * min(ny, 1 << 20) * min(nz, 1 << 20);
+// Units (of 1 << shift cells) from cell lo to cell hi, or a number past any
+// limit where these span more than the grid's period: particles of one tile are
+// only alike modulo the grid, and a box that holds two of them a period apart
+// would stage the cells between them twice.  (64 bits: lo and hi are anything.)
+__device__ __forceinline__ int box_extent(int lo, int hi, int shift) {
+    const int64_t e = (int64_t)(hi >> shift) - (lo >> shift) + 1;
+    return e > (kCellsPerDim >> shift) ? 1 << 20 : (int)e;
 }
+__device__ __forceinline__ int64_t box_units(int nx, int ny, int nz) { return (int64_t)nx * ny * nz; }
 
 // The particle's h is final: note it when the lists of its neighbours may lack
 // it (a little early, for the rounding of the lists' squared reach; NaN counts
@@ -704,8 +708,8 @@ __device__ __forceinline__ void mark_grown(const DensityArgs &a, uint32_t p, flo
 template <int U>
 __device__ __forceinline__ int unit_shift(const int (&box)[6]) {
     if (U == 0) return 0;
-    return box_units((box[3] >> 1) - (box[0] >> 1) + 1, (box[4] >> 1) - (box[1] >> 1) + 1,
-                     (box[5] >> 1) - (box[2] >> 1) + 1) <= kTileCellsMax
+    return box_units(box_extent(box[0], box[3], 1), box_extent(box[1], box[4], 1), box_extent(box[2], box[5], 1)) <=
+                   kTileCellsMax
                ? 1
                : kUnitShift;
 }
@@ -1231,7 +1235,8 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
             }
             const int us = unit_shift<U>(S.box);
             const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
-            const int nx = (S.box[3] >> us) - lo0 + 1, ny = (S.box[4] >> us) - lo1 + 1, nz = (S.box[5] >> us) - lo2 + 1;
+            const int nx = box_extent(S.box[0], S.box[3], us), ny = box_extent(S.box[1], S.box[4], us),
+                      nz = box_extent(S.box[2], S.box[5], us);
             const bool too_many = box_units(nx, ny, nz) > kTileCellsMax;
             const int ncell = too_many ? 0 : nx * ny * nz;
             // unit counts (kPer consecutive units per thread) and their
@@ -2225,13 +2230,12 @@ __global__ void __launch_bounds__(kTileThreads, 2)
             const bool any = S.box[0] <= S.box[3];
             const int us = unit_shift<U>(S.box);
             const int lo0 = S.box[0] >> us, lo1 = S.box[1] >> us, lo2 = S.box[2] >> us;
-            const int nx = any ? (S.box[3] >> us) - lo0 + 1 : 0, ny = any ? (S.box[4] >> us) - lo1 + 1 : 0,
-                      nz = any ? (S.box[5] >> us) - lo2 + 1 : 0;
+            const int nx = any ? box_extent(S.box[0], S.box[3], us) : 0, ny = any ? box_extent(S.box[1], S.box[4], us) : 0,
+                      nz = any ? box_extent(S.box[2], S.box[5], us) : 0;
             int ncell = 0;
             if (any) {
-                // (pack_cell's range: such a box holds particles of cells that
-                // are only alike modulo the grid)
-                if (box_units(nx, ny, nz) > kTileCellsMax || max(nx, max(ny, nz)) > (kBoxCellsMax >> us)) {
+                static_assert(kCellsPerDim <= kBoxCellsMax, "a box that is staged has cells within pack_cell's range");
+                if (box_units(nx, ny, nz) > kTileCellsMax) {
                     if (tid == 0) S.defer_all = 1;
                 } else {
                     ncell = nx * ny * nz;

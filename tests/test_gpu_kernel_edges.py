@@ -200,3 +200,86 @@ def test_hydro_matches_the_parity_build(cuda, pkg, n, scale, masses, squeeze, pr
         assert e.max() <= tol[f], (f, float(e.max()))
     # a step whose limit lies on a power of two may fall to either side
     assert np.mean(a["next_active_time"][keep] != b["next_active_time"][keep]) <= 1e-4
+
+
+def _hydro(pkg, ic, parity, forms=None, prepare=None):
+    with pkg.Compute(ic, max_children_in_leaf=32, parity=parity) as c:
+        if forms:
+            c.set_form(**forms)
+        if prepare:
+            prepare(c)
+        c.sort()
+        c.densityPass()
+        c.accelerationPass()
+        c.synchronize()
+        assert c.health() == 0
+        return {f: c.download(f) for f in HYDRO_FIELDS + ("next_active_time", "dt")}
+
+
+HYDRO_FIELDS = ("h", "rho", "grad_term", "pressure", "sound_speed", "balsara", "acc", "du", "dhdt")
+
+
+def _assert_hydro(a, b, pos, few=1e-3):
+    """a (product) against b (parity build): the bounds of
+    test_hydro_matches_the_parity_build."""
+    n = len(pos)
+    flip = np.abs(a["h"].astype(np.float64) / b["h"] - 1.0) > 1e-5
+    assert flip.sum() <= max(5, int(few * n))
+    keep = np.ones(n, bool)
+    if flip.any():
+        from scipy.spatial import cKDTree
+
+        p = pos.astype(np.float64)
+        near = cKDTree(p).query_ball_point(p[flip], r=2.0 * float(b["h"].max()))
+        keep[np.unique(np.concatenate([np.asarray(q, np.int64) for q in near]))] = False
+    tol = {"h": 1e-5, "rho": 1e-5, "grad_term": 1e-5, "pressure": 5e-4, "sound_speed": 5e-4, "balsara": 1e-3,
+           "acc": 1e-3, "du": 1e-3, "dhdt": 1e-3}
+    for f in HYDRO_FIELDS:
+        sel = ~flip if f in HYDRO_FIELDS[:6] else keep
+        if f in ("balsara", "du", "dhdt"):
+            e = np.abs(a[f][sel].astype(np.float64) - b[f][sel]) / np.sqrt(np.mean(b[f].astype(np.float64) ** 2))
+        else:
+            e = _rel(a[f][sel], b[f][sel])
+        assert e.max() <= tol[f], (f, float(e.max()))
+    assert np.mean(a["next_active_time"][keep] != b["next_active_time"][keep]) <= 1e-4
+
+
+# Cells are numbered modulo the grid of 256, so a tile can hold particles a whole
+# period (46.08 Mm) apart: here every other particle of the target's middle is
+# moved by one.  The staged boxes of some 160 units of the coarse tiles (6e4
+# particles, h of 2.2 cells) would span more than the period.
+@pytest.mark.parametrize("n,axis,scale", [(60000, 0, 1.0), (60000, 2, 1.0), (100000, 1, 1.0)])
+def test_hydro_of_particles_a_grid_period_apart(cuda, pkg, n, axis, scale):
+    ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=5)
+    rng = np.random.default_rng(0)
+    ic["vel"] = (ic["vel"] + rng.normal(size=(n, 3)) * 1e-3).astype(np.float32)
+    near = np.linalg.norm(ic["pos"] - np.float32(318.55), axis=1) < 2.5
+    move = near & (rng.random(n) < 0.5)
+    assert move.sum() > 1000
+    ic["pos"][move, axis] += np.float32(256 * 0.18)
+    a, b = (_hydro(pkg, ic, parity) for parity in (False, True))
+    _assert_hydro(a, b, ic["pos"])
+
+
+# A position beyond what an int of cells holds (a run that blew up), in the same
+# cells modulo the grid as the body's
+@pytest.mark.parametrize("n,x", [(20480, -1e30), (60000, -1e30), (400000, -1e30), (60000, 3e9)])
+def test_hydro_beside_a_position_out_of_any_range(cuda, pkg, n, x):
+    ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=5)
+    cell = np.floor(ic["pos"][:, 0] / CELL).astype(np.int64) % 256
+    inner = np.linalg.norm(ic["pos"] - np.float32(318.55), axis=1) < 5.0
+    far = np.flatnonzero(inner & (cell < 4))[:3]  # such a position's cell is 0
+    assert len(far) == 3
+    ic["pos"][far, 0] = np.float32(x)
+    ic["vel"] = (ic["vel"] + np.random.default_rng(n).normal(size=(n, 3)) * 1e-3).astype(np.float32)
+    out = []
+    for parity in (False, True):
+        with pkg.Compute(ic, max_children_in_leaf=32, parity=parity) as c:
+            c.sort()
+            c.densityPass()
+            c.accelerationPass()
+            assert c._lib.sph_synchronize(c._h, None) in (0, 5)  # their own density may be no number
+            out.append({f: c.download(f) for f in HYDRO_FIELDS + ("next_active_time", "dt")})
+    rest = np.setdiff1d(np.arange(n), far)
+    a, b = ({f: v[rest] if len(v) == n else v for f, v in o.items()} for o in out)
+    _assert_hydro(a, b, ic["pos"][rest])

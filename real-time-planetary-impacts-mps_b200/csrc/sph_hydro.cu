@@ -1174,6 +1174,12 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
         const bool splittable = (a.skey[tstart] >> kSplit) != (a.skey[tend - 1] >> kSplit);
         int level = 0;  // 0 the tile, 1 its octets, 2 their cells
         uint32_t r0 = tstart;
+        // on to what follows the range: behind the last cell of an octet that
+        // was taken cell by cell, to the next octet as a whole
+        auto advance = [&](uint32_t to) {
+            r0 = to;
+            if (level == 2 && r0 < tend && ((a.skey[r0] ^ a.skey[r0 - 1u]) >> kSplit) != 0u) level = 1;
+        };
         while (r0 < tend) {
             __syncthreads();
             if (tid == 0) {
@@ -1230,7 +1236,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
             }
             __syncthreads();
             if (!S.need) {  // nothing in the range for this pass
-                r0 = end;
+                advance(end);
                 continue;
             }
             const int us = unit_shift<U>(S.box);
@@ -1281,7 +1287,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
             __syncthreads();
             if (S.defer_all) {
                 if (level < 2) level = level == 0 && splittable ? 1 : 2;
-                else r0 = end;  // its particles are left without a list
+                else advance(end);  // its particles are left without a list
                 continue;
             }
             float hmax = 0.f;
@@ -1303,8 +1309,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
                 if (start + j >= end) break;
                 lists_tile_warp<U>(a, S, start + j, end, lane);
             }
-            r0 = end;
-            if (level == 2 && r0 < tend && ((a.skey[r0] ^ a.skey[r0 - 1u]) >> kSplit) != 0u) level = 1;
+            advance(end);
         }
     }
 }

@@ -283,3 +283,38 @@ def test_hydro_beside_a_position_out_of_any_range(cuda, pkg, n, x):
     rest = np.setdiff1d(np.arange(n), far)
     a, b = ({f: v[rest] if len(v) == n else v for f, v in o.items()} for o in out)
     _assert_hydro(a, b, ic["pos"][rest])
+
+
+# Octets whose box is too full even cell by cell (beside a cell of 3500
+# particles) leave their particles to the walk, and no others: the octet behind
+# them in the tile is searched whole again, with the second, wider search that
+# every particle of this lattice needs (h 12 % below its fixed point, a density
+# that does not foretell it).  So as many particles are left as with tiles of
+# single octets.
+def test_an_overfull_octet_does_not_cost_the_next_one_its_wider_search(cuda, pkg):
+    s, k = 0.1, 44
+    rng = np.random.default_rng(1)
+    cell0 = 1764  # the lattice starts on a 64-cell block; its 16-cell quarters (93 particles) are tiles
+    g = (np.arange(k) + 0.5) * s + cell0 * 0.18
+    lattice = np.stack(np.meshgrid(g, g, g, indexing="ij"), axis=-1).reshape(-1, 3)
+    # cells just before a tile's first along x
+    full = np.array([(x - 1, y, z) for x in (4, 12) for y in (4, 12, 20) for z in (4, 12, 20)])
+    dense = ((cell0 + full) * 0.18)[:, None, :] + rng.uniform(0.01, 0.17, size=(len(full), 3500, 3))
+    pos = np.concatenate([lattice, dense.reshape(-1, 3)])
+    n = len(pos)
+    ic = pkg.ic.make_cube(n, seed=0)
+    ic["pos"] = np.ascontiguousarray(pos, np.float32)
+    ic["mass"][:] = 1.0
+    ic["h"][:] = 0.88 * 1.2348 * s
+    ic["rho"][:] = 4.0 / s ** 3
+    deferred = []
+    for tiling in ({}, dict(block_max=1, half_max=1)):
+        with pkg.Compute(ic, max_children_in_leaf=32) as c:
+            if tiling:
+                c.set_tiling(**tiling)
+            c.sort()
+            c.densityPass()
+            c.synchronize()
+            deferred.append(c.hseed_stats()["deferred"])
+    assert len(dense) * 3500 <= deferred[0] < 0.5 * n + len(dense) * 3500
+    assert deferred[0] == deferred[1]

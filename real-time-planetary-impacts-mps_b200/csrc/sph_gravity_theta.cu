@@ -368,9 +368,7 @@ __device__ __forceinline__ void eval_parts(const PartPair *part, int np, float4 
         const F2 r2 = fma2(rz, rz, fma2(ry, ry, rx * rx));
         float r2a, r2b;
         unpack(r2, r2a, r2b);
-        // (both compared, so that a NaN position takes the other branch, where
-        // its pair is left out)
-        if (r2a >= soft2x4 && r2b >= soft2x4) {
+        if (fminf(r2a, r2b) >= soft2x4) {
             const F2 rinv = f2(rsqrt_hw(r2a), rsqrt_hw(r2b));
             const F2 mr = at2(q.c[3]) * rinv;
             const F2 s = mr * rinv * rinv;
@@ -383,8 +381,6 @@ __device__ __forceinline__ void eval_parts(const PartPair *part, int np, float4 
             unpack(rx, xa, xb);
             unpack(ry, ya, yb);
             unpack(rz, za, zb);
-            if (!(r2a > 0.f)) xa = ya = za = 0.f;
-            if (!(r2b > 0.f)) xb = yb = zb = 0.f;
             const float2 a = near_pair(r2a, q.c[3][0]), b = near_pair(r2b, q.c[3][1]);
             sx += a.x * xa + b.x * xb;
             sy += a.x * ya + b.x * yb;
@@ -476,7 +472,10 @@ __global__ void __launch_bounds__(32 * kWalkWarps, 6) k_walk(WalkArgs a) {
 #pragma unroll
                     for (int step = kLeafCap / 2; step > 0; step >>= 1)
                         if (q + step < nleaf && s_loff[w][q + step] <= j) q += step;
-                    const float4 p = a.kp4[s_leaf[w][q].x + (j - s_loff[w][q])];
+                    float4 p = a.kp4[s_leaf[w][q].x + (j - s_loff[w][q])];
+                    // a position that is no number (a run that blew up) would make
+                    // every target's sums none: left out here, once for 32 targets
+                    if (!(fabsf(p.x + p.y + p.z) < 1e30f)) p = make_float4(1e18f, 1e18f, 1e18f, 0.f);
                     PartPair &to = s_part[w][lane >> 1];
                     to.c[0][lane & 1] = -p.x;
                     to.c[1][lane & 1] = -p.y;

@@ -960,6 +960,11 @@ sph_status sph_set_form(sph_ctx *ctx, const sph_form *f) {
     }
     cudaSetDevice(ctx->device);
     drop_graphs(ctx);
+    // (the walk's positions here, not in the first pass)
+    if (f->gravity == SPH_GRAVITY_THETA && !ctx->tb.kp4) {
+        const cudaError_t e = cudaMalloc(&ctx->tb.kp4, sizeof(float4) * (size_t)ctx->n);
+        if (e != cudaSuccess) return cuda_status(e, "sph_set_form: positions of the walk");
+    }
     const bool enter_mixed = f->precision == SPH_PRECISION_MIXED && ctx->form.precision != SPH_PRECISION_MIXED;
     ctx->form = *f;
     if (enter_mixed) {
@@ -1097,13 +1102,27 @@ sph_status sph_step(sph_ctx *ctx, void *stream) {
 
 namespace sph {
 
-// The other streams and the events of a step (created once).
-sph_status ensure_streams(sph_ctx *ctx) {
+// The other streams and the events of a step (created once): side, the input
+// copies' and the seed's refresh; gravity, the tree and gravity passes'.
+static sph_status ensure_streams(sph_ctx *ctx, bool side, bool gravity) {
     cudaError_t e = cudaSuccess;
-    for (cudaStream_t *s : {&ctx->side_stream, &ctx->gravity_stream})
-        if (e == cudaSuccess && !*s) e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
-    for (cudaEvent_t *v : {&ctx->ev_fork, &ctx->ev_join, &ctx->ev_gfork, &ctx->ev_up, &ctx->ev_gjoin})
-        if (e == cudaSuccess && !*v) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+    auto stream = [&](cudaStream_t &s) {
+        if (e == cudaSuccess && !s) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    };
+    auto event = [&](cudaEvent_t &v) {
+        if (e == cudaSuccess && !v) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
+    };
+    if (side) {
+        stream(ctx->side_stream);
+        event(ctx->ev_fork);
+        event(ctx->ev_join);
+    }
+    if (gravity) {
+        stream(ctx->gravity_stream);
+        event(ctx->ev_gfork);
+        event(ctx->ev_up);
+        event(ctx->ev_gjoin);
+    }
     return cuda_status(e, "step streams");
 }
 
@@ -1118,7 +1137,20 @@ sph_status ensure_streams(sph_ctx *ctx) {
 // `inputs` (may be null): joined before the density pass.  fork false: all on
 // st (an ensemble's instances already run beside one another).
 static sph_status step_passes(sph_ctx *ctx, cudaStream_t st, cudaEvent_t inputs, bool fork) {
-    cudaStream_t gs = fork ? ctx->gravity_stream : st;
+    if (!fork) {
+        sph_status s = SPH_OK;
+        if (ctx->params.tree_source == SPH_TREE_GPU) s = launch_tree_build(ctx, st);
+        if (s == SPH_OK) s = gravity_pass(ctx, st);
+        if (s == SPH_OK) s = launch_sort(ctx, st);
+        const cudaError_t ei = inputs ? cudaStreamWaitEvent(st, inputs, 0) : cudaSuccess;
+        if (s == SPH_OK) s = cuda_status(ei, "step join");
+        if (s == SPH_OK) s = launch_density(ctx, st);
+        ctx->hs.trained_ahead = false;
+        if (s == SPH_OK) s = launch_acceleration(ctx, st);
+        if (s == SPH_OK) s = launch_step(ctx, st);
+        return s;
+    }
+    cudaStream_t gs = ctx->gravity_stream;
     cudaError_t e = cudaEventRecord(ctx->ev_gfork, st);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(gs, ctx->ev_gfork, 0);
     sph_status s = cuda_status(e, "step fork");
@@ -1147,12 +1179,12 @@ static sph_status step_passes(sph_ctx *ctx, cudaStream_t st, cudaEvent_t inputs,
 
 // One full step on `st`.
 sph_status full_step(sph_ctx *ctx, cudaStream_t st, bool fork) {
-    sph_status s = ensure_streams(ctx);
-    if (s != SPH_OK) return s;
     // the learned seed's online refresh runs beside the tree, sort and
     // gravity passes (it reads the previous density pass's pairs and writes
     // only the network) and is joined before the density pass
     const bool ahead = hseed_online_due(ctx);
+    sph_status s = ensure_streams(ctx, ahead, fork);
+    if (s != SPH_OK) return s;
     if (ahead) {
         cudaError_t e = cudaEventRecord(ctx->ev_fork, st);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->side_stream, ctx->ev_fork, 0);
@@ -1331,7 +1363,7 @@ sph_status sph_step_host(sph_ctx *ctx, const sph_host_state *in, const sph_host_
     cudaError_t e = cudaSuccess;
     if (!ctx->own_stream) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_status(e, "sph_step_host stream");
-    sph_status s = ensure_streams(ctx);
+    sph_status s = ensure_streams(ctx, true, true);
     if (s != SPH_OK) return s;
     const bool same = ctx->host_graph && std::memcmp(&ctx->host_in, in, sizeof(*in)) == 0 &&
                       std::memcmp(&ctx->host_out, out, sizeof(*out)) == 0;

@@ -44,10 +44,11 @@ constexpr uint32_t kTileCandidates[] = {128u, 320u, 640u};
 constexpr int kTuneTargets = 512;
 constexpr float kTuneGravityBound = 1e-3f;
 
-// Mean milliseconds of `steps` full steps of ctx after `warm` untimed ones.
+// Mean milliseconds of `steps` full steps of ctx, as the ensemble runs them, after
+// `warm` untimed ones.
 sph_status time_steps(sph_ctx *ctx, cudaStream_t st, int warm, int steps, float &ms) {
     for (int i = 0; i < warm; ++i) {
-        sph_status s = full_step(ctx, st);
+        sph_status s = full_step(ctx, st, false);
         if (s != SPH_OK) return s;
     }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -55,7 +56,7 @@ sph_status time_steps(sph_ctx *ctx, cudaStream_t st, int warm, int steps, float 
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
     sph_status s = SPH_OK;
-    for (int i = 0; i < steps && s == SPH_OK; ++i) s = full_step(ctx, st);
+    for (int i = 0; i < steps && s == SPH_OK; ++i) s = full_step(ctx, st, false);
     cudaEventRecord(e1, st);
     cudaError_t e = cudaEventSynchronize(e1);
     float t = 0.f;

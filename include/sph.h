@@ -206,6 +206,22 @@ typedef struct {
 sph_status sph_set_tiling(sph_ctx *ctx, const sph_tiling *t);
 sph_status sph_get_tiling(const sph_ctx *ctx, sph_tiling *t);
 
+/* Storage of the neighbour lists: 768 B for each of `particles` particles (any
+ * number from the context's particle count on: all of them; 0: none).  With
+ * lists of all particles the acceleration pass reads what the density pass
+ * found; with fewer, density takes that many particles at a time and the
+ * acceleration pass searches for itself; with none, density walks the cells
+ * particle by particle.  Nothing else depends on it.  sph_create takes lists of
+ * all particles while half of the device's memory stays free beside them, else
+ * of a quarter of them or of 65536 when it can; a program that fills the device
+ * gives them back here.
+ * SPH_ERR_OOM: they could not be had, and there are none now.  Waits for the
+ * device and drops a captured step graph; work that a caller captured itself
+ * must not be replayed after it.  SPH_ERR_UNSUPPORTED for an ensemble's
+ * instances, whose lists are taken when all of them have been made. */
+sph_status sph_set_list_storage(sph_ctx *ctx, int64_t particles);
+int64_t sph_get_list_storage(const sph_ctx *ctx);
+
 /* FP64 direct-sum gravity at n_targets particles (host array of particle
  * indices), from the current positions and masses of all particles, with the
  * cubic-spline softened kernel and its exact coefficients: out receives

@@ -203,6 +203,8 @@ def load(parity: bool = False) -> C.CDLL:
         "sph_set_form": (st, [vp, C.POINTER(SphForm)]),
         "sph_get_form": (st, [vp, C.POINTER(SphForm)]),
         "sph_set_tiling": (st, [vp, C.POINTER(SphTiling)]),
+        "sph_set_list_storage": (st, [vp, C.c_int64]),
+        "sph_get_list_storage": (C.c_int64, [vp]),
         "sph_get_tiling": (st, [vp, C.POINTER(SphTiling)]),
         "sph_gravity_direct_f64": (st, [vp, _ip, C.c_int32, C.POINTER(C.c_double), vp]),
         "sph_diagnostics": (st, [vp, vp, C.c_float, C.POINTER(SphDiag)]),

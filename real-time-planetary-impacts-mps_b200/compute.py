@@ -264,6 +264,15 @@ class Compute:
             t.coarse = 1 if coarse else 0
         self._check(self._lib.sph_set_tiling(self._h, C.byref(t)), "sph_set_tiling")
 
+    def set_list_storage(self, particles: int | None = None):
+        """Storage for the neighbour lists of this many particles, 768 B each
+        (sph_set_list_storage); None: of all."""
+        self._check(self._lib.sph_set_list_storage(self._h, self.nParticles if particles is None else int(particles)),
+                    "sph_set_list_storage")
+
+    def get_list_storage(self) -> int:
+        return int(self._lib.sph_get_list_storage(self._h))
+
     def get_tiling(self) -> dict:
         t = _lib.SphTiling()
         self._check(self._lib.sph_get_tiling(self._h, C.byref(t)), "sph_get_tiling")

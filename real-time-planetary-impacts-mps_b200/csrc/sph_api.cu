@@ -327,7 +327,57 @@ sph_status sph_destroy(sph_ctx *ctx) {
     return SPH_OK;
 }
 
-sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out) {
+}  // extern "C"
+
+namespace sph {
+
+// The smallest slice of lists that is taken by itself (48 MiB).
+constexpr int kListSlice = 1 << 16;
+
+static sph_status list_storage(sph_ctx *ctx, int64_t particles) {
+    const int room = (int)std::min<int64_t>(particles, ctx->n);
+    cudaFree(ctx->nlist);
+    ctx->nlist = nullptr;
+    ctx->list_room = 0;
+    // (what the counts say was in the lists)
+    cudaError_t e = cudaMemset(ctx->nlist_count, 0xff, (size_t)ctx->n);
+    if (e == cudaSuccess && room > 0) e = dmalloc(&ctx->nlist, neighbour_list_entries(room));
+    if (e != cudaSuccess) {
+        ctx->nlist = nullptr;
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        return cuda_status(e, "neighbour lists");
+    }
+    ctx->list_room = room;
+    return SPH_OK;
+}
+
+// The lists of all particles (768 B each) make the density and the acceleration
+// pass faster but are not needed: with a slice's, density takes the particles a
+// slice at a time and the acceleration tiles search for themselves (N = 1e6,
+// density: whole lists 2.07 ms, slices of n / 4 2.72, n / 8 3.49, n / 15 4.84,
+// none 6.1; every slice ends with the last tiles of its search).  So they are
+// taken only while half of the device's memory stays free for contexts and
+// tensors that are still to come, and a slice's while 256 B a particle do (FP64
+// positions, the learned seed's records, a larger tree).
+void default_list_storage(sph_ctx *ctx) {
+    size_t free_bytes = 0, total_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    const int n = ctx->n;
+    auto fits = [&](int particles, size_t reserve) {
+        return free_bytes > reserve && neighbour_list_entries(particles) * sizeof(uint32_t) <= free_bytes - reserve;
+    };
+    const size_t own = 256 * (size_t)n;
+    if (fits(n, std::max(own, total_bytes / 2)) && list_storage(ctx, n) == SPH_OK) return;
+    for (int slice : {std::max(n / 4 + 1, kListSlice), kListSlice}) {
+        slice = std::min(slice, n);
+        if (fits(slice, own) && list_storage(ctx, slice) == SPH_OK) return;
+    }
+}
+
+sph_status create_context(const sph_params *params, const sph_ic *ic, sph_ctx **out) {
     if (!out || !ic || ic->n <= 0 || !ic->pos || !ic->vel || !ic->rho || !ic->u || !ic->mass || !ic->h ||
         !ic->material) {
         set_error("sph_create: missing initial conditions");
@@ -424,19 +474,6 @@ sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out)
         sph_destroy(ctx);
         return s;
     }
-    // The neighbour lists (768 B a particle) are worth their storage but not
-    // needed: without it density walks the cells particle by particle and the
-    // acceleration tiles search for themselves.  Taken only when 256 B a
-    // particle stay free for what is allocated later (FP64 positions, the
-    // learned seed's records, a larger tree).
-    size_t free_bytes = 0, total_bytes = 0;
-    const size_t entries = neighbour_list_entries(n);
-    if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess ||
-        free_bytes / 256 < entries * sizeof(uint32_t) / 256 + (size_t)n ||
-        dmalloc(&ctx->nlist, entries) != cudaSuccess) {
-        cudaGetLastError();
-        ctx->nlist = nullptr;
-    }
     if (e == cudaSuccess) e = cudaMemset(ctx->nlist_count, 0xff, (size_t)n);
     if (e == cudaSuccess) e = cudaMemset(ctx->grown, 0, sizeof(int) * kNumUnits);
     // EOS tables and the derived lookup constants (density.metal:45-46)
@@ -484,6 +521,34 @@ sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out)
     *out = ctx;
     return SPH_OK;
 }
+
+}  // namespace sph
+
+extern "C" {
+
+sph_status sph_create(const sph_params *params, const sph_ic *ic, sph_ctx **out) {
+    const sph_status s = create_context(params, ic, out);
+    if (s == SPH_OK) default_list_storage(*out);
+    return s;
+}
+
+sph_status sph_set_list_storage(sph_ctx *ctx, int64_t particles) {
+    if (!ctx || particles < 0) {
+        set_error("sph_set_list_storage: a number of particles from 0 on is wanted");
+        return SPH_ERR_INVALID_ARG;
+    }
+    if (ctx->in_ensemble) {
+        set_error("sph_set_list_storage: an ensemble's instances keep the lists they were made with");
+        return SPH_ERR_UNSUPPORTED;
+    }
+    cudaSetDevice(ctx->device);
+    const cudaError_t e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) return cuda_status(e, "sph_set_list_storage");
+    drop_graphs(ctx);
+    return list_storage(ctx, particles);
+}
+
+int64_t sph_get_list_storage(const sph_ctx *ctx) { return ctx ? ctx->list_room : 0; }
 
 sph_status sph_upload_async(sph_ctx *ctx, sph_field field, const void *host, size_t count, void *stream) {
     if (!ctx || !host) {

@@ -227,12 +227,16 @@ sph_status sph_ensemble_create(const sph_params *params, int32_t n_instances, co
         if (autotune) s = tune_instance(p, ics[i], f, e->capture, t);
         if (s != SPH_OK) break;
         sph_ctx *c = nullptr;
-        s = sph_create(&p, &ics[i], &c);
+        s = create_context(&p, &ics[i], &c);
         if (s != SPH_OK) break;
+        c->in_ensemble = true;
         e->inst.push_back(c);
         s = sph_set_form(c, &f);
         if (s == SPH_OK) apply_tuning(c, t);
     }
+    // (the lists when every instance has what it needs)
+    if (s == SPH_OK)
+        for (sph_ctx *c : e->inst) default_list_storage(c);
     if (s == SPH_OK) {
         err = cudaStreamSynchronize(e->capture);
         if (err != cudaSuccess) s = cuda_status(err, "ensemble create");

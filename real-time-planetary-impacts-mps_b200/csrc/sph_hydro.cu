@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "sph_f32x2.cuh"
 #include "sph_internal.h"
@@ -274,7 +275,8 @@ __device__ __forceinline__ int group_collect(float px, float py, float pz, float
 // kTileListReach: the largest such h is kept per 64-cell unit in `grown`, and a
 // particle's list is complete as long as that h reaches no further than it.
 struct NeighbourLists {
-    uint32_t *entries;  // [n][kTileList] sorted indices
+    uint32_t *entries;  // [last - first][kTileList] sorted indices
+    int first, last;    // the sorted particles whose lists are in it
     uint8_t *count;     // [n], kNoList: none
     float *reach2;      // [n] everything within this squared distance is listed;
                         // negative: nothing else is (no use to the acceleration pass)
@@ -1038,7 +1040,8 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
             ny2[k] = f2(-__shfl_sync(kFull, me.y, 2 * k * L), -__shfl_sync(kFull, me.y, (2 * k + 1) * L));
             nz2[k] = f2(-__shfl_sync(kFull, me.z, 2 * k * L), -__shfl_sync(kFull, me.z, (2 * k + 1) * L));
         }
-        uint32_t *const out = a.lists.entries + (size_t)p0 * kTileList;  // of particle k: + k kTileList
+        uint32_t *const out =
+            a.lists.entries + (size_t)(p0 - (uint32_t)a.lists.first) * kTileList;  // of particle k: + k kTileList
         int cnt[kTileGpw] = {};
         const unsigned below = (1u << lane) - 1u;
         uint32_t *const rows_of = S.rows[threadIdx.x >> 5];
@@ -1158,13 +1161,14 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
             S.tile = t;
             if (t < ntiles) {
                 const uint2 r = tiles[t];
-                S.start = r.x;
-                S.end = r.y;
+                S.start = max(r.x, (uint32_t)a.lists.first);
+                S.end = min(r.y, (uint32_t)a.lists.last);
             }
         }
         __syncthreads();
         if (S.tile >= ntiles) break;
         const uint32_t tstart = S.start, tend = S.end;
+        if (tstart >= tend) continue;  // a tile of another slice
         // a tile whose staged box overflows shared memory is taken again as
         // its octets (coarse tiles: its units), one at a time, an octet that
         // still does as its cells (a unit: its octets) and without the margin
@@ -1321,15 +1325,19 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
 // k_density_deferred takes them from the start.  The iteration is
 // density_particle's with the neighbour cache never in use (h < MAX_H
 // throughout, so the reference's int max_h stays 0).
+// only: kAllModes, or whether the particles of the coarse tiles are taken
+// (kUnitShift) or those of all other modes (0).
+constexpr int kAllModes = -1;
 constexpr int kListThreads = 256;
 __global__ void __launch_bounds__(kListThreads, 4)
-    k_density_list(DensityArgs a, uint32_t *__restrict__ deferred, uint32_t *dctr) {
+    k_density_list(DensityArgs a, int only, uint32_t *__restrict__ deferred, uint32_t *dctr) {
     constexpr int L = kTileLanes;
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31, sub = lane & (L - 1);
-    const int p = (int)((blockIdx.x * (unsigned)kListThreads + threadIdx.x) / L);
-    const uint8_t mode = p < a.n ? a.mode[p] : kModeInactive;
-    bool live = p < a.n;  // the group iterates its particle (uniform within the group)
+    const int p = a.lists.first + (int)((blockIdx.x * (unsigned)kListThreads + threadIdx.x) / L);
+    const uint8_t mode = p < a.lists.last ? a.mode[p] : kModeInactive;
+    // the group iterates its particle (uniform within the group)
+    bool live = p < a.lists.last && (only == kAllModes || (mode == kUnitShift) == (only == kUnitShift));
     uint32_t ind = 0u;
     float4 me = make_float4(0.f, 0.f, 0.f, 0.f), mv = me;
     float h_plain = 0.5f;
@@ -1360,7 +1368,7 @@ __global__ void __launch_bounds__(kListThreads, 4)
         }
         live = false;
     };
-    const uint32_t *list = a.lists.entries + (size_t)(p < a.n ? p : 0) * kTileList;
+    const uint32_t *list = a.lists.entries + (size_t)(p < a.lists.last ? p - a.lists.first : 0) * kTileList;
     float hi = 0.5f, list_r2 = 0.f;
     bool seeded = false;
     if (live) {
@@ -2637,7 +2645,7 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     a.coarse = ctx->tile_coarse;
     a.mode = ctx->tile_mode;
     a.start_h = ctx->tile_h;
-    a.lists = NeighbourLists{ctx->nlist, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
+    a.lists = NeighbourLists{ctx->nlist, 0, n, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     a.sp4 = ctx->sp4;
     a.sv4 = ctx->sv4;
     a.h = ctx->h;
@@ -2688,19 +2696,52 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     cudaMemsetAsync(ctx->grown, 0, sizeof(int) * kNumUnits, st);
     k_density_plan<<<(n + 255) / 256, 256, 0, st>>>(a, ctx->tiles, ctr, ctx->tile_block_max, ctx->tile_half_max,
                                                     ctx->tile_big_max);
-    // (without the lists' storage every particle is left to the walk)
-    if (ctx->nlist)
-        k_lists<0><<<tile_grid(n, sms * ListTile<0>::kCtas), ListTile<0>::kThreads, sizeof(ListShared<0>), st>>>(
-            a, ctx->tiles, ctr);
-    if (ctx->nlist && a.coarse) {
-        constexpr int U = kUnitShift;
+    auto search = [&](auto unit, uint32_t *c) {
+        constexpr int U = decltype(unit)::value;
+        k_lists<U><<<tile_grid(n, sms * ListTile<U>::kCtas), ListTile<U>::kThreads, sizeof(ListShared<U>), st>>>(
+            a, ctx->tiles, c);
+    };
+    auto iterate = [&](int only) {
+        const unsigned grid =
+            (unsigned)(((int64_t)(a.lists.last - a.lists.first) * kTileLanes + kListThreads - 1) / kListThreads);
+        k_density_list<<<grid, kListThreads, 0, st>>>(a, only, ctx->deferred, ctr + 2);
+    };
+    auto coarse_starts = [&]() {
         k_coarse_starts<<<(n + 255) / 256, 256, 0, st>>>(n, a.skey, ctx->units, ctx->coarse_flags, ctx->tiles,
                                                          ctr + 4);
-        k_lists<U><<<tile_grid(n, sms * ListTile<U>::kCtas), ListTile<U>::kThreads, sizeof(ListShared<U>), st>>>(
-            a, ctx->tiles, ctr + 4);
+    };
+    using Cells = std::integral_constant<int, 0>;
+    using Units = std::integral_constant<int, kUnitShift>;
+    const int room = ctx->nlist ? std::min(ctx->list_room, n) : 0;
+    if (room == n) {
+        search(Cells{}, ctr);
+        if (a.coarse) {
+            coarse_starts();
+            search(Units{}, ctr + 4);
+        }
+        iterate(kAllModes);
+    } else if (room == 0) {
+        // (every particle is left to the walk; the coarse tiles' flags stay for
+        // the acceleration pass, which sets the same and more)
+        iterate(kAllModes);
+    } else {
+        // lists of a slice of the sorted order at a time; the tile list holds
+        // one kind of tiles, so first all slices of the one, then of the other
+        auto slices = [&](auto unit, uint32_t *c) {
+            for (int64_t first = 0; first < n; first += room) {
+                a.lists.first = (int)first;
+                a.lists.last = (int)std::min<int64_t>(n, first + room);
+                if (first > 0) cudaMemsetAsync(c + 1, 0, sizeof(uint32_t), st);
+                search(unit, c);
+                iterate(decltype(unit)::value);
+            }
+        };
+        slices(Cells{}, ctr);
+        if (a.coarse) {
+            coarse_starts();
+            slices(Units{}, ctr + 4);
+        }
     }
-    const unsigned lgrid = (unsigned)(((int64_t)n * kTileLanes + kListThreads - 1) / kListThreads);
-    k_density_list<<<lgrid, kListThreads, 0, st>>>(a, ctx->deferred, ctr + 2);
     k_density_deferred<kWalkLanes><<<tile_grid(n, sms * 2) * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(
         a, ctx->deferred, ctr + 2);
 #endif
@@ -2722,7 +2763,8 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     a.cflags = ctx->coarse_flags;
     a.coarse = ctx->tile_coarse;
     a.mode = ctx->tile_mode;
-    a.lists = NeighbourLists{ctx->nlist, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
+    const bool whole = ctx->nlist && ctx->list_room >= n;  // every particle's list is there
+    a.lists = NeighbourLists{whole ? ctx->nlist : nullptr, 0, n, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     a.sA = ctx->sA;
     a.sB = ctx->sB;
     a.sC = ctx->sC;
@@ -2753,7 +2795,7 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
                                                          ctx->tile_half_max, ctx->tile_big_max);
     const unsigned tgrid = tile_grid(n, sms * 2);
     const size_t tsm = sizeof(TileAccShared);
-    if (ctx->nlist) {
+    if (whole) {
         const unsigned lgrid = (unsigned)(((int64_t)n * kTileLanes + kListThreads - 1) / kListThreads);
         if (kahan) k_acceleration_list<true><<<lgrid, kListThreads, 0, st>>>(a);
         else k_acceleration_list<false><<<lgrid, kListThreads, 0, st>>>(a);

@@ -179,9 +179,11 @@ struct sph_ctx {
     uint32_t *deferred = nullptr;
     uint8_t *tile_mode = nullptr;  // [n] the pass that takes each sorted particle
     float *tile_h = nullptr;       // [n] density: the h its staged box is built for
-    // neighbour lists of the density tiles, read by the acceleration pass
-    // (none when their storage could not be had: the tiles look again)
+    // neighbour lists of the density tiles: of all particles, and then read by
+    // the acceleration pass, or of list_room at a time (sph_set_list_storage)
     uint32_t *nlist = nullptr;
+    int list_room = 0;
+    bool in_ensemble = false;
     uint8_t *nlist_count = nullptr;
     float *nlist_reach2 = nullptr;
     int *grown = nullptr;          // per 64-cell unit
@@ -285,6 +287,9 @@ void tree_free(sph_ctx *ctx);
 sph_status launch_tree_build(sph_ctx *ctx, cudaStream_t st, bool withhold = false);
 
 // sph_api.cu
+// sph_create without the neighbour lists' storage, and what it then takes by itself
+sph_status create_context(const sph_params *params, const sph_ic *ic, sph_ctx **out);
+void default_list_storage(sph_ctx *ctx);
 // One full step (tree, sort, gravity, density, acceleration, step) on st.
 // fork: the tree and gravity passes on a stream of their own.
 sph_status full_step(sph_ctx *ctx, cudaStream_t st, bool fork = true);

@@ -244,6 +244,58 @@ def _assert_hydro(a, b, pos, few=1e-3):
     assert np.mean(a["next_active_time"][keep] != b["next_active_time"][keep]) <= 1e-4
 
 
+# The lists of a slice of the particles at a time (slices that end inside tiles
+# and warps, of both kinds of tile), and none at all: the results of the whole
+# lists up to the order of the sums.
+@pytest.mark.parametrize("n,room", [(20480, 20480), (20480, 20479), (20480, 8192), (20480, 1003), (20480, 0),
+                                    (100001, 33333), (400000, 65536), (60000, 0), (400000, 0), (33, 1), (33, 32)])
+@pytest.mark.parametrize("coarse", [True, False])
+def test_hydro_with_less_list_storage(cuda, pkg, n, room, coarse):
+    if not coarse and (n > 100001 or n == 33):
+        pytest.skip("the coarse tiles off: the small bodies, whose particles they take")
+    ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=5)
+    rng = np.random.default_rng(n)
+    ic["h"] = np.minimum(ic["h"] * rng.uniform(0.95, 1.05, n), 0.99).astype(np.float32)
+    ic["vel"] = (ic["vel"] + rng.normal(size=(n, 3)) * 1e-3).astype(np.float32)
+
+    def prepare(c):
+        c.set_tiling(coarse=coarse)
+
+    def less(c):
+        prepare(c)
+        c.step_all(2)  # (a captured step reads the old storage: dropped)
+        c.set_list_storage(room)
+        assert c.get_list_storage() == room
+        for f in ("pos", "vel", "u", "rho", "h"):
+            c.upload(f, ic[f])
+        c.upload("acc", np.zeros((n, 3), np.float32))
+        c.upload("global_time", np.zeros(1, np.int32))
+
+    a, b = _hydro(pkg, ic, False, prepare=less), _hydro(pkg, ic, False, prepare=prepare)
+    _assert_hydro(a, b, ic["pos"])
+
+
+def test_list_storage_arguments(cuda, pkg):
+    ic = pkg.ic.make_impact(2048, 512, seed=4)
+    with pkg.Compute(ic) as c:
+        assert c.get_list_storage() == 2560
+        with pytest.raises(pkg.SphError):
+            c.set_list_storage(-1)
+        c.set_list_storage(0)
+        c.step()
+        c.synchronize()
+        c.set_list_storage()
+        assert c.get_list_storage() == 2560
+        c.step_all(3)
+        c.synchronize()
+    with pkg.Ensemble([ic, ic]) as e:
+        assert [c.get_list_storage() for c in e.instances] == [2560, 2560]
+        with pytest.raises(pkg.SphError):
+            e.instances[0].set_list_storage(0)
+        e.step(2)
+        e.synchronize()
+
+
 # Cells are numbered modulo the grid of 256, so a tile can hold particles a whole
 # period (46.08 Mm) apart: here every other particle of the target's middle is
 # moved by one.  The staged boxes of some 160 units of the coarse tiles (6e4

@@ -316,7 +316,7 @@ sph_status sph_destroy(sph_ctx *ctx) {
                     ctx->health, ctx->cell_range, ctx->sp4, ctx->sv4, ctx->sA, ctx->sB, ctx->sC,
                     ctx->eos_forsterite, ctx->eos_fe, ctx->stage, ctx->snapshot, ctx->pos64, ctx->dglob,
                     ctx->diag, ctx->tiles, ctx->tile_ctr, ctx->deferred, ctx->units, ctx->coarse_flags,
-                    ctx->tile_mode, ctx->tile_h, ctx->octets,
+                    ctx->tile_mode, ctx->tile_h, ctx->tile_first_h, ctx->octets,
                     ctx->nlist, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     for (void *b : bufs) cudaFree(b);
     sort_free(ctx->cell_sort);
@@ -448,6 +448,7 @@ sph_status create_context(const sph_params *params, const sph_ic *ic, sph_ctx **
     chk(dmalloc(&ctx->deferred, (size_t)n));
     chk(dmalloc(&ctx->tile_mode, (size_t)n));
     chk(dmalloc(&ctx->tile_h, (size_t)n));
+    chk(dmalloc(&ctx->tile_first_h, (size_t)n));
     chk(dmalloc(&ctx->nlist_count, (size_t)n));
     chk(dmalloc(&ctx->nlist_reach2, (size_t)n));
     chk(dmalloc(&ctx->grown, (size_t)kNumUnits));

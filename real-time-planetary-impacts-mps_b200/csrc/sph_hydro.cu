@@ -294,6 +294,7 @@ struct DensityArgs {
     uint8_t *cflags;       // per 512-cell block: holds a coarse-tile particle
     int coarse;            // coarse tiles on
     uint8_t *mode;         // [n] the pass that takes each sorted particle (kMode*), written by k_density_plan
+    float *first_h;        // [n] the largest h its first sweep can have, and
     float *start_h;        // [n] the h its staged box is built for, written by k_density_plan
     NeighbourLists lists;  // out, for the acceleration pass
     const float4 *sp4, *sv4;
@@ -629,6 +630,9 @@ constexpr float kTileListReach = SPH_TILE_LIST_REACH;
 // staged box radius / (2 h): room for the second, wider search of a particle
 // that finds too few neighbours
 constexpr float kTileStageReach = 1.25f;
+// list and box radius / (2 h) of lists that serve a first sweep and no more, and
+// the h whose kTileListReach is that, for h = 1
+constexpr float kFirstReach = 1.00001f, kNarrow = kFirstReach / kTileListReach;
 // neighbours within 2 kTileListReach h of a particle at its fixed point,
 // 4/3 pi (2 RESOLUTION_ETA kTileListReach)^3
 constexpr float kListFull = 4.18879f * 8.f * kResolutionEta * kResolutionEta * kResolutionEta * kTileListReach *
@@ -663,7 +667,8 @@ struct ListShared {
     uint32_t start, end, tile, next;
     int defer_all;
     int need;                              // some particle of the range needs the warp pass
-    float reach;                           // staged box radius / (2 h)
+    int narrow;                            // lists of first sweeps only
+    float reach;                           // staged box radius / (2 h), h the first sweep's when narrow
 };
 
 // The list box of a tile particle at smoothing length hb: the cells within
@@ -896,6 +901,7 @@ __global__ void __launch_bounds__(256) k_density_plan(DensityArgs a, uint2 *tile
         const bool on = a.active[ind];
         bool seeded;
         float hb = fmaxf(tile_start_h(a, ind, h_plain, seeded), h_plain);
+        a.first_h[p] = hb;
         // the list is built for the h the iteration is on its way to, as the
         // last pass's density (moved on by the step) has it
         if (on && hb < kMaxH) {
@@ -999,13 +1005,13 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
     const int ny = hi1 - lo1 + 1, nz = hi2 - lo2 + 1;
     if (want) {
         me = a.sp4[p];
-        hb = a.start_h[p];
+        hb = S.narrow ? kNarrow * a.first_h[p] : a.start_h[p];
     }
     // a second search: wider, for the particles that found too few neighbours
     // for their h to stay within the first one's reach (a body's surface at its
     // first step), or just as far as the iteration's first sweep needs, for
     // those that found more than a list holds (a body that contracts)
-    float hscale = kFar2;  // 0: the neighbours' own reach does not count
+    float hscale = S.narrow ? 0.f : kFar2;  // 0: the neighbours' own reach does not count
     bool narrow = false;
     for (int round = 0; round < 2; ++round) {
         CellBox b;
@@ -1015,7 +1021,7 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
             tile_box(me.x, me.y, me.z, hb, b);
             if (round == 1 && !narrow && ((b.lo0 >> us) < lo0 || (b.lo1 >> us) < lo1 || (b.lo2 >> us) < lo2 ||
                                (b.hi0 >> us) > hi0 || (b.hi1 >> us) > hi1 || (b.hi2 >> us) > hi2)) {
-                hb = a.start_h[p] * (S.reach / kTileListReach);  // what is staged for it
+                hb = a.start_h[p] * (kTileStageReach / kTileListReach);  // what is staged for it
                 tile_box(me.x, me.y, me.z, hb, b);
             }
             b.lo0 = max(b.lo0 >> us, lo0), b.lo1 = max(b.lo1 >> us, lo1), b.lo2 = max(b.lo2 >> us, lo2);
@@ -1126,15 +1132,8 @@ __device__ __forceinline__ void lists_tile_warp(const DensityArgs &a, ListShared
             }
             const float to = hb * cbrtf(kListFull / (float)max(c, 1));
             narrow = c > kTileList;
-            want = round == 0 && (narrow || (to > kTileListReach * hb && to < kMaxH && S.reach > kTileListReach));
-            if (want && narrow) {
-                const uint32_t ind = a.cidx[p];
-                const float h_plain = a.h[ind];
-                bool seeded;
-                hb = fmaxf(tile_start_h(a, ind, h_plain, seeded), h_plain) * (1.00001f / kTileListReach);
-            } else if (want) {
-                hb = fminf(1.02f * to, 0.999f * kMaxH);
-            }
+            want = round == 0 && !S.narrow && (narrow || (to > kTileListReach * hb && to < kMaxH));
+            if (want) hb = narrow ? kNarrow * a.first_h[p] : fminf(1.02f * to, 0.999f * kMaxH);
         }
         // (a warp's second searches are alike: rare, and the test of a slot
         // stays the same for all)
@@ -1170,31 +1169,31 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
         const uint32_t tstart = S.start, tend = S.end;
         if (tstart >= tend) continue;  // a tile of another slice
         // a tile whose staged box overflows shared memory is taken again as
-        // its octets (coarse tiles: its units), one at a time, an octet that
-        // still does as its cells (a unit: its octets) and without the margin
-        // for wider searches (a body under compression); what overflows even
-        // so is left to the per-particle pass
-        constexpr int kSplit = U == 0 ? 3 : 3 * U, kSplit2 = kSplit - 3;
+        // its octets (coarse tiles: its units), one at a time, and an octet that
+        // still does once more for lists that reach just as far as its particles'
+        // first sweeps (a body under compression, whose h shrinks); what overflows
+        // even so is left to the per-particle pass.  (Octets taken cell by cell
+        // instead: eight boxes one after another for little less of a box, and
+        // often in vain; free run of N = 1e5, density passes of steps 11 and 46
+        // 2.2 and 2.6 ms instead of 1.4 and 1.0; N = 1e6, first 26 passes 92 ms
+        // instead of 87, while a settled one is 2.06 with it and 2.07 so.)
+        constexpr int kSplit = U == 0 ? 3 : 3 * U;
         const bool splittable = (a.skey[tstart] >> kSplit) != (a.skey[tend - 1] >> kSplit);
-        int level = 0;  // 0 the tile, 1 its octets, 2 their cells
+        int level = 0;  // 0 the tile, 1 its octets, 2 an octet once more
         uint32_t r0 = tstart;
-        // on to what follows the range: behind the last cell of an octet that
-        // was taken cell by cell, to the next octet as a whole
         auto advance = [&](uint32_t to) {
             r0 = to;
-            if (level == 2 && r0 < tend && ((a.skey[r0] ^ a.skey[r0 - 1u]) >> kSplit) != 0u) level = 1;
+            level = min(level, 1);
         };
         while (r0 < tend) {
             __syncthreads();
             if (tid == 0) {
                 uint32_t r1 = tend;
-                if (level == 1) {  // the rest of r0's octet / unit
+                if (level > 0)  // the rest of r0's octet / unit
                     r1 = (U == 0 ? a.octets : a.units)[a.skey[r0] >> kSplit].y + 1u;
-                } else if (level == 2) {
-                    r1 = (U == 0 ? a.cells : a.octets)[a.skey[r0] >> kSplit2].y + 1u;
-                }
                 r1 = min(max(r0 + 1u, r1), tend);
-                S.reach = level < 2 ? kTileStageReach : kTileListReach;
+                S.narrow = level == 2;
+                S.reach = level == 2 ? kFirstReach : kTileStageReach;
                 S.end = r1;
                 S.next = 0u;
                 S.box[0] = S.box[1] = S.box[2] = 0x7fffffff;
@@ -1214,7 +1213,7 @@ __global__ void __launch_bounds__(ListTile<U>::kThreads, ListTile<U>::kCtas)
                     need = true;
                     const float4 me = a.sp4[p];
                     CellBox cb;
-                    tile_box(me.x, me.y, me.z, a.start_h[p], cb, S.reach);
+                    tile_box(me.x, me.y, me.z, (S.narrow ? a.first_h : a.start_h)[p], cb, S.reach);
                     b[0] = min(b[0], cb.lo0);
                     b[1] = min(b[1], cb.lo1);
                     b[2] = min(b[2], cb.lo2);
@@ -2644,6 +2643,7 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     a.cflags = ctx->coarse_flags;
     a.coarse = ctx->tile_coarse;
     a.mode = ctx->tile_mode;
+    a.first_h = ctx->tile_first_h;
     a.start_h = ctx->tile_h;
     a.lists = NeighbourLists{ctx->nlist, 0, n, ctx->nlist_count, ctx->nlist_reach2, ctx->grown};
     a.sp4 = ctx->sp4;

@@ -179,6 +179,7 @@ struct sph_ctx {
     uint32_t *deferred = nullptr;
     uint8_t *tile_mode = nullptr;  // [n] the pass that takes each sorted particle
     float *tile_h = nullptr;       // [n] density: the h its staged box is built for
+    float *tile_first_h = nullptr; // [n] density: the largest h of its first sweep
     // neighbour lists of the density tiles: of all particles, and then read by
     // the acceleration pass, or of list_room at a time (sph_set_list_storage)
     uint32_t *nlist = nullptr;

@@ -219,7 +219,7 @@ def _hydro(pkg, ic, parity, forms=None, prepare=None):
 HYDRO_FIELDS = ("h", "rho", "grad_term", "pressure", "sound_speed", "balsara", "acc", "du", "dhdt")
 
 
-def _assert_hydro(a, b, pos, few=1e-3):
+def _assert_hydro(a, b, pos, few=1e-3, cancelling=("balsara", "du", "dhdt")):
     """a (product) against b (parity build): the bounds of
     test_hydro_matches_the_parity_build."""
     n = len(pos)
@@ -236,7 +236,7 @@ def _assert_hydro(a, b, pos, few=1e-3):
            "acc": 1e-3, "du": 1e-3, "dhdt": 1e-3}
     for f in HYDRO_FIELDS:
         sel = ~flip if f in HYDRO_FIELDS[:6] else keep
-        if f in ("balsara", "du", "dhdt"):
+        if f in cancelling:
             e = np.abs(a[f][sel].astype(np.float64) - b[f][sel]) / np.sqrt(np.mean(b[f].astype(np.float64) ** 2))
         else:
             e = _rel(a[f][sel], b[f][sel])
@@ -294,6 +294,33 @@ def test_list_storage_arguments(cuda, pkg):
             e.instances[0].set_list_storage(0)
         e.step(2)
         e.synchronize()
+
+
+# States that a free impact comes to: particles whose h outgrows their list, and
+# regions under compression, where lists and staged boxes overflow at the h of the
+# step before (N = 1e5, step 46: 8.7 % of the particles outgrow theirs).  Inside
+# such a body the pressure terms of a particle cancel to a thousandth of their sum
+# (N = 1e5, step 11: they are 170 to 1800 times the acceleration where it differs
+# most, and each build is within 1e-7 of its own terms' 64-bit sum), so what the
+# equation of state does to the terms (up to 5e-4) is held to 1e-3 of the root mean
+# square of the accelerations and not of each one.
+@pytest.mark.parametrize("n,steps", [(20000, 3), (20000, 47), (100000, 11), (100000, 46), (100000, 58)])
+def test_hydro_along_a_free_impact(cuda, pkg, n, steps):
+    ic = pkg.ic.make_impact(n - n // 5, n // 5, seed=0)
+    with pkg.Compute(ic, max_children_in_leaf=32) as c:
+        c.step_all(steps)
+        c.synchronize()
+        state = {f: c.download(f) for f in ("pos", "vel", "u", "rho", "h")}
+        c.sort()
+        c.densityPass()
+        c.synchronize()
+        deferred = c.hseed_stats()["deferred"]
+    assert deferred <= 0.2 * n
+    if steps >= 11:
+        assert deferred > 0
+    ic = {**ic, **state}
+    a, b = (_hydro(pkg, ic, parity) for parity in (False, True))
+    _assert_hydro(a, b, ic["pos"], cancelling=("balsara", "acc", "du", "dhdt"))
 
 
 # Cells are numbered modulo the grid of 256, so a tile can hold particles a whole

@@ -341,6 +341,7 @@ static sph_status list_storage(sph_ctx *ctx, int64_t particles) {
     ctx->list_room = 0;
     // (what the counts say was in the lists)
     cudaError_t e = cudaMemset(ctx->nlist_count, 0xff, (size_t)ctx->n);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // before any other stream's next pass
     if (e == cudaSuccess && room > 0) e = dmalloc(&ctx->nlist, neighbour_list_entries(room));
     if (e != cudaSuccess) {
         ctx->nlist = nullptr;

@@ -5,20 +5,24 @@
 // step         SPH/Shaders/step.metal:12-46            (Compute.cpp:242-263)
 // snapshot     SPH/Shaders/render.metal:49-66          (Compute.cpp:396-448)
 //
-// A small group of lanes per particle in sorted (Morton cell) order (see
-// group_walk), so a warp's groups walk neighbouring cells together.
-// Neighbour data are read from sorted, 16-byte records (sp4/sv4, then
-// sA/sB/sC written by the density epilogue), so every cell's particles are
-// one contiguous run of float4 loads instead of the reference's index-chased
-// float3 gathers.  The neighbour walks visit the reference's cells and
-// particles; each lane sums its slice in the reference's order and the slices
-// are combined at the end (with one lane per particle, in the parity build,
-// the order is the reference's exactly).
+// Particles are taken in sorted (Morton cell) order, and neighbour data are read
+// from sorted, 16-byte records (sp4/sv4, then sA/sB/sC written by the density
+// epilogue), so every cell's particles are one contiguous run of float4 loads
+// instead of the reference's index-chased float3 gathers.
 //
-// The reference's 128-entry per-thread neighbour cache (density.metal:67-70)
-// is replaced by rescanning the same cell box with the same filters: the
-// visited set and order are identical (see k_density), and no thread carries
-// 1 KiB of local memory.
+// Product build: the density pass searches once, over tiles of cells staged in
+// shared memory, and writes every particle's neighbour list (k_lists); eight
+// lanes a particle iterate h over the list (k_density_list) and sum the
+// acceleration over the same list (k_acceleration_list), or over one that the
+// acceleration tiles search for (k_acceleration_tile).  Particles that no tile
+// or list serves are walked for, a warp each (k_density_deferred,
+// k_acceleration_deferred; group_walk).
+//
+// Parity build: one thread a particle walks the reference's cells in its order
+// (k_density, k_acceleration).  The reference's 128-entry per-thread neighbour
+// cache (density.metal:67-70) is replaced by rescanning the same cell box with
+// the same filters: the visited set and order are identical (density_particle),
+// and no thread carries 1 KiB of local memory.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -68,16 +72,9 @@ __device__ __forceinline__ float pdiv(float a, float b) {
 #endif
 }
 
-// Lanes per particle in the density and acceleration walks.  The parity
-// build (SPH_PARITY) uses one, which sums in the reference's sequential order.
-#ifdef SPH_PARITY
-constexpr int kLanesPerParticle = 1;
-#else
-#ifndef SPH_HYDRO_LANES
-#define SPH_HYDRO_LANES 8
-#endif
-constexpr int kLanesPerParticle = SPH_HYDRO_LANES;
-#endif
+// Lanes per particle of the parity build's passes: one, which sums in the
+// reference's sequential order.
+constexpr int kParityLanes = 1;
 // Lanes per particle of the deferred particles' walk, a whole warp: its cost
 // is the walk over the thousands of cells of a box that no tile can hold, one
 // look-up per lane at a time, and a few particles at the end of a pass are
@@ -106,16 +103,15 @@ __global__ void k_gather(int n, const uint32_t *__restrict__ cidx, const float4 
 
 // ---- neighbour walk shared by the lanes of one particle -------------------
 //
-// Each particle gets a group of L consecutive lanes (L = 1, 2, 4 or 8); a
-// warp holds 32 / L consecutive particles of the sorted order.  The group
+// Each particle gets a group of L consecutive lanes (the parity build's one or
+// the deferred walk's whole warp).  The group
 // walks the particle's own cell box of radius 2h in the reference's order
 // (x outer, z inner; sorted index within a cell): its lanes look up L cells
 // at a time (cells farther than the search radius are not looked up), the
 // particles of those cells are numbered consecutively, and lane `sub` takes
 // every L-th of them.  So each lane sees a slice of exactly the candidates the
 // reference's box walk visits, the lanes stay busy although a cell holds only
-// a few particles, and the cell table is read once per cell and particle
-// group instead of once per lane.  Partial sums are combined across the
+// a few particles.  Partial sums are combined across the
 // group by a butterfly (every lane ends with the same bits).  With L = 1 the
 // walk is the reference's sequential order exactly.
 
@@ -553,6 +549,7 @@ __device__ __forceinline__ void density_particle(const DensityArgs &a, int index
     a.sC[index] = make_float4(mi, (fi * pc.x / (dens * dens)), dens, bal);
 }
 
+#ifdef SPH_PARITY
 // One lane group per sorted particle, every particle.
 template <int L>
 __global__ void __launch_bounds__(parts_per_block<L>() * L) k_density(DensityArgs a) {
@@ -566,6 +563,7 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L) k_density(DensityArg
     density_particle<L>(a, index, sub, group_mask<L>(lane), gbase, s_off + (threadIdx.x & ~31),
                         s_start + (threadIdx.x & ~31), s_lists + (size_t)(threadIdx.x / L) * kListMax);
 }
+#endif
 
 // The particles the tile pass handed on (sorted indices idx[0, *count)),
 // one lane group each, grid-stride.
@@ -809,7 +807,7 @@ __device__ __forceinline__ float tile_start_h(const DensityArgs &a, uint32_t ind
     return h_plain;
 }
 
-// The pass that takes a sorted particle, decided once per pass by k_tile_plan
+// The pass that takes a sorted particle, decided once per pass by tile_plan
 // from the particle's starting h: the density pass changes h as it goes, so a
 // second look could give a particle to two passes (10 % of them on a 2e5
 // impact) or to none.
@@ -1832,6 +1830,7 @@ __device__ __forceinline__ void block_min_dt(int idt, int32_t *dt) {
     }
 }
 
+#ifdef SPH_PARITY
 template <int L, bool KAHAN>
 __global__ void __launch_bounds__(parts_per_block<L>() * L) k_acceleration(AccelArgs a) {
     extern __shared__ uint32_t s_lists[];
@@ -1846,6 +1845,7 @@ __global__ void __launch_bounds__(parts_per_block<L>() * L) k_acceleration(Accel
                                        s_lists + (size_t)(threadIdx.x / L) * kListMax);
     block_min_dt(idt, a.globals + 1);
 }
+#endif
 
 // The particles the tile pass handed on (sorted indices idx[0, *count)).
 template <int L, bool KAHAN>
@@ -2572,25 +2572,28 @@ __global__ void k_snapshot(int n, const float4 *__restrict__ pos4, const int32_t
     atomicMax(img + pixel, mat[i]);
 }
 
-// Dynamic shared memory of the list kernels; above 48 KiB (the one-lane
-// parity build) it needs the per-device opt-in, set once per device.
-size_t list_smem_opt_in() {
-    const size_t smem = sizeof(uint32_t) * parts_per_block<kLanesPerParticle>() * kListMax;
+// Dynamic shared memory of the walks' lists.
+template <int L>
+constexpr size_t list_smem() {
+    return sizeof(uint32_t) * parts_per_block<L>() * kListMax;
+}
+#ifdef SPH_PARITY
+// Above 48 KiB: the per-device opt-in, set once per device.
+void list_smem_opt_in() {
+    constexpr int smem = (int)list_smem<kParityLanes>();
     static bool done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (smem > 48 * 1024 && dev >= 0 && dev < 64 && !done[dev]) {
-        cudaFuncSetAttribute(k_density<kLanesPerParticle>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(k_acceleration<kLanesPerParticle, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        cudaFuncSetAttribute(k_acceleration<kLanesPerParticle, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    if (dev >= 0 && dev < 64 && !done[dev]) {
+        cudaFuncSetAttribute(k_density<kParityLanes>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_acceleration<kParityLanes, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaFuncSetAttribute(k_acceleration<kParityLanes, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         done[dev] = true;
     }
-    return smem;
 }
+#endif
 
-// Shared memory of the tile kernel (above 48 KiB: the per-device opt-in) and
+// Shared memory of the tile kernels (above 48 KiB: the per-device opt-in) and
 // the device's SM count, set up once per device.
 int tile_smem_opt_in() {
     static int sms[64] = {};
@@ -2680,12 +2683,11 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
     if (s != SPH_OK) return s;
     a.nn_out = ctx->hs.nn;
     a.stats = ctx->hs.stats;
-    const size_t smem = list_smem_opt_in();
-    static_assert(parts_per_block<kWalkLanes>() <= parts_per_block<kLanesPerParticle>(), "the lists' shared memory");
 #ifdef SPH_PARITY
-    constexpr int parts = parts_per_block<kLanesPerParticle>();
-    // one lane per particle, in the reference's order
-    k_density<kLanesPerParticle><<<(unsigned)((n + parts - 1) / parts), parts * kLanesPerParticle, smem, st>>>(a);
+    constexpr int parts = parts_per_block<kParityLanes>();
+    list_smem_opt_in();
+    k_density<kParityLanes><<<(unsigned)((n + parts - 1) / parts), parts * kParityLanes, list_smem<kParityLanes>(),
+                              st>>>(a);
 #else
     // the lists over cell tiles, then over the coarse tiles of the flagged
     // blocks (the tile list is reused); the iteration; the per-particle pass
@@ -2742,8 +2744,9 @@ sph_status launch_density(sph_ctx *ctx, cudaStream_t st) {
             slices(Units{}, ctr + 4);
         }
     }
-    k_density_deferred<kWalkLanes><<<tile_grid(n, sms * 2) * 4, parts_per_block<kWalkLanes>() * kWalkLanes, smem, st>>>(
-        a, ctx->deferred, ctr + 2);
+    k_density_deferred<kWalkLanes>
+        <<<tile_grid(n, sms * 2) * 4, parts_per_block<kWalkLanes>() * kWalkLanes, list_smem<kWalkLanes>(), st>>>(
+            a, ctx->deferred, ctr + 2);
 #endif
     if (ctx->hs.capture) s = launch_hseed_targets(ctx, st);
     if (s != SPH_OK) return s;
@@ -2775,17 +2778,18 @@ sph_status launch_acceleration(sph_ctx *ctx, cudaStream_t st) {
     a.active = ctx->active;
     a.globals = ctx->globals;
     a.individual = ctx->form.timestep == SPH_TIMESTEP_INDIVIDUAL;
-    const size_t smem = list_smem_opt_in();
     const bool kahan = ctx->form.precision == SPH_PRECISION_MIXED;
 #ifdef SPH_PARITY
-    constexpr int parts = parts_per_block<kLanesPerParticle>();
-    // one lane per particle, in the reference's order
+    constexpr int parts = parts_per_block<kParityLanes>();
+    constexpr size_t smem = list_smem<kParityLanes>();
     const unsigned blocks = (unsigned)((n + parts - 1) / parts);
+    list_smem_opt_in();
     if (kahan)
-        k_acceleration<kLanesPerParticle, true><<<blocks, parts * kLanesPerParticle, smem, st>>>(a);
+        k_acceleration<kParityLanes, true><<<blocks, parts * kParityLanes, smem, st>>>(a);
     else
-        k_acceleration<kLanesPerParticle, false><<<blocks, parts * kLanesPerParticle, smem, st>>>(a);
+        k_acceleration<kParityLanes, false><<<blocks, parts * kParityLanes, smem, st>>>(a);
 #else
+    constexpr size_t smem = list_smem<kWalkLanes>();
     // the density pass's tiles, rebuilt so the pass also stands alone; its own
     // counters (tile_ctr[8..15]); then the coarse tiles and the deferred
     const int sms = tile_smem_opt_in();

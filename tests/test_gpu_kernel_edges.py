@@ -101,6 +101,26 @@ def test_reference_gravity_matches_the_parity_build(cuda, pkg, n, leaf, depth, u
     assert np.array_equal(got[0][1], got[1][1])
 
 
+# The same near the origin, where the moments lose nothing to the distance: the
+# builds differ by the rounding of sums of some thousand terms (sqrt(1000) 2^-24 of
+# terms up to ten times the mean, 2e-5), while one term left out is 1e-3
+@pytest.mark.parametrize("n,leaf,depth,unchecked", [(3000, 4, 7, 1024), (3000, 4, 7, 16), (5000, 16, 3, 1024),
+                                                    (2000, 1, 7, 1024), (20000, 100, 7, 1024), (20000, 4, 7, 1024)])
+def test_reference_gravity_near_the_origin(cuda, pkg, n, leaf, depth, unchecked):
+    ic = pkg.ic.make_cube(n, seed=3)
+    ic["pos"] = (ic["pos"] - np.float32(318.55)).astype(np.float32)
+    got = []
+    for parity in (False, True):
+        with pkg.Compute(ic, max_children_in_leaf=leaf, max_tree_depth=depth, max_unchecked_pointers=unchecked,
+                         parity=parity) as c:
+            c.upload("grav_norm", np.full(n, 0.1, np.float32))
+            c.gravitationalPass()
+            c.synchronize()
+            got.append(c.download("acc").astype(np.float64))
+    scale = np.sqrt(np.mean(np.sum(got[1] ** 2, axis=1)))
+    assert np.max(np.linalg.norm(got[0] - got[1], axis=1)) <= 2e-5 * scale
+
+
 # odd counts of staged nodes and particles, groups that are not full, and pairs
 # inside the softening
 @pytest.mark.parametrize("n,leaf,side", [(1, 4, 10.0), (2, 1, 0.05), (31, 4, 10.0), (33, 32, 0.3), (65, 1, 10.0),

@@ -57,7 +57,7 @@ PASSES = ("tree", "sort", "gravity", "density", "acceleration", "step")
 # compulsory HBM bytes per particle per pass (each array touched once)
 ALGO_BYTES = {"tree": 76, "sort": 92, "gravity": 44, "density": 65, "acceleration": 88, "step": 92}
 PASS_KERNELS = {
-    "tree": "k_bbox, k_tree_keys, k_onesweep x3, k_mark, k_write, k_link",
+    "tree": "k_bbox, k_tree_keys, k_onesweep x3, k_tree_mark, k_tree_write, k_tree_link",
     "sort": "k_hash_hist, k_onesweep x3, k_cells",
     "gravity": "plain: k_up_all, k_down x8; chosen: k_up_theta, k_gather_key_order, k_walk",
     "density": "k_gather, [k_mlp (learned seed)], k_density_plan, k_lists, k_density_list, k_density_deferred",
@@ -70,7 +70,7 @@ def launches_per_step(depth: int, chosen: bool, online_iters: int = 0, seed: boo
     """Kernels of one step (memsets excluded), counted from the pass structure
     (matches the ncu launch list: 37 plain, 52 chosen with 8 online Adam
     steps, at depth 7)."""
-    tree = 3 + 3 + 3                     # box (2), keys, 3 sort passes, marks, write, link
+    tree = 3 + (3 * depth + 7) // 8 + 3  # box (2), keys, sort passes of 8 bits, marks, write, link
     sort = 1 + 3 + 1                     # hash, 3 passes, cells
     gravity = 3 if chosen else 1 + (depth + 1)
     # gather, plan, lists, coarse starts, coarse lists, iteration, deferred pass
